@@ -574,13 +574,21 @@ __global__ void __launch_bounds__(kStagedMaxThreads, kStagedMinBlocks) trace_sta
   w.stk = stack;
   w.pin_base = pin_ok ? smem_u32(smem0) : 0u;
   w.pin_root = pin_ok ? a.pin_root : 0u;
-  bool have = false, exhausted = false;
+  bool have = false, ended = false, exhausted = false;
   uint32_t r = 0, it = 0;
   unsigned long long bytes = 0, staged = 0, stagings = 0, sreads = 0, greads = 0;
   for (;; ++it) {
-    // --- refill idle lanes (as run_persistent)
+    // --- records of finished rays, then new rays for idle lanes (as run_persistent)
     const uint32_t need = __ballot_sync(0xffffffffu, !have);
-    if (!exhausted && need && (__popc(need) >= (int)a.refill || need == 0xffffffffu)) {
+    if (need == 0xffffffffu || (!exhausted && __popc(need) >= (int)a.refill)) {
+      if (ended) {
+        w.finish(a, r);
+        bytes += w.rec.bytes;
+        sreads += w.smem_reads;
+        greads += w.gmem_reads;
+        ended = false;
+      }
+      if (exhausted) break;  // every lane is idle
       const int leader = __ffs(need) - 1;
       uint32_t base = 0;
       if ((int)lane == leader) base = atomicAdd(a.queue, (uint32_t)__popc(need));
@@ -591,18 +599,10 @@ __global__ void __launch_bounds__(kStagedMaxThreads, kStagedMinBlocks) trace_sta
         if (rr < a.n) {
           r = rr;
           w.init(a, r);
-          have = true;
-          if (!w.active()) {
-            w.finish(a, r);
-            bytes += w.rec.bytes;
-            have = false;
-          }
+          have = w.active();
+          ended = !have;
         }
       }
-    }
-    if (!__any_sync(0xffffffffu, have)) {
-      if (exhausted) break;
-      continue;
     }
     // --- staging: land a finished copy, then vote for the next one
     if (SLOTS && slots > 0 && (it % a.epoch) == 0) {
@@ -663,11 +663,8 @@ __global__ void __launch_bounds__(kStagedMaxThreads, kStagedMinBlocks) trace_sta
       if (SLOTS) w.step(a, r, lookup);
       else w.step(a, r);
       if (!w.active()) {
-        w.finish(a, r);
-        bytes += w.rec.bytes;
-        sreads += w.smem_reads;
-        greads += w.gmem_reads;
         have = false;
+        ended = true;
       }
     }
   }
