@@ -29,7 +29,7 @@ rt_status fail(rt_status s, const std::string& msg) {
   return s;
 }
 
-bool validate_blob(const uint8_t* b, uint64_t n, std::string* err) {
+bool validate_blob(const uint8_t* b, uint64_t n, std::string* err, bool* ordered) {
   auto bad = [&](const std::string& m) {
     if (err) *err = m;
     return false;
@@ -43,6 +43,7 @@ bool validate_blob(const uint8_t* b, uint64_t n, std::string* err) {
     return v;
   };
   std::vector<uint8_t> seen(units, 0);
+  bool in_order = true;
   struct Item {
     uint64_t unit;
     bool top;
@@ -69,6 +70,8 @@ bool validate_blob(const uint8_t* b, uint64_t n, std::string* err) {
       const uint32_t sz = rtf::child_size_units(info), ty = rtf::child_type(info);
       if (sz) {
         if (c + sz > units) return bad("child outside the blob");
+        for (uint32_t k = 0; k < 3; ++k)
+          in_order &= p[rtf::IN_LO_X + 12 * k + i] <= p[rtf::IN_HI_X + 12 * k + i];
         if (ty == rtf::CT_INTERNAL) {
           work.push_back({c, it.top});
         } else if (it.top) {
@@ -88,6 +91,7 @@ bool validate_blob(const uint8_t* b, uint64_t n, std::string* err) {
       c += sz;
     }
   }
+  if (ordered) *ordered = in_order;
   return true;
 }
 
@@ -111,6 +115,7 @@ struct rt_scene {
   uint8_t* d_blob = nullptr;
   uint64_t blob_bytes = 0;
   uint32_t n_units = 0;
+  bool ordered = false;  // no child box has a quantized lower bound above its upper one
   // treelets
   bool has_treelets = false;
   rtt::Partition part;
@@ -656,7 +661,8 @@ rt_status rt_scene_create(rt_ctx* ctx, const rt_blob* blob, rt_scene** out) {
   if (!ctx || !blob || !out) return rti::fail(RT_ERR_INVALID, "rt_scene_create: NULL argument");
   *out = nullptr;
   std::string err;
-  if (!rti::validate_blob(blob->bytes.data(), blob->bytes.size(), &err)) return rti::fail(RT_ERR_BLOB, err);
+  bool ordered = false;
+  if (!rti::validate_blob(blob->bytes.data(), blob->bytes.size(), &err, &ordered)) return rti::fail(RT_ERR_BLOB, err);
   if (blob->bytes.size() / 64 >= (1ull << 29))
     return rti::fail(RT_ERR_TOO_LARGE, "rt_scene_create: blobs are limited to 2^29 units of 64 bytes");
   RT_CUDA(cudaSetDevice(ctx->device));
@@ -665,6 +671,7 @@ rt_status rt_scene_create(rt_ctx* ctx, const rt_blob* blob, rt_scene** out) {
   s->host_blob = blob->bytes;
   s->blob_bytes = blob->bytes.size();
   s->n_units = (uint32_t)(s->blob_bytes / 64);
+  s->ordered = ordered;
   rt_status st = dalloc(&s->d_blob, s->blob_bytes);
   if (st == RT_OK) st = dalloc(&s->d_stats, sizeof(unsigned long long) * rtk::ST_COUNT);
   if (st == RT_OK) st = dalloc(&s->d_status, sizeof(uint32_t));
@@ -877,6 +884,7 @@ rt_status trace_launch(rt_scene* s, const rt_ray* rays, const uint32_t* flags, u
   rtk::TraceArgs a{};
   a.blob = reinterpret_cast<const uint4*>(s->d_blob);
   a.n_units = s->n_units;
+  a.ordered = s->ordered;
   a.rays = rays;
   a.flags = flags;
   a.default_flags = default_flags;
@@ -1319,7 +1327,7 @@ rt_status batch_args(rt_batch* b, const rt_ray* rays, const uint32_t* flags, uin
   bool stale = false;
   for (size_t i = 0; i < b->scenes.size(); ++i) {
     const rt_scene* s = b->scenes[i];
-    const rtk::SceneView nv{reinterpret_cast<const uint4*>(s->d_blob), s->d_meta, s->d_route, s->n_units};
+    const rtk::SceneView nv{reinterpret_cast<const uint4*>(s->d_blob), s->d_meta, s->d_route, s->n_units, s->ordered};
     const rtk::SceneView& ov = b->views[i];
     if (nv.blob != ov.blob || nv.meta != ov.meta || nv.route != ov.route || nv.n_units != ov.n_units) {
       b->views[i] = nv;
@@ -1413,7 +1421,7 @@ rt_status rt_batch_create(rt_ctx* ctx, rt_scene* const* scenes, uint32_t n_scene
       return rti::fail(RT_ERR_INVALID, "rt_batch_create: NULL scene or scene on another device");
     }
     v[i] = rtk::SceneView{reinterpret_cast<const uint4*>(scenes[i]->d_blob), scenes[i]->d_meta, scenes[i]->d_route,
-                          scenes[i]->n_units};
+                          scenes[i]->n_units, scenes[i]->ordered};
   }
   cudaError_t e = cudaMemcpy(b->d_views, v.data(), sizeof(rtk::SceneView) * n_scenes, cudaMemcpyHostToDevice);
   b->views = v;

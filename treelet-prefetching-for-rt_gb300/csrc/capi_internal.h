@@ -23,7 +23,7 @@ void set_error(const std::string& msg);
 rt_status fail(rt_status s, const std::string& msg);
 
 // Host-side structural check of a blob; returns false with a message.
-bool validate_blob(const uint8_t* b, uint64_t n, std::string* err);
+bool validate_blob(const uint8_t* b, uint64_t n, std::string* err, bool* ordered = nullptr);
 
 // After the scene's traces have finished: RT_ERR_TIMEOUT if a bounded device
 // wait of the last launch gave up, else RT_OK.

@@ -39,11 +39,13 @@ struct SceneView {
   const uint2* meta;      // per unit: x = treelet root unit, y = dense << 10 | slot
   const uint16_t* route;  // per unit: routing bits of the treelet-ordered walk (treelets.h)
   uint32_t n_units;
+  uint32_t ordered;       // every child box's quantized lower bounds are at most its upper ones
 };
 
 struct TraceArgs {
   const uint4* blob;
   uint32_t n_units;
+  uint32_t ordered;
   // several scenes in one launch: rays [item_begin[k], item_begin[k+1]) use
   // scenes[item_scene[k]]; n_items == 0 means every ray uses blob / meta
   const SceneView* scenes;
@@ -169,7 +171,7 @@ __device__ __forceinline__ void load_ray(const rt_ray* rays, uint32_t r, rtm::V3
 // whose tables are the launch arguments themselves.
 template <bool MULTI>
 __device__ __forceinline__ SceneView scene_of(const TraceArgs& a, uint32_t r) {
-  if (!MULTI || a.n_items == 0) return SceneView{a.blob, a.meta, a.route, a.n_units};
+  if (!MULTI || a.n_items == 0) return SceneView{a.blob, a.meta, a.route, a.n_units, a.ordered};
   uint32_t lo = 0, hi = a.n_items;  // last item with item_begin <= r
   while (hi - lo > 1) {
     const uint32_t mid = (lo + hi) >> 1;
@@ -182,6 +184,7 @@ __device__ __forceinline__ SceneView scene_of(const TraceArgs& a, uint32_t r) {
   v.meta = reinterpret_cast<const uint2*>(__ldg(reinterpret_cast<const unsigned long long*>(&s->meta)));
   v.route = reinterpret_cast<const uint16_t*>(__ldg(reinterpret_cast<const unsigned long long*>(&s->route)));
   v.n_units = __ldg(&s->n_units);
+  v.ordered = __ldg(&s->ordered);
   return v;
 }
 
@@ -381,7 +384,7 @@ struct PlainWalker {
     ic.unit = kNone;
     ic_fast = false;
     idir = rtm::calculate_idir(D);
-    fast = rtd::finite_ray(O, D, tmin, tmax);
+    fast = v.ordered && rtd::finite_ray(O, D, tmin, tmax);
     rec.rec<TRACED>(a, 0, rtf::TX_STRUCTURE);
     const uint4 h0 = __ldg(v.blob), h1 = __ldg(v.blob + 1);
     const uint64_t root_off = (uint64_t)h0.x | ((uint64_t)h0.y << 32);
@@ -405,8 +408,8 @@ struct PlainWalker {
     const rtm::V3 o = inblas ? ic.o : O, id = inblas ? ic.idir : idir;
     const float t0 = inblas ? ic.tmin : tmin, t1 = inblas ? ic.tmax : tmax;
     const float cull = inblas ? min_thit * ic.mult : min_thit;
-    const rtd::ChildHits ch = f ? rtd::test_children<true>(nd, unit, o, id, t0, t1, cull)
-                                : rtd::test_children<false>(nd, unit, o, id, t0, t1, cull);
+    const rtd::ChildHits ch = f ? rtd::test_children<true>(nd, v.blob + (uint64_t)unit * 4, unit, o, id, t0, t1, cull)
+                                : rtd::test_children<false>(nd, v.blob + (uint64_t)unit * 4, unit, o, id, t0, t1, cull);
     const uint32_t level = inblas ? 0u : kTop;
     uint32_t c = ch.child_unit, nn = kNone;
 #pragma unroll
@@ -462,7 +465,7 @@ struct PlainWalker {
     const uint4 h0 = __ldg(v.blob + (hdr >> 4));
     const uint64_t broot = hdr + ((uint64_t)h0.x | ((uint64_t)h0.y << 32));
     enter_instance(in, unit, O, D, tmin, tmax, ic);
-    ic_fast = rtd::finite_ray(ic.o, ic.d, ic.tmin, ic.tmax);
+    ic_fast = v.ordered && rtd::finite_ray(ic.o, ic.d, ic.tmin, ic.tmax);
     push(a, (uint32_t)(broot >> 6) << 2);
     inblas = true;
     if (status & RT_RAY_STACK_OVERFLOW) stop(0);

@@ -184,7 +184,7 @@ struct Walker {
     smem_reads = gmem_reads = 0;
     const rtm::V3 id = rtm::calculate_idir(D);
     set_world(o, id);
-    fast = rtd::finite_ray(o, D, tmin, tmax);
+    fast = v.ordered && rtd::finite_ray(o, D, tmin, tmax);
     ic_fast = false;
     record(a, r, 0, rtf::TX_STRUCTURE);
     const uint4 h0 = __ldg(v.blob), h1 = __ldg(v.blob + 1);
@@ -241,7 +241,7 @@ struct Walker {
     ic_fast = false;
     smem_reads = gmem_reads = 0;
     set_world(o, rtm::calculate_idir(D));
-    fast = rtd::finite_ray(o, D, tmin, tmax);
+    fast = v.ordered && rtd::finite_ray(o, D, tmin, tmax);
   }
 
   // True while the walk is inside its current treelet: the next pop would
@@ -281,10 +281,11 @@ struct Walker {
     // the first 64 bytes (or the whole pinned record of an instance leaf), for
     // every kind of node at once, so the warp's lanes issue one load
     rtd::Node64 nd;
+    const uint4* src = g;
     if (STAGED) {
       // one generic load for lanes reading shared memory and lanes reading
       // global memory, instead of both load paths for a mixed warp
-      const uint4* src = saddr ? reinterpret_cast<const uint4*>(__cvta_shared_to_generic(saddr)) : g;
+      if (saddr) src = reinterpret_cast<const uint4*>(__cvta_shared_to_generic(saddr));
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         const uint4 w = src[k];
@@ -317,7 +318,7 @@ struct Walker {
     }
     if (enter != kNone) {
       enter_instance(in, enter, world_o(), dir(), tmin, tmax, ic);
-      ic_fast = rtd::finite_ray(ic.o, ic.d, ic.tmin, ic.tmax);
+      ic_fast = v.ordered && rtd::finite_ray(ic.o, ic.d, ic.tmin, ic.tmax);
     }
     if (!leaf) {  // internal node, top (:1758-1869) or bottom (:1954-2070)
       record(a, r, unit, rtf::TX_INTERNAL);
@@ -336,8 +337,8 @@ struct Walker {
       const rtm::V3 o = top ? world_o() : ic.o, id = top ? world_idir() : ic.idir;
       const float t0 = top ? tmin : ic.tmin, t1 = top ? tmax : ic.tmax;
       const float cull = top ? min_thit : min_thit * ic.mult;
-      const rtd::ChildHits ch = f ? rtd::test_children<true>(nd, unit, o, id, t0, t1, cull)
-                                  : rtd::test_children<false>(nd, unit, o, id, t0, t1, cull);
+      const rtd::ChildHits ch = f ? rtd::test_children<true>(nd, src, unit, o, id, t0, t1, cull)
+                                  : rtd::test_children<false>(nd, src, unit, o, id, t0, t1, cull);
       const uint32_t hit = ch.hit_mask;
       const uint64_t info = ch.info;
       const uint32_t same = rbits >> (rsh * kRouteOther);
