@@ -141,22 +141,6 @@ __device__ __forceinline__ void trace_drain(const TraceArgs& a, uint32_t* vrow, 
   }
 }
 
-struct Recorder {
-  uint32_t* vrow;
-  uint32_t* trow;
-  uint32_t cap;
-  uint32_t n;
-  uint32_t bytes;
-  const uint2* meta;
-  // TRACED = false: a launch without traces, whose walk only counts.
-  template <bool TRACED>
-  __device__ __forceinline__ void rec(const TraceArgs& a, uint32_t unit, uint32_t type) {
-    if (TRACED && n < cap) trace_put(a, vrow, trow, n, rtf::pack_visit(unit, type), trow ? meta[unit].x : 0u);
-    n++;
-    bytes += rtf::tx_bytes(type);
-  }
-};
-
 __device__ __forceinline__ void load_ray(const rt_ray* rays, uint32_t r, rtm::V3& o, float& tmin, rtm::V3& d,
                                          float& tmax) {
   const float4* p = reinterpret_cast<const float4*>(rays + r);
@@ -191,7 +175,7 @@ __device__ __forceinline__ SceneView scene_of(const TraceArgs& a, uint32_t r) {
 // Hit record from the closest leaf / instance (vulkan_ray_tracing.cc:2990-3028).
 __device__ __forceinline__ void write_hit(const TraceArgs& a, const SceneView& v, uint32_t r, bool hit, float min_thit, rtm::V3 O,
                                           rtm::V3 D, float tmin, float tmax, uint32_t c_leaf, uint32_t c_inst,
-                                          float c_tobj, const Recorder& rec, uint32_t status) {
+                                          float c_tobj, uint32_t n_visits, uint32_t status) {
   rt_hit h;
   h.hit_geometry = 0;
   h.geometry_index = 0;
@@ -228,29 +212,41 @@ __device__ __forceinline__ void write_hit(const TraceArgs& a, const SceneView& v
     h.closest_leaf = c_leaf;
     h.closest_instance = c_inst;
   }
-  h.n_visits = rec.n;
-  h.status = status | (rec.cap && rec.n > rec.cap ? RT_RAY_TRACE_OVERFLOW : 0u);
+  h.n_visits = n_visits;
+  h.status = status | (a.cap && n_visits > a.cap ? RT_RAY_TRACE_OVERFLOW : 0u);
   a.hits[r] = h;
 }
 
-// Object-space ray of one instance (make_transformed_ray).
-struct InstCtx {
+// The ray a walk tests nodes with: the world ray at top-level nodes (unit
+// kNone, mult 1), an instance's object ray (make_transformed_ray) in its BLAS.
+// A walk keeps one of them in registers and changes it when the next node
+// needs the other, instead of holding both and selecting per node.  The
+// interval is the world ray's times mult in either case (mult = 1 is exact).
+struct RayCtx {
   uint32_t unit;
   rtm::V3 o, d, idir;
-  float tmin, tmax, mult;
+  float mult;
+  bool fast;  // the box test may tell planes apart by the direction's sign
 };
 
 __device__ __forceinline__ void enter_instance(const rtd::Instance& in, uint32_t unit, rtm::V3 O, rtm::V3 D, float tmin,
-                                               float tmax, InstCtx& c) {
+                                               float tmax, bool ordered, RayCtx& c) {
   const rtm::ObjRay r = rtm::make_transformed_ray(in.w2o, O, D, tmin, tmax);
   c.unit = unit;
   c.o = r.o;
   c.d = r.d;
-  c.tmin = r.tmin;
-  c.tmax = r.tmax;
   c.mult = r.mult;
   c.idir = rtm::calculate_idir(r.d);
+  c.fast = ordered && rtd::finite_ray(r.o, r.d, r.tmin, r.tmax);
 }
+
+// Flags of a walk, above the RT_RAY_* status bits of its hit record.
+constexpr uint32_t kRayTerminate = 0x100u, kRayOpaque = 0x200u, kRayWorldFast = 0x400u, kRayStatusMask = 0xffu;
+
+// Node bytes a ray reads: 64 per transaction, but 128 for an instance leaf and
+// 8 for a leaf descriptor.  A walk counts transactions per ray and, per
+// thread, the difference in units of 8 bytes.
+constexpr int kInstanceExtra = 8, kDescriptorExtra = -7;
 
 // Adds v summed over the calling warp's active lanes with one atomic.
 __device__ __forceinline__ void add_warp_total(unsigned long long* dst, uint32_t v) {
@@ -288,7 +284,7 @@ __device__ __forceinline__ void run_persistent(const TraceArgs& a, W& w, unsigne
     if (need == 0xffffffffu || (!exhausted && __popc(need) >= (int)a.refill)) {
       if (ended) {
         w.finish(a, r);
-        bytes += w.rec.bytes;
+        bytes += 64ull * w.n_tx;
         ended = false;
       }
       if (exhausted) break;  // every lane is idle
@@ -315,16 +311,18 @@ __device__ __forceinline__ void run_persistent(const TraceArgs& a, W& w, unsigne
       }
     }
   }
-  bytes_out = bytes;
+  bytes_out = bytes + (unsigned long long)(8ll * w.extra);
 }
 
 // ----------------------------------------------------------------- plain
 
 // A ray's traceRay walk (vulkan_ray_tracing.cc:2309-3076) as a sequence of
 // node visits.  One LIFO stack of unit << 2 | top | leaf entries; `next` is
-// the internal node descended next (the first hit internal child, :2570-2578);
-// leaves and further children are pushed.  A top-level instance leaf is
-// followed by its whole BLAS before the next top-level entry (:2602-2679).
+// the internal node descended next (the first hit internal child, :2570-2578),
+// as an entry, 0 for none (no entry is 0: unit 0 is the TLAS header); leaves
+// and further children are pushed.  A top-level instance leaf is followed by
+// its whole BLAS before the next top-level entry (:2602-2679), so a
+// bottom-level entry always belongs to the instance entered last.
 // The warp-synchronous short stack (SHORT): entries 0..kShortStack-1 of each
 // ray's stack in its warp's shared memory, entry k of the warp's 32 rays in
 // one 128-byte row (lane l in bank l, so a warp's pushes and pops at any mix
@@ -332,24 +330,48 @@ __device__ __forceinline__ void run_persistent(const TraceArgs& a, W& w, unsigne
 constexpr int kShortStack = 16;
 constexpr uint32_t kShortStackWarpBytes = kShortStack * 32 * 4;
 
+// Entries past CAP that a visit may write before its depth is checked: a
+// node's children are pushed without a check each.
+constexpr int kStackPad = 8;
+// Words after the stack entries: what a step rarely needs stays in local
+// memory (the stack array is indexed at run time, so the compiler leaves all
+// of it there), so that the walk's registers hold the ray it tests with.
+constexpr int kPlainCold = 12;
+
 // TRACED = false compiles the walk of a launch without traces (no trace
 // code at all); TRACED = true writes the rows.  SHORT keeps the bottom of the
 // stack in shared memory (rt_tuning.short_stack).
 template <int CAP, bool MULTI, bool TRACED, bool SHORT = false>
 struct PlainWalker {
-  rtm::V3 O, D, idir;
-  float tmin, tmax, min_thit, c_tobj;
-  bool opaque, terminate, inblas, fast;
-  uint32_t next, c_leaf, c_inst, status;
+  RayCtx cx;
+  float tmin, tmax, min_thit;
+  uint32_t next, flags;
   int sp;
-  uint32_t stk[CAP];
-  InstCtx ic;
-  bool ic_fast;
-  Recorder rec;
+  uint32_t n_tx;  // the ray's transactions
+  int extra;      // the thread's byte difference (kInstanceExtra)
+  uint32_t* stk;  // CAP + kStackPad + kPlainCold words, a local array of the kernel
   SceneView v;
 
-  __device__ __forceinline__ bool active() const { return next != kNone || sp > 0; }
+  __device__ __forceinline__ bool active() const { return next != 0 || sp > 0; }
 
+  // ---- the cold words
+  __device__ __forceinline__ uint32_t& cold(int k) const { return stk[CAP + kStackPad + k]; }
+  __device__ __forceinline__ rtm::V3 cold3(int k) const {
+    return rtm::v3(__uint_as_float(cold(k)), __uint_as_float(cold(k + 1)), __uint_as_float(cold(k + 2)));
+  }
+  __device__ __forceinline__ void set_cold3(int k, rtm::V3 x) {
+    cold(k) = __float_as_uint(x.x);
+    cold(k + 1) = __float_as_uint(x.y);
+    cold(k + 2) = __float_as_uint(x.z);
+  }
+  __device__ __forceinline__ rtm::V3 world_d() const { return cold3(0); }
+  __device__ __forceinline__ rtm::V3 world_o() const { return cold3(3); }
+  __device__ __forceinline__ rtm::V3 world_idir() const { return cold3(6); }
+  __device__ __forceinline__ void set_hit(uint32_t leaf, uint32_t inst, float tobj) {
+    cold(9) = leaf;
+    cold(10) = inst;
+    cold(11) = __float_as_uint(tobj);
+  }
 
   // entry i of the stack (the short stack's rows for i < kShortStack)
   __device__ __forceinline__ uint32_t* slot(const TraceArgs& a, int i) {
@@ -360,101 +382,108 @@ struct PlainWalker {
     }
     return stk + i;
   }
-  __device__ __forceinline__ void push(const TraceArgs& a, uint32_t e) {
-    if (sp < CAP) *slot(a, sp++) = e;
-    else status |= RT_RAY_STACK_OVERFLOW;
+
+  __device__ __forceinline__ void record(const TraceArgs& a, uint32_t r, uint32_t unit, uint32_t type) {
+    if (TRACED && n_tx < a.cap) {
+      uint32_t* vrow = a.visits ? a.visits + (uint64_t)r * a.cap : nullptr;
+      uint32_t* trow = a.tl_trace ? a.tl_trace + (uint64_t)r * a.cap : nullptr;
+      trace_put(a, vrow, trow, n_tx, rtf::pack_visit(unit, type), trow ? v.meta[unit].x : 0u);
+    }
+    n_tx++;
   }
-  __device__ __forceinline__ uint32_t pop(const TraceArgs& a) { return *slot(a, --sp); }
 
   __device__ __forceinline__ void init(const TraceArgs& a, uint32_t r) {
     v = scene_of<MULTI>(a, r);
+    rtm::V3 O, D;
     load_ray(a.rays, r, O, tmin, D, tmax);
-    const uint32_t flags = a.flags ? a.flags[r] : a.default_flags;
-    terminate = flags & rtf::RAY_FLAG_TERMINATE_ON_FIRST_HIT;
-    opaque = flags & rtf::RAY_FLAG_OPAQUE;
-    rec = Recorder{a.visits ? a.visits + (uint64_t)r * a.cap : nullptr,
-                   a.tl_trace ? a.tl_trace + (uint64_t)r * a.cap : nullptr, a.cap, 0u, 0u, v.meta};
-    status = 0;
+    const uint32_t f = a.flags ? a.flags[r] : a.default_flags;
+    flags = (f & rtf::RAY_FLAG_TERMINATE_ON_FIRST_HIT ? kRayTerminate : 0u) | (f & rtf::RAY_FLAG_OPAQUE ? kRayOpaque : 0u);
+    n_tx = 0;
     sp = 0;
-    next = kNone;
-    inblas = false;
+    next = 0;
     min_thit = tmax;
-    c_leaf = c_inst = 0;
-    c_tobj = 0.0f;
-    ic.unit = kNone;
-    ic_fast = false;
-    idir = rtm::calculate_idir(D);
-    fast = v.ordered && rtd::finite_ray(O, D, tmin, tmax);
-    rec.rec<TRACED>(a, 0, rtf::TX_STRUCTURE);
+    const rtm::V3 id = rtm::calculate_idir(D);
+    set_cold3(0, D);
+    set_cold3(3, O);
+    set_cold3(6, id);
+    set_hit(0, 0, 0.0f);
+    if (v.ordered && rtd::finite_ray(O, D, tmin, tmax)) flags |= kRayWorldFast;
+    world();
+    record(a, r, 0, rtf::TX_STRUCTURE);
     const uint4 h0 = __ldg(v.blob), h1 = __ldg(v.blob + 1);
     const uint64_t root_off = (uint64_t)h0.x | ((uint64_t)h0.y << 32);
     const rtm::V3 bmin = rtm::v3(__uint_as_float(h0.z), __uint_as_float(h0.w), __uint_as_float(h1.x));
     const rtm::V3 bmax = rtm::v3(__uint_as_float(h1.y), __uint_as_float(h1.z), __uint_as_float(h1.w));
     float th;
-    if (rtm::ray_box_test(bmin, bmax, idir, O, tmin, tmax, th)) push(a, ((uint32_t)(root_off >> 6) << 2) | kTop);
+    if (rtm::ray_box_test(bmin, bmax, id, O, tmin, tmax, th)) next = ((uint32_t)(root_off >> 6) << 2) | kTop;
+  }
+
+  // The world ray as the ray tested with (its direction is not: only
+  // bottom-level leaves and instance entries read one).
+  __device__ __forceinline__ void world() {
+    cx.unit = kNone;
+    cx.o = world_o();
+    cx.idir = world_idir();
+    cx.mult = 1.0f;
+    cx.fast = (flags & kRayWorldFast) != 0;
   }
 
   __device__ __forceinline__ void stop(uint32_t bits) {
-    status |= bits;
+    flags |= bits;
     sp = 0;
-    next = kNone;
+    next = 0;
   }
 
-  __device__ __forceinline__ void visit_internal(const TraceArgs& a, uint32_t unit, const rtd::Node64& nd) {
-    // one box test for both levels (the world ray, or the instance's object
-    // ray with the culling distance scaled into object space): lanes at TLAS
-    // and BLAS nodes run it together
-    const bool f = inblas ? ic_fast : fast;
-    const rtm::V3 o = inblas ? ic.o : O, id = inblas ? ic.idir : idir;
-    const float t0 = inblas ? ic.tmin : tmin, t1 = inblas ? ic.tmax : tmax;
-    const float cull = inblas ? min_thit * ic.mult : min_thit;
-    const rtd::ChildHits ch = f ? rtd::test_children<true>(nd, v.blob + (uint64_t)unit * 4, unit, o, id, t0, t1, cull)
-                                : rtd::test_children<false>(nd, v.blob + (uint64_t)unit * 4, unit, o, id, t0, t1, cull);
-    const uint32_t level = inblas ? 0u : kTop;
-    uint32_t c = ch.child_unit, nn = kNone;
+  __device__ __forceinline__ void visit_internal(const TraceArgs& a, uint32_t unit, uint32_t level,
+                                                 const rtd::Node64& nd) {
+    const float t0 = tmin * cx.mult, t1 = tmax * cx.mult, cull = min_thit * cx.mult;
+    const uint4* src = v.blob + (uint64_t)unit * 4;
+    const rtd::ChildHits ch = cx.fast ? rtd::test_children<true>(nd, src, unit, cx.o, cx.idir, t0, t1, cull)
+                                      : rtd::test_children<false>(nd, src, unit, cx.o, cx.idir, t0, t1, cull);
+    uint32_t c = ch.child_unit, nn = 0;
 #pragma unroll
     for (int i = 0; i < 6; ++i) {
       // the first hit internal child becomes `next`; other hit children are
       // pushed (one predicated store, no branch per child)
       const uint32_t info = ch.info_of(i);
       const bool h = (ch.hit_mask >> i) & 1u, internal = (info >> 2) == rtf::CT_INTERNAL;
-      const bool take = h && internal && nn == kNone, store = h && !take, ok = sp < CAP;
-      if (store && ok) *slot(a, sp) = (c << 2) | level | (internal ? 0u : kLeaf);
-      if (store && !ok) status |= RT_RAY_STACK_OVERFLOW;
-      sp += (store && ok) ? 1 : 0;
-      nn = take ? c : nn;
+      const uint32_t e = (c << 2) | level | (internal ? 0u : kLeaf);
+      const bool take = h && internal && nn == 0, store = h && !take;
+      if (store) *slot(a, sp) = e;
+      sp += store ? 1 : 0;
+      nn = take ? e : nn;
       c += info & 3u;
     }
     next = nn;
-    if (status & RT_RAY_STACK_OVERFLOW) stop(0);
+    if (sp > CAP) stop(RT_RAY_STACK_OVERFLOW);
   }
 
   // Returns the transaction type of the leaf's second record.
   __device__ __forceinline__ uint32_t visit_leaf(const TraceArgs& a, uint32_t unit, const rtd::Node64& q) {
+    extra += kDescriptorExtra;
     if (rtf::leaf_type_of(q.w[1]) == 0) {
       const rtm::V3 v0 = rtm::v3(__uint_as_float(q.w[4]), __uint_as_float(q.w[5]), __uint_as_float(q.w[6]));
       const rtm::V3 v1 = rtm::v3(__uint_as_float(q.w[7]), __uint_as_float(q.w[8]), __uint_as_float(q.w[9]));
       const rtm::V3 v2 = rtm::v3(__uint_as_float(q.w[10]), __uint_as_float(q.w[11]), __uint_as_float(q.w[12]));
       float t = 0.0f;
-      const bool hit = rtm::ray_triangle_test(v0, v1, v2, ic.o, ic.d, t);
-      const float wt = t / ic.mult;
+      const bool hit = rtm::ray_triangle_test(v0, v1, v2, cx.o, cx.d, t);
+      const float wt = t / cx.mult;
       if (hit && tmin <= wt && wt <= tmax) {  // :2843-2859
-        if (opaque && wt < min_thit) min_thit = t / ic.mult;
-        c_leaf = unit;
-        c_inst = ic.unit;
-        c_tobj = t;
-        if (terminate) sp = 0;
+        if ((flags & kRayOpaque) && wt < min_thit) min_thit = wt;
+        set_hit(unit, cx.unit, t);
+        if (flags & kRayTerminate) sp = 0;
         return rtf::TX_QUAD_LEAF_HIT;
       }
       return rtf::TX_QUAD_LEAF;
     }
-    status |= RT_RAY_HIT_PROCEDURAL;
+    flags |= RT_RAY_HIT_PROCEDURAL;
     return rtf::TX_PROCEDURAL_LEAF;
   }
 
   // Returns the unit of the instance's second record (its BLAS header), or
   // kNone when the header lies outside the blob.
   __device__ __forceinline__ uint32_t visit_instance(const TraceArgs& a, uint32_t unit, const rtd::Node64& q) {
+    extra += kInstanceExtra;
     rtd::Instance in;
     rtd::instance_from(q, v.blob + (uint64_t)unit * 4, 0, in);
     const uint64_t hdr = (uint64_t)unit * 64 + in.bvh_address;
@@ -464,88 +493,64 @@ struct PlainWalker {
     }
     const uint4 h0 = __ldg(v.blob + (hdr >> 4));
     const uint64_t broot = hdr + ((uint64_t)h0.x | ((uint64_t)h0.y << 32));
-    enter_instance(in, unit, O, D, tmin, tmax, ic);
-    ic_fast = v.ordered && rtd::finite_ray(ic.o, ic.d, ic.tmin, ic.tmax);
-    push(a, (uint32_t)(broot >> 6) << 2);
-    inblas = true;
-    if (status & RT_RAY_STACK_OVERFLOW) stop(0);
+    enter_instance(in, unit, world_o(), world_d(), tmin, tmax, v.ordered, cx);
+    if (sp < CAP) next = (uint32_t)(broot >> 6) << 2;
+    else stop(RT_RAY_STACK_OVERFLOW);
     return (uint32_t)(hdr >> 6);
   }
 
-  // One node visit (the caller checks active() first).  The node to visit is
-  // found first and its first 64 bytes loaded once for every kind, so a
-  // warp's lanes at internal nodes, leaves and instance leaves issue one load.
-  __device__ __forceinline__ void step(const TraceArgs& a) {
-    uint32_t unit, kind;  // 0 internal node, 1 primitive leaf, 2 instance leaf
-    for (;;) {
-      if (next != kNone) {
-        unit = next;
-        kind = 0;
-        break;
-      }
-      if (inblas) {
-        if (sp > 0 && !(*slot(a, sp - 1) & kTop)) {
-          const uint32_t e = pop(a);
-          if (e & kLeaf) {
-            unit = e >> 2;
-            kind = 1;
-            break;
-          }
-          next = e >> 2;
-          continue;
-        }
-        inblas = false;
-        continue;
-      }
-      if (sp == 0) return;
-      const uint32_t e = pop(a);
-      if (!(e & kLeaf)) {
-        next = e >> 2;
-        continue;
-      }
-      unit = e >> 2;
-      kind = 2;
-      break;
-    }
-    if (unit + (kind == 2 ? 1u : 0u) >= v.n_units) return stop(RT_RAY_BAD_NODE);
+  // One node visit (the caller checks active() first).  The node's first 64
+  // bytes are loaded once for every kind, so a warp's lanes at internal
+  // nodes, leaves and instance leaves issue one load.
+  __device__ __forceinline__ void step(const TraceArgs& a, uint32_t r) {
+    uint32_t e = next;
+    next = 0;
+    if (!e) e = *slot(a, --sp);
+    const bool top = e & kTop, leaf = e & kLeaf;
+    const uint32_t unit = e >> 2;
+    if (unit + ((top && leaf) ? 1u : 0u) >= v.n_units) return stop(RT_RAY_BAD_NODE);
     rtd::Node64 q;
     rtd::load64(v.blob + (uint64_t)unit * 4, 0, q);
     // a visit records one or two transactions; two call sites for all kinds
     // keep the recording code (staged through shared memory) out of every
     // branch
-    rec.rec<TRACED>(a, unit, kind == 0 ? rtf::TX_INTERNAL : (kind == 1 ? rtf::TX_LEAF_DESC : rtf::TX_INSTANCE_LEAF));
+    record(a, r, unit, !leaf ? rtf::TX_INTERNAL : (top ? rtf::TX_INSTANCE_LEAF : rtf::TX_LEAF_DESC));
     uint32_t unit2 = unit, type2 = rtf::TX_STRUCTURE;
-    if (kind == 0) {
-      visit_internal(a, unit, q);
+    if (!leaf) {
+      if (top && cx.unit != kNone) world();
+      visit_internal(a, unit, e & kTop, q);
       unit2 = kNone;
-    } else if (kind == 1) {
+    } else if (!top) {
       type2 = visit_leaf(a, unit, q);
     } else {
       unit2 = visit_instance(a, unit, q);
     }
-    if (unit2 != kNone) rec.rec<TRACED>(a, unit2, type2);
+    if (unit2 != kNone) record(a, r, unit2, type2);
   }
 
-  // (the walk keeps its own rows in the recorder; the ray index is not needed)
-  __device__ __forceinline__ void step(const TraceArgs& a, uint32_t) { step(a); }
-
   __device__ __forceinline__ void finish(const TraceArgs& a, uint32_t r) {
-    const bool bad = status & (RT_RAY_STACK_OVERFLOW | RT_RAY_BAD_NODE);
-    if (TRACED) trace_drain(a, rec.vrow, rec.trow, min(rec.n, rec.cap));
-    write_hit(a, v, r, !bad && (min_thit < tmax), min_thit, O, D, tmin, tmax, c_leaf, c_inst, c_tobj, rec, status);
+    const bool bad = flags & (RT_RAY_STACK_OVERFLOW | RT_RAY_BAD_NODE);
+    if (TRACED)
+      trace_drain(a, a.visits ? a.visits + (uint64_t)r * a.cap : nullptr,
+                  a.tl_trace ? a.tl_trace + (uint64_t)r * a.cap : nullptr, min(n_tx, a.cap));
+    write_hit(a, v, r, !bad && (min_thit < tmax), min_thit, world_o(), world_d(), tmin, tmax, cold(9), cold(10),
+              __uint_as_float(cold(11)), n_tx, flags & kRayStatusMask);
   }
 };
 
-// The plain walk keeps its stack inside the walker, whose fields the compiler
-// then leaves in local memory: 48 registers and five 256-thread CTAs per SM
-// (the launch bound holds it there: with the trace staging the compiler
-// would take 54 registers and fit four CTAs, 2-8% slower untraced and 7%
-// slower traced on bounce rays).
-// Its fields in registers (90, or capped at 51-85 with spills) measured
-// 40-45% slower, while the treelet walks gained from them (below).
+// Four 256-thread CTAs per SM, 64 registers.  With one ray context in
+// registers and the rest in the stack's cold words, 2M bounce rays of the
+// 2M-triangle terrain take 3.23 ms on a GB300; five CTAs at 48 registers
+// spill and take 3.52 ms, three 3.34 ms.  (With both the world ray and the
+// object ray live the walk took 90 registers, and did best with all its
+// fields left in local memory at 48: 4.27 ms, bound by those loads.)
+constexpr int kPlainMinBlocks = 4;
 template <int CAP, bool MULTI, bool TRACED, bool SHORT = false>
-__global__ void __launch_bounds__(256, 5) trace_plain_kernel(TraceArgs a) {
+__global__ void __launch_bounds__(256, kPlainMinBlocks) trace_plain_kernel(TraceArgs a) {
+  uint32_t stack[CAP + kStackPad + kPlainCold];
   PlainWalker<CAP, MULTI, TRACED, SHORT> w;
+  w.stk = stack;
+  w.extra = 0;
   unsigned long long bytes = 0;
   run_persistent(a, w, bytes);
   if (a.stats) add_warp_total64(a.stats + ST_NODE_BYTES, bytes);

@@ -105,12 +105,15 @@ __global__ void __launch_bounds__(kStagedMaxThreads, kStagedMinBlocks) trace_que
     const uint32_t u = loc & ((1u << kSlotBitsDev) - 1u);
     return u < slot_units[warp] ? slot_base + u * 64u : 0u;
   };
-  unsigned long long stack[CAP + kColdWords];
-  Walker<CAP, true, false, true> w;
+  using W = Walker<CAP, true, false, true>;
+  unsigned long long stack[W::kWords];
+  W w;
   w.stk = stack;
+  w.extra = 0;
+  w.smem_reads = w.gmem_reads = 0;
   w.pin_base = 0;
   w.pin_root = 0;
-  unsigned long long bytes = 0, staged = 0, stagings = 0, sreads = 0, greads = 0;
+  unsigned long long bytes = 0, staged = 0, stagings = 0;
 
   if (FINAL) {
     // every ray still walking goes to its end, one node visit per iteration,
@@ -134,7 +137,7 @@ __global__ void __launch_bounds__(kStagedMaxThreads, kStagedMinBlocks) trace_que
             have = true;
             if (!w.active()) {
               w.finish(a, r);
-              bytes += w.rec.bytes;
+              bytes += 64ull * w.n_tx;
               have = false;
             }
           }
@@ -148,9 +151,7 @@ __global__ void __launch_bounds__(kStagedMaxThreads, kStagedMinBlocks) trace_que
         w.step(a, r, lookup);
         if (!w.active()) {
           w.finish(a, r);
-          bytes += w.rec.bytes;
-          sreads += w.smem_reads;
-          greads += w.gmem_reads;
+          bytes += 64ull * w.n_tx;
           have = false;
         }
       }
@@ -230,11 +231,7 @@ __global__ void __launch_bounds__(kStagedMaxThreads, kStagedMinBlocks) trace_que
       const bool cont = live && w.active();
       if (valid && !cont) {
         w.finish(a, r);
-        bytes += w.rec.bytes;
-      }
-      if (valid) {
-        sreads += w.smem_reads;
-        greads += w.gmem_reads;
+        bytes += 64ull * w.n_tx;
       }
       // rays that go on: state out, queued for the next round
       const uint32_t cmask = __ballot_sync(0xffffffffu, cont);
@@ -259,9 +256,9 @@ __global__ void __launch_bounds__(kStagedMaxThreads, kStagedMinBlocks) trace_que
   }
   __syncwarp();
   if (a.stats) {
-    add_warp_total64(a.stats + ST_NODE_BYTES, bytes);
-    add_warp_total64(a.stats + ST_SMEM_READS, sreads);
-    add_warp_total64(a.stats + ST_GMEM_READS, greads);
+    add_warp_total64(a.stats + ST_NODE_BYTES, bytes + (unsigned long long)(8ll * w.extra));
+    add_warp_total64(a.stats + ST_SMEM_READS, w.smem_reads);
+    add_warp_total64(a.stats + ST_GMEM_READS, w.gmem_reads);
     add_warp_total64(a.stats + ST_STAGED_BYTES, staged);
     add_warp_total64(a.stats + ST_STAGINGS, stagings);
   }

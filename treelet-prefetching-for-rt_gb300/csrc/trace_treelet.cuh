@@ -16,9 +16,9 @@ constexpr uint32_t kRouteOther = 6, kRouteInst = 12;  // route bits (treelets.h)
 
 // A ray's treelet-ordered walk.  Two LIFO stacks as in the reference
 // (push_front / pop_front on std::list, :1708-1709): `cu` holds nodes of the
-// current treelet, `ot` the rest (:1821-1856).  Both live in one local
-// array (cu at [0, CAP), ot at [CAP, 2 CAP)), so that a push goes to either
-// with one predicated store instead of a branch per child.  Which stack a child goes to
+// current treelet, `ot` the rest (:1821-1856).  Both live in one local array
+// (cu first, then ot), so that a push goes to either with one predicated
+// store instead of a branch per child.  Which stack a child goes to
 // is read from the per-node route bits (treelets.h): a node popped from `cu`
 // is in the current treelet, and a node popped from `ot` becomes the current
 // treelet root, so the reference's addrToTreeletID comparison is fixed per
@@ -27,16 +27,11 @@ constexpr uint32_t kRouteOther = 6, kRouteInst = 12;  // route bits (treelets.h)
 // warp has a staged slot; pinned nodes are named by their record.
 //
 // Fields a step rarely needs live in the tail of the stack array, in local
-// memory, instead of registers (kColdWords 64-bit words after the 2 CAP stack
-// entries): the world direction, the closest hit and, in the unstaged walk,
-// the world origin and inverse direction, which only TLAS nodes and instance
-// entries read.  The trace rows are found from the ray index, which the
-// kernel's loop holds anyway, instead of from the tail (two local loads per
-// recorded transaction before).  Fewer live registers let the treelet
-// walk run four CTAs per SM at 64 registers: +5% on bounce rays, +2% on
-// primary rays; the staged walk, with its pinned-record state, measured best
-// with the world ray in registers at three CTAs per SM.
-constexpr int kColdWords = 7;
+// memory, instead of registers (kColdWords 64-bit words): the world ray, read
+// when the walk comes back to a top-level node or enters an instance, and the
+// closest hit.  The trace rows are found from the ray index, which the
+// kernel's loop holds anyway.
+constexpr int kColdWords = 6;
 
 // SLAB = true keeps the other-treelet stack in a per-ray slab of global
 // memory (`ot`, CAP entries) instead of the local array, so that a ray can
@@ -47,89 +42,86 @@ constexpr int kColdWords = 7;
 // at all).
 template <int CAP, bool STAGED, bool MULTI, bool SLAB = false, bool TRACED = true>
 struct Walker {
-  static constexpr bool kColdWorld = !STAGED;
-  static constexpr int kOtLocal = SLAB ? 0 : CAP;  // other-stack entries in the local array
-  rtm::V3 O, idir;  // world ray (registers only when !kColdWorld)
+  // local array: cu, ot (unless SLAB), each with room for the entries a visit
+  // may push before its depths are checked, then the cold words
+  static constexpr int kOt = CAP + kStackPad, kCold = SLAB ? kOt : kOt + CAP + kStackPad;
+  static constexpr int kWords = kCold + kColdWords;
+  RayCtx cx;
   float tmin, tmax, min_thit;
-  bool terminate, fast, ic_fast;  // FAST min/max allowed for the world / object ray
-  uint32_t status;
-  unsigned long long* stk;  // CAP + kOtLocal + kColdWords entries, a local array of the kernel
+  uint32_t flags;
+  unsigned long long* stk;  // kWords entries, a local array of the kernel
   unsigned long long* ot;   // SLAB: the ray's other-treelet stack in global memory
   int ncu, not_;            // entries on cu and on ot
   // The top of `cu` when it was pushed by the previous node visit: the node
   // the walk pops next, kept in a register instead of a local-memory round
   // trip (0 = none; no stack entry is 0, a blob's unit 0 is its TLAS header).
   unsigned long long nxt;
-  InstCtx ic;
-  // Visit recording: the counts in registers, the trace rows in the cold tail.
-  struct Counts {
-    uint32_t cap, n, bytes;
-  } rec;
+  uint32_t n_tx;  // the ray's transactions
+  int extra;      // the thread's byte difference (kInstanceExtra)
   SceneView v;
-  uint32_t smem_reads, gmem_reads;
+  uint32_t smem_reads, gmem_reads;  // the thread's node reads (staged walks)
   uint32_t pin_base;  // shared address of the pinned records, 0 = none
   uint32_t pin_root;  // record of the TLAS root node, 0 = not pinned
 
-  __device__ __forceinline__ bool active() const { return nxt != 0 || (ncu | not_) != 0; }
+  __device__ __forceinline__ bool active() const { return (ncu | not_) != 0; }
 
   __device__ __forceinline__ void clear() {
     nxt = 0;
     ncu = not_ = 0;
   }
 
-  // ---- the cold tail: stk[CAP + kOtLocal + k]
-  __device__ __forceinline__ unsigned long long& cold(int k) const { return stk[CAP + kOtLocal + k]; }
+  // ---- the cold words
+  __device__ __forceinline__ unsigned long long& cold(int k) const { return stk[kCold + k]; }
   // ---- entry i of the other-treelet stack
-  __device__ __forceinline__ unsigned long long& ot_at(int i) const { return SLAB ? ot[i] : stk[CAP + i]; }
+  __device__ __forceinline__ unsigned long long& ot_at(int i) const { return SLAB ? ot[i] : stk[kOt + i]; }
   static __device__ __forceinline__ unsigned long long pack(float a, float b) {
     return (unsigned long long)__float_as_uint(a) | ((unsigned long long)__float_as_uint(b) << 32);
   }
   static __device__ __forceinline__ float lo(unsigned long long w) { return __uint_as_float((uint32_t)w); }
   static __device__ __forceinline__ float hi(unsigned long long w) { return __uint_as_float((uint32_t)(w >> 32)); }
-  __device__ __forceinline__ void set_dir(rtm::V3 d) {
+  __device__ __forceinline__ void set_world(rtm::V3 o, rtm::V3 d, rtm::V3 id) {
     cold(0) = pack(d.x, d.y);
-    cold(1) = pack(d.z, 0.0f);
+    reinterpret_cast<uint32_t*>(&cold(1))[0] = __float_as_uint(d.z);
+    cold(3) = pack(o.x, o.y);
+    cold(4) = pack(o.z, id.x);
+    cold(5) = pack(id.y, id.z);
   }
   __device__ __forceinline__ rtm::V3 dir() const {
     const unsigned long long a = cold(0), b = cold(1);
     return rtm::v3(lo(a), hi(a), lo(b));
   }
-  __device__ __forceinline__ void set_hit(uint32_t leaf, uint32_t inst, float tobj) {
-    cold(2) = (unsigned long long)leaf | ((unsigned long long)inst << 32);
-    cold(3) = pack(tobj, 0.0f);
-  }
-  __device__ __forceinline__ void set_world(rtm::V3 o, rtm::V3 id) {
-    if (kColdWorld) {
-      cold(4) = pack(o.x, o.y);
-      cold(5) = pack(o.z, id.x);
-      cold(6) = pack(id.y, id.z);
-    } else {
-      O = o;
-      idir = id;
-    }
-  }
   __device__ __forceinline__ rtm::V3 world_o() const {
-    if (!kColdWorld) return O;
-    const unsigned long long a = cold(4), b = cold(5);
+    const unsigned long long a = cold(3), b = cold(4);
     return rtm::v3(lo(a), hi(a), lo(b));
   }
   __device__ __forceinline__ rtm::V3 world_idir() const {
-    if (!kColdWorld) return idir;
-    const unsigned long long b = cold(5), c = cold(6);
+    const unsigned long long b = cold(4), c = cold(5);
     return rtm::v3(hi(b), lo(c), hi(c));
+  }
+  // the closest hit: word 2 its leaf and instance, the high half of word 1 its object-space t
+  __device__ __forceinline__ void set_hit(uint32_t leaf, uint32_t inst, float tobj) {
+    cold(2) = (unsigned long long)leaf | ((unsigned long long)inst << 32);
+    reinterpret_cast<uint32_t*>(&cold(1))[1] = __float_as_uint(tobj);
+  }
+  // The world ray as the ray tested with (RayCtx).
+  __device__ __forceinline__ void world() {
+    cx.unit = kNone;
+    cx.o = world_o();
+    cx.idir = world_idir();
+    cx.mult = 1.0f;
+    cx.fast = (flags & kRayWorldFast) != 0;
   }
   // one visit of the trace (the reference's MemoryTransactionRecord)
   // The rows are written entry by entry: staging them through shared memory
   // as the plain walk does measured 15-30% slower here (eight inlined
   // copies of the staging code in the traced walk).
   __device__ __forceinline__ void record(const TraceArgs& a, uint32_t r, uint32_t unit, uint32_t type) {
-    if (TRACED && rec.n < rec.cap) {
-      const uint64_t at = (uint64_t)r * a.cap + rec.n;
+    if (TRACED && n_tx < a.cap) {
+      const uint64_t at = (uint64_t)r * a.cap + n_tx;
       if (a.visits) a.visits[at] = rtf::pack_visit(unit, type);
       if (a.tl_trace) a.tl_trace[at] = v.meta[unit].x;
     }
-    rec.n++;
-    rec.bytes += rtf::tx_bytes(type);
+    n_tx++;
   }
 
   // Staged location (dense treelet << 10 | slot) of the node the ray visits
@@ -145,26 +137,25 @@ struct Walker {
     return unit < v.n_units ? __ldg(reinterpret_cast<const uint32_t*>(v.meta) + 2ull * unit + 1) : kNone;
   }
 
+  // Pushes an entry onto cu (same treelet; it becomes nxt too) or ot.  Depths
+  // are checked once per visit (too_deep); a slab has no room past CAP, so an
+  // entry beyond it is not written (the ray is flagged and its stacks cleared).
   __device__ __forceinline__ void push(bool same, uint32_t code, uint32_t inst) {
     const unsigned long long e = (unsigned long long)code | ((unsigned long long)inst << 32);
-    // same treelet: e becomes nxt and the previous nxt (if any) goes to cu;
-    // else e goes to ot.  One predicated store instead of a branch per child
-    // (treelet walk +5% on bounce rays, staged walk +4%).
-    const bool store = !same || nxt != 0;
-    const int cnt = same ? ncu : not_;
-    const bool ok = cnt < CAP;
-    if (store && ok) {
-      if (SLAB) *(same ? stk + cnt : ot + cnt) = same ? nxt : e;
-      else stk[same ? cnt : CAP + cnt] = same ? nxt : e;
+    if (SLAB) {
+      if (same || not_ < CAP) *(same ? stk + ncu : ot + not_) = e;
+    } else {
+      stk[same ? ncu : kOt + not_] = e;
     }
-    if (store && !ok) status |= RT_RAY_STACK_OVERFLOW;
-    ncu += (same && store && ok) ? 1 : 0;
-    not_ += (!same && ok) ? 1 : 0;
+    ncu += same ? 1 : 0;
+    not_ += same ? 0 : 1;
     nxt = same ? e : nxt;
   }
+  // CAP entries per stack, one more on cu for the entry held in nxt
+  __device__ __forceinline__ bool too_deep() const { return ncu > CAP + 1 || not_ > CAP; }
 
   __device__ __forceinline__ void bad_node() {
-    status |= RT_RAY_BAD_NODE;
+    flags |= RT_RAY_BAD_NODE;
     clear();
   }
 
@@ -172,20 +163,16 @@ struct Walker {
     v = scene_of<MULTI>(a, r);
     rtm::V3 o, D;
     load_ray(a.rays, r, o, tmin, D, tmax);
-    const uint32_t flags = a.flags ? a.flags[r] : a.default_flags;
-    terminate = flags & rtf::RAY_FLAG_TERMINATE_ON_FIRST_HIT;
-    rec = Counts{a.cap, 0u, 0u};
-    status = 0;
+    const uint32_t f = a.flags ? a.flags[r] : a.default_flags;
+    flags = f & rtf::RAY_FLAG_TERMINATE_ON_FIRST_HIT ? kRayTerminate : 0u;
+    n_tx = 0;
     clear();
     min_thit = tmax;
-    set_hit(0, 0, 0.0f);
-    set_dir(D);
-    ic.unit = kNone;
-    smem_reads = gmem_reads = 0;
     const rtm::V3 id = rtm::calculate_idir(D);
-    set_world(o, id);
-    fast = v.ordered && rtd::finite_ray(o, D, tmin, tmax);
-    ic_fast = false;
+    set_world(o, D, id);
+    set_hit(0, 0, 0.0f);
+    if (v.ordered && rtd::finite_ray(o, D, tmin, tmax)) flags |= kRayWorldFast;
+    world();
     record(a, r, 0, rtf::TX_STRUCTURE);
     const uint4 h0 = __ldg(v.blob), h1 = __ldg(v.blob + 1);
     const uint64_t root_off = (uint64_t)h0.x | ((uint64_t)h0.y << 32);
@@ -203,7 +190,7 @@ struct Walker {
 
   // ---- the treelet-queued walk (SLAB): a ray's state between two treelets,
   // 64 bytes: the ray (origin, tmin, direction, tmax), then min_thit, status
-  // (bit 31: terminate on first hit), transactions and bytes recorded, the
+  // (bit 31: terminate on first hit), transactions, a spare word, the
   // closest leaf, its instance, its object-space t, and the other-treelet
   // stack's size.  The current-treelet stack is empty between treelets.
   static constexpr uint32_t kTerminateBit = 0x80000000u;
@@ -216,8 +203,9 @@ struct Walker {
 
   __device__ __forceinline__ void suspend(uint4* st) const {
     const unsigned long long h = cold(2);
-    st[2] = make_uint4(__float_as_uint(min_thit), status | (terminate ? kTerminateBit : 0u), rec.n, rec.bytes);
-    st[3] = make_uint4((uint32_t)h, (uint32_t)(h >> 32), (uint32_t)cold(3), (uint32_t)not_);
+    st[2] = make_uint4(__float_as_uint(min_thit),
+                       (flags & kRayStatusMask) | ((flags & kRayTerminate) ? kTerminateBit : 0u), n_tx, 0u);
+    st[3] = make_uint4((uint32_t)h, (uint32_t)(h >> 32), (uint32_t)(cold(1) >> 32), (uint32_t)not_);
   }
 
   __device__ __forceinline__ void resume(const TraceArgs& a, uint32_t r, const uint4* st) {
@@ -228,37 +216,30 @@ struct Walker {
     tmin = __uint_as_float(q0.w);
     tmax = __uint_as_float(q1.w);
     min_thit = __uint_as_float(q2.x);
-    status = q2.y & ~kTerminateBit;
-    terminate = (q2.y & kTerminateBit) != 0;
-    rec = Counts{a.cap, q2.z, q2.w};
-    cold(2) = (unsigned long long)q3.x | ((unsigned long long)q3.y << 32);
-    cold(3) = (unsigned long long)q3.z;
+    flags = (q2.y & kRayStatusMask) | ((q2.y & kTerminateBit) ? kRayTerminate : 0u);
+    n_tx = q2.z;
+    set_world(o, D, rtm::calculate_idir(D));
+    set_hit(q3.x, q3.y, __uint_as_float(q3.z));
     nxt = 0;
     ncu = 0;
     not_ = (int)q3.w;
-    set_dir(D);
-    ic.unit = kNone;
-    ic_fast = false;
-    smem_reads = gmem_reads = 0;
-    set_world(o, rtm::calculate_idir(D));
-    fast = v.ordered && rtd::finite_ray(o, D, tmin, tmax);
+    if (v.ordered && rtd::finite_ray(o, D, tmin, tmax)) flags |= kRayWorldFast;
+    world();
   }
 
   // True while the walk is inside its current treelet: the next pop would
   // come from the current-treelet stack.
-  __device__ __forceinline__ bool in_treelet() const { return nxt != 0 || ncu > 0; }
+  __device__ __forceinline__ bool in_treelet() const { return ncu > 0; }
 
   // Visits one node; `lookup(unit, meta)` returns the shared-memory address
   // of a node staged in a warp slot, else 0.
   template <class Lookup>
   __device__ __forceinline__ void step(const TraceArgs& a, uint32_t r, Lookup&& lookup) {
-    const bool from_cu = nxt != 0 || ncu > 0;  // :1748-1754
+    const bool from_cu = ncu > 0;  // :1748-1754
     unsigned long long e = nxt;
-    if (!nxt) {
-      e = SLAB ? (from_cu ? stk[ncu - 1] : ot[not_ - 1]) : stk[from_cu ? ncu - 1 : CAP + not_ - 1];
-      ncu -= from_cu ? 1 : 0;
-      not_ -= from_cu ? 0 : 1;
-    }
+    if (!e) e = SLAB ? (from_cu ? stk[ncu - 1] : ot[not_ - 1]) : stk[from_cu ? ncu - 1 : kOt + not_ - 1];
+    ncu -= from_cu ? 1 : 0;
+    not_ -= from_cu ? 0 : 1;
     nxt = 0;
     const uint32_t code = (uint32_t)e, inst = (uint32_t)(e >> 32);
     const bool top = code & kTop, leaf = code & kLeaf, pinned = STAGED && (code & kEPin);
@@ -297,11 +278,12 @@ struct Walker {
     } else {
       rtd::load64(g, 0, nd);
     }
-    // The instance context, once for every kind of node: an instance leaf
-    // enters its own instance; a BLAS node needs its instance's object ray,
+    // The ray context, once for every kind of node: an instance leaf enters
+    // its own instance; a BLAS node needs its instance's object ray,
     // recomputed when the walk comes back from another instance's nodes
     // (make_transformed_ray is deterministic, so recomputing gives the
-    // reference's stored objectRay).  Lanes of all kinds switch together.
+    // reference's stored objectRay); a top-level node needs the world ray.
+    // Lanes of all kinds switch together.
     rtd::Instance in;
     uint32_t enter = kNone;
     if (top && leaf) {
@@ -312,15 +294,13 @@ struct Walker {
         rtd::instance_from(nd, g, saddr, in);
       }
       enter = unit;
-    } else if (!top && inst != ic.unit) {
+    } else if (!top && inst != cx.unit) {
       rtd::load_instance(v.blob + (uint64_t)inst * 4, 0, in);
       enter = inst;
     }
-    if (enter != kNone) {
-      enter_instance(in, enter, world_o(), dir(), tmin, tmax, ic);
-      ic_fast = v.ordered && rtd::finite_ray(ic.o, ic.d, ic.tmin, ic.tmax);
-    }
+    if (enter != kNone) enter_instance(in, enter, world_o(), dir(), tmin, tmax, v.ordered, cx);
     if (!leaf) {  // internal node, top (:1758-1869) or bottom (:1954-2070)
+      if (top && cx.unit != kNone) world();
       record(a, r, unit, rtf::TX_INTERNAL);
       uint32_t soff01 = 0, soff23 = 0, soff45 = 0;
       if (pinned) {  // route bits in bytes 16..17, child records in the tail
@@ -332,13 +312,9 @@ struct Walker {
       } else {
         rbits = __ldg(v.route + unit);
       }
-      // one box test for both levels, so lanes at TLAS and BLAS nodes run it together
-      const bool f = top ? fast : ic_fast;
-      const rtm::V3 o = top ? world_o() : ic.o, id = top ? world_idir() : ic.idir;
-      const float t0 = top ? tmin : ic.tmin, t1 = top ? tmax : ic.tmax;
-      const float cull = top ? min_thit : min_thit * ic.mult;
-      const rtd::ChildHits ch = f ? rtd::test_children<true>(nd, src, unit, o, id, t0, t1, cull)
-                                  : rtd::test_children<false>(nd, src, unit, o, id, t0, t1, cull);
+      const float t0 = tmin * cx.mult, t1 = tmax * cx.mult, cull = min_thit * cx.mult;
+      const rtd::ChildHits ch = cx.fast ? rtd::test_children<true>(nd, src, unit, cx.o, cx.idir, t0, t1, cull)
+                                        : rtd::test_children<false>(nd, src, unit, cx.o, cx.idir, t0, t1, cull);
       const uint32_t hit = ch.hit_mask;
       const uint64_t info = ch.info;
       const uint32_t same = rbits >> (rsh * kRouteOther);
@@ -358,6 +334,7 @@ struct Walker {
       }
     } else if (top) {  // instance leaf (:1870-1953)
       record(a, r, unit, rtf::TX_INSTANCE_LEAF);
+      extra += kInstanceExtra;
       uint32_t hdr_unit, broot_unit, broot_soff = 0;
       if (pinned) {  // the 64-byte record: units, route bits, BLAS root record, rows
         hdr_unit = nd.w[rtp::IL_HDR_UNIT / 4];
@@ -378,28 +355,32 @@ struct Walker {
       push((rbits >> (kRouteInst + rsh)) & 1u, cc, unit);
     } else {  // primitive leaf (:2071-2196)
       record(a, r, unit, rtf::TX_LEAF_DESC);
+      extra += kDescriptorExtra;
       const rtd::Node64& q = nd;
       if (rtf::leaf_type_of(q.w[1]) == 0) {
         const rtm::V3 v0 = rtm::v3(__uint_as_float(q.w[4]), __uint_as_float(q.w[5]), __uint_as_float(q.w[6]));
         const rtm::V3 v1 = rtm::v3(__uint_as_float(q.w[7]), __uint_as_float(q.w[8]), __uint_as_float(q.w[9]));
         const rtm::V3 v2 = rtm::v3(__uint_as_float(q.w[10]), __uint_as_float(q.w[11]), __uint_as_float(q.w[12]));
         float t = 0.0f;
-        const bool hit = rtm::ray_triangle_test(v0, v1, v2, ic.o, ic.d, t);
-        const float wt = t / ic.mult;
+        const bool hit = rtm::ray_triangle_test(v0, v1, v2, cx.o, cx.d, t);
+        const float wt = t / cx.mult;
         if (hit && tmin <= wt && wt <= tmax && wt < min_thit) {  // :2127-2141
-          min_thit = t / ic.mult;
+          min_thit = wt;
           set_hit(unit, inst, t);
           record(a, r, unit, rtf::TX_QUAD_LEAF_HIT);
-          if (terminate) clear();
+          if (flags & kRayTerminate) clear();
         } else {
           record(a, r, unit, rtf::TX_QUAD_LEAF);
         }
       } else {
-        status |= RT_RAY_HIT_PROCEDURAL;
+        flags |= RT_RAY_HIT_PROCEDURAL;
         record(a, r, unit, rtf::TX_PROCEDURAL_LEAF);
       }
     }
-    if (status & RT_RAY_STACK_OVERFLOW) clear();
+    if (too_deep()) {
+      flags |= RT_RAY_STACK_OVERFLOW;
+      clear();
+    }
   }
 
   __device__ __forceinline__ void step(const TraceArgs& a, uint32_t r) {
@@ -407,25 +388,28 @@ struct Walker {
   }
 
   __device__ __forceinline__ void finish(const TraceArgs& a, uint32_t r) {
-    const bool bad = status & (RT_RAY_STACK_OVERFLOW | RT_RAY_BAD_NODE);
+    const bool bad = flags & (RT_RAY_STACK_OVERFLOW | RT_RAY_BAD_NODE);
     const unsigned long long h = cold(2);
-    const Recorder counts{nullptr, nullptr, rec.cap, rec.n, rec.bytes, v.meta};
     write_hit(a, v, r, !bad && (min_thit < tmax), min_thit, world_o(), dir(), tmin, tmax, (uint32_t)h,
-              (uint32_t)(h >> 32), lo(cold(3)), counts, status);
+              (uint32_t)(h >> 32), hi(cold(1)), n_tx, flags & kRayStatusMask);
   }
 };
 
 // The walker's stacks are a separate local array so that its fields stay in
-// registers (+5% over the walker with its stacks inside, whose fields the
-// compiler left in local memory); with its rarely used fields in the stack's
-// cold tail it fits four 256-thread CTAs per SM at 64 registers.
+// registers (stacks inside it would leave every field in local memory); with
+// one ray context in registers (RayCtx) and the rarely used fields in the
+// cold words it fits four 256-thread CTAs per SM at 64 registers: 2M any-hit
+// rays 1.86 ms on a GB300 (three CTAs 1.93, five at 48 registers 2.15; with
+// the world ray and the object ray both held, 2.13).
 constexpr int kTreeletMinBlocks = 4;
 
 template <int CAP, bool MULTI, bool TRACED>
 __global__ void __launch_bounds__(256, kTreeletMinBlocks) trace_treelet_kernel(TraceArgs a) {
-  unsigned long long stack[2 * CAP + kColdWords];
-  Walker<CAP, false, MULTI, false, TRACED> w;
+  using W = Walker<CAP, false, MULTI, false, TRACED>;
+  unsigned long long stack[W::kWords];
+  W w;
   w.stk = stack;
+  w.extra = 0;
   w.pin_base = 0;
   w.pin_root = 0;
   unsigned long long bytes = 0;
@@ -488,9 +472,9 @@ __device__ __forceinline__ void bulk_copy_g2s(void* dst, const void* src, uint32
 
 constexpr int kMaxSlots = 8;  // slots per warp
 constexpr uint32_t kWaitTries = 1u << 22;
-// Three 256-thread CTAs per SM, 85 registers a thread as the treelet walk:
-// measured against one 512-thread CTA per SM (108 registers, no spills),
-// +3% on primary rays and +2% on bounce rays.
+// Three 256-thread CTAs per SM, at most 85 registers a thread (no spills with
+// one ray context held): 2M primary rays 2.86 ms on a GB300 against 3.12 ms
+// with both rays held and 52 bytes of spills.
 constexpr int kStagedMaxThreads = 256;
 constexpr int kStagedMinBlocks = 3;
 constexpr uint32_t kPinChunk = 32768;  // bytes per bulk copy of the pinned image
@@ -570,23 +554,24 @@ __global__ void __launch_bounds__(kStagedMaxThreads, kStagedMinBlocks) trace_sta
       if (st.resident[s] == d && u < st.units[s]) return slot_base + s * a.slot_bytes + u * 64u;
     return 0u;
   };
-  unsigned long long stack[2 * CAP + kColdWords];
-  Walker<CAP, true, false, false, TRACED> w;  // staged launches trace one scene
+  using W = Walker<CAP, true, false, false, TRACED>;  // staged launches trace one scene
+  unsigned long long stack[W::kWords];
+  W w;
   w.stk = stack;
+  w.extra = 0;
+  w.smem_reads = w.gmem_reads = 0;
   w.pin_base = pin_ok ? smem_u32(smem0) : 0u;
   w.pin_root = pin_ok ? a.pin_root : 0u;
   bool have = false, ended = false, exhausted = false;
   uint32_t r = 0, it = 0;
-  unsigned long long bytes = 0, staged = 0, stagings = 0, sreads = 0, greads = 0;
+  unsigned long long bytes = 0, staged = 0, stagings = 0;
   for (;; ++it) {
     // --- records of finished rays, then new rays for idle lanes (as run_persistent)
     const uint32_t need = __ballot_sync(0xffffffffu, !have);
     if (need == 0xffffffffu || (!exhausted && __popc(need) >= (int)a.refill)) {
       if (ended) {
         w.finish(a, r);
-        bytes += w.rec.bytes;
-        sreads += w.smem_reads;
-        greads += w.gmem_reads;
+        bytes += 64ull * w.n_tx;
         ended = false;
       }
       if (exhausted) break;  // every lane is idle
@@ -678,9 +663,9 @@ __global__ void __launch_bounds__(kStagedMaxThreads, kStagedMinBlocks) trace_sta
   }
   __syncwarp();
   if (a.stats) {
-    add_warp_total64(a.stats + ST_NODE_BYTES, bytes);
-    add_warp_total64(a.stats + ST_SMEM_READS, sreads);
-    add_warp_total64(a.stats + ST_GMEM_READS, greads);
+    add_warp_total64(a.stats + ST_NODE_BYTES, bytes + (unsigned long long)(8ll * w.extra));
+    add_warp_total64(a.stats + ST_SMEM_READS, w.smem_reads);
+    add_warp_total64(a.stats + ST_GMEM_READS, w.gmem_reads);
     add_warp_total64(a.stats + ST_STAGED_BYTES, staged);
     add_warp_total64(a.stats + ST_STAGINGS, stagings);
   }
