@@ -262,8 +262,49 @@ __device__ __forceinline__ void add_warp_total64(unsigned long long* dst, unsign
   if ((threadIdx.x & 31u) == 0) atomicAdd(dst, v);
 }
 
+// One turn of a warp's lanes (all 32 call it; `have`: the lane walks a ray).
+// A lane's next node is an internal node, a primitive leaf, or an entry: an
+// instance leaf, or a node of another instance than the one whose ray the
+// lane holds.  The three kinds cost about 300, 150 and 250 instructions, and
+// most nodes are internal; a warp that visits one node of every lane per turn
+// spends half its issue slots on leaves and entries with few lanes active.
+// So internal nodes are visited again and again while at least
+// kInternalShare / 16 of the walking lanes are at one; leaf and entry lanes
+// wait, and are then visited together.  Every ray's own visit order is
+// unchanged.  A lane whose ray is over gets have = false, ended = true; the
+// turn ends early once `spare` lanes have no ray.
+// Measured on a GB300 (2M-triangle terrain, 1M-triangle blobs; ms): one visit of
+// every lane per turn 3.23 for 2M bounce rays plain, 3.12 for 1M traced bounce
+// rays in treelet order, 1.86 for 2M any-hit rays; share 4 3.57 / 3.07 / 2.34,
+// 8 2.98 / 2.83 / 1.88, 11 2.86 / 2.84 / 1.72, 12 2.90 / 2.88 / 1.71,
+// 13 2.97 / 2.94 / 1.72, 16 3.49 / 3.30 / 2.04.  Letting entries wait for more
+// lanes, or running only the larger of leaves and entries, changed nothing
+// (2.88-2.90 / 2.85-2.88 / 1.74).
+constexpr int kInternalShare = 11;
+
+template <class W, class Lookup>
+__device__ __forceinline__ void warp_turn(const TraceArgs& a, W& w, uint32_t r, bool& have, bool& ended, int spare,
+                                          Lookup&& lookup) {
+  for (;;) {
+    if (have && !w.pop(a)) {
+      have = false;
+      ended = true;
+    }
+    const bool in = have && w.at_internal();
+    const int m = __popc(__ballot_sync(0xffffffffu, in)), busy = __popc(__ballot_sync(0xffffffffu, have));
+    if (m == 0 || 16 * m < kInternalShare * busy || 32 - busy >= spare) break;
+    if (in) w.internal(a, r, lookup);
+  }
+  if (have && w.at_leaf()) w.leaf(a, r, lookup);
+  else if (have && w.at_entry()) w.entry(a, r, lookup);
+}
+
+struct NoLookup {
+  __device__ __forceinline__ uint32_t operator()(uint32_t, const uint2*) const { return 0u; }
+};
+
 // Finds a ray for every idle lane of the warp (one atomic per refill) and
-// runs each lane's walker one node visit per iteration.  A lane that finishes
+// runs the lanes' walkers turn by turn.  A lane that finishes
 // its ray gets a new one as soon as `refill` lanes of its warp are idle, so
 // warps stay full while rays of very different lengths finish (persistent
 // threads with dynamic ray fetch).  Every ray's own visit order is unchanged.
@@ -298,18 +339,11 @@ __device__ __forceinline__ void run_persistent(const TraceArgs& a, W& w, unsigne
         if (rr < a.n) {
           r = rr;
           w.init(a, r);
-          have = w.active();
-          ended = !have;
+          have = true;
         }
       }
     }
-    if (have) {
-      w.step(a, r);
-      if (!w.active()) {
-        have = false;
-        ended = true;
-      }
-    }
+    warp_turn(a, w, r, have, ended, exhausted ? 33 : (int)a.refill, NoLookup());
   }
   bytes_out = bytes + (unsigned long long)(8ll * w.extra);
 }
@@ -317,10 +351,10 @@ __device__ __forceinline__ void run_persistent(const TraceArgs& a, W& w, unsigne
 // ----------------------------------------------------------------- plain
 
 // A ray's traceRay walk (vulkan_ray_tracing.cc:2309-3076) as a sequence of
-// node visits.  One LIFO stack of unit << 2 | top | leaf entries; `next` is
-// the internal node descended next (the first hit internal child, :2570-2578),
-// as an entry, 0 for none (no entry is 0: unit 0 is the TLAS header); leaves
-// and further children are pushed.  A top-level instance leaf is followed by
+// node visits.  One LIFO stack of unit << 2 | top | leaf entries; `e` is the
+// entry visited next once popped: the first hit internal child (:2570-2578)
+// or the stack's top, 0 for none yet (no entry is 0: unit 0 is the TLAS
+// header); leaves and further children are pushed.  A top-level instance leaf is followed by
 // its whole BLAS before the next top-level entry (:2602-2679), so a
 // bottom-level entry always belongs to the instance entered last.
 // The warp-synchronous short stack (SHORT): entries 0..kShortStack-1 of each
@@ -345,14 +379,24 @@ template <int CAP, bool MULTI, bool TRACED, bool SHORT = false>
 struct PlainWalker {
   RayCtx cx;
   float tmin, tmax, min_thit;
-  uint32_t next, flags;
+  uint32_t e, flags;
   int sp;
   uint32_t n_tx;  // the ray's transactions
   int extra;      // the thread's byte difference (kInstanceExtra)
   uint32_t* stk;  // CAP + kStackPad + kPlainCold words, a local array of the kernel
   SceneView v;
 
-  __device__ __forceinline__ bool active() const { return next != 0 || sp > 0; }
+  // The next node to visit into e; false when the walk is over.
+  __device__ __forceinline__ bool pop(const TraceArgs& a) {
+    if (e) return true;
+    if (sp == 0) return false;
+    e = *slot(a, --sp);
+    return true;
+  }
+  // a bottom-level entry always belongs to the instance entered last
+  __device__ __forceinline__ bool at_internal() const { return !(e & kLeaf); }
+  __device__ __forceinline__ bool at_leaf() const { return (e & (kLeaf | kTop)) == kLeaf; }
+  __device__ __forceinline__ bool at_entry() const { return (e & (kLeaf | kTop)) == (kLeaf | kTop); }
 
   // ---- the cold words
   __device__ __forceinline__ uint32_t& cold(int k) const { return stk[CAP + kStackPad + k]; }
@@ -400,7 +444,7 @@ struct PlainWalker {
     flags = (f & rtf::RAY_FLAG_TERMINATE_ON_FIRST_HIT ? kRayTerminate : 0u) | (f & rtf::RAY_FLAG_OPAQUE ? kRayOpaque : 0u);
     n_tx = 0;
     sp = 0;
-    next = 0;
+    e = 0;
     min_thit = tmax;
     const rtm::V3 id = rtm::calculate_idir(D);
     set_cold3(0, D);
@@ -415,7 +459,7 @@ struct PlainWalker {
     const rtm::V3 bmin = rtm::v3(__uint_as_float(h0.z), __uint_as_float(h0.w), __uint_as_float(h1.x));
     const rtm::V3 bmax = rtm::v3(__uint_as_float(h1.y), __uint_as_float(h1.z), __uint_as_float(h1.w));
     float th;
-    if (rtm::ray_box_test(bmin, bmax, id, O, tmin, tmax, th)) next = ((uint32_t)(root_off >> 6) << 2) | kTop;
+    if (rtm::ray_box_test(bmin, bmax, id, O, tmin, tmax, th)) e = ((uint32_t)(root_off >> 6) << 2) | kTop;
   }
 
   // The world ray as the ray tested with (its direction is not: only
@@ -431,11 +475,29 @@ struct PlainWalker {
   __device__ __forceinline__ void stop(uint32_t bits) {
     flags |= bits;
     sp = 0;
-    next = 0;
+    e = 0;
   }
 
-  __device__ __forceinline__ void visit_internal(const TraceArgs& a, uint32_t unit, uint32_t level,
-                                                 const rtd::Node64& nd) {
+  // The entry's unit, and the node's first 64 bytes; false (and the ray
+  // stopped) when it lies outside the blob.
+  __device__ __forceinline__ bool load(uint32_t& unit, uint32_t units, rtd::Node64& q) {
+    unit = e >> 2;
+    if (unit + units > v.n_units) {
+      stop(RT_RAY_BAD_NODE);
+      return false;
+    }
+    rtd::load64(v.blob + (uint64_t)unit * 4, 0, q);
+    return true;
+  }
+
+  template <class Lookup>
+  __device__ __forceinline__ void internal(const TraceArgs& a, uint32_t r, Lookup&&) {
+    uint32_t unit;
+    rtd::Node64 nd;
+    if (!load(unit, 1, nd)) return;
+    const uint32_t level = e & kTop;
+    record(a, r, unit, rtf::TX_INTERNAL);
+    if (level && cx.unit != kNone) world();
     const float t0 = tmin * cx.mult, t1 = tmax * cx.mult, cull = min_thit * cx.mult;
     const uint4* src = v.blob + (uint64_t)unit * 4;
     const rtd::ChildHits ch = cx.fast ? rtd::test_children<true>(nd, src, unit, cx.o, cx.idir, t0, t1, cull)
@@ -443,89 +505,69 @@ struct PlainWalker {
     uint32_t c = ch.child_unit, nn = 0;
 #pragma unroll
     for (int i = 0; i < 6; ++i) {
-      // the first hit internal child becomes `next`; other hit children are
+      // the first hit internal child is visited next; other hit children are
       // pushed (one predicated store, no branch per child)
       const uint32_t info = ch.info_of(i);
       const bool h = (ch.hit_mask >> i) & 1u, internal = (info >> 2) == rtf::CT_INTERNAL;
-      const uint32_t e = (c << 2) | level | (internal ? 0u : kLeaf);
+      const uint32_t ce = (c << 2) | level | (internal ? 0u : kLeaf);
       const bool take = h && internal && nn == 0, store = h && !take;
-      if (store) *slot(a, sp) = e;
+      if (store) *slot(a, sp) = ce;
       sp += store ? 1 : 0;
-      nn = take ? e : nn;
+      nn = take ? ce : nn;
       c += info & 3u;
     }
-    next = nn;
+    e = nn;
     if (sp > CAP) stop(RT_RAY_STACK_OVERFLOW);
   }
 
-  // Returns the transaction type of the leaf's second record.
-  __device__ __forceinline__ uint32_t visit_leaf(const TraceArgs& a, uint32_t unit, const rtd::Node64& q) {
+  template <class Lookup>
+  __device__ __forceinline__ void leaf(const TraceArgs& a, uint32_t r, Lookup&&) {
+    uint32_t unit;
+    rtd::Node64 q;
+    if (!load(unit, 1, q)) return;
+    e = 0;
+    record(a, r, unit, rtf::TX_LEAF_DESC);
     extra += kDescriptorExtra;
+    uint32_t type = rtf::TX_PROCEDURAL_LEAF;
     if (rtf::leaf_type_of(q.w[1]) == 0) {
       const rtm::V3 v0 = rtm::v3(__uint_as_float(q.w[4]), __uint_as_float(q.w[5]), __uint_as_float(q.w[6]));
       const rtm::V3 v1 = rtm::v3(__uint_as_float(q.w[7]), __uint_as_float(q.w[8]), __uint_as_float(q.w[9]));
       const rtm::V3 v2 = rtm::v3(__uint_as_float(q.w[10]), __uint_as_float(q.w[11]), __uint_as_float(q.w[12]));
       float t = 0.0f;
-      const bool hit = rtm::ray_triangle_test(v0, v1, v2, cx.o, cx.d, t);
-      const float wt = t / cx.mult;
-      if (hit && tmin <= wt && wt <= tmax) {  // :2843-2859
-        if ((flags & kRayOpaque) && wt < min_thit) min_thit = wt;
-        set_hit(unit, cx.unit, t);
-        if (flags & kRayTerminate) sp = 0;
-        return rtf::TX_QUAD_LEAF_HIT;
+      type = rtf::TX_QUAD_LEAF;
+      if (rtm::ray_triangle_test(v0, v1, v2, cx.o, cx.d, t)) {
+        const float wt = t / cx.mult;
+        if (tmin <= wt && wt <= tmax) {  // :2843-2859
+          if ((flags & kRayOpaque) && wt < min_thit) min_thit = wt;
+          set_hit(unit, cx.unit, t);
+          if (flags & kRayTerminate) sp = 0;
+          type = rtf::TX_QUAD_LEAF_HIT;
+        }
       }
-      return rtf::TX_QUAD_LEAF;
+    } else {
+      flags |= RT_RAY_HIT_PROCEDURAL;
     }
-    flags |= RT_RAY_HIT_PROCEDURAL;
-    return rtf::TX_PROCEDURAL_LEAF;
+    record(a, r, unit, type);
   }
 
-  // Returns the unit of the instance's second record (its BLAS header), or
-  // kNone when the header lies outside the blob.
-  __device__ __forceinline__ uint32_t visit_instance(const TraceArgs& a, uint32_t unit, const rtd::Node64& q) {
+  // an instance leaf
+  template <class Lookup>
+  __device__ __forceinline__ void entry(const TraceArgs& a, uint32_t r, Lookup&&) {
+    uint32_t unit;
+    rtd::Node64 q;
+    if (!load(unit, 2, q)) return;
+    record(a, r, unit, rtf::TX_INSTANCE_LEAF);
     extra += kInstanceExtra;
     rtd::Instance in;
     rtd::instance_from(q, v.blob + (uint64_t)unit * 4, 0, in);
     const uint64_t hdr = (uint64_t)unit * 64 + in.bvh_address;
-    if ((hdr & 63) || hdr / 64 >= v.n_units) {
-      stop(RT_RAY_BAD_NODE);
-      return kNone;
-    }
+    if ((hdr & 63) || hdr / 64 >= v.n_units) return stop(RT_RAY_BAD_NODE);
     const uint4 h0 = __ldg(v.blob + (hdr >> 4));
     const uint64_t broot = hdr + ((uint64_t)h0.x | ((uint64_t)h0.y << 32));
     enter_instance(in, unit, world_o(), world_d(), tmin, tmax, v.ordered, cx);
-    if (sp < CAP) next = (uint32_t)(broot >> 6) << 2;
+    if (sp < CAP) e = (uint32_t)(broot >> 6) << 2;
     else stop(RT_RAY_STACK_OVERFLOW);
-    return (uint32_t)(hdr >> 6);
-  }
-
-  // One node visit (the caller checks active() first).  The node's first 64
-  // bytes are loaded once for every kind, so a warp's lanes at internal
-  // nodes, leaves and instance leaves issue one load.
-  __device__ __forceinline__ void step(const TraceArgs& a, uint32_t r) {
-    uint32_t e = next;
-    next = 0;
-    if (!e) e = *slot(a, --sp);
-    const bool top = e & kTop, leaf = e & kLeaf;
-    const uint32_t unit = e >> 2;
-    if (unit + ((top && leaf) ? 1u : 0u) >= v.n_units) return stop(RT_RAY_BAD_NODE);
-    rtd::Node64 q;
-    rtd::load64(v.blob + (uint64_t)unit * 4, 0, q);
-    // a visit records one or two transactions; two call sites for all kinds
-    // keep the recording code (staged through shared memory) out of every
-    // branch
-    record(a, r, unit, !leaf ? rtf::TX_INTERNAL : (top ? rtf::TX_INSTANCE_LEAF : rtf::TX_LEAF_DESC));
-    uint32_t unit2 = unit, type2 = rtf::TX_STRUCTURE;
-    if (!leaf) {
-      if (top && cx.unit != kNone) world();
-      visit_internal(a, unit, e & kTop, q);
-      unit2 = kNone;
-    } else if (!top) {
-      type2 = visit_leaf(a, unit, q);
-    } else {
-      unit2 = visit_instance(a, unit, q);
-    }
-    if (unit2 != kNone) record(a, r, unit2, type2);
+    record(a, r, (uint32_t)(hdr >> 6), rtf::TX_STRUCTURE);
   }
 
   __device__ __forceinline__ void finish(const TraceArgs& a, uint32_t r) {

@@ -180,8 +180,8 @@ __global__ void __launch_bounds__(kStagedMaxThreads, kStagedMinBlocks) trace_que
       const bool live = valid && w.active();
       uint32_t want = key;
       if (round0 && live) {
-        // the node the ray visits first (nxt, or the top of the other stack)
-        const unsigned long long e = w.nxt ? w.nxt : w.ot_at(w.not_ - 1);
+        // the node the ray visits first (e, or the top of the other stack)
+        const unsigned long long e = w.e ? w.e : w.ot_at(w.not_ - 1);
         const uint32_t loc = __ldg(reinterpret_cast<const uint32_t*>(a.meta) + 2ull * ((uint32_t)e >> kEShift) + 1);
         want = loc == kNone ? kNone : loc >> kSlotBitsDev;
       }

@@ -52,10 +52,13 @@ struct Walker {
   unsigned long long* stk;  // kWords entries, a local array of the kernel
   unsigned long long* ot;   // SLAB: the ray's other-treelet stack in global memory
   int ncu, not_;            // entries on cu and on ot
-  // The top of `cu` when it was pushed by the previous node visit: the node
-  // the walk pops next, kept in a register instead of a local-memory round
-  // trip (0 = none; no stack entry is 0, a blob's unit 0 is its TLAS header).
-  unsigned long long nxt;
+  // The entry popped (`popped` != 0) and visited next, or the top of `cu` when
+  // the previous node visit pushed it, kept in a register instead of a
+  // local-memory round trip (0 = none; no stack entry is 0, a blob's unit 0 is
+  // its TLAS header).
+  unsigned long long e;
+  uint32_t popped;  // 0 no, else 1 + which route bits apply: kPopCu from cu, kPopOt from ot (:1748-1754)
+  static constexpr uint32_t kPopCu = 1u, kPopOt = 2u;
   uint32_t n_tx;  // the ray's transactions
   int extra;      // the thread's byte difference (kInstanceExtra)
   SceneView v;
@@ -66,8 +69,31 @@ struct Walker {
   __device__ __forceinline__ bool active() const { return (ncu | not_) != 0; }
 
   __device__ __forceinline__ void clear() {
-    nxt = 0;
+    e = 0;
+    popped = 0;
     ncu = not_ = 0;
+  }
+
+  // The next node to visit into e; false when the walk is over.
+  __device__ __forceinline__ bool pop(const TraceArgs&) {
+    if (popped) return true;
+    if ((ncu | not_) == 0) return false;
+    const bool from_cu = ncu > 0;
+    if (!e) e = SLAB ? (from_cu ? stk[ncu - 1] : ot[not_ - 1]) : stk[from_cu ? ncu - 1 : kOt + not_ - 1];
+    ncu -= from_cu ? 1 : 0;
+    not_ -= from_cu ? 0 : 1;
+    popped = from_cu ? kPopCu : kPopOt;
+    return true;
+  }
+  // Kinds of the popped entry: a bottom-level node of another instance than
+  // the one whose ray is held is an entry first.
+  __device__ __forceinline__ bool other_inst() const {
+    return !((uint32_t)e & kTop) && (uint32_t)(e >> 32) != cx.unit;
+  }
+  __device__ __forceinline__ bool at_internal() const { return !((uint32_t)e & kLeaf) && !other_inst(); }
+  __device__ __forceinline__ bool at_leaf() const { return ((uint32_t)e & (kLeaf | kTop)) == kLeaf && !other_inst(); }
+  __device__ __forceinline__ bool at_entry() const {
+    return ((uint32_t)e & (kLeaf | kTop)) == (kLeaf | kTop) || other_inst();
   }
 
   // ---- the cold words
@@ -127,31 +153,32 @@ struct Walker {
   // Staged location (dense treelet << 10 | slot) of the node the ray visits
   // next, i.e. its first pending access; kNone for a pinned node.
   __device__ __forceinline__ uint32_t next_loc() const {
-    unsigned long long e;
-    if (nxt) e = nxt;
-    else if (ncu > 0) e = stk[ncu - 1];
-    else if (not_ > 0) e = ot_at(not_ - 1);
-    else return kNone;
-    if ((uint32_t)e & kEPin) return kNone;
-    const uint32_t unit = (uint32_t)e >> kEShift;
+    unsigned long long x = e;  // popped, or the cached top of cu
+    if (!x) {
+      if (ncu > 0) x = stk[ncu - 1];
+      else if (not_ > 0) x = ot_at(not_ - 1);
+      else return kNone;
+    }
+    if ((uint32_t)x & kEPin) return kNone;
+    const uint32_t unit = (uint32_t)x >> kEShift;
     return unit < v.n_units ? __ldg(reinterpret_cast<const uint32_t*>(v.meta) + 2ull * unit + 1) : kNone;
   }
 
-  // Pushes an entry onto cu (same treelet; it becomes nxt too) or ot.  Depths
+  // Pushes an entry onto cu (same treelet; it becomes e too) or ot.  Depths
   // are checked once per visit (too_deep); a slab has no room past CAP, so an
   // entry beyond it is not written (the ray is flagged and its stacks cleared).
   __device__ __forceinline__ void push(bool same, uint32_t code, uint32_t inst) {
-    const unsigned long long e = (unsigned long long)code | ((unsigned long long)inst << 32);
+    const unsigned long long x = (unsigned long long)code | ((unsigned long long)inst << 32);
     if (SLAB) {
-      if (same || not_ < CAP) *(same ? stk + ncu : ot + not_) = e;
+      if (same || not_ < CAP) *(same ? stk + ncu : ot + not_) = x;
     } else {
-      stk[same ? ncu : kOt + not_] = e;
+      stk[same ? ncu : kOt + not_] = x;
     }
     ncu += same ? 1 : 0;
     not_ += same ? 0 : 1;
-    nxt = same ? e : nxt;
+    e = same ? x : e;
   }
-  // CAP entries per stack, one more on cu for the entry held in nxt
+  // CAP entries per stack, one more on cu for the entry held in e
   __device__ __forceinline__ bool too_deep() const { return ncu > CAP + 1 || not_ > CAP; }
 
   __device__ __forceinline__ void bad_node() {
@@ -220,8 +247,7 @@ struct Walker {
     n_tx = q2.z;
     set_world(o, D, rtm::calculate_idir(D));
     set_hit(q3.x, q3.y, __uint_as_float(q3.z));
-    nxt = 0;
-    ncu = 0;
+    clear();
     not_ = (int)q3.w;
     if (v.ordered && rtd::finite_ray(o, D, tmin, tmax)) flags |= kRayWorldFast;
     world();
@@ -231,38 +257,32 @@ struct Walker {
   // come from the current-treelet stack.
   __device__ __forceinline__ bool in_treelet() const { return ncu > 0; }
 
-  // Visits one node; `lookup(unit, meta)` returns the shared-memory address
-  // of a node staged in a warp slot, else 0.
+  // Where a popped node is: its unit, and the address of its pinned record or
+  // staged copy in shared memory (`lookup(unit, meta)`: a node staged in a
+  // warp slot), 0 when it is read from the blob.  Loads its first 64 bytes
+  // (or the whole pinned record of an instance leaf).  False, and the ray
+  // stopped, when it lies outside the blob.
   template <class Lookup>
-  __device__ __forceinline__ void step(const TraceArgs& a, uint32_t r, Lookup&& lookup) {
-    const bool from_cu = ncu > 0;  // :1748-1754
-    unsigned long long e = nxt;
-    if (!e) e = SLAB ? (from_cu ? stk[ncu - 1] : ot[not_ - 1]) : stk[from_cu ? ncu - 1 : kOt + not_ - 1];
-    ncu -= from_cu ? 1 : 0;
-    not_ -= from_cu ? 0 : 1;
-    nxt = 0;
-    const uint32_t code = (uint32_t)e, inst = (uint32_t)(e >> 32);
-    const bool top = code & kTop, leaf = code & kLeaf, pinned = STAGED && (code & kEPin);
-    const uint32_t rsh = from_cu ? 0u : 1u;  // which route bit applies
-    uint32_t unit, rbits, saddr = 0;
-    if (pinned) {
+  __device__ __forceinline__ bool load(uint32_t code, uint32_t units, Lookup&& lookup, uint32_t& unit, uint32_t& saddr,
+                                       const uint4*& src, rtd::Node64& nd) {
+    saddr = 0;
+    if (STAGED && (code & kEPin)) {
       saddr = pin_base + (code >> kEShift) * 16u;
-      unit = rtd::ld_shared_u32(saddr + (leaf ? 0u : rtp::IN_UNIT));
+      unit = rtd::ld_shared_u32(saddr + ((code & kLeaf) ? 0u : rtp::IN_UNIT));
       ++smem_reads;
     } else {
       unit = code >> kEShift;
-      if (unit + ((top && leaf) ? 1u : 0u) >= v.n_units) return bad_node();
+      if (unit + units > v.n_units) {
+        bad_node();
+        return false;
+      }
       if (STAGED) {
         saddr = lookup(unit, v.meta);
         if (saddr) ++smem_reads;
         else ++gmem_reads;
       }
     }
-    const uint4* g = v.blob + (uint64_t)unit * 4;
-    // the first 64 bytes (or the whole pinned record of an instance leaf), for
-    // every kind of node at once, so the warp's lanes issue one load
-    rtd::Node64 nd;
-    const uint4* src = g;
+    src = v.blob + (uint64_t)unit * 4;
     if (STAGED) {
       // one generic load for lanes reading shared memory and lanes reading
       // global memory, instead of both load paths for a mixed warp
@@ -276,115 +296,159 @@ struct Walker {
         nd.w[4 * k + 3] = w.w;
       }
     } else {
-      rtd::load64(g, 0, nd);
+      rtd::load64(src, 0, nd);
     }
-    // The ray context, once for every kind of node: an instance leaf enters
-    // its own instance; a BLAS node needs its instance's object ray,
-    // recomputed when the walk comes back from another instance's nodes
-    // (make_transformed_ray is deterministic, so recomputing gives the
-    // reference's stored objectRay); a top-level node needs the world ray.
-    // Lanes of all kinds switch together.
+    return true;
+  }
+
+  // internal node, top (:1758-1869) or bottom (:1954-2070)
+  template <class Lookup>
+  __device__ __forceinline__ void internal(const TraceArgs& a, uint32_t r, Lookup&& lookup) {
+    const uint32_t code = (uint32_t)e, inst = (uint32_t)(e >> 32), level = code & kTop;
+    const uint32_t rsh = popped - kPopCu;  // which route bit applies
+    uint32_t unit, saddr, rbits;
+    const uint4* src;
+    rtd::Node64 nd;
+    if (!load(code, 1, lookup, unit, saddr, src, nd)) return;
+    e = 0;
+    popped = 0;
+    if (level && cx.unit != kNone) world();
+    record(a, r, unit, rtf::TX_INTERNAL);
+    uint32_t soff01 = 0, soff23 = 0, soff45 = 0;
+    if (STAGED && (code & kEPin)) {  // route bits in bytes 16..17, child records in the tail
+      const uint4 t = rtd::ld_shared_v4(saddr + rtp::IN_UNIT);
+      rbits = nd.w[rtp::IN_ROUTE / 4] & 0xffffu;
+      soff01 = t.y;
+      soff23 = t.z;
+      soff45 = t.w;
+    } else {
+      rbits = __ldg(v.route + unit);
+    }
+    const float t0 = tmin * cx.mult, t1 = tmax * cx.mult, cull = min_thit * cx.mult;
+    const rtd::ChildHits ch = cx.fast ? rtd::test_children<true>(nd, src, unit, cx.o, cx.idir, t0, t1, cull)
+                                      : rtd::test_children<false>(nd, src, unit, cx.o, cx.idir, t0, t1, cull);
+    const uint32_t hit = ch.hit_mask;
+    const uint64_t info = ch.info;
+    const uint32_t same = rbits >> (rsh * kRouteOther);
+    uint32_t c = ch.child_unit;
+#pragma unroll
+    for (int i = 0; i < 6; ++i) {
+      const uint32_t ci = (uint32_t)(info >> (8 * i)) & 0x3fu;
+      if ((hit >> i) & 1u) {
+        const uint32_t lf = ((ci >> 2) != rtf::CT_INTERNAL) ? kLeaf : 0u;
+        const uint32_t sw = i < 2 ? soff01 : (i < 4 ? soff23 : soff45);
+        const uint32_t so = (sw >> (16 * (i & 1))) & 0xffffu;
+        const uint32_t cc = so ? ((so << kEShift) | kEPin | level | lf) : ((c << kEShift) | level | lf);
+        push((same >> i) & 1u, cc, inst);
+      }
+      c += ci & 3u;
+    }
+    check_depth();
+  }
+
+  // primitive leaf (:2071-2196)
+  template <class Lookup>
+  __device__ __forceinline__ void leaf(const TraceArgs& a, uint32_t r, Lookup&& lookup) {
+    uint32_t unit, saddr;
+    const uint4* src;
+    rtd::Node64 q;
+    if (!load((uint32_t)e, 1, lookup, unit, saddr, src, q)) return;
+    e = 0;
+    popped = 0;
+    record(a, r, unit, rtf::TX_LEAF_DESC);
+    extra += kDescriptorExtra;
+    uint32_t type = rtf::TX_PROCEDURAL_LEAF;
+    if (rtf::leaf_type_of(q.w[1]) == 0) {
+      const rtm::V3 v0 = rtm::v3(__uint_as_float(q.w[4]), __uint_as_float(q.w[5]), __uint_as_float(q.w[6]));
+      const rtm::V3 v1 = rtm::v3(__uint_as_float(q.w[7]), __uint_as_float(q.w[8]), __uint_as_float(q.w[9]));
+      const rtm::V3 v2 = rtm::v3(__uint_as_float(q.w[10]), __uint_as_float(q.w[11]), __uint_as_float(q.w[12]));
+      float t = 0.0f;
+      type = rtf::TX_QUAD_LEAF;
+      if (rtm::ray_triangle_test(v0, v1, v2, cx.o, cx.d, t)) {
+        const float wt = t / cx.mult;
+        if (tmin <= wt && wt <= tmax && wt < min_thit) {  // :2127-2141
+          min_thit = wt;
+          set_hit(unit, cx.unit, t);
+          type = rtf::TX_QUAD_LEAF_HIT;
+          if (flags & kRayTerminate) clear();
+        }
+      }
+    } else {
+      flags |= RT_RAY_HIT_PROCEDURAL;
+    }
+    record(a, r, unit, type);
+  }
+
+  // The ray context for the popped entry: an instance leaf (:1870-1953)
+  // enters its own instance; a BLAS node's instance is entered again when the
+  // walk comes back to it from another instance's nodes or from the TLAS
+  // (make_transformed_ray is deterministic, so recomputing gives the
+  // reference's stored objectRay), and the node itself stays popped.
+  template <class Lookup>
+  __device__ __forceinline__ void entry(const TraceArgs& a, uint32_t r, Lookup&& lookup) {
+    const uint32_t code = (uint32_t)e;
+    const bool top = code & kTop, pinned = STAGED && (code & kEPin);
     rtd::Instance in;
-    uint32_t enter = kNone;
-    if (top && leaf) {
+    rtd::Node64 nd;
+    uint32_t unit = (uint32_t)(e >> 32), saddr = 0;
+    const uint4* src;
+    if (top) {
+      if (!load(code, 2, lookup, unit, saddr, src, nd)) return;
       if (pinned) {
 #pragma unroll
         for (int k = 0; k < 12; ++k) in.w2o.m[k / 3][k % 3] = __uint_as_float(nd.w[rtp::IL_W2O / 4 + k]);
       } else {
-        rtd::instance_from(nd, g, saddr, in);
+        rtd::instance_from(nd, v.blob + (uint64_t)unit * 4, saddr, in);
       }
-      enter = unit;
-    } else if (!top && inst != cx.unit) {
-      rtd::load_instance(v.blob + (uint64_t)inst * 4, 0, in);
-      enter = inst;
+    } else {
+      rtd::load_instance(v.blob + (uint64_t)unit * 4, 0, in);
     }
-    if (enter != kNone) enter_instance(in, enter, world_o(), dir(), tmin, tmax, v.ordered, cx);
-    if (!leaf) {  // internal node, top (:1758-1869) or bottom (:1954-2070)
-      if (top && cx.unit != kNone) world();
-      record(a, r, unit, rtf::TX_INTERNAL);
-      uint32_t soff01 = 0, soff23 = 0, soff45 = 0;
-      if (pinned) {  // route bits in bytes 16..17, child records in the tail
-        const uint4 t = rtd::ld_shared_v4(saddr + rtp::IN_UNIT);
-        rbits = nd.w[rtp::IN_ROUTE / 4] & 0xffffu;
-        soff01 = t.y;
-        soff23 = t.z;
-        soff45 = t.w;
-      } else {
-        rbits = __ldg(v.route + unit);
-      }
-      const float t0 = tmin * cx.mult, t1 = tmax * cx.mult, cull = min_thit * cx.mult;
-      const rtd::ChildHits ch = cx.fast ? rtd::test_children<true>(nd, src, unit, cx.o, cx.idir, t0, t1, cull)
-                                        : rtd::test_children<false>(nd, src, unit, cx.o, cx.idir, t0, t1, cull);
-      const uint32_t hit = ch.hit_mask;
-      const uint64_t info = ch.info;
-      const uint32_t same = rbits >> (rsh * kRouteOther);
-      const uint32_t level = top ? kTop : 0u;
-      uint32_t c = ch.child_unit;
-#pragma unroll
-      for (int i = 0; i < 6; ++i) {
-        const uint32_t ci = (uint32_t)(info >> (8 * i)) & 0x3fu;
-        if ((hit >> i) & 1u) {
-          const uint32_t lf = ((ci >> 2) != rtf::CT_INTERNAL) ? kLeaf : 0u;
-          const uint32_t sw = i < 2 ? soff01 : (i < 4 ? soff23 : soff45);
-          const uint32_t so = (sw >> (16 * (i & 1))) & 0xffffu;
-          const uint32_t cc = so ? ((so << kEShift) | kEPin | level | lf) : ((c << kEShift) | level | lf);
-          push((same >> i) & 1u, cc, inst);
-        }
-        c += ci & 3u;
-      }
-    } else if (top) {  // instance leaf (:1870-1953)
-      record(a, r, unit, rtf::TX_INSTANCE_LEAF);
-      extra += kInstanceExtra;
-      uint32_t hdr_unit, broot_unit, broot_soff = 0;
-      if (pinned) {  // the 64-byte record: units, route bits, BLAS root record, rows
-        hdr_unit = nd.w[rtp::IL_HDR_UNIT / 4];
-        broot_unit = nd.w[rtp::IL_BROOT_UNIT / 4];
-        rbits = nd.w[rtp::IL_ROUTE / 4] & 0xffffu;
-        broot_soff = nd.w[rtp::IL_ROUTE / 4] >> 16;
-      } else {
-        rbits = __ldg(v.route + unit);
-        const uint64_t hdr = (uint64_t)unit * 64 + in.bvh_address;
-        if ((hdr & 63) || hdr / 64 >= v.n_units) return bad_node();
-        hdr_unit = (uint32_t)(hdr >> 6);
-        const uint4 h0 = __ldg(v.blob + (hdr >> 4));
-        const uint64_t broot = hdr + ((uint64_t)h0.x | ((uint64_t)h0.y << 32));
-        broot_unit = (uint32_t)(broot >> 6);
-      }
-      record(a, r, hdr_unit, rtf::TX_STRUCTURE);
-      const uint32_t cc = broot_soff ? ((broot_soff << kEShift) | kEPin) : (broot_unit << kEShift);
-      push((rbits >> (kRouteInst + rsh)) & 1u, cc, unit);
-    } else {  // primitive leaf (:2071-2196)
-      record(a, r, unit, rtf::TX_LEAF_DESC);
-      extra += kDescriptorExtra;
-      const rtd::Node64& q = nd;
-      if (rtf::leaf_type_of(q.w[1]) == 0) {
-        const rtm::V3 v0 = rtm::v3(__uint_as_float(q.w[4]), __uint_as_float(q.w[5]), __uint_as_float(q.w[6]));
-        const rtm::V3 v1 = rtm::v3(__uint_as_float(q.w[7]), __uint_as_float(q.w[8]), __uint_as_float(q.w[9]));
-        const rtm::V3 v2 = rtm::v3(__uint_as_float(q.w[10]), __uint_as_float(q.w[11]), __uint_as_float(q.w[12]));
-        float t = 0.0f;
-        const bool hit = rtm::ray_triangle_test(v0, v1, v2, cx.o, cx.d, t);
-        const float wt = t / cx.mult;
-        if (hit && tmin <= wt && wt <= tmax && wt < min_thit) {  // :2127-2141
-          min_thit = wt;
-          set_hit(unit, inst, t);
-          record(a, r, unit, rtf::TX_QUAD_LEAF_HIT);
-          if (flags & kRayTerminate) clear();
-        } else {
-          record(a, r, unit, rtf::TX_QUAD_LEAF);
-        }
-      } else {
-        flags |= RT_RAY_HIT_PROCEDURAL;
-        record(a, r, unit, rtf::TX_PROCEDURAL_LEAF);
-      }
+    enter_instance(in, unit, world_o(), dir(), tmin, tmax, v.ordered, cx);
+    if (!top) return;
+    const uint32_t rsh = popped - kPopCu;
+    e = 0;
+    popped = 0;
+    record(a, r, unit, rtf::TX_INSTANCE_LEAF);
+    extra += kInstanceExtra;
+    uint32_t hdr_unit, broot_unit, broot_soff = 0, rbits;
+    if (pinned) {  // the 64-byte record: units, route bits, BLAS root record, rows
+      hdr_unit = nd.w[rtp::IL_HDR_UNIT / 4];
+      broot_unit = nd.w[rtp::IL_BROOT_UNIT / 4];
+      rbits = nd.w[rtp::IL_ROUTE / 4] & 0xffffu;
+      broot_soff = nd.w[rtp::IL_ROUTE / 4] >> 16;
+    } else {
+      rbits = __ldg(v.route + unit);
+      const uint64_t hdr = (uint64_t)unit * 64 + in.bvh_address;
+      if ((hdr & 63) || hdr / 64 >= v.n_units) return bad_node();
+      hdr_unit = (uint32_t)(hdr >> 6);
+      const uint4 h0 = __ldg(v.blob + (hdr >> 4));
+      const uint64_t broot = hdr + ((uint64_t)h0.x | ((uint64_t)h0.y << 32));
+      broot_unit = (uint32_t)(broot >> 6);
     }
+    record(a, r, hdr_unit, rtf::TX_STRUCTURE);
+    const uint32_t cc = broot_soff ? ((broot_soff << kEShift) | kEPin) : (broot_unit << kEShift);
+    push((rbits >> (kRouteInst + rsh)) & 1u, cc, unit);
+    check_depth();
+  }
+
+  __device__ __forceinline__ void check_depth() {
     if (too_deep()) {
       flags |= RT_RAY_STACK_OVERFLOW;
       clear();
     }
   }
 
-  __device__ __forceinline__ void step(const TraceArgs& a, uint32_t r) {
-    step(a, r, [](uint32_t, const uint2*) -> uint32_t { return 0u; });
+  // One node visit (the caller checks active() first).
+  template <class Lookup>
+  __device__ __forceinline__ void step(const TraceArgs& a, uint32_t r, Lookup&& lookup) {
+    pop(a);
+    if (at_entry()) {
+      const bool top = (uint32_t)e & kTop;
+      entry(a, r, lookup);
+      if (top) return;
+    }
+    if ((uint32_t)e & kLeaf) leaf(a, r, lookup);
+    else internal(a, r, lookup);
   }
 
   __device__ __forceinline__ void finish(const TraceArgs& a, uint32_t r) {
@@ -585,8 +649,7 @@ __global__ void __launch_bounds__(kStagedMaxThreads, kStagedMinBlocks) trace_sta
         if (rr < a.n) {
           r = rr;
           w.init(a, r);
-          have = w.active();
-          ended = !have;
+          have = true;
         }
       }
     }
@@ -600,7 +663,7 @@ __global__ void __launch_bounds__(kStagedMaxThreads, kStagedMinBlocks) trace_sta
       }
       __syncwarp();
       if (st.pending_slot == kNone && !st.disabled) {
-        const uint32_t nl = (have && w.active()) ? w.next_loc() : kNone;
+        const uint32_t nl = have ? w.next_loc() : kNone;
         uint32_t key = nl == kNone ? kNone : (nl >> kSlotBitsDev);
         if (a.hint && key != kNone) {
           // vote for the treelet predicted to follow the one the ray enters next
@@ -644,15 +707,9 @@ __global__ void __launch_bounds__(kStagedMaxThreads, kStagedMinBlocks) trace_sta
       }
       __syncwarp();
     }
-    // --- one node visit per lane
-    if (have) {
-      if (SLOTS) w.step(a, r, lookup);
-      else w.step(a, r);
-      if (!w.active()) {
-        have = false;
-        ended = true;
-      }
-    }
+    // --- node visits
+    if (SLOTS) warp_turn(a, w, r, have, ended, exhausted ? 33 : (int)a.refill, lookup);
+    else warp_turn(a, w, r, have, ended, exhausted ? 33 : (int)a.refill, NoLookup());
   }
   // copies still in flight must land before the CTA's shared memory goes away
   if (lane == 0 && st.pending_slot != kNone) {
