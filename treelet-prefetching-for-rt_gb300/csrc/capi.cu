@@ -503,15 +503,11 @@ rt_status launch_cap(rtk::TraceArgs& a, uint32_t mode, const rt_tuning& t, uint3
   }
   RT_CUDA(cudaMemsetAsync(a.queue, 0, sizeof(uint32_t), st));
   // A launch that writes traces runs the walks compiled with the trace code
-  // (TRACED).  The plain walk writes its rows a whole 32-byte sector at a
-  // time through shared memory (rtk::trace_put) when every row starts on a
-  // 32-byte boundary, else entry by entry; the treelet walks write entry by
-  // entry (staging their rows through shared memory, inline at each
-  // recording site or through a per-lane ring written once per node visit,
-  // measured 5-31% slower on their traced launches).
+  // (TRACED).  They write their rows a whole 32-byte sector at a time through
+  // shared memory (rtk::trace_put) when every row starts on a 32-byte
+  // boundary, else entry by entry.
   const bool traced = a.cap != 0;
-  const bool stage_rows = traced && mode == RT_MODE_PLAIN && (a.cap % 8u) == 0 &&
-                          ((uintptr_t)a.visits & 31u) == 0 && ((uintptr_t)a.tl_trace & 31u) == 0;
+  const bool stage_rows = traced && (a.cap % 8u) == 0 && ((uintptr_t)a.rows & 31u) == 0;
   const uint32_t stage_warp_bytes = rtk::kTraceBufWarpBytes;
   a.tbuf_off = rtk::kNone;
   a.ss_off = rtk::kNone;
@@ -558,7 +554,12 @@ rt_status launch_cap(rtk::TraceArgs& a, uint32_t mode, const rt_tuning& t, uint3
     a.slots = slots;
     a.slot_bytes = slot_bytes;
     a.min_votes = t.staged_min_votes;
-    const size_t dyn = (size_t)a.pin_bytes + (size_t)warps * slots * slot_bytes + 128;
+    size_t dyn = (size_t)a.pin_bytes + (size_t)warps * slots * slot_bytes + 128;
+    // the trace staging area after the slots, when there is room for it
+    if (stage_rows && dyn + (size_t)warps * stage_warp_bytes <= limit) {
+      a.tbuf_off = a.pin_bytes + warps * slots * slot_bytes;
+      dyn += (size_t)warps * stage_warp_bytes;
+    }
     auto kern = slots ? (traced ? rtk::trace_staged_kernel<CAP, true, true> : rtk::trace_staged_kernel<CAP, true, false>)
                       : (traced ? rtk::trace_staged_kernel<CAP, false, true> : rtk::trace_staged_kernel<CAP, false, false>);
     RT_CUDA(ensure_dyn_smem((const void*)kern, dyn));
@@ -890,9 +891,11 @@ rt_status trace_launch(rt_scene* s, const rt_ray* rays, const uint32_t* flags, u
   a.default_flags = default_flags;
   a.n = n;
   a.hits = hits;
-  a.visits = trace ? trace->visits : nullptr;
-  a.tl_trace = trace ? trace->treelets : nullptr;
-  a.cap = (trace && (trace->visits || trace->treelets)) ? trace->capacity : 0;
+  uint32_t* const visits = trace ? trace->visits : nullptr;
+  uint32_t* const treelets = trace ? trace->treelets : nullptr;
+  a.rows = visits ? visits : treelets;
+  a.rows_tl = visits ? 0u : 1u;
+  a.cap = a.rows ? trace->capacity : 0;
   a.meta = s->d_meta;
   a.route = s->d_route;
   if (mode == RT_MODE_STAGED && s->d_pin) {
@@ -907,12 +910,17 @@ rt_status trace_launch(rt_scene* s, const rt_ray* rays, const uint32_t* flags, u
   a.status = s->d_status;
   a.queue = queue;
   a.hint = s->d_hint;
-  if (allow_queues && queued(s, mode)) {
-    rt_status qst = ensure_queue_scratch(s, n);
-    if (qst != RT_OK) return qst;
-    return launch_trace(a, mode, s->tuning, s->slot_bytes, st, keep, &s->qs);
+  rt_status rs = RT_OK;
+  const bool queues = allow_queues && queued(s, mode);
+  if (queues) rs = ensure_queue_scratch(s, n);
+  if (rs == RT_OK) rs = launch_trace(a, mode, s->tuning, s->slot_bytes, st, keep, queues ? &s->qs : nullptr);
+  if (rs == RT_OK && visits && treelets) {
+    auto ids = rtk::trace_treelet_ids_kernel;
+    ids<<<persistent_grid((const void*)ids, 256, (uint32_t)std::min<uint64_t>(32ull * n, 0xffffffffull)), 256, 0, st>>>(
+        visits, hits, s->d_meta, n, a.cap, treelets);
+    RT_CUDA(cudaGetLastError());
   }
-  return launch_trace(a, mode, s->tuning, s->slot_bytes, st, keep);
+  return rs;
 }
 
 // The device address of a page-locked, mapped host array (cudaHostAlloc or
@@ -1561,8 +1569,9 @@ __global__ void trace_offsets_kernel(uint32_t* __restrict__ off, const uint32_t*
 
 // One warp per ray: the ray's global offset (base + chunk offset) into
 // `goff`, and the used prefix of its trace rows to its place in the packed
-// staging arrays (NULL: not written).
-__global__ void trace_pack_kernel(const uint32_t* __restrict__ vis_rows, const uint32_t* __restrict__ tl_rows,
+// staging arrays (NULL: not written).  The rows are visits when `vis` is
+// written (a treelet id is then looked up for each), else treelet ids.
+__global__ void trace_pack_kernel(const uint32_t* __restrict__ rows, const uint2* __restrict__ meta, bool rows_tl,
                                   const uint32_t* __restrict__ off, uint32_t n, uint32_t cap, uint32_t chunk_total,
                                   unsigned long long base, unsigned long long* __restrict__ goff,
                                   uint32_t* __restrict__ vis, uint32_t* __restrict__ tl) {
@@ -1574,8 +1583,9 @@ __global__ void trace_pack_kernel(const uint32_t* __restrict__ vis_rows, const u
     if (lane == 0) goff[r] = base + o;
     const uint64_t row = (uint64_t)r * cap;
     for (uint32_t j = lane; j < m; j += 32) {
-      if (vis) vis[o + j] = vis_rows[row + j];
-      if (tl) tl[o + j] = tl_rows[row + j];
+      const uint32_t x = __ldcs(rows + row + j);
+      if (vis) vis[o + j] = x;
+      if (tl) tl[o + j] = rows_tl ? x : meta[x >> 3].x;
     }
   }
 }
@@ -1628,8 +1638,7 @@ extern "C" rt_status rt_trace_host_packed(rt_scene* s, const rt_ray* rays, const
   const size_t b_blk = al(sizeof(uint32_t) * rtk::kBinScanItems) * rti::kHostChunks;
   const size_t b_goff = al(sizeof(unsigned long long) * (size_t)n);
   const size_t b_tot = al(sizeof(unsigned long long) * rti::kHostChunks);
-  const size_t need = b_rays + b_flags + b_hits + (visits ? b_row : 0) + (treelets ? b_row : 0) + 2 * b_cnt + b_blk +
-                      b_goff + b_tot;
+  const size_t need = b_rays + b_flags + b_hits + b_row + 2 * b_cnt + b_blk + b_goff + b_tot;
   if (need > s->io_bytes) {
     cudaFree(s->d_io);
     s->d_io = nullptr;
@@ -1654,8 +1663,7 @@ extern "C" rt_status rt_trace_host_packed(rt_scene* s, const rt_ray* rays, const
   rt_ray* d_rays = (rt_ray*)take(b_rays);
   uint32_t* d_flags = flags ? (uint32_t*)take(b_flags) : nullptr;
   rt_hit* d_hits = (rt_hit*)take(b_hits);
-  uint32_t* d_vis = visits ? (uint32_t*)take(b_row) : nullptr;
-  uint32_t* d_tl = treelets ? (uint32_t*)take(b_row) : nullptr;
+  uint32_t* d_rows = (uint32_t*)take(b_row);  // visits, or treelet ids when only they are asked for
   uint32_t* d_cnt = (uint32_t*)take(b_cnt);
   uint32_t* d_off = (uint32_t*)take(b_cnt);
   uint32_t* d_blk = (uint32_t*)take(b_blk);
@@ -1683,7 +1691,7 @@ extern "C" rt_status rt_trace_host_packed(rt_scene* s, const rt_ray* rays, const
     cudaStream_t cs = (c & 1) ? s->stream2 : s->stream;
     e = cudaStreamWaitEvent(cs, s->ev_in[c], 0);
     if (e != cudaSuccess) return false;
-    rt_trace_buf rows{d_vis ? d_vis + lo * cap : nullptr, d_tl ? d_tl + lo * cap : nullptr, cap};
+    rt_trace_buf rows{visits ? d_rows + lo * cap : nullptr, visits ? nullptr : d_rows + lo * cap, cap};
     st = trace_launch(s, d_rays + lo, d_flags ? d_flags + lo : nullptr, default_flags, m, mode, d_hits + lo, &rows, cs,
                       s->d_queue + c, true);
     if (st != RT_OK) return false;
@@ -1736,8 +1744,7 @@ extern "C" rt_status rt_trace_host_packed(rt_scene* s, const rt_ray* rays, const
     if (e != cudaSuccess) break;
     unsigned long long* goff = d_goff + lo;
     trace_pack_kernel<<<std::min<uint32_t>((m + 3) / 4, 152 * 8), 128, 0, s->xout>>>(
-        d_vis ? d_vis + lo * cap : nullptr, d_tl ? d_tl + lo * cap : nullptr, d_off + lo, m, cap, (uint32_t)tot_c, base,
-        goff, dst_vis, dst_tl);
+        d_rows + lo * cap, s->d_meta, !visits, d_off + lo, m, cap, (uint32_t)tot_c, base, goff, dst_vis, dst_tl);
     e = cudaGetLastError();
     if (e == cudaSuccess && c + 1 < chunks && !trace_chunk(c + 1)) break;
     if (e == cudaSuccess)

@@ -57,8 +57,8 @@ struct TraceArgs {
   uint32_t default_flags;
   uint32_t n;
   rt_hit* hits;
-  uint32_t* visits;
-  uint32_t* tl_trace;
+  uint32_t* rows;              // traced: n rows of `cap` entries, visits or (rows_tl) treelet ids, or null
+  uint32_t rows_tl;
   uint32_t cap;
   const uint2* meta;           // per unit: x = treelet root unit, y = dense << 10 | slot
   const uint16_t* route;       // per unit: routing bits of the treelet-ordered walk
@@ -78,21 +78,26 @@ struct TraceArgs {
   uint32_t min_votes;          // lanes that must want a treelet before a warp stages it
   const uint32_t* hint;        // staged: predicted next treelet per (treelet, direction octant), or null
   uint32_t wait_tries;         // staged: probes of the wait for the pinned image before staging stops
-  uint32_t tbuf_off;           // plain walk: byte offset of the trace staging area in dynamic shared
+  uint32_t tbuf_off;           // byte offset of the trace staging area in dynamic shared
                                // memory (128-aligned base), kNone: trace entries go straight to the rows
   uint32_t ss_off;             // plain walk with SHORT: byte offset of the short stacks, likewise
 };
 
-// Trace staging (the plain walk).  A lane writing its ray's trace rows one
-// 4-byte entry at a time leaves partly written 32-byte sectors that L2 fills
-// from DRAM and writes back again and again (4.5x the entries' bytes
-// written, as many read, on bounce rays).  Instead each lane keeps its ray's
-// next 8 entries of each row in its warp's 2 KiB staging area ([visit |
-// treelet][entry 0..7][lane] words: lanes hit distinct banks) and writes them
-// as one whole, aligned sector.  Used when the row capacity is a multiple of
-// 8 and the rows start on 32-byte boundaries; the last partial sector is
+// Access traces.  A walk writes one row per ray: the visits, or the treelet
+// ids when only they are asked for.  With both asked for the treelet ids are
+// filled in from the visits afterwards (trace_treelet_ids_kernel): looked up
+// in the walk each cost a dependent load, a second scattered store and L1
+// room.
+//
+// Staging.  A lane writing its ray's row one 4-byte entry at a time leaves
+// partly written 32-byte sectors that L2 fills from DRAM and writes back again
+// and again (4.5x the entries' bytes written, as many read, on bounce rays).
+// Instead each lane keeps its ray's next 8 entries in its warp's 1 KiB staging
+// area ([entry 0..7][lane] words: lanes hit distinct banks) and writes
+// them as one whole, aligned sector.  Used when the row capacity is a multiple
+// of 8 and the rows start on 32-byte boundaries; the last partial sector is
 // written when the ray ends.
-constexpr uint32_t kTraceBufWarpBytes = 2048;
+constexpr uint32_t kTraceBufWarpBytes = 1024;
 
 extern __shared__ __align__(128) uint8_t rt_dyn_smem[];
 
@@ -102,42 +107,43 @@ __device__ __forceinline__ uint32_t* trace_buf(uint32_t off) {
   return reinterpret_cast<uint32_t*>(base + off + (threadIdx.x >> 5) * kTraceBufWarpBytes) + (threadIdx.x & 31u);
 }
 
-// Entry n (< capacity) of a ray's visit and treelet rows (either row may be null).
-__device__ __forceinline__ void trace_put(const TraceArgs& a, uint32_t* vrow, uint32_t* trow, uint32_t n, uint32_t vis,
-                                          uint32_t tl) {
+// Records entry n (< capacity) of ray r's row.
+__device__ __forceinline__ void trace_put(const TraceArgs& a, uint32_t r, uint32_t n, uint32_t x) {
   if (a.tbuf_off == kNone) {
-    if (vrow) vrow[n] = vis;
-    if (trow) trow[n] = tl;
+    a.rows[(uint64_t)r * a.cap + n] = x;
     return;
   }
   uint32_t* b = trace_buf(a.tbuf_off);
   const uint32_t j = n & 7u;
-  if (vrow) b[j * 32] = vis;
-  if (trow) b[256 + j * 32] = tl;
+  b[j * 32] = x;
   if (j == 7u) {
-    if (vrow) {
-      uint4* d = reinterpret_cast<uint4*>(vrow + (n - 7u));
-      __stcs(d, make_uint4(b[0], b[32], b[64], b[96]));
-      __stcs(d + 1, make_uint4(b[128], b[160], b[192], b[224]));
-    }
-    if (trow) {
-      uint4* d = reinterpret_cast<uint4*>(trow + (n - 7u));
-      __stcs(d, make_uint4(b[256], b[288], b[320], b[352]));
-      __stcs(d + 1, make_uint4(b[384], b[416], b[448], b[480]));
-    }
+    uint4* d = reinterpret_cast<uint4*>(a.rows + (uint64_t)r * a.cap + (n - 7u));
+    __stcs(d, make_uint4(b[0], b[32], b[64], b[96]));
+    __stcs(d + 1, make_uint4(b[128], b[160], b[192], x));
   }
 }
 
 // Writes the staged entries of a ray's last partial sector; m = entries
 // recorded (at most the capacity).
-__device__ __forceinline__ void trace_drain(const TraceArgs& a, uint32_t* vrow, uint32_t* trow, uint32_t m) {
+__device__ __forceinline__ void trace_drain(const TraceArgs& a, uint32_t r, uint32_t m) {
   const uint32_t k = m & 7u;
   if (a.tbuf_off == kNone || k == 0) return;
   const uint32_t* b = trace_buf(a.tbuf_off);
-  const uint32_t base = m - k;
-  for (uint32_t j = 0; j < k; ++j) {
-    if (vrow) vrow[base + j] = b[j * 32];
-    if (trow) trow[base + j] = b[256 + j * 32];
+  uint32_t* row = a.rows + (uint64_t)r * a.cap + (m - k);
+  for (uint32_t j = 0; j < k; ++j) row[j] = b[j * 32];
+}
+
+// The treelet id of every recorded visit (one warp per ray): reads and writes
+// whole rows in order, the scattered part is the 8-byte table entry.
+__global__ void __launch_bounds__(256) trace_treelet_ids_kernel(const uint32_t* __restrict__ visits,
+                                                                const rt_hit* __restrict__ hits,
+                                                                const uint2* __restrict__ meta, uint32_t n,
+                                                                uint32_t cap, uint32_t* __restrict__ treelets) {
+  const uint32_t lane = threadIdx.x & 31u, warps = (gridDim.x * blockDim.x) >> 5;
+  for (uint32_t r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < n; r += warps) {
+    const uint32_t m = min(hits[r].n_visits, cap);
+    const uint64_t row = (uint64_t)r * cap;
+    for (uint32_t j = lane; j < m; j += 32) __stcs(treelets + row + j, meta[__ldcs(visits + row + j) >> 3].x);
   }
 }
 
@@ -428,11 +434,7 @@ struct PlainWalker {
   }
 
   __device__ __forceinline__ void record(const TraceArgs& a, uint32_t r, uint32_t unit, uint32_t type) {
-    if (TRACED && n_tx < a.cap) {
-      uint32_t* vrow = a.visits ? a.visits + (uint64_t)r * a.cap : nullptr;
-      uint32_t* trow = a.tl_trace ? a.tl_trace + (uint64_t)r * a.cap : nullptr;
-      trace_put(a, vrow, trow, n_tx, rtf::pack_visit(unit, type), trow ? v.meta[unit].x : 0u);
-    }
+    if (TRACED && n_tx < a.cap) trace_put(a, r, n_tx, a.rows_tl ? v.meta[unit].x : rtf::pack_visit(unit, type));
     n_tx++;
   }
 
@@ -572,9 +574,7 @@ struct PlainWalker {
 
   __device__ __forceinline__ void finish(const TraceArgs& a, uint32_t r) {
     const bool bad = flags & (RT_RAY_STACK_OVERFLOW | RT_RAY_BAD_NODE);
-    if (TRACED)
-      trace_drain(a, a.visits ? a.visits + (uint64_t)r * a.cap : nullptr,
-                  a.tl_trace ? a.tl_trace + (uint64_t)r * a.cap : nullptr, min(n_tx, a.cap));
+    if (TRACED) trace_drain(a, r, min(n_tx, a.cap));
     write_hit(a, v, r, !bad && (min_thit < tmax), min_thit, world_o(), world_d(), tmin, tmax, cold(9), cold(10),
               __uint_as_float(cold(11)), n_tx, flags & kRayStatusMask);
   }

@@ -138,15 +138,8 @@ struct Walker {
     cx.fast = (flags & kRayWorldFast) != 0;
   }
   // one visit of the trace (the reference's MemoryTransactionRecord)
-  // The rows are written entry by entry: staging them through shared memory
-  // as the plain walk does measured 15-30% slower here (eight inlined
-  // copies of the staging code in the traced walk).
   __device__ __forceinline__ void record(const TraceArgs& a, uint32_t r, uint32_t unit, uint32_t type) {
-    if (TRACED && n_tx < a.cap) {
-      const uint64_t at = (uint64_t)r * a.cap + n_tx;
-      if (a.visits) a.visits[at] = rtf::pack_visit(unit, type);
-      if (a.tl_trace) a.tl_trace[at] = v.meta[unit].x;
-    }
+    if (TRACED && n_tx < a.cap) trace_put(a, r, n_tx, a.rows_tl ? v.meta[unit].x : rtf::pack_visit(unit, type));
     n_tx++;
   }
 
@@ -454,6 +447,7 @@ struct Walker {
   __device__ __forceinline__ void finish(const TraceArgs& a, uint32_t r) {
     const bool bad = flags & (RT_RAY_STACK_OVERFLOW | RT_RAY_BAD_NODE);
     const unsigned long long h = cold(2);
+    if (TRACED) trace_drain(a, r, min(n_tx, a.cap));
     write_hit(a, v, r, !bad && (min_thit < tmax), min_thit, world_o(), dir(), tmin, tmax, (uint32_t)h,
               (uint32_t)(h >> 32), hi(cold(1)), n_tx, flags & kRayStatusMask);
   }
