@@ -67,3 +67,30 @@ def test_unordered_boxes_and_nonfinite_rays(ctx, every):
         finite = np.isfinite(rays["origin"]).all(axis=1) & np.isfinite(rays["dir"]).all(axis=1)
         assert_hits_equal(hits[finite], oh[finite], f"hits, mode {mode}")
     scene.close()
+
+
+def test_unit_that_is_node_and_leaf(ctx):
+    """A unit one parent lists as an internal node and another as a quad leaf."""
+    import treelet_rt as rt
+    from oracle import oracle as orc
+
+    b = rt.Blob.gen(rt.SCENE_CUBE, 2000, 3).bytes()
+    top = int(b[:8].view(np.uint64)[0]) // 64
+    leaf = top + int(b[top * 64 + 12:top * 64 + 16].view(np.int32)[0])  # the TLAS root's instance leaf
+    hdr = leaf + int(b[leaf * 64 + 64:leaf * 64 + 72].view(np.uint64)[0]) // 64
+    root = hdr + int(b[hdr * 64:hdr * 64 + 8].view(np.uint64)[0]) // 64
+    child = root + int(b[root * 64 + 12:root * 64 + 16].view(np.int32)[0])
+    info = b[child * 64 + 22:child * 64 + 28]
+    assert (b[root * 64 + 22] >> 2) & 15 == 0 and info[0] & 3  # the root's first child is internal
+    # the first child's children become its siblings, read as quad leaves
+    b[child * 64 + 12:child * 64 + 16] = np.array([1], np.int32).view(np.uint8)
+    for i in range(6):
+        if info[i] & 3:
+            info[i] = 4 << 2 | 1
+    rays = rt.camera_rays(rt.default_camera(rt.SCENE_CUBE), 40, 31, 1, 2, 1e-4, 1e30)
+    scene = rt.Scene(ctx, rt.Blob.wrap(b))
+    hits, vis, _ = scene.trace_host(rays, rt.MODE_PLAIN, capacity=CAP, want_visits=True)
+    oh, ov, _ = orc.trace(b, rays, 0, None, capacity=CAP, want_visits=True)
+    assert np.array_equal(hits["n_visits"], oh["n_visits"])
+    assert_traces_equal(vis, ov, oh["n_visits"], "visits")
+    scene.close()

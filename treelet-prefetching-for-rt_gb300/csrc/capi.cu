@@ -16,6 +16,7 @@
 #include "trace_queued.cuh"
 #include "trace_treelet.cuh"
 #include "treelets.h"
+#include "walk_node.h"
 
 namespace rti {
 
@@ -29,7 +30,7 @@ rt_status fail(rt_status s, const std::string& msg) {
   return s;
 }
 
-bool validate_blob(const uint8_t* b, uint64_t n, std::string* err, bool* ordered) {
+bool validate_blob(const uint8_t* b, uint64_t n, std::string* err, BlobRoles* roles) {
   auto bad = [&](const std::string& m) {
     if (err) *err = m;
     return false;
@@ -43,7 +44,15 @@ bool validate_blob(const uint8_t* b, uint64_t n, std::string* err, bool* ordered
     return v;
   };
   std::vector<uint8_t> seen(units, 0);
-  bool in_order = true;
+  // roles: bit 0 internal node, bit 1 read as the blob's bytes (headers, leaves)
+  constexpr uint8_t kInternal = 1, kRaw = 2;
+  std::vector<uint8_t> role(units, 0);
+  bool mixed = false;
+  auto take = [&](uint64_t u, uint8_t r) {
+    role[u] |= r;
+    mixed |= role[u] == (kInternal | kRaw);
+  };
+  take(0, kRaw);
   struct Item {
     uint64_t unit;
     bool top;
@@ -55,6 +64,7 @@ bool validate_blob(const uint8_t* b, uint64_t n, std::string* err, bool* ordered
   while (!work.empty()) {
     const Item it = work.back();
     work.pop_back();
+    take(it.unit, kInternal);
     if (seen[it.unit]) continue;
     seen[it.unit] = 1;
     const uint8_t* p = b + it.unit * 64;
@@ -70,28 +80,34 @@ bool validate_blob(const uint8_t* b, uint64_t n, std::string* err, bool* ordered
       const uint32_t sz = rtf::child_size_units(info), ty = rtf::child_type(info);
       if (sz) {
         if (c + sz > units) return bad("child outside the blob");
-        for (uint32_t k = 0; k < 3; ++k)
-          in_order &= p[rtf::IN_LO_X + 12 * k + i] <= p[rtf::IN_HI_X + 12 * k + i];
         if (ty == rtf::CT_INTERNAL) {
           work.push_back({c, it.top});
         } else if (it.top) {
           if (ty != rtf::CT_INSTANCE || sz != 2) return bad("top-level leaf that is not a 128-byte instance leaf");
+          take(c, kRaw);
+          take(c + 1, kRaw);
           if (!seen[c]) {
             seen[c] = 1;
             const uint64_t hdr = c * 64 + rd64(c * 64 + rtf::IL_BVH_ADDRESS);
             if (hdr % 64 || hdr / 64 >= units) return bad("instance BVHAddress out of range");
             const uint64_t broot = hdr + rd64(hdr + rtf::HDR_ROOT_OFFSET);
             if (broot % 64 || broot / 64 >= units || broot <= hdr) return bad("BLAS RootNodeOffset out of range");
+            take(hdr / 64, kRaw);
             work.push_back({broot / 64, false});
           }
         } else {
           if (ty != rtf::CT_QUAD && ty != rtf::CT_PROCEDURAL) return bad("bottom-level leaf of unknown type");
+          for (uint32_t k = 0; k < sz; ++k) take(c + k, kRaw);
         }
       }
       c += sz;
     }
   }
-  if (ordered) *ordered = in_order;
+  if (roles) {
+    roles->mixed = mixed;
+    roles->internal.assign((units + 31) / 32, 0);
+    for (uint64_t u = 0; u < units; ++u) roles->internal[u / 32] |= (uint32_t)(role[u] & kInternal) << (u % 32);
+  }
   return true;
 }
 
@@ -113,9 +129,14 @@ struct rt_scene {
   rt_ctx* ctx = nullptr;
   std::vector<uint8_t> host_blob;
   uint8_t* d_blob = nullptr;
+  // The blob as the walks read it: internal nodes as walk nodes (walk_node.h),
+  // the rest as it is.  When a unit has both uses (mixed_roles) it holds walk
+  // nodes only, and leaves and headers are read from the blob.
+  uint8_t* d_walk = nullptr;
+  uint32_t* d_internal = nullptr;  // BlobRoles::internal, null when mixed_roles
+  bool mixed_roles = false;
   uint64_t blob_bytes = 0;
   uint32_t n_units = 0;
-  bool ordered = false;  // no child box has a quantized lower bound above its upper one
   // treelets
   bool has_treelets = false;
   rtt::Partition part;
@@ -299,8 +320,17 @@ void drop_pin_cache(rt_scene* s) {
   s->pin_cache.clear();
 }
 
+// Writes the scene's walk nodes with the given route bits (null: none) and
+// waits for them.
+cudaError_t make_walk_nodes(rt_scene* s, const uint16_t* d_route) {
+  rtk::walk_nodes_kernel<<<(s->n_units + 255) / 256, 256>>>(reinterpret_cast<const uint4*>(s->d_blob), s->d_internal,
+                                                            d_route, s->n_units, reinterpret_cast<uint4*>(s->d_walk));
+  const cudaError_t e = cudaGetLastError();
+  return e != cudaSuccess ? e : cudaStreamSynchronize(nullptr);
+}
+
 // Computes the route bits of the walk (treelets.h) into s->route, uploads
-// them and rebuilds the pinned image that embeds them.  With a nonzero
+// them, writes them into the walk nodes and rebuilds the pinned image that embeds them.  With a nonzero
 // device_offset the reference's comparisons stop matching at the first pop
 // from the other-treelet stack (vulkan_ray_tracing.cc:1752); the current
 // stack is empty then and nothing is pushed to it again, so every later node
@@ -313,6 +343,7 @@ rt_status upload_route(rt_scene* s) {
   if (s->offset_quirk)
     for (uint16_t& r : s->route) r &= (uint16_t)~((0x3Fu << rtt::kRouteOtherShift) | (2u << rtt::kRouteInstShift));
   RT_CUDA(cudaMemcpy(s->d_route, s->route.data(), sizeof(uint16_t) * s->route.size(), cudaMemcpyHostToDevice));
+  RT_CUDA(make_walk_nodes(s, s->d_route));
   drop_pin_cache(s);
   return rebuild_pinned(s);
 }
@@ -354,6 +385,13 @@ rt_status rebuild_pinned(rt_scene* s, bool keep_current) {
   rtt::build_pinned(s->host_blob.data(), s->blob_bytes, s->part, s->route,
                     s->pin_order.empty() ? s->pin_default : s->pin_order, budget, pin);
   if (pin.bytes.empty()) return RT_OK;
+  // internal nodes' records hold walk nodes on the device
+  for (const auto& [at, unit] : pin.internal) {
+    uint32_t raw[16], node[16];
+    std::memcpy(raw, s->host_blob.data() + (uint64_t)unit * 64, 64);
+    rtw::walk_node(raw, unit, s->route[unit], node);
+    std::memcpy(pin.bytes.data() + at, node, 64);
+  }
   rt_status st = dalloc(&s->d_pin, pin.bytes.size());
   if (st != RT_OK) return st;
   RT_CUDA(cudaMemcpy(s->d_pin, pin.bytes.data(), pin.bytes.size(), cudaMemcpyHostToDevice));
@@ -662,8 +700,8 @@ rt_status rt_scene_create(rt_ctx* ctx, const rt_blob* blob, rt_scene** out) {
   if (!ctx || !blob || !out) return rti::fail(RT_ERR_INVALID, "rt_scene_create: NULL argument");
   *out = nullptr;
   std::string err;
-  bool ordered = false;
-  if (!rti::validate_blob(blob->bytes.data(), blob->bytes.size(), &err, &ordered)) return rti::fail(RT_ERR_BLOB, err);
+  rti::BlobRoles roles;
+  if (!rti::validate_blob(blob->bytes.data(), blob->bytes.size(), &err, &roles)) return rti::fail(RT_ERR_BLOB, err);
   if (blob->bytes.size() / 64 >= (1ull << 29))
     return rti::fail(RT_ERR_TOO_LARGE, "rt_scene_create: blobs are limited to 2^29 units of 64 bytes");
   RT_CUDA(cudaSetDevice(ctx->device));
@@ -672,8 +710,10 @@ rt_status rt_scene_create(rt_ctx* ctx, const rt_blob* blob, rt_scene** out) {
   s->host_blob = blob->bytes;
   s->blob_bytes = blob->bytes.size();
   s->n_units = (uint32_t)(s->blob_bytes / 64);
-  s->ordered = ordered;
   rt_status st = dalloc(&s->d_blob, s->blob_bytes);
+  if (st == RT_OK) st = dalloc(&s->d_walk, s->blob_bytes);
+  s->mixed_roles = roles.mixed;
+  if (st == RT_OK && !roles.mixed) st = dalloc(&s->d_internal, sizeof(uint32_t) * roles.internal.size());
   if (st == RT_OK) st = dalloc(&s->d_stats, sizeof(unsigned long long) * rtk::ST_COUNT);
   if (st == RT_OK) st = dalloc(&s->d_status, sizeof(uint32_t));
   if (st == RT_OK) st = dalloc(&s->d_queue, sizeof(uint32_t) * rti::kHostChunks);
@@ -682,6 +722,9 @@ rt_status rt_scene_create(rt_ctx* ctx, const rt_blob* blob, rt_scene** out) {
     return st;
   }
   cudaError_t e = cudaMemcpy(s->d_blob, blob->bytes.data(), s->blob_bytes, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess && s->d_internal)
+    e = cudaMemcpy(s->d_internal, roles.internal.data(), sizeof(uint32_t) * roles.internal.size(), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = make_walk_nodes(s, nullptr);
   if (e == cudaSuccess) e = cudaMemset(s->d_stats, 0, sizeof(unsigned long long) * rtk::ST_COUNT);
   if (e == cudaSuccess) e = cudaMemset(s->d_status, 0, sizeof(uint32_t));
   for (cudaStream_t* x : {&s->stream, &s->stream2, &s->xin, &s->xout})
@@ -703,6 +746,8 @@ rt_status rt_scene_destroy(rt_scene* s) {
   cudaSetDevice(s->ctx->device);
   free_treelets(s);
   cudaFree(s->d_blob);
+  cudaFree(s->d_walk);
+  cudaFree(s->d_internal);
   cudaFree(s->d_stats);
   cudaFree(s->d_status);
   cudaFree(s->d_queue);
@@ -877,15 +922,23 @@ rt_status check_trace(const rt_scene* s, uint32_t mode, const rt_trace_buf* trac
   return RT_OK;
 }
 
+rtk::SceneView scene_view(const rt_scene* s) {
+  const uint4* raw = reinterpret_cast<const uint4*>(s->d_blob);
+  const uint4* walk = reinterpret_cast<const uint4*>(s->d_walk);
+  return rtk::SceneView{s->mixed_roles ? raw : walk, walk, raw, s->d_meta, s->d_route, s->n_units};
+}
+
 // Launches one trace over device arrays.  `queue` is the ray hand-out
 // counter of this launch; `keep` adds the counters to the previous launch's.
 rt_status trace_launch(rt_scene* s, const rt_ray* rays, const uint32_t* flags, uint32_t default_flags, uint32_t n,
                        uint32_t mode, rt_hit* hits, const rt_trace_buf* trace, cudaStream_t st, uint32_t* queue,
                        bool keep, bool allow_queues = true) {
   rtk::TraceArgs a{};
-  a.blob = reinterpret_cast<const uint4*>(s->d_blob);
+  const rtk::SceneView view = scene_view(s);
+  a.blob = view.blob;
+  a.raw = view.raw;
   a.n_units = s->n_units;
-  a.ordered = s->ordered;
+  a.walk = view.walk;
   a.rays = rays;
   a.flags = flags;
   a.default_flags = default_flags;
@@ -1335,9 +1388,10 @@ rt_status batch_args(rt_batch* b, const rt_ray* rays, const uint32_t* flags, uin
   bool stale = false;
   for (size_t i = 0; i < b->scenes.size(); ++i) {
     const rt_scene* s = b->scenes[i];
-    const rtk::SceneView nv{reinterpret_cast<const uint4*>(s->d_blob), s->d_meta, s->d_route, s->n_units, s->ordered};
+    const rtk::SceneView nv = scene_view(s);
     const rtk::SceneView& ov = b->views[i];
-    if (nv.blob != ov.blob || nv.meta != ov.meta || nv.route != ov.route || nv.n_units != ov.n_units) {
+    if (nv.blob != ov.blob || nv.walk != ov.walk || nv.raw != ov.raw || nv.meta != ov.meta || nv.route != ov.route ||
+        nv.n_units != ov.n_units) {
       b->views[i] = nv;
       stale = true;
     }
@@ -1428,8 +1482,7 @@ rt_status rt_batch_create(rt_ctx* ctx, rt_scene* const* scenes, uint32_t n_scene
       rt_batch_destroy(b);
       return rti::fail(RT_ERR_INVALID, "rt_batch_create: NULL scene or scene on another device");
     }
-    v[i] = rtk::SceneView{reinterpret_cast<const uint4*>(scenes[i]->d_blob), scenes[i]->d_meta, scenes[i]->d_route,
-                          scenes[i]->n_units, scenes[i]->ordered};
+    v[i] = scene_view(scenes[i]);
   }
   cudaError_t e = cudaMemcpy(b->d_views, v.data(), sizeof(rtk::SceneView) * n_scenes, cudaMemcpyHostToDevice);
   b->views = v;

@@ -22,8 +22,17 @@ namespace rti {
 void set_error(const std::string& msg);
 rt_status fail(rt_status s, const std::string& msg);
 
+// What a blob's units are to the walks.  internal: bit u % 32 of word u / 32
+// for every unit reached as an internal node; mixed: some unit is reached as
+// an internal node and also read as something else (then `internal` may miss
+// some).
+struct BlobRoles {
+  std::vector<uint32_t> internal;
+  bool mixed = false;
+};
+
 // Host-side structural check of a blob; returns false with a message.
-bool validate_blob(const uint8_t* b, uint64_t n, std::string* err, bool* ordered = nullptr);
+bool validate_blob(const uint8_t* b, uint64_t n, std::string* err, BlobRoles* roles = nullptr);
 
 // After the scene's traces have finished: RT_ERR_TIMEOUT if a bounded device
 // wait of the last launch gave up, else RT_OK.

@@ -7,6 +7,7 @@
 
 #include "format.h"
 #include "rtmath.h"
+#include "walk_node.h"
 
 namespace rtd {
 
@@ -26,6 +27,12 @@ __device__ __forceinline__ uint4 ld_shared_v4(uint32_t saddr) {
 __device__ __forceinline__ uint32_t ld_shared_u32(uint32_t saddr) {
   uint32_t v;
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(saddr));
+  return v;
+}
+
+__device__ __forceinline__ uint32_t ld_shared_u16(uint32_t saddr) {
+  uint16_t v;
+  asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(saddr));
   return v;
 }
 
@@ -60,16 +67,7 @@ __device__ __forceinline__ uint4 load16(const uint4* g, uint32_t saddr, int q) {
   return saddr ? ld_shared_v4(saddr + 16u * q) : ld_global_nc(g + q);
 }
 
-__device__ __forceinline__ uint32_t byte_at(const Node64& n, int b) { return (n.w[b >> 2] >> ((b & 3) * 8)) & 0xffu; }
 __device__ __forceinline__ float f32_at(const Node64& n, int b) { return __uint_as_float(n.w[b >> 2]); }
-
-// Result of testing one internal node's children against a ray.
-struct ChildHits {
-  uint32_t hit_mask;    // bit i: child i hit and not culled
-  uint32_t child_unit;  // unit index of child 0's block
-  uint64_t info;        // child i's info byte (bits 0-1 size, 2-5 type) at bits 8i..8i+7
-  __device__ __forceinline__ uint32_t info_of(int i) const { return (uint32_t)(info >> (8 * i)) & 0x3fu; }
-};
 
 // Two-wide FP32 arithmetic (add / sub / mul / fma .rn.f32x2, sm_100 and
 // later): one instruction computes two lanes, each rounded exactly as the
@@ -128,9 +126,10 @@ __device__ __forceinline__ float min3(float a, float b, float c) {
   return r;
 }
 
-// The quantized bounds of one axis, sorted into the plane a ray meets first
-// and the other by the sign of its direction: children 0..3 in the bytes of
-// `near4` and `far4`, children 4 and 5 in `rest` (near 4, near 5, far 4, far 5).
+// The quantized bounds of one axis of a walk node, sorted into the plane a
+// ray meets first and the other by the sign of its direction: children 0..3
+// in the bytes of `near4` and `far4`, children 4 and 5 in `rest` (near 4,
+// near 5, far 4, far 5).
 struct AxisBytes {
   uint32_t near4, far4, rest;
   __device__ __forceinline__ uint32_t near_bits(int i) const {
@@ -140,27 +139,44 @@ struct AxisBytes {
     return __byte_perm(i < 4 ? far4 : rest, 0x4B000000u, (uint32_t)(i < 4 ? i : i - 2) | 0x7540u);
   }
 };
-
-// Axis k's six lower bounds are bytes 28 + 12k .. 33 + 12k, the upper ones
-// the six bytes after them.
 __device__ __forceinline__ AxisBytes axis_bytes(const Node64& n, int k, float idir) {
-  const uint32_t a = n.w[7 + 3 * k], b = n.w[8 + 3 * k], c = n.w[9 + 3 * k];
-  const uint32_t hi4 = __byte_perm(b, c, 0x5432);
+  const uint32_t lo4 = n.w[7 + 3 * k], rest = n.w[8 + 3 * k], hi4 = n.w[9 + 3 * k];
   const bool up = idir > 0.0f;
-  return AxisBytes{up ? a : hi4, up ? hi4 : a, __byte_perm(b, c, up ? 0x7610u : 0x1076u)};
+  return AxisBytes{up ? lo4 : hi4, up ? hi4 : lo4, __byte_perm(rest, 0, up ? 0x3210u : 0x1032u)};
 }
 
 // The box tests of an internal node (vulkan_ray_tracing.cc:2518-2553 and the
 // bottom-level twin :2714-2741): children with ChildSize > 0 are slab-tested
 // with the ray's [tmin, tmax]; a hit at thit >= cull is dropped.  Bounds are
-// Origin + ldexpf(q, exp - 8) (asu.h:499-508, child_bound), slab values
-// (b - o) * idir (vulkan_ray_tracing.cc:199-218), reduced as magic_max7 /
-// magic_min7.
+// Origin + ldexpf(q, exp - 8) (asu.h:499-508), slab values (b - o) * idir
+// (vulkan_ray_tracing.cc:199-218), reduced as magic_max7 / magic_min7.
+// Returns bit i for a hit child i.
 //
-// FAST = false uses the reference's ternary MIN/MAX macros in its order, and
-// reads the bounds from `src`, where the node was loaded from.
-// FAST = true is for a finite ray (finite_ray) in a scene whose quantized
-// boxes are ordered.  Every slab value then is one monotone function of its
+// hit_children_exact reads the blob's node and uses the reference's ternary
+// MIN/MAX macros in its order.
+__device__ __forceinline__ uint32_t hit_children_exact(const uint4* raw, rtm::V3 o, rtm::V3 idir, float tmin,
+                                                       float tmax, float cull) {
+  const uint8_t* b = reinterpret_cast<const uint8_t*>(raw);
+  const float* org = reinterpret_cast<const float*>(raw);
+  const float s[3] = {rtm::exp2_int((int)(int8_t)b[rtf::IN_EXP] - 8), rtm::exp2_int((int)(int8_t)b[rtf::IN_EXP + 1] - 8),
+                      rtm::exp2_int((int)(int8_t)b[rtf::IN_EXP + 2] - 8)};
+  uint32_t mask = 0;
+#pragma unroll 1
+  for (int i = 0; i < 6; ++i) {
+    if (!(b[rtf::IN_CHILD_INFO + i] & 3u)) continue;
+    const uint8_t* q = b + rtf::IN_LO_X + i;
+    const rtm::V3 lo = rtm::v3(__fmaf_rn((float)q[0], s[0], org[0]), __fmaf_rn((float)q[12], s[1], org[1]),
+                               __fmaf_rn((float)q[24], s[2], org[2]));
+    const rtm::V3 hi = rtm::v3(__fmaf_rn((float)q[6], s[0], org[0]), __fmaf_rn((float)q[18], s[1], org[1]),
+                               __fmaf_rn((float)q[30], s[2], org[2]));
+    float tn;
+    if (rtm::ray_box_test(lo, hi, idir, o, tmin, tmax, tn) && !(tn >= cull)) mask |= 1u << i;
+  }
+  return mask;
+}
+
+// hit_children is for a finite ray (finite_ray) and a walk node without
+// kExact.  Every slab value then is one monotone function of its
 // bound (two roundings, a finite nonzero idir), so the lower plane's value is
 // the smaller one when idir > 0 and the larger one when idir < 0: the two
 // planes are told apart once per node and axis by the sign of idir instead of
@@ -172,38 +188,18 @@ __device__ __forceinline__ AxisBytes axis_bytes(const Node64& n, int k, float id
 // bound by the integer / minmax pipe (63% busy in the staged walk): against
 // six minima and maxima and one branch a child, 2M primary rays staged went
 // from 3.29 to 3.12 ms on a GB300 and small frames gained 2-6%.
-template <bool FAST>
-__device__ __forceinline__ ChildHits test_children(const Node64& n, const uint4* src, uint32_t node_unit,
-                                                   rtm::V3 o, rtm::V3 idir, float tmin, float tmax, float cull) {
-  ChildHits r;
+__device__ __forceinline__ uint32_t hit_children(const Node64& n, rtm::V3 o, rtm::V3 idir, float tmin, float tmax,
+                                                 float cull) {
   const float ox = f32_at(n, 0), oy = f32_at(n, 4), oz = f32_at(n, 8);
-  const int child_off = (int)n.w[3];
-  const int ex = (int)(int8_t)byte_at(n, 18), ey = (int)(int8_t)byte_at(n, 19), ez = (int)(int8_t)byte_at(n, 20);
-  const float sx = rtm::exp2_int(ex - 8), sy = rtm::exp2_int(ey - 8), sz = rtm::exp2_int(ez - 8);
-  r.hit_mask = 0;
-  r.info = ((uint64_t)n.w[6] << 16) | (n.w[5] >> 16);  // bytes 22..27
-  r.info &= 0x3f3f3f3f3f3full;
-  r.child_unit = (uint32_t)((int)node_unit + child_off);
-  if (!FAST) {
-#pragma unroll 1
-    for (int i = 0; i < 6; ++i) {
-      if (!(r.info_of(i) & 3u)) continue;
-      // read again from memory: indexed by a run-time i the node's words would leave registers
-      const uint8_t* row = reinterpret_cast<const uint8_t*>(src) + rtf::IN_LO_X + i;
-      auto q = [&](int k) { return (float)row[6 * k]; };
-      const rtm::V3 lo = rtm::v3(__fmaf_rn(q(0), sx, ox), __fmaf_rn(q(2), sy, oy), __fmaf_rn(q(4), sz, oz));
-      const rtm::V3 hi = rtm::v3(__fmaf_rn(q(1), sx, ox), __fmaf_rn(q(3), sy, oy), __fmaf_rn(q(5), sz, oz));
-      float tn;
-      if (rtm::ray_box_test(lo, hi, idir, o, tmin, tmax, tn) && !(tn >= cull)) r.hit_mask |= 1u << i;
-    }
-    return r;
-  }
+  const float sx = __uint_as_float((n.w[4] << 23) & 0x7f800000u), sy = __uint_as_float((n.w[4] << 15) & 0x7f800000u),
+              sz = __uint_as_float((n.w[4] << 7) & 0x7f800000u);
   const AxisBytes bx = axis_bytes(n, 0, idir.x), by = axis_bytes(n, 1, idir.y), bz = axis_bytes(n, 2, idir.z);
   // x and y in two-wide FP32, and the two z planes: the same roundings, half the instructions
   const unsigned long long s_xy = f2_pack(sx, sy), o_xy = f2_pack(ox, oy), s_z = f2_pack(sz, sz), o_z = f2_pack(oz, oz);
   const unsigned long long org_xy = f2_pack(o.x, o.y), id_xy = f2_pack(idir.x, idir.y);
   const unsigned long long org_z = f2_pack(o.z, o.z), id_z = f2_pack(idir.z, idir.z);
   const unsigned long long two23 = f2_pack(8388608.0f, 8388608.0f);
+  uint32_t mask = 0;
 #pragma unroll
   for (int i = 0; i < 6; ++i) {
     // q as an exact float (bits - 2^23), Origin + q * 2^(e-8) fused, then (b - o) * idir
@@ -217,17 +213,12 @@ __device__ __forceinline__ ChildHits test_children(const Node64& n, const uint4*
     slab(bx.far_bits(i), by.far_bits(i), s_xy, o_xy, org_xy, id_xy, fx, fy);
     slab(bz.near_bits(i), bz.far_bits(i), s_z, o_z, org_z, id_z, nz, fz);
     const float tn = fmaxf(max3(nx, ny, nz), tmin), tf = fminf(min3(fx, fy, fz), tmax);
-    if (tn <= tf && !(tn >= cull)) r.hit_mask |= 1u << i;
+    if (tn <= tf && !(tn >= cull)) mask |= 1u << i;
   }
-  // children with ChildSize 0 are no children: bit i of `valid` for byte i of the info
-  const uint32_t v03 = ((uint32_t)r.info | ((uint32_t)r.info >> 1)) & 0x01010101u;
-  const uint32_t v45 = ((uint32_t)(r.info >> 32) | ((uint32_t)(r.info >> 33))) & 0x0101u;
-  const uint32_t valid = ((v03 * 0x01020408u) >> 24 & 0xfu) | (v45 & 1u) << 4 | (v45 >> 8) << 5;
-  r.hit_mask &= valid;
-  return r;
+  return mask & (n.w[5] | (n.w[5] >> rtw::kLeafShift)) & rtw::kChildMask;
 }
 
-// True when the slab test may use the FAST min/max (see mn2).
+// True when the slab test may tell planes apart by the direction's sign (hit_children).
 __device__ __forceinline__ bool finite_ray(rtm::V3 o, rtm::V3 d, float tmin, float tmax) {
   return isfinite(o.x) && isfinite(o.y) && isfinite(o.z) && isfinite(d.x) && isfinite(d.y) && isfinite(d.z) &&
          !isnan(tmin) && !isnan(tmax);

@@ -35,17 +35,43 @@ constexpr uint32_t kStatusTimeout = 1u;
 
 // What a walk needs of one scene.
 struct SceneView {
-  const uint4* blob;
+  const uint4* blob;      // headers, leaves and instance leaves
+  const uint4* walk;      // walk nodes (walk_node.h); the same array unless a unit has both uses
+  const uint4* raw;       // the blob as uploaded
   const uint2* meta;      // per unit: x = treelet root unit, y = dense << 10 | slot
   const uint16_t* route;  // per unit: routing bits of the treelet-ordered walk (treelets.h)
   uint32_t n_units;
-  uint32_t ordered;       // every child box's quantized lower bounds are at most its upper ones
 };
+
+// The walks' copy of the blob: units marked in `internal` as walk nodes
+// (walk_node.h), the others as they are; without marks every unit is taken as
+// an internal node.
+__global__ void __launch_bounds__(256) walk_nodes_kernel(const uint4* __restrict__ blob,
+                                                         const uint32_t* __restrict__ internal,
+                                                         const uint16_t* __restrict__ route, uint32_t n_units,
+                                                         uint4* __restrict__ walk) {
+  const uint32_t u = blockIdx.x * blockDim.x + threadIdx.x;
+  if (u >= n_units) return;
+  uint32_t raw[16], node[16];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const uint4 x = __ldcs(blob + (uint64_t)u * 4 + q);
+    raw[4 * q] = x.x, raw[4 * q + 1] = x.y, raw[4 * q + 2] = x.z, raw[4 * q + 3] = x.w;
+  }
+  rtw::walk_node(raw, u, route ? route[u] : 0u, node);
+  const bool keep = internal && !((internal[u >> 5] >> (u & 31u)) & 1u);
+#pragma unroll
+  for (int q = 0; q < 16; ++q) node[q] = keep ? raw[q] : node[q];
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+    walk[(uint64_t)u * 4 + q] = make_uint4(node[4 * q], node[4 * q + 1], node[4 * q + 2], node[4 * q + 3]);
+}
 
 struct TraceArgs {
   const uint4* blob;
+  const uint4* walk;
+  const uint4* raw;
   uint32_t n_units;
-  uint32_t ordered;
   // several scenes in one launch: rays [item_begin[k], item_begin[k+1]) use
   // scenes[item_scene[k]]; n_items == 0 means every ray uses blob / meta
   const SceneView* scenes;
@@ -161,7 +187,7 @@ __device__ __forceinline__ void load_ray(const rt_ray* rays, uint32_t r, rtm::V3
 // whose tables are the launch arguments themselves.
 template <bool MULTI>
 __device__ __forceinline__ SceneView scene_of(const TraceArgs& a, uint32_t r) {
-  if (!MULTI || a.n_items == 0) return SceneView{a.blob, a.meta, a.route, a.n_units, a.ordered};
+  if (!MULTI || a.n_items == 0) return SceneView{a.blob, a.walk, a.raw, a.meta, a.route, a.n_units};
   uint32_t lo = 0, hi = a.n_items;  // last item with item_begin <= r
   while (hi - lo > 1) {
     const uint32_t mid = (lo + hi) >> 1;
@@ -171,10 +197,11 @@ __device__ __forceinline__ SceneView scene_of(const TraceArgs& a, uint32_t r) {
   const SceneView* s = a.scenes + __ldg(a.item_scene + lo);
   SceneView v;
   v.blob = reinterpret_cast<const uint4*>(__ldg(reinterpret_cast<const unsigned long long*>(&s->blob)));
+  v.walk = reinterpret_cast<const uint4*>(__ldg(reinterpret_cast<const unsigned long long*>(&s->walk)));
+  v.raw = reinterpret_cast<const uint4*>(__ldg(reinterpret_cast<const unsigned long long*>(&s->raw)));
   v.meta = reinterpret_cast<const uint2*>(__ldg(reinterpret_cast<const unsigned long long*>(&s->meta)));
   v.route = reinterpret_cast<const uint16_t*>(__ldg(reinterpret_cast<const unsigned long long*>(&s->route)));
   v.n_units = __ldg(&s->n_units);
-  v.ordered = __ldg(&s->ordered);
   return v;
 }
 
@@ -236,14 +263,14 @@ struct RayCtx {
 };
 
 __device__ __forceinline__ void enter_instance(const rtd::Instance& in, uint32_t unit, rtm::V3 O, rtm::V3 D, float tmin,
-                                               float tmax, bool ordered, RayCtx& c) {
+                                               float tmax, RayCtx& c) {
   const rtm::ObjRay r = rtm::make_transformed_ray(in.w2o, O, D, tmin, tmax);
   c.unit = unit;
   c.o = r.o;
   c.d = r.d;
   c.mult = r.mult;
   c.idir = rtm::calculate_idir(r.d);
-  c.fast = ordered && rtd::finite_ray(r.o, r.d, r.tmin, r.tmax);
+  c.fast = rtd::finite_ray(r.o, r.d, r.tmin, r.tmax);
 }
 
 // Flags of a walk, above the RT_RAY_* status bits of its hit record.
@@ -290,7 +317,7 @@ constexpr int kInternalShare = 11;
 
 template <class W, class Lookup>
 __device__ __forceinline__ void warp_turn(const TraceArgs& a, W& w, uint32_t r, bool& have, bool& ended, int spare,
-                                          Lookup&& lookup) {
+                                          const Lookup& lookup) {
   for (;;) {
     if (have && !w.pop(a)) {
       have = false;
@@ -306,6 +333,7 @@ __device__ __forceinline__ void warp_turn(const TraceArgs& a, W& w, uint32_t r, 
 }
 
 struct NoLookup {
+  static constexpr bool kSlots = false;
   __device__ __forceinline__ uint32_t operator()(uint32_t, const uint2*) const { return 0u; }
 };
 
@@ -453,7 +481,7 @@ struct PlainWalker {
     set_cold3(3, O);
     set_cold3(6, id);
     set_hit(0, 0, 0.0f);
-    if (v.ordered && rtd::finite_ray(O, D, tmin, tmax)) flags |= kRayWorldFast;
+    if (rtd::finite_ray(O, D, tmin, tmax)) flags |= kRayWorldFast;
     world();
     record(a, r, 0, rtf::TX_STRUCTURE);
     const uint4 h0 = __ldg(v.blob), h1 = __ldg(v.blob + 1);
@@ -480,53 +508,67 @@ struct PlainWalker {
     e = 0;
   }
 
-  // The entry's unit, and the node's first 64 bytes; false (and the ray
-  // stopped) when it lies outside the blob.
-  __device__ __forceinline__ bool load(uint32_t& unit, uint32_t units, rtd::Node64& q) {
+  // The entry's unit, and 64 bytes of its node in `from` (the walk nodes or
+  // the blob); false (and the ray stopped) when it lies outside the blob.
+  __device__ __forceinline__ bool load(const uint4* from, uint32_t& unit, uint32_t units, rtd::Node64& q) {
     unit = e >> 2;
     if (unit + units > v.n_units) {
       stop(RT_RAY_BAD_NODE);
       return false;
     }
-    rtd::load64(v.blob + (uint64_t)unit * 4, 0, q);
+    rtd::load64(from + (uint64_t)unit * 4, 0, q);
     return true;
   }
 
   template <class Lookup>
-  __device__ __forceinline__ void internal(const TraceArgs& a, uint32_t r, Lookup&&) {
+  __device__ __forceinline__ void internal(const TraceArgs& a, uint32_t r, const Lookup&) {
     uint32_t unit;
     rtd::Node64 nd;
-    if (!load(unit, 1, nd)) return;
+    if (!load(v.walk, unit, 1, nd)) return;
+    // the stack's top, read while the node is on its way: 40% of the visits
+    // end with it as the next entry (2M bounce rays 2.71 against 2.81 ms on a
+    // GB300; the treelet walk, with two stacks to choose from, gained nothing)
+    const uint32_t below = sp > 0 ? *slot(a, sp - 1) : 0u;
     const uint32_t level = e & kTop;
     record(a, r, unit, rtf::TX_INTERNAL);
     if (level && cx.unit != kNone) world();
     const float t0 = tmin * cx.mult, t1 = tmax * cx.mult, cull = min_thit * cx.mult;
-    const uint4* src = v.blob + (uint64_t)unit * 4;
-    const rtd::ChildHits ch = cx.fast ? rtd::test_children<true>(nd, src, unit, cx.o, cx.idir, t0, t1, cull)
-                                      : rtd::test_children<false>(nd, src, unit, cx.o, cx.idir, t0, t1, cull);
-    uint32_t c = ch.child_unit, nn = 0;
-#pragma unroll
-    for (int i = 0; i < 6; ++i) {
-      // the first hit internal child is visited next; other hit children are
-      // pushed (one predicated store, no branch per child)
-      const uint32_t info = ch.info_of(i);
-      const bool h = (ch.hit_mask >> i) & 1u, internal = (info >> 2) == rtf::CT_INTERNAL;
-      const uint32_t ce = (c << 2) | level | (internal ? 0u : kLeaf);
-      const bool take = h && internal && nn == 0, store = h && !take;
-      if (store) *slot(a, sp) = ce;
-      sp += store ? 1 : 0;
-      nn = take ? ce : nn;
-      c += info & 3u;
+    uint32_t hit = cx.fast && !(nd.w[5] & rtw::kExact)
+                       ? rtd::hit_children(nd, cx.o, cx.idir, t0, t1, cull)
+                       : rtd::hit_children_exact(v.raw + (uint64_t)unit * 4, cx.o, cx.idir, t0, t1, cull);
+    // the first hit internal child is visited next; the other hit children
+    // are pushed in order (1.2 hits a visit, so a loop over the bits is
+    // shorter than six predicated pushes: 2.81 against 2.92 ms for 2M bounce
+    // rays on a GB300)
+    auto entry_of = [&](int i) {
+      return ((nd.w[3] + ((nd.w[6] >> (4 * i)) & 15u)) << 2) | level | ((nd.w[5] >> (i + rtw::kLeafShift)) & kLeaf);
+    };
+    const uint32_t inner = hit & nd.w[5];
+    e = 0;
+    if (inner) {
+      const int i = __ffs(inner) - 1;
+      e = entry_of(i);
+      hit &= ~(1u << i);
     }
-    e = nn;
-    if (sp > CAP) stop(RT_RAY_STACK_OVERFLOW);
+    uint32_t last = 0;
+#pragma unroll 1
+    for (; hit; hit &= hit - 1u) {
+      last = entry_of(__ffs(hit) - 1);
+      *slot(a, sp++) = last;
+    }
+    const bool deep = sp > CAP;
+    if (!e && sp > 0) {
+      e = last ? last : below;
+      --sp;
+    }
+    if (deep) stop(RT_RAY_STACK_OVERFLOW);
   }
 
   template <class Lookup>
-  __device__ __forceinline__ void leaf(const TraceArgs& a, uint32_t r, Lookup&&) {
+  __device__ __forceinline__ void leaf(const TraceArgs& a, uint32_t r, const Lookup&) {
     uint32_t unit;
     rtd::Node64 q;
-    if (!load(unit, 1, q)) return;
+    if (!load(v.blob, unit, 1, q)) return;
     e = 0;
     record(a, r, unit, rtf::TX_LEAF_DESC);
     extra += kDescriptorExtra;
@@ -554,10 +596,10 @@ struct PlainWalker {
 
   // an instance leaf
   template <class Lookup>
-  __device__ __forceinline__ void entry(const TraceArgs& a, uint32_t r, Lookup&&) {
+  __device__ __forceinline__ void entry(const TraceArgs& a, uint32_t r, const Lookup&) {
     uint32_t unit;
     rtd::Node64 q;
-    if (!load(unit, 2, q)) return;
+    if (!load(v.blob, unit, 2, q)) return;
     record(a, r, unit, rtf::TX_INSTANCE_LEAF);
     extra += kInstanceExtra;
     rtd::Instance in;
@@ -566,7 +608,7 @@ struct PlainWalker {
     if ((hdr & 63) || hdr / 64 >= v.n_units) return stop(RT_RAY_BAD_NODE);
     const uint4 h0 = __ldg(v.blob + (hdr >> 4));
     const uint64_t broot = hdr + ((uint64_t)h0.x | ((uint64_t)h0.y << 32));
-    enter_instance(in, unit, world_o(), world_d(), tmin, tmax, v.ordered, cx);
+    enter_instance(in, unit, world_o(), world_d(), tmin, tmax, cx);
     if (sp < CAP) e = (uint32_t)(broot >> 6) << 2;
     else stop(RT_RAY_STACK_OVERFLOW);
     record(a, r, (uint32_t)(hdr >> 6), rtf::TX_STRUCTURE);
@@ -580,12 +622,13 @@ struct PlainWalker {
   }
 };
 
-// Four 256-thread CTAs per SM, 64 registers.  With one ray context in
+// Four 256-thread CTAs per SM, 64 registers: with one ray context in
 // registers and the rest in the stack's cold words, 2M bounce rays of the
-// 2M-triangle terrain take 3.23 ms on a GB300; five CTAs at 48 registers
-// spill and take 3.52 ms, three 3.34 ms.  (With both the world ray and the
-// object ray live the walk took 90 registers, and did best with all its
-// fields left in local memory at 48: 4.27 ms, bound by those loads.)
+// 2M-triangle terrain take 2.70 ms on a GB300 (56 registers 2.73, 72 2.80; when
+// the node test took more registers, 48 were 9% and 85 4% slower than 64).
+// With both the world ray and the object ray live the walk took 90 registers,
+// and did best with all its fields left in local memory at 48: 4.27 ms, bound
+// by those loads.
 constexpr int kPlainMinBlocks = 4;
 template <int CAP, bool MULTI, bool TRACED, bool SHORT = false>
 __global__ void __launch_bounds__(256, kPlainMinBlocks) trace_plain_kernel(TraceArgs a) {

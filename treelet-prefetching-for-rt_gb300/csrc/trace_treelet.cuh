@@ -191,7 +191,7 @@ struct Walker {
     const rtm::V3 id = rtm::calculate_idir(D);
     set_world(o, D, id);
     set_hit(0, 0, 0.0f);
-    if (v.ordered && rtd::finite_ray(o, D, tmin, tmax)) flags |= kRayWorldFast;
+    if (rtd::finite_ray(o, D, tmin, tmax)) flags |= kRayWorldFast;
     world();
     record(a, r, 0, rtf::TX_STRUCTURE);
     const uint4 h0 = __ldg(v.blob), h1 = __ldg(v.blob + 1);
@@ -242,7 +242,7 @@ struct Walker {
     set_hit(q3.x, q3.y, __uint_as_float(q3.z));
     clear();
     not_ = (int)q3.w;
-    if (v.ordered && rtd::finite_ray(o, D, tmin, tmax)) flags |= kRayWorldFast;
+    if (rtd::finite_ray(o, D, tmin, tmax)) flags |= kRayWorldFast;
     world();
   }
 
@@ -252,12 +252,12 @@ struct Walker {
 
   // Where a popped node is: its unit, and the address of its pinned record or
   // staged copy in shared memory (`lookup(unit, meta)`: a node staged in a
-  // warp slot), 0 when it is read from the blob.  Loads its first 64 bytes
-  // (or the whole pinned record of an instance leaf).  False, and the ray
-  // stopped, when it lies outside the blob.
+  // warp slot), 0 when it is read from `from` (the walk nodes or the blob).
+  // Loads its first 64 bytes (or the whole pinned record of an instance leaf).
+  // False, and the ray stopped, when it lies outside the blob.
   template <class Lookup>
-  __device__ __forceinline__ bool load(uint32_t code, uint32_t units, Lookup&& lookup, uint32_t& unit, uint32_t& saddr,
-                                       const uint4*& src, rtd::Node64& nd) {
+  __device__ __forceinline__ bool load(const uint4* from, uint32_t code, uint32_t units, const Lookup& lookup,
+                                       uint32_t& unit, uint32_t& saddr, rtd::Node64& nd) {
     saddr = 0;
     if (STAGED && (code & kEPin)) {
       saddr = pin_base + (code >> kEShift) * 16u;
@@ -275,7 +275,7 @@ struct Walker {
         else ++gmem_reads;
       }
     }
-    src = v.blob + (uint64_t)unit * 4;
+    const uint4* src = from + (uint64_t)unit * 4;
     if (STAGED) {
       // one generic load for lanes reading shared memory and lanes reading
       // global memory, instead of both load paths for a mixed warp
@@ -296,56 +296,48 @@ struct Walker {
 
   // internal node, top (:1758-1869) or bottom (:1954-2070)
   template <class Lookup>
-  __device__ __forceinline__ void internal(const TraceArgs& a, uint32_t r, Lookup&& lookup) {
+  __device__ __forceinline__ void internal(const TraceArgs& a, uint32_t r, const Lookup& lookup) {
     const uint32_t code = (uint32_t)e, inst = (uint32_t)(e >> 32), level = code & kTop;
-    const uint32_t rsh = popped - kPopCu;  // which route bit applies
-    uint32_t unit, saddr, rbits;
-    const uint4* src;
+    // which route bits apply
+    const uint32_t shift = popped == kPopCu ? rtw::kSameShift : rtw::kOtherShift;
+    const bool pinned = STAGED && (code & kEPin);
+    uint32_t unit, saddr;
     rtd::Node64 nd;
-    if (!load(code, 1, lookup, unit, saddr, src, nd)) return;
+    if (!load(v.walk, code, 1, lookup, unit, saddr, nd)) return;
+    if (STAGED && Lookup::kSlots && saddr && !pinned) {  // a warp slot holds the blob's bytes
+      uint32_t raw[16];
+#pragma unroll
+      for (int k = 0; k < 16; ++k) raw[k] = nd.w[k];
+      rtw::walk_node(raw, unit, __ldg(v.route + unit), nd.w);
+    }
     e = 0;
     popped = 0;
     if (level && cx.unit != kNone) world();
     record(a, r, unit, rtf::TX_INTERNAL);
-    uint32_t soff01 = 0, soff23 = 0, soff45 = 0;
-    if (STAGED && (code & kEPin)) {  // route bits in bytes 16..17, child records in the tail
-      const uint4 t = rtd::ld_shared_v4(saddr + rtp::IN_UNIT);
-      rbits = nd.w[rtp::IN_ROUTE / 4] & 0xffffu;
-      soff01 = t.y;
-      soff23 = t.z;
-      soff45 = t.w;
-    } else {
-      rbits = __ldg(v.route + unit);
-    }
     const float t0 = tmin * cx.mult, t1 = tmax * cx.mult, cull = min_thit * cx.mult;
-    const rtd::ChildHits ch = cx.fast ? rtd::test_children<true>(nd, src, unit, cx.o, cx.idir, t0, t1, cull)
-                                      : rtd::test_children<false>(nd, src, unit, cx.o, cx.idir, t0, t1, cull);
-    const uint32_t hit = ch.hit_mask;
-    const uint64_t info = ch.info;
-    const uint32_t same = rbits >> (rsh * kRouteOther);
-    uint32_t c = ch.child_unit;
-#pragma unroll
-    for (int i = 0; i < 6; ++i) {
-      const uint32_t ci = (uint32_t)(info >> (8 * i)) & 0x3fu;
-      if ((hit >> i) & 1u) {
-        const uint32_t lf = ((ci >> 2) != rtf::CT_INTERNAL) ? kLeaf : 0u;
-        const uint32_t sw = i < 2 ? soff01 : (i < 4 ? soff23 : soff45);
-        const uint32_t so = (sw >> (16 * (i & 1))) & 0xffffu;
-        const uint32_t cc = so ? ((so << kEShift) | kEPin | level | lf) : ((c << kEShift) | level | lf);
-        push((same >> i) & 1u, cc, inst);
-      }
-      c += ci & 3u;
+    uint32_t hit = cx.fast && !(nd.w[5] & rtw::kExact)
+                       ? rtd::hit_children(nd, cx.o, cx.idir, t0, t1, cull)
+                       : rtd::hit_children_exact(v.raw + (uint64_t)unit * 4, cx.o, cx.idir, t0, t1, cull);
+    // 1.2 hits a visit: a loop over the bits is shorter than six predicated
+    // pushes (2M any-hit rays 1.64 against 1.70 ms on a GB300)
+#pragma unroll 1
+    for (; hit; hit &= hit - 1u) {
+      const int i = __ffs(hit) - 1;
+      const uint32_t lf = (nd.w[5] >> (i + rtw::kLeafShift)) & kLeaf;
+      uint32_t so = 0;  // a pinned parent names its pinned children's records
+      if (pinned) so = rtd::ld_shared_u16(saddr + rtp::IN_CHILD_SOFF + 2u * i);
+      const uint32_t c = nd.w[3] + ((nd.w[6] >> (4 * i)) & 15u);
+      push((nd.w[5] >> (shift + i)) & 1u, (so ? (so << kEShift) | kEPin : c << kEShift) | level | lf, inst);
     }
     check_depth();
   }
 
   // primitive leaf (:2071-2196)
   template <class Lookup>
-  __device__ __forceinline__ void leaf(const TraceArgs& a, uint32_t r, Lookup&& lookup) {
+  __device__ __forceinline__ void leaf(const TraceArgs& a, uint32_t r, const Lookup& lookup) {
     uint32_t unit, saddr;
-    const uint4* src;
     rtd::Node64 q;
-    if (!load((uint32_t)e, 1, lookup, unit, saddr, src, q)) return;
+    if (!load(v.blob, (uint32_t)e, 1, lookup, unit, saddr, q)) return;
     e = 0;
     popped = 0;
     record(a, r, unit, rtf::TX_LEAF_DESC);
@@ -378,15 +370,14 @@ struct Walker {
   // (make_transformed_ray is deterministic, so recomputing gives the
   // reference's stored objectRay), and the node itself stays popped.
   template <class Lookup>
-  __device__ __forceinline__ void entry(const TraceArgs& a, uint32_t r, Lookup&& lookup) {
+  __device__ __forceinline__ void entry(const TraceArgs& a, uint32_t r, const Lookup& lookup) {
     const uint32_t code = (uint32_t)e;
     const bool top = code & kTop, pinned = STAGED && (code & kEPin);
     rtd::Instance in;
     rtd::Node64 nd;
     uint32_t unit = (uint32_t)(e >> 32), saddr = 0;
-    const uint4* src;
     if (top) {
-      if (!load(code, 2, lookup, unit, saddr, src, nd)) return;
+      if (!load(v.blob, code, 2, lookup, unit, saddr, nd)) return;
       if (pinned) {
 #pragma unroll
         for (int k = 0; k < 12; ++k) in.w2o.m[k / 3][k % 3] = __uint_as_float(nd.w[rtp::IL_W2O / 4 + k]);
@@ -396,7 +387,7 @@ struct Walker {
     } else {
       rtd::load_instance(v.blob + (uint64_t)unit * 4, 0, in);
     }
-    enter_instance(in, unit, world_o(), dir(), tmin, tmax, v.ordered, cx);
+    enter_instance(in, unit, world_o(), dir(), tmin, tmax, cx);
     if (!top) return;
     const uint32_t rsh = popped - kPopCu;
     e = 0;
@@ -433,7 +424,7 @@ struct Walker {
 
   // One node visit (the caller checks active() first).
   template <class Lookup>
-  __device__ __forceinline__ void step(const TraceArgs& a, uint32_t r, Lookup&& lookup) {
+  __device__ __forceinline__ void step(const TraceArgs& a, uint32_t r, const Lookup& lookup) {
     pop(a);
     if (at_entry()) {
       const bool top = (uint32_t)e & kTop;
@@ -454,15 +445,14 @@ struct Walker {
 };
 
 // The walker's stacks are a separate local array so that its fields stay in
-// registers (stacks inside it would leave every field in local memory); with
-// one ray context in registers (RayCtx) and the rarely used fields in the
-// cold words it fits four 256-thread CTAs per SM at 64 registers: 2M any-hit
-// rays 1.86 ms on a GB300 (three CTAs 1.93, five at 48 registers 2.15; with
-// the world ray and the object ray both held, 2.13).
-constexpr int kTreeletMinBlocks = 4;
+// registers (stacks inside it would leave every field in local memory).
+// 72 registers: seven 128-thread CTAs per SM.  GB300, ms for 1M traced bounce
+// rays / 2M any-hit rays: 2.36 / 1.64; 64 registers (eight CTAs) 2.44 / 1.64,
+// 56 2.51 / 1.67, 85 2.49 / 1.76.
+constexpr int kTreeletRegs = 72;
 
 template <int CAP, bool MULTI, bool TRACED>
-__global__ void __launch_bounds__(256, kTreeletMinBlocks) trace_treelet_kernel(TraceArgs a) {
+__global__ void __maxnreg__(kTreeletRegs) trace_treelet_kernel(TraceArgs a) {
   using W = Walker<CAP, false, MULTI, false, TRACED>;
   unsigned long long stack[W::kWords];
   W w;
@@ -526,6 +516,18 @@ __device__ __forceinline__ void bulk_copy_g2s(void* dst, const void* src, uint32
       "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
       "l"(src), "r"(bytes), "r"(smem_u32(bar))
       : "memory");
+}
+
+// A lookup of nodes staged in warp slots (Walker::load).
+template <class F>
+struct SlotLookup {
+  static constexpr bool kSlots = true;
+  F f;
+  __device__ __forceinline__ uint32_t operator()(uint32_t unit, const uint2* meta) const { return f(unit, meta); }
+};
+template <class F>
+__device__ __forceinline__ SlotLookup<F> slot_lookup(F f) {
+  return SlotLookup<F>{f};
 }
 
 constexpr int kMaxSlots = 8;  // slots per warp
@@ -601,7 +603,7 @@ __global__ void __launch_bounds__(kStagedMaxThreads, kStagedMinBlocks) trace_sta
   }
   __syncthreads();
   // the node's location is read only while some slot of the warp is resident
-  auto lookup = [&](uint32_t unit, const uint2* meta) -> uint32_t {
+  const auto lookup = slot_lookup([&](uint32_t unit, const uint2* meta) -> uint32_t {
     bool any = false;
     for (uint32_t s = 0; s < slots; ++s) any |= st.resident[s] != kNone;
     if (!any) return 0u;
@@ -611,7 +613,7 @@ __global__ void __launch_bounds__(kStagedMaxThreads, kStagedMinBlocks) trace_sta
     for (uint32_t s = 0; s < slots; ++s)
       if (st.resident[s] == d && u < st.units[s]) return slot_base + s * a.slot_bytes + u * 64u;
     return 0u;
-  };
+  });
   using W = Walker<CAP, true, false, false, TRACED>;  // staged launches trace one scene
   unsigned long long stack[W::kWords];
   W w;

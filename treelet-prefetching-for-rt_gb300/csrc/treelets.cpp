@@ -436,6 +436,7 @@ void build_pinned(const uint8_t* blob, uint64_t n_bytes, const Partition& p, con
     const uint64_t at = (uint64_t)soff[u] * 16, off = (uint64_t)u * 64;
     const uint8_t r = role[u];
     if (r == kTopInternal || r == kBotInternal) {
+      out.internal.push_back({(uint32_t)at, u});
       std::memcpy(out.bytes.data() + at, blob + off, 64);
       put<uint16_t>(out.bytes, at + rtp::IN_ROUTE, route[u]);
       put<uint32_t>(out.bytes, at + rtp::IN_UNIT, u);

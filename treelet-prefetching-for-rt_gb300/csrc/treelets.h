@@ -4,6 +4,7 @@
 #include <stdint.h>
 
 #include <string>
+#include <utility>
 #include <vector>
 
 namespace rtt {
@@ -57,6 +58,7 @@ struct Pinned {
   uint32_t root_soff = 0;      // record of the TLAS root node, 0 if it is not pinned
   uint32_t n_treelets = 0;
   uint32_t n_records = 0;
+  std::vector<std::pair<uint32_t, uint32_t>> internal;  // byte offset and unit of the internal nodes' records
 };
 
 // Dense treelet ids by estimated visit frequency: the TLAS treelet first,
