@@ -1,6 +1,8 @@
-"""The walks' box test against the oracle where its planes cannot be told
-apart by the direction's sign (a scene with quantized lower bounds above the
-upper ones) and for rays that are not finite."""
+"""The walks against the oracle where their kernels branch: the box test of a
+scene whose planes cannot be told apart by the direction's sign (quantized
+lower bounds above the upper ones) and of rays that are not finite, nodes used
+in two roles, and launches on both sides of the sizes at which a ray gets eight
+lanes, and a warp fewer rays."""
 import numpy as np
 import pytest
 
@@ -93,4 +95,47 @@ def test_unit_that_is_node_and_leaf(ctx):
     oh, ov, _ = orc.trace(b, rays, 0, None, capacity=CAP, want_visits=True)
     assert np.array_equal(hits["n_visits"], oh["n_visits"])
     assert_traces_equal(vis, ov, oh["n_visits"], "visits")
+    scene.close()
+
+
+@pytest.mark.parametrize("n", [1, 7, 33, 4864, 4865, 9729, 32768, 32769, 40001])
+def test_launch_sizes(ctx, n):
+    """Eight lanes a ray (one, two or four rays a warp) up to 32,768 rays, one
+    lane a ray above: hits and traces, any-hit rays among them, with a row
+    capacity that some rays exceed and rows that start off a 32-byte boundary."""
+    import torch
+
+    import treelet_rt as rt
+    from oracle import oracle as orc
+
+    blob = rt.Blob.gen(rt.SCENE_TERRAIN_INSTANCES, 2 * 40 * 40, 5)
+    scene = rt.Scene(ctx, blob)
+    scene.form_treelets(2048)
+    tl = orc.Treelets(blob.bytes(), 2048)
+    rays = rt.camera_rays(rt.default_camera(rt.SCENE_TERRAIN_INSTANCES), 250, 161, 1, 3, 1e-4, 1e30)
+    rays = np.ascontiguousarray(rays[np.random.default_rng(n).permutation(len(rays))[:n]])
+    flags = np.random.default_rng(n + 1).choice(np.array([0, 1, 5], np.uint32), size=n)
+    d_rays = torch.from_numpy(rays.view(np.uint8).copy()).cuda()
+    d_flags = torch.from_numpy(flags.view(np.uint8).copy()).cuda()
+    for mode, omode in ((rt.MODE_PLAIN, 0), (rt.MODE_TREELET, 1)):
+        for cap, skew in ((48, 0), (48, 1), (45, 0)):
+            d_hits = torch.zeros(n * 64, dtype=torch.uint8, device="cuda")
+            d_vis = torch.zeros(n * cap + skew, dtype=torch.int32, device="cuda")[skew:]
+            d_tl = torch.zeros(n * cap, dtype=torch.int32, device="cuda")
+            scene.trace(d_rays, d_hits, mode, flags=d_flags, visits=d_vis, treelets=d_tl, capacity=cap, n=n)
+            torch.cuda.synchronize()
+            hits = np.frombuffer(d_hits.cpu().numpy().tobytes(), rt.HIT_DTYPE)
+            oh, ov, ot = orc.trace(blob.bytes(), rays, omode, tl, flags=flags, capacity=cap, want_visits=True,
+                                   want_treelets=True, threads=8)
+            assert_hits_equal(hits, oh, f"hits, mode {mode}, {n} rays")
+            assert_traces_equal(d_vis.cpu().numpy().view(np.uint32).reshape(n, cap), ov, oh["n_visits"], "visits")
+            assert_traces_equal(d_tl.cpu().numpy().view(np.uint32).reshape(n, cap), ot, oh["n_visits"], "treelet ids")
+            node_bytes = scene.stats()["node_bytes"]
+        untraced = torch.zeros(n * 64, dtype=torch.uint8, device="cuda")
+        scene.trace(d_rays, untraced, mode, flags=d_flags, n=n)
+        torch.cuda.synchronize()
+        got = np.frombuffer(untraced.cpu().numpy().tobytes(), rt.HIT_DTYPE).copy()
+        got["status"] |= np.where(got["n_visits"] > cap, rt.RAY_TRACE_OVERFLOW, 0).astype(np.uint32)
+        assert_hits_equal(got, hits, f"untraced hits, mode {mode}, {n} rays")
+        assert scene.stats()["node_bytes"] == node_bytes
     scene.close()

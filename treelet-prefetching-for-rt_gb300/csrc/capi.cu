@@ -13,6 +13,7 @@
 #include "trace_kernels.cuh"
 #include "prefetch_kernels.cuh"
 #include "replay_kernel.cuh"
+#include "trace_group.cuh"
 #include "trace_queued.cuh"
 #include "trace_treelet.cuh"
 #include "treelets.h"
@@ -527,6 +528,43 @@ rt_status launch_queued(rtk::TraceArgs& a, const rt_tuning& t, uint32_t largest_
   return RT_OK;
 }
 
+// Rays up to which a launch walks each with eight lanes (trace_group.cuh)
+// instead of one.  GB300, us of a launch, eight lanes / one:
+//                                    32        1,024      4,096      16,384     30,976     49,152
+//   131K-tri terrain, bounce, plain  69 / 126  126 / 281  158 / 321  210 / 369  298 / 372  440 / 370
+//   the same, treelet order          79 / 210  124 / 315  153 / 340  259 / 380  360 / 444  495 / 417
+//   16K-tri cube, bounce, plain      28 / 55   44 / 96    49 / 108   66 / 115   94 / 117   105 / 120
+//   the same, treelet order          31 / 65   44 / 106   50 / 114   67 / 116   107 / 126  124 / 117
+// Longer launches have enough rays to fill the lanes, and eight lanes a ray
+// then cost more instructions than one.
+constexpr uint32_t kGroupRays = 1u << 15;
+// A warp holds one ray up to this many, then two, then four: 32 warps of 64-72
+// registers are resident on each of 152 SMs (twice as many rays a warp from
+// the start: 9,216 bounce rays 303 against 257 us).
+constexpr uint32_t kGroupRaysPerSplit = 152 * 32;
+
+bool group_launch(const rtk::TraceArgs& a, uint32_t mode, const rt_tuning& t) {
+  if (a.n_items || t.short_stack == 1) return false;
+  return (mode == RT_MODE_PLAIN || mode == RT_MODE_TREELET) && a.n <= kGroupRays;
+}
+
+rt_status launch_group(rtk::TraceArgs& a, bool treelet, uint32_t depth, cudaStream_t st) {
+  void (*kern)(rtk::TraceArgs, uint32_t, uint32_t);
+  if (treelet) kern = a.cap ? rtk::trace_group_kernel<true, true> : rtk::trace_group_kernel<true, false>;
+  else kern = a.cap ? rtk::trace_group_kernel<false, true> : rtk::trace_group_kernel<false, false>;
+  const uint32_t warps = rtk::kGroupThreads / 32;
+  uint32_t rpw = 1;
+  while (rpw < 4 && a.n > rpw * kGroupRaysPerSplit) rpw *= 2;
+  const size_t dyn = (size_t)warps * rpw * rtk::group_stack_bytes(treelet, depth);
+  RT_CUDA(ensure_dyn_smem((const void*)kern, dyn));
+  // CTAs for every ray, or as many as are resident at once
+  const uint32_t full = persistent_grid((const void*)kern, rtk::kGroupThreads, 0xffffffffu, dyn);
+  const uint32_t need = (a.n + warps * rpw - 1) / (warps * rpw);
+  kern<<<std::min(full, need), rtk::kGroupThreads, dyn, st>>>(a, depth, rpw);
+  RT_CUDA(cudaGetLastError());
+  return RT_OK;
+}
+
 // Zeroes the launch's queue (and its counters unless `keep` is set: chunks of
 // one call add up), then launches the kernel of `mode` with stack depth CAP.
 template <int CAP>
@@ -549,6 +587,7 @@ rt_status launch_cap(rtk::TraceArgs& a, uint32_t mode, const rt_tuning& t, uint3
   const uint32_t stage_warp_bytes = rtk::kTraceBufWarpBytes;
   a.tbuf_off = rtk::kNone;
   a.ss_off = rtk::kNone;
+  if (group_launch(a, mode, t)) return launch_group(a, mode == RT_MODE_TREELET, (uint32_t)CAP, st);
   if (mode == RT_MODE_PLAIN || mode == RT_MODE_TREELET) {
     const uint32_t bt = t.block_threads;
     size_t dyn = stage_rows ? (size_t)(bt / 32) * stage_warp_bytes + 128 : 0;

@@ -36,6 +36,14 @@ __device__ __forceinline__ uint32_t ld_shared_u16(uint32_t saddr) {
   return v;
 }
 
+// Brings the 32-byte sector of p into L1: a 4-byte asynchronous copy to a
+// scratch word of shared memory that nobody reads.  The thread must wait for
+// its copies (touch_l1_done) before it exits.
+__device__ __forceinline__ void touch_l1(uint32_t scratch, const void* p) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(scratch), "l"(p) : "memory");
+}
+__device__ __forceinline__ void touch_l1_done() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // One 32-byte read-only load from global memory (256-bit loads exist on
 // sm_100 and later, for the global state space only): a 64-byte node takes
 // two load instructions instead of four.  p must be 32-byte aligned; nodes are
@@ -153,16 +161,16 @@ __device__ __forceinline__ AxisBytes axis_bytes(const Node64& n, int k, float id
 // Returns bit i for a hit child i.
 //
 // hit_children_exact reads the blob's node and uses the reference's ternary
-// MIN/MAX macros in its order.
+// MIN/MAX macros in its order, for children [first, end).
 __device__ __forceinline__ uint32_t hit_children_exact(const uint4* raw, rtm::V3 o, rtm::V3 idir, float tmin,
-                                                       float tmax, float cull) {
+                                                       float tmax, float cull, uint32_t first = 0, uint32_t end = 6) {
   const uint8_t* b = reinterpret_cast<const uint8_t*>(raw);
   const float* org = reinterpret_cast<const float*>(raw);
   const float s[3] = {rtm::exp2_int((int)(int8_t)b[rtf::IN_EXP] - 8), rtm::exp2_int((int)(int8_t)b[rtf::IN_EXP + 1] - 8),
                       rtm::exp2_int((int)(int8_t)b[rtf::IN_EXP + 2] - 8)};
   uint32_t mask = 0;
 #pragma unroll 1
-  for (int i = 0; i < 6; ++i) {
+  for (uint32_t i = first; i < end; ++i) {
     if (!(b[rtf::IN_CHILD_INFO + i] & 3u)) continue;
     const uint8_t* q = b + rtf::IN_LO_X + i;
     const rtm::V3 lo = rtm::v3(__fmaf_rn((float)q[0], s[0], org[0]), __fmaf_rn((float)q[12], s[1], org[1]),
