@@ -249,6 +249,7 @@ __global__ void __launch_bounds__(kStagedMaxThreads, kStagedMinBlocks) trace_que
       __syncwarp();
     }
   }
+  rtd::touch_l1_done();
   // a copy still in flight after a wait that gave up must land before the
   // CTA's shared memory goes away
   if (!FINAL && lane == 0 && inflight) {

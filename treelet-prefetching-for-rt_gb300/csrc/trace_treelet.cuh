@@ -328,6 +328,7 @@ struct Walker {
       if (pinned) so = rtd::ld_shared_u16(saddr + rtp::IN_CHILD_SOFF + 2u * i);
       const uint32_t c = nd.w[3] + ((nd.w[6] >> (4 * i)) & 15u);
       push((nd.w[5] >> (shift + i)) & 1u, (so ? (so << kEShift) | kEPin : c << kEShift) | level | lf, inst);
+      if (!so) touch_node(v.walk, c);
     }
     check_depth();
   }
@@ -462,6 +463,7 @@ __global__ void __maxnreg__(kTreeletRegs) trace_treelet_kernel(TraceArgs a) {
   w.pin_root = 0;
   unsigned long long bytes = 0;
   run_persistent(a, w, bytes);
+  rtd::touch_l1_done();
   if (a.stats) add_warp_total64(a.stats + ST_NODE_BYTES, bytes);
 }
 
@@ -707,6 +709,7 @@ __global__ void __launch_bounds__(kStagedMaxThreads, kStagedMinBlocks) trace_sta
     if (SLOTS) warp_turn(a, w, r, have, ended, exhausted ? 33 : (int)a.refill, lookup);
     else warp_turn(a, w, r, have, ended, exhausted ? 33 : (int)a.refill, NoLookup());
   }
+  rtd::touch_l1_done();
   // copies still in flight must land before the CTA's shared memory goes away
   if (lane == 0 && st.pending_slot != kNone) {
     if (!mbar_wait(&st.bar, st.phase, kWaitTries)) atomicOr(a.status, kStatusTimeout);
