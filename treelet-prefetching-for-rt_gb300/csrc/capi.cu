@@ -1331,6 +1331,8 @@ extern "C" rt_status rt_unit_replay(rt_scene* s, const rt_hit* hits, const uint3
   off = align(off + sizeof(rtr::QueuedEntry) * (1ull << tab_log2));
   a.off_pq = off;
   off = align(off + 16ull * pq_cap);
+  a.off_pq_next = off;
+  off = align(off + 4ull * pq_cap);
   a.off_dead = off;
   off = align(off + pq_cap);
   a.off_meta = off;

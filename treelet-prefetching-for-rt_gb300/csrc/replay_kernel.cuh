@@ -23,11 +23,17 @@
 //             through the sector it filled or, once evicted, as the sector's
 //             most recently evicted one, so the classification needs these
 //             counts and no record list
-//   queued    open-addressing map: live queued prefetch requests per address
-//             (so a demand request scans the prefetch queue only when it can
-//             match)
-//   pq        the prefetch queue: a ring of (address, base) with tombstones
+//   queued    open-addressing map: the oldest and newest live queued prefetch
+//             request of each address (a demand request finds its queued
+//             copies there instead of scanning the queue)
+//   pq        the prefetch queue: a ring of (address, base) with tombstones;
+//             pq_next links the live requests of one address, oldest first
 //   metaret   metadata fills in flight
+//
+// What a unit does in a cycle in which nothing is sent, retired or decided is
+// known in advance, so the model steps from event to event: idle cycles are
+// skipped (more than half of all cycles), rounds are retired when the earliest
+// one is due, and a decision that can change nothing is only counted.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -64,8 +70,7 @@ struct SectorEntry {
 
 struct QueuedEntry {
   unsigned long long key;  // address + 1, 0 = empty
-  uint32_t count;
-  uint32_t pad;
+  uint32_t first, last;    // queue position + 1 of its oldest / newest live request, first 0 = none
 };
 
 struct Request {
@@ -102,6 +107,8 @@ struct UnitState {
   uint32_t mr_head, mr_tail;
   // histogram summary of the lanes' next treelets
   uint32_t n_keys, best, best_cnt, total, distinct, best_dense, best_nodes, second, hist_dirty;
+  uint32_t quiet;         // deciding again changes nothing until the histogram does
+  uint32_t next_retire;   // earliest cycle at which a round is retired or a warp leaves
   uint32_t full, next_gid, local;
 };
 
@@ -126,7 +133,7 @@ struct ReplayArgs {
   uint32_t sec_log2, queued_log2, pq_cap;
   uint32_t cycle_cap;     // per unit: the model's own bound on its cycles (or max_cycles)
   uint32_t lines_shared;  // 1: the L1 lines live in shared memory
-  unsigned long long off_lines, off_sec, off_queued, off_pq, off_dead, off_meta;
+  unsigned long long off_lines, off_sec, off_queued, off_pq, off_pq_next, off_dead, off_meta;
 };
 
 // Dynamic shared memory of one unit (one warp per CTA).
@@ -181,6 +188,7 @@ struct WUnit {
   SectorEntry* sec;
   QueuedEntry* queued;
   unsigned long long* pq;  // pairs (addr, base)
+  uint32_t* pq_next;       // queue position + 1 of the address's next live request, 0 = none
   uint8_t* dead;
   MetaReturn* metaret;
 
@@ -191,6 +199,7 @@ struct WUnit {
     sec = reinterpret_cast<SectorEntry*>(base + a.off_sec);
     queued = reinterpret_cast<QueuedEntry*>(base + a.off_queued);
     pq = reinterpret_cast<unsigned long long*>(base + a.off_pq);
+    pq_next = reinterpret_cast<uint32_t*>(base + a.off_pq_next);
     dead = base + a.off_dead;
     metaret = reinterpret_cast<MetaReturn*>(base + a.off_meta);
   }
@@ -377,10 +386,14 @@ struct WUnit {
     pq[2 * i] = addr;
     pq[2 * i + 1] = base;
     dead[i] = 0;
-    ++S.pq_tail;
+    pq_next[i] = 0;
+    const uint32_t at = ++S.pq_tail;  // position + 1
     ++S.pq_live;
     QueuedEntry* q = queued_entry(addr, true);
-    if (q) q->count++;
+    if (!q) return;
+    if (q->first) pq_next[(q->last - 1u) % a.pq_cap] = at;
+    else q->first = at;
+    q->last = at;
   }
 
   __device__ void pq_drop_dead() {  // lane 0
@@ -388,46 +401,37 @@ struct WUnit {
   }
 
   // Erases queued prefetches of `addr`, stepping past the entry that follows
-  // each erased one (shader.cc:4657-4668 as written).  Lanes read 32 queue
-  // entries at a time; lane 0 walks their live ones in order.
+  // each erased one (shader.cc:4657-4668 as written): of two matches with no
+  // live entry between them the second stays.  Follows the address's own
+  // requests (almost always one).
   __device__ void remove_queued(unsigned long long addr) {
-    uint32_t scan = 0;
-    QueuedEntry* q = nullptr;
     if (lane == 0) {
-      q = queued_entry(addr, false);
-      scan = (q && q->count) ? 1u : 0u;
-    }
-    scan = __shfl_sync(kFull, scan, 0);
-    if (!scan) return;
-    const uint32_t head = S.pq_head, tail = S.pq_tail;
-    bool skip = false;
-    for (uint32_t p0 = head; p0 != tail; p0 += (tail - p0 < 32u ? tail - p0 : 32u)) {
-      const uint32_t p = p0 + lane;
-      const bool in = p - head < tail - head;
-      const uint32_t i = p % a.pq_cap;
-      const bool live = in && !dead[i];
-      const bool match = live && pq[2 * i] == addr;
-      const uint32_t lm = __ballot_sync(kFull, live), mm = __ballot_sync(kFull, match);
-      __syncwarp();
-      if (lane == 0) {
-        for (uint32_t m = lm; m; m &= m - 1) {
-          const uint32_t b = __ffs(m) - 1;
-          if (skip) {
-            skip = false;
-            continue;
-          }
-          if ((mm >> b) & 1u) {
-            dead[(p0 + b) % a.pq_cap] = 1;
-            --S.pq_live;
-            q->count--;
-            S.st.prefetch_removed++;
-            skip = true;
+      QueuedEntry* q = queued_entry(addr, false);
+      uint32_t at = q ? q->first : 0u;
+      if (at) {
+        uint32_t kept = 0;  // last live request kept, position + 1
+        q->first = 0;
+        while (at) {
+          const uint32_t i = (at - 1u) % a.pq_cap, next = pq_next[i];
+          dead[i] = 1;
+          --S.pq_live;
+          S.st.prefetch_removed++;
+          uint32_t p = at;  // the entry stepped past: the next live one (positions at .. tail - 1)
+          while (p != S.pq_tail && dead[p % a.pq_cap]) ++p;
+          at = next;
+          if (next && p + 1u == next) {  // it is the address's next request: it stays
+            const uint32_t k = p % a.pq_cap;
+            if (kept) pq_next[(kept - 1u) % a.pq_cap] = next;
+            else q->first = next;
+            kept = next;
+            at = pq_next[k];
           }
         }
+        if (kept) pq_next[(kept - 1u) % a.pq_cap] = 0;
+        q->last = kept;
+        pq_drop_dead();
       }
-      __syncwarp();
     }
-    if (lane == 0) pq_drop_dead();
     __syncwarp();
   }
 
@@ -539,9 +543,11 @@ struct WUnit {
   // The RT unit's decision (shader.cc:3419-3683; as prefetch_decide_kernel).
   __device__ void decide() {
     if (S.hist_dirty) rebuild_histogram();
+    else if (S.quiet) return;
     const rt_prefetch_params& p = cfg.decision;
+    __syncwarp();
     if (lane == 0) {
-      S.st.decisions++;
+      bool quiet = true;
       const uint32_t best = S.best;
       bool submit = false;
       int num_nodes = 0;
@@ -567,6 +573,7 @@ struct WUnit {
       if (submit && best != kNone && bd != kNone && S.ds.last_prefetched != best && S.ds.last_prefetched_second != best) {
         const bool partial = p.heuristic == RT_PREFETCH_PARTIAL || p.heuristic == RT_PREFETCH_LATTER;
         const int num = partial ? num_nodes : n_nodes;
+        quiet = false;  // submitted, or waiting for room in the queue
         if ((unsigned long long)num + queue <= p.max_queue) {
           const int j0 = p.heuristic == RT_PREFETCH_LATTER ? n_nodes - num : 0;
           const int j1 = p.heuristic == RT_PREFETCH_LATTER ? n_nodes : num;
@@ -579,6 +586,10 @@ struct WUnit {
           S.st.treelets_prefetched++;
         }
       }
+      // the second treelet may follow as soon as the queue is empty
+      if (p.second_prefetch && S.total > 0 && S.distinct > 1 && S.second != kNone &&
+          S.ds.last_prefetched_second != S.second)
+        quiet = false;
       if (p.second_prefetch && queue == 0 && S.total > 0 && S.distinct > 1 && S.ds.last_prefetched == best &&
           best != kNone) {
         // the first maximum among treelets other than the last prefetched one,
@@ -593,6 +604,7 @@ struct WUnit {
           S.st.treelets_prefetched++;
         }
       }
+      S.quiet = quiet ? 1u : 0u;
     }
     __syncwarp();
   }
@@ -718,6 +730,7 @@ struct WUnit {
       if (S.ch_head == S.ch_tail) {
         w.all_sent = 1;
         w.ready += w.ilat;
+        S.next_retire = min(S.next_retire, w.ready);
         S.serving = kNone;
       }
     }
@@ -795,6 +808,17 @@ struct WUnit {
       }
       __syncwarp();
     }
+    // when to look again: the earliest round due, or the next cycle for a
+    // warp that came in without a transaction
+    uint32_t due = 0xFFFFFFFFu;
+    if (lane < S.n_res) {
+      const WarpSlot& w = sh.warps[S.order[lane]];
+      if (w.in_flight && w.all_sent) due = w.ready;
+      else if (!w.in_flight && w.live == 0) due = t + 1;
+    }
+    due = __reduce_min_sync(kFull, due);
+    if (lane == 0) S.next_retire = due;
+    __syncwarp();
   }
 
   __device__ void run(uint32_t u) {
@@ -814,6 +838,8 @@ struct WUnit {
       S.best_cnt = S.total = S.distinct = S.best_nodes = 0;
       S.best_dense = S.second = kNone;
       S.hist_dirty = 1;
+      S.quiet = 0;
+      S.next_retire = 0;
       S.full = 0;
       S.next_gid = u;
       S.local = 0;
@@ -823,8 +849,11 @@ struct WUnit {
       for (uint32_t i = lane; i < cfg.l1_sets * cfg.l1_ways; i += 32) lines[i].flags = 0;
     __syncwarp();
     const uint32_t tcap = a.cycle_cap;
+    const bool treelets = cfg.prefetcher == RT_UNIT_PF_TREELET;
+    unsigned long long decisions = 0;
+    uint32_t next_decide = 0;  // the next multiple of prefetch_delay
     for (uint32_t t = 0;; ++t) {
-      retire_and_admit(t, n_warps);
+      if (t >= S.next_retire) retire_and_admit(t, n_warps);
       if (S.n_res == 0) {
         if (lane == 0) S.st.cycles = t;
         break;
@@ -836,13 +865,19 @@ struct WUnit {
         }
         break;
       }
-      if (lane == 0)
-        while (S.mr_head != S.mr_tail && metaret[S.mr_head % kMetaRing].t <= t) {
-          S.most_recent_metadata = metaret[S.mr_head % kMetaRing].base;
-          ++S.mr_head;
-        }
-      __syncwarp();
-      if (cfg.prefetcher == RT_UNIT_PF_TREELET && t % cfg.prefetch_delay == 0) decide();
+      if (cfg.load_metadata) {
+        if (lane == 0)
+          while (S.mr_head != S.mr_tail && metaret[S.mr_head % kMetaRing].t <= t) {
+            S.most_recent_metadata = metaret[S.mr_head % kMetaRing].base;
+            ++S.mr_head;
+          }
+        __syncwarp();
+      }
+      if (treelets && t == next_decide) {
+        decide();
+        ++decisions;
+        next_decide += cfg.prefetch_delay;
+      }
       if (S.ch_head != S.ch_tail) {
         send_demand(t);
         continue;
@@ -853,8 +888,8 @@ struct WUnit {
         send_demand(t);
         continue;
       }
+      uint32_t go = 0;
       if (cfg.prefetcher != RT_UNIT_PF_NONE && S.pq_live > 0) {
-        uint32_t go = 0;
         unsigned long long addr = 0, base = 0;
         if (lane == 0 && prefetch_issuable()) {
           const uint32_t i = S.pq_head % a.pq_cap;
@@ -863,7 +898,7 @@ struct WUnit {
           dead[i] = 1;
           --S.pq_live;
           QueuedEntry* q = queued_entry(addr, false);
-          if (q) q->count--;
+          if (q) q->first = pq_next[i];  // the queue's head is its address's oldest request
           pq_drop_dead();
           go = 1;
         }
@@ -875,7 +910,24 @@ struct WUnit {
           prefetch(addr, base, t);
         }
       }
+      if (go) continue;
+      // An idle cycle: every resident warp waits for its round (schedule()
+      // found none ready and no request is left to send).  Until the earliest
+      // round is due nothing happens but decisions that change nothing and
+      // metadata returns, which matter to a queued request that waits for one.
+      uint32_t until = min(S.next_retire, tcap);
+      if (treelets && (S.hist_dirty || !S.quiet)) until = min(until, next_decide);
+      if (S.pq_live > 0 && S.mr_head != S.mr_tail) until = min(until, metaret[S.mr_head % kMetaRing].t);
+      if (until > t + 1) {
+        if (treelets && next_decide < until) {
+          const uint32_t k = (until - next_decide + cfg.prefetch_delay - 1u) / cfg.prefetch_delay;
+          decisions += k;
+          next_decide += k * cfg.prefetch_delay;
+        }
+        t = until - 1u;
+      }
     }
+    if (lane == 0) S.st.decisions = decisions;
     __syncwarp();
     // final tally (gpu-sim.cc:1749-1790): lanes take sector-map slices
     const uint32_t n_sec = 1u << a.sec_log2;
