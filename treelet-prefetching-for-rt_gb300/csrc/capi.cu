@@ -150,6 +150,7 @@ struct rt_scene {
   uint32_t* d_members = nullptr;
   uint32_t* d_hint = nullptr;  // staged-mode predictions (8 per treelet) or null
   uint32_t slot_bytes = 0;
+  bool members_apart = false;   // no 128-byte member covers the unit of another node
   std::vector<uint16_t> route;  // routing bits of the treelet-ordered walk
   bool offset_quirk = false;    // walk as the reference does with a nonzero device_offset
   uint16_t* d_route = nullptr;
@@ -853,6 +854,11 @@ rt_status rt_treelets_form(rt_scene* s, uint32_t max_treelet_bytes, rt_treelet_i
     RT_CUDA(cudaMemcpy(s->d_members, p.members.data(), sizeof(uint32_t) * p.members.size(), cudaMemcpyHostToDevice));
   s->slot_bytes = (p.largest_image + 127u) & ~127u;
   s->part = std::move(p);
+  s->members_apart = true;
+  for (size_t j = 0; j < s->part.members.size() && s->members_apart; ++j)
+    for (uint32_t k = 1; k < (s->part.member_bytes[j] + 63u) / 64u; ++k)
+      s->members_apart &= s->part.members[j] + k >= s->n_units ||
+                          s->part.node_root[s->part.members[j] + k] == rtt::kNoTreelet;
   st = dalloc(&s->d_route, sizeof(uint16_t) * (s->blob_bytes / 64));
   if (st != RT_OK) {
     free_treelets(s);
@@ -1361,6 +1367,7 @@ extern "C" rt_status rt_unit_replay(rt_scene* s, const rt_hit* hits, const uint3
   a.members = s->d_members;
   a.member_bytes = s->d_member_bytes;
   a.n_treelets = (uint32_t)n_treelets;
+  a.members_apart = s->members_apart;
   a.meta_base = meta_base;
   a.meta_size = meta_size;
   a.scratch = scratch;

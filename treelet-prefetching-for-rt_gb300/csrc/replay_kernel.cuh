@@ -17,8 +17,8 @@
 //   lines     sectored L1 (128 B lines, 4 x 32 B sectors, LRU stamps), when
 //             they do not fit in shared memory
 //   sectors   open-addressing map keyed by 32 B sector: prefetch records of
-//             the sector still unclassified, per-class counts of classified
-//             ones, and the state of the sector's most recently evicted
+//             the sector still unclassified, whether one has been
+//             classified, and the state of the sector's most recently evicted
 //             prefetch record.  A prefetch record is only ever classified
 //             through the sector it filled or, once evicted, as the sector's
 //             most recently evicted one, so the classification needs these
@@ -39,6 +39,7 @@
 #include <stdint.h>
 
 #include "../../include/treelet_rt.h"
+#include "device_nodes.cuh"
 #include "format.h"
 
 namespace rtr {
@@ -47,7 +48,7 @@ constexpr uint32_t kNone = 0xFFFFFFFFu;
 constexpr uint32_t kFull = 0xFFFFFFFFu;
 constexpr uint32_t kChunkCap = 32 * 4;     // a round: 32 lanes x 128 B
 constexpr uint32_t kMaxResident = 16;
-constexpr uint32_t kMaxKeys = 32 * kMaxResident;
+constexpr uint32_t kHistLog2 = 10, kHistSize = 1u << kHistLog2;  // at most 512 roots at a time
 constexpr uint32_t kMetaRing = 4096;       // > miss latency: metadata fills in flight
 constexpr uint32_t kStrideEntries = 33;    // a stride table grows while it has <= 32 entries
 constexpr uint32_t kTimeCap = 0xF0000000u; // cycles are 32-bit
@@ -64,8 +65,8 @@ struct Line {
 struct SectorEntry {
   unsigned long long key;  // sector + 1, 0 = empty
   uint32_t n_unclassified;
-  uint32_t count[4];       // RT_PF_TOO_LATE .. RT_PF_TOO_EARLY
-  uint32_t evicted;        // 0 none, 1 most recent evicted record unclassified, 2 classified
+  uint16_t classified;     // 1 once a record of the sector has been classified
+  uint16_t evicted;        // 0 none, 1 most recent evicted record unclassified, 2 classified
 };
 
 struct QueuedEntry {
@@ -82,6 +83,7 @@ struct WarpSlot {
   uint32_t gid, wid, in_flight, all_sent, ready, ilat, issued;
   uint32_t live;  // lanes with transactions left
   uint32_t ptr[32], end[32];
+  uint32_t next[32], root[32];  // each lane's next transaction (visit entry) and its treelet root
 };
 
 struct StrideTable {
@@ -98,7 +100,6 @@ struct MetaReturn {
 
 // The unit's scalar state (shared memory; lane 0 writes, __syncwarp, all read).
 struct UnitState {
-  rt_unit_stats st;
   unsigned long long most_recent_metadata;
   rt_prefetch_state ds;
   uint32_t pq_head, pq_tail, pq_live;
@@ -106,7 +107,7 @@ struct UnitState {
   uint32_t order[kMaxResident], n_res, free_mask;
   uint32_t mr_head, mr_tail;
   // histogram summary of the lanes' next treelets
-  uint32_t n_keys, best, best_cnt, total, distinct, best_dense, best_nodes, second, hist_dirty;
+  uint32_t hist_used, best, best_cnt, total, distinct, best_of, best_dense, best_nodes, second, hist_dirty;
   uint32_t quiet;         // deciding again changes nothing until the histogram does
   uint32_t next_retire;   // earliest cycle at which a round is retired or a warp leaves
   uint32_t full, next_gid, local;
@@ -133,6 +134,7 @@ struct ReplayArgs {
   uint32_t sec_log2, queued_log2, pq_cap;
   uint32_t cycle_cap;     // per unit: the model's own bound on its cycles (or max_cycles)
   uint32_t lines_shared;  // 1: the L1 lines live in shared memory
+  uint32_t members_apart; // no two members of a treelet share an address
   unsigned long long off_lines, off_sec, off_queued, off_pq, off_pq_next, off_dead, off_meta;
 };
 
@@ -141,12 +143,17 @@ struct UnitShared {
   UnitState s;
   WarpSlot warps[kMaxResident];
   Request chunk[kChunkCap];
-  uint32_t keys[kMaxKeys];
+  uint32_t hist_key[kHistSize], hist_cnt[kHistSize];
+  uint32_t scratch;  // touch_l1's word
   StrideTable stride[kMaxResident];
 };
 
-__device__ __forceinline__ uint32_t hash_slot(unsigned long long key, uint32_t log2) {
-  return (uint32_t)((key * 0x9E3779B97F4A7C15ull) >> (64 - log2));
+// Table slot of a 32-byte sector: the 16 sectors of 512 bytes get neighbouring
+// slots, so that the requests of one node, or of nodes next to each other,
+// find their entries in a few cache lines (the tables of all units together are
+// larger than L2, and a probe of its own per sector was a DRAM access).
+__device__ __forceinline__ uint32_t hash_slot(unsigned long long sector, uint32_t log2) {
+  return ((uint32_t)(((sector >> 4) * 0x9E3779B97F4A7C15ull) >> (68 - log2)) << 4) | (uint32_t)(sector & 15u);
 }
 
 __device__ __forceinline__ uint32_t tx_size(uint32_t type) { return type == 2 ? 128u : (type == 3 ? 8u : 64u); }
@@ -191,6 +198,10 @@ struct WUnit {
   uint32_t* pq_next;       // queue position + 1 of the address's next live request, 0 = none
   uint8_t* dead;
   MetaReturn* metaret;
+  // lane 0's: the counters, and the records not yet classified, in all and in
+  // sectors that have a classified one
+  rt_unit_stats st;
+  unsigned long long uncl, uncl_accessed;
 
   __device__ WUnit(const ReplayArgs& args, uint32_t u, UnitShared& shm, Line* smem_lines)
       : a(args), cfg(args.cfg), lane(threadIdx.x & 31u), sh(shm), S(shm.s) {
@@ -202,13 +213,15 @@ struct WUnit {
     pq_next = reinterpret_cast<uint32_t*>(base + a.off_pq_next);
     dead = base + a.off_dead;
     metaret = reinterpret_cast<MetaReturn*>(base + a.off_meta);
+    st = rt_unit_stats{};
+    uncl = uncl_accessed = 0;
   }
 
   // ------------------------------------------------------------ tables (lane 0)
   __device__ SectorEntry* sector_entry(unsigned long long sector, bool create) {
     const unsigned long long key = sector + 1;
     const uint32_t mask = (1u << a.sec_log2) - 1u;
-    uint32_t i = hash_slot(key, a.sec_log2);
+    uint32_t i = hash_slot(sector, a.sec_log2);
     for (uint32_t probe = 0; probe <= mask; ++probe, i = (i + 1) & mask) {
       SectorEntry& e = sec[i];
       if (e.key == key) return &e;
@@ -225,7 +238,7 @@ struct WUnit {
   __device__ QueuedEntry* queued_entry(unsigned long long addr, bool create) {
     const unsigned long long key = addr + 1;
     const uint32_t mask = (1u << a.queued_log2) - 1u;
-    uint32_t i = hash_slot(key, a.queued_log2);
+    uint32_t i = hash_slot(addr >> 5, a.queued_log2);
     for (uint32_t probe = 0; probe <= mask; ++probe, i = (i + 1) & mask) {
       QueuedEntry& e = queued[i];
       if (e.key == key) return &e;
@@ -239,11 +252,32 @@ struct WUnit {
     return nullptr;
   }
 
+  // Starts the table entries of a request on their way to L1.
+  __device__ void touch_tables(unsigned long long addr) {
+    const uint32_t word = (uint32_t)__cvta_generic_to_shared(&sh.scratch);
+    rtd::touch_l1(word, queued + hash_slot(addr >> 5, a.queued_log2));
+    rtd::touch_l1(word, sec + hash_slot(addr >> 5, a.sec_log2));
+  }
+
+  // One of the sector's records is classified.  The final tally
+  // (gpu-sim.cc:1749-1790) needs, besides the classes' counts, the
+  // unclassified records of the sectors with a classified one and of the
+  // others; both are kept here (scanning the table at the end took a fifth of
+  // a replay).
+  __device__ void classify(SectorEntry* e, uint32_t cls) {  // lane 0
+    e->n_unclassified--;
+    --uncl;
+    st.effectiveness[cls]++;
+    if (e->classified) {
+      --uncl_accessed;
+    } else {
+      e->classified = 1;
+      uncl_accessed += e->n_unclassified;
+    }
+  }
   __device__ void classify(unsigned long long sector, uint32_t cls) {
     SectorEntry* e = sector_entry(sector, false);
-    if (!e) return;
-    e->n_unclassified--;
-    e->count[cls]++;
+    if (e) classify(e, cls);
   }
 
   // ------------------------------------------------------------ cache (warp)
@@ -295,20 +329,20 @@ struct WUnit {
     uint32_t ret = 0;
     if (lane == 0) {
       const unsigned long long sector = addr >> 5;
-      S.st.demand_requests++;
+      st.demand_requests++;
       if (sector_valid) {
         Line* l = set + way;
         l->lru = t;
         const bool pf_uncl = (l->flags >> (4 + k)) & (l->flags >> (8 + k)) & 1u;
         if (l->ready[k] <= t) {
-          S.st.demand_hits++;
+          st.demand_hits++;
           if (pf_uncl) {
             classify(sector, RT_PF_TIMELY);
             l->flags &= ~(1u << (8 + k));
           }
           ret = t + cfg.hit_latency;
         } else {
-          S.st.demand_hit_reserved++;
+          st.demand_hit_reserved++;
           if (pf_uncl) {
             classify(sector, RT_PF_LATE);
             l->flags &= ~(1u << (8 + k));
@@ -316,11 +350,10 @@ struct WUnit {
           ret = l->ready[k];
         }
       } else {
-        S.st.demand_misses++;
+        st.demand_misses++;
         SectorEntry* e = sector_entry(sector, false);
         if (e && e->evicted == 1u) {
-          e->n_unclassified--;
-          e->count[RT_PF_TOO_EARLY]++;
+          classify(e, RT_PF_TOO_EARLY);
           e->evicted = 2u;
         }
         Line* l = way >= 0 ? set + way : install(block, vic, t);
@@ -346,18 +379,22 @@ struct WUnit {
     const bool sector_valid = way >= 0 && ((set[way].flags >> k) & 1u);
     const int vic = (way < 0) ? victim_way(block) : -1;
     if (lane == 0) {
-      S.st.prefetch_issued++;
+      st.prefetch_issued++;
       SectorEntry* e = sector_entry(addr >> 5, true);
-      if (e) e->n_unclassified++;
+      if (e) {
+        e->n_unclassified++;
+        ++uncl;
+        uncl_accessed += e->classified;
+      }
       if (sector_valid) {
         Line* l = set + way;
         l->lru = t;
         // a fresh record is unclassified, so the TOO_LATE rule of
         // gpu-cache.cc:2101-2116 never applies to it
-        if (l->ready[k] <= t) S.st.prefetch_present++;
-        else S.st.prefetch_merged++;
+        if (l->ready[k] <= t) st.prefetch_present++;
+        else st.prefetch_merged++;
       } else {
-        S.st.prefetch_filled++;
+        st.prefetch_filled++;
         Line* l = way >= 0 ? set + way : install(block, vic, t);
         l->lru = t;
         l->flags |= (1u << k) | (1u << (4 + k)) | (1u << (8 + k));
@@ -377,7 +414,7 @@ struct WUnit {
 
   // ------------------------------------------------------------ prefetch queue
   __device__ void pq_push(unsigned long long addr, unsigned long long base) {  // lane 0
-    S.st.prefetch_queued++;
+    st.prefetch_queued++;
     if (S.pq_tail - S.pq_head >= a.pq_cap) {  // ring full (live + erased entries)
       S.full = 1;
       return;
@@ -415,7 +452,7 @@ struct WUnit {
           const uint32_t i = (at - 1u) % a.pq_cap, next = pq_next[i];
           dead[i] = 1;
           --S.pq_live;
-          S.st.prefetch_removed++;
+          st.prefetch_removed++;
           uint32_t p = at;  // the entry stepped past: the next live one (positions at .. tail - 1)
           while (p != S.pq_tail && dead[p % a.pq_cap]) ++p;
           at = next;
@@ -452,7 +489,7 @@ struct WUnit {
       const unsigned long long ma = a.meta_base + (unsigned long long)(d == kNone ? 0u : d) * a.meta_size;
       for (unsigned long long i = 0; i < a.meta_size / 32; ++i) {
         pq_push(ma + i * 32, ma);
-        S.st.metadata_queued++;
+        st.metadata_queued++;
       }
     }
     const unsigned long long addr = (unsigned long long)m * 64;
@@ -460,81 +497,159 @@ struct WUnit {
     for (uint32_t i = 0; i < (b + 31) / 32; ++i) pq_push(addr + 32ull * i, addr);
   }
 
-  // ------------------------------------------------------------ decision
-  __device__ uint32_t lane_root(const WarpSlot& w, uint32_t l) const {
-    const uint32_t r = w.gid * 32 + l;
-    const uint32_t unit = __ldg(a.visits + (unsigned long long)r * a.capacity + w.ptr[l]) >> 3;
-    return unit < a.n_units ? __ldg(&a.meta[unit].x) : kNone;
-  }
-
-  // Run summary of the sorted keys, skipping `skip_key`: (count << 32 | ~key)
-  // of the first maximum in ascending key order, and the number of runs.
-  __device__ unsigned long long best_run(uint32_t skip_key, uint32_t* runs) const {
-    const uint32_t n = S.n_keys;
-    unsigned long long best = 0;
-    uint32_t nr = 0;
-    for (uint32_t i = lane; i < n; i += 32) {
-      const uint32_t k = sh.keys[i];
-      if (i > 0 && sh.keys[i - 1] == k) continue;
-      ++nr;
-      if (k == skip_key) continue;
-      uint32_t lo = i + 1, hi = n;  // end of the run
-      while (lo < hi) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (sh.keys[mid] == k) lo = mid + 1;
-        else hi = mid;
+  // Queues members [j0, j1) of the member lists, each as its 32-byte requests,
+  // one member per lane.  Their addresses are distinct (a.members_apart), so
+  // the lanes' table entries are too and only their keys need a
+  // compare-and-swap.  False when the ring has no room for all of them.
+  __device__ bool push_members(unsigned long long j0, unsigned long long j1) {
+    for (unsigned long long jb = j0; jb < j1; jb += 32) {
+      const unsigned long long j = jb + lane;
+      const bool in = j < j1;
+      const unsigned long long addr = in ? (unsigned long long)__ldg(a.members + j) * 64 : 0ull;
+      const uint32_t n = in ? (__ldg(a.member_bytes + j) + 31u) / 32u : 0u;
+      uint32_t incl = n;
+#pragma unroll
+      for (int s = 1; s < 32; s <<= 1) {
+        const uint32_t o = __shfl_up_sync(kFull, incl, s);
+        if ((int)lane >= s) incl += o;
       }
-      const unsigned long long v = ((unsigned long long)(lo - i) << 32) | (unsigned long long)(~k);
-      best = v > best ? v : best;
+      const uint32_t total = __shfl_sync(kFull, incl, 31);
+      const uint32_t tail = S.pq_tail;
+      if (tail - S.pq_head + total > a.pq_cap) return jb == j0 ? false : push_rest(jb, j1);
+      for (uint32_t i = 0; i < n; ++i) {
+        const unsigned long long at_addr = addr + 32ull * i;
+        const uint32_t p = tail + incl - n + i, k = p % a.pq_cap;
+        pq[2 * k] = at_addr;
+        pq[2 * k + 1] = addr;
+        dead[k] = 0;
+        pq_next[k] = 0;
+        touch_tables(at_addr);
+        QueuedEntry* q = queued_claim(at_addr);
+        if (!q) continue;
+        if (q->first) pq_next[(q->last - 1u) % a.pq_cap] = p + 1u;
+        else q->first = p + 1u;
+        q->last = p + 1u;
+      }
+      __syncwarp();
+      if (lane == 0) {
+        S.pq_tail = tail + total;
+        S.pq_live += total;
+        st.prefetch_queued += total;
+      }
+      __syncwarp();
     }
-    if (runs) *runs = warp_sum(nr);
-    return warp_max64(best);
+    return true;
+  }
+  // The rest of a list that no longer fits the ring: one request at a time.
+  __device__ bool push_rest(unsigned long long j0, unsigned long long j1) {
+    if (lane == 0)
+      for (unsigned long long j = j0; j < j1; ++j) push_member(j, false);
+    __syncwarp();
+    return true;
   }
 
-  __device__ void rebuild_histogram() {
-    uint32_t n = 0;
+  // queued_entry(addr, true) for lanes that claim entries at the same time.
+  __device__ QueuedEntry* queued_claim(unsigned long long addr) {
+    const unsigned long long key = addr + 1;
+    const uint32_t mask = (1u << a.queued_log2) - 1u;
+    uint32_t i = hash_slot(addr >> 5, a.queued_log2);
+    for (uint32_t probe = 0; probe <= mask; ++probe, i = (i + 1) & mask) {
+      unsigned long long k = *reinterpret_cast<volatile unsigned long long*>(&queued[i].key);
+      if (k == 0) k = atomicCAS(&queued[i].key, 0ull, key);
+      if (k == 0 || k == key) return &queued[i];
+    }
+    S.full = 1;
+    return nullptr;
+  }
+
+  // ------------------------------------------------------------ decision
+  // Reads the calling lane's next transaction of a warp (when it has one).
+  __device__ void fetch_next(WarpSlot& w) const {
+    if (w.ptr[lane] >= w.end[lane]) return;
+    const uint32_t v = __ldg(a.visits + (unsigned long long)(w.gid * 32 + lane) * a.capacity + w.ptr[lane]);
+    w.next[lane] = v;
+    w.root[lane] = (v >> 3) < a.n_units ? __ldg(&a.meta[v >> 3].x) : kNone;
+  }
+
+  // ------------------------------------------------------------ histogram
+  // Lanes per treelet root over the resident warps' next transactions, kept
+  // up to date as rounds retire and warps come in: an open-addressing table
+  // of roots and counts (a root whose count is 0 keeps its slot until the
+  // table is built anew).  Sorting up to 512 roots after every round was a
+  // third of the replay's instructions.
+  __device__ uint32_t hist_slot(uint32_t root) const {
+    uint32_t i = (root * 0x9E3779B1u) >> (32 - kHistLog2);
+    for (;; i = (i + 1) & (kHistSize - 1)) {
+      const uint32_t k = sh.hist_key[i];
+      if (k == root) return i;
+      if (k == kNone && atomicCAS(&sh.hist_key[i], kNone, root) == kNone) {
+        atomicAdd(&S.hist_used, 1u);
+        return i;
+      }
+      if (sh.hist_key[i] == root) return i;
+    }
+  }
+  // Adds 1 (or -1) per calling lane with `on`; all 32 lanes call.
+  __device__ void hist_add(uint32_t root, bool on, uint32_t one) {
+    const uint32_t key = on ? root : kNone;
+    const uint32_t peers = __match_any_sync(kFull, key);
+    if (key != kNone && (uint32_t)(__ffs(peers) - 1) == lane)
+      atomicAdd(&sh.hist_cnt[hist_slot(key)], one * (uint32_t)__popc(peers));
+    __syncwarp();
+  }
+  __device__ bool has_next(const WarpSlot& w) const { return w.ptr[lane] < w.end[lane]; }
+  // Room for 32 new roots, or the table built anew from the resident warps'
+  // lanes (true then: they are all counted).
+  __device__ bool hist_renew() {
+    if (S.hist_used + 32u <= kHistSize * 3 / 4) return false;
+    __syncwarp();
+    hist_clear();
     for (uint32_t o = 0; o < S.n_res; ++o) {
       const WarpSlot& w = sh.warps[S.order[o]];
-      const uint32_t k = (w.ptr[lane] < w.end[lane]) ? lane_root(w, lane) : kNone;
-      const uint32_t b = __ballot_sync(kFull, k != kNone);
-      if (k != kNone) sh.keys[n + __popc(b & lanemask_lt())] = k;
-      n += __popc(b);
+      hist_add(w.root[lane], has_next(w), 1u);
     }
-    uint32_t P = 1;
-    while (P < n) P <<= 1;
-    for (uint32_t i = n + lane; i < P; i += 32) sh.keys[i] = kNone;
+    return true;
+  }
+  __device__ void hist_clear() {
+    for (uint32_t i = lane; i < kHistSize; i += 32) {
+      sh.hist_key[i] = kNone;
+      sh.hist_cnt[i] = 0;
+    }
+    if (lane == 0) S.hist_used = 0;
     __syncwarp();
-    for (uint32_t size = 2; size <= P; size <<= 1)
-      for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
-        for (uint32_t i = lane; i < P; i += 32) {
-          const uint32_t j = i ^ stride;
-          if (j > i) {
-            const bool up = (i & size) == 0;
-            const uint32_t x = sh.keys[i], y = sh.keys[j];
-            if ((x > y) == up) {
-              sh.keys[i] = y;
-              sh.keys[j] = x;
-            }
-          }
-        }
-        __syncwarp();
-      }
-    if (lane == 0) S.n_keys = n;
-    __syncwarp();
-    uint32_t runs = 0;
-    const unsigned long long b = best_run(kNone, &runs);
-    unsigned long long b2 = 0;
-    if (cfg.decision.second_prefetch && n) b2 = best_run(~(uint32_t)(b & 0xffffffffu), nullptr);
+  }
+
+  // The most popular root (ties to the lowest) and the next one, the number
+  // of roots and of lanes.
+  __device__ void summarize_histogram() {
+    unsigned long long best = 0, second = 0;
+    uint32_t runs = 0, total = 0;
+    for (uint32_t i = lane; i < kHistSize; i += 32) {
+      const uint32_t c = sh.hist_cnt[i];
+      if (!c) continue;
+      ++runs;
+      total += c;
+      const unsigned long long v = ((unsigned long long)c << 32) | (unsigned long long)(~sh.hist_key[i]);
+      second = v > best ? best : (v > second ? v : second);
+      best = v > best ? v : best;
+    }
+    const unsigned long long b = warp_max64(best);
+    const unsigned long long b2 = warp_max64(best == b ? second : best);
+    runs = warp_sum(runs);
+    total = warp_sum(total);
     if (lane == 0) {
-      S.second = b2 ? ~(uint32_t)(b2 & 0xffffffffu) : kNone;
-      S.total = n;
+      S.second = (cfg.decision.second_prefetch && b2) ? ~(uint32_t)(b2 & 0xffffffffu) : kNone;
+      S.total = total;
       S.distinct = runs;
-      S.best = n ? ~(uint32_t)(b & 0xffffffffu) : kNone;
+      S.best = total ? ~(uint32_t)(b & 0xffffffffu) : kNone;
       S.best_cnt = (uint32_t)(b >> 32);
-      S.best_dense = S.best == kNone ? kNone : dense_of(S.best);
-      S.best_nodes = S.best_dense == kNone
-                         ? 0u
-                         : (uint32_t)(__ldg(a.member_first + S.best_dense + 1) - __ldg(a.member_first + S.best_dense));
+      if (S.best != S.best_of) {
+        S.best_of = S.best;
+        S.best_dense = S.best == kNone ? kNone : dense_of(S.best);
+        S.best_nodes = S.best_dense == kNone
+                           ? 0u
+                           : (uint32_t)(__ldg(a.member_first + S.best_dense + 1) - __ldg(a.member_first + S.best_dense));
+      }
       S.hist_dirty = 0;
     }
     __syncwarp();
@@ -542,12 +657,14 @@ struct WUnit {
 
   // The RT unit's decision (shader.cc:3419-3683; as prefetch_decide_kernel).
   __device__ void decide() {
-    if (S.hist_dirty) rebuild_histogram();
+    if (S.hist_dirty) summarize_histogram();
     else if (S.quiet) return;
     const rt_prefetch_params& p = cfg.decision;
     __syncwarp();
+    // lane 0 decides which members are queued: [from, to) of the lists
+    unsigned long long from = 0, to = 0;
+    bool quiet = true;
     if (lane == 0) {
-      bool quiet = true;
       const uint32_t best = S.best;
       bool submit = false;
       int num_nodes = 0;
@@ -569,23 +686,33 @@ struct WUnit {
           submit = true;
         }
       }
-      unsigned long long queue = S.pq_live;
       if (submit && best != kNone && bd != kNone && S.ds.last_prefetched != best && S.ds.last_prefetched_second != best) {
         const bool partial = p.heuristic == RT_PREFETCH_PARTIAL || p.heuristic == RT_PREFETCH_LATTER;
         const int num = partial ? num_nodes : n_nodes;
         quiet = false;  // submitted, or waiting for room in the queue
-        if ((unsigned long long)num + queue <= p.max_queue) {
+        if ((unsigned long long)num + S.pq_live <= p.max_queue) {
           const int j0 = p.heuristic == RT_PREFETCH_LATTER ? n_nodes - num : 0;
           const int j1 = p.heuristic == RT_PREFETCH_LATTER ? n_nodes : num;
           const unsigned long long mf = __ldg(a.member_first + bd);
-          for (int j = j0; j < j1; ++j) {
-            queue += (__ldg(a.member_bytes + mf + j) + 31u) / 32u;
-            push_member(mf + j, true);
-          }
+          from = mf + j0;
+          to = mf + j1;
           S.ds.last_prefetched = best;
-          S.st.treelets_prefetched++;
+          st.treelets_prefetched++;
         }
       }
+    }
+    from = __shfl_sync(kFull, from, 0);
+    to = __shfl_sync(kFull, to, 0);
+    const unsigned long long live = S.pq_live;
+    push_list(from, to, true);
+    unsigned long long from2 = 0, to2 = 0;
+    if (lane == 0) {
+      const uint32_t best = S.best;
+      // the queue length the decision sees: requests of the members submitted
+      // count whether or not the ring had room, metadata requests do not
+      unsigned long long queue = live;
+      if (p.second_prefetch && live == 0)
+        for (unsigned long long j = from; j < to; ++j) queue += (__ldg(a.member_bytes + j) + 31u) / 32u;
       // the second treelet may follow as soon as the queue is empty
       if (p.second_prefetch && S.total > 0 && S.distinct > 1 && S.second != kNone &&
           S.ds.last_prefetched_second != S.second)
@@ -597,15 +724,29 @@ struct WUnit {
         const uint32_t second = S.second;
         if (second != kNone && S.ds.last_prefetched_second != second) {
           const uint32_t sd = dense_of(second);
-          if (sd != kNone)
-            for (unsigned long long j = __ldg(a.member_first + sd); j < __ldg(a.member_first + sd + 1); ++j)
-              push_member(j, false);
+          if (sd != kNone) {
+            from2 = __ldg(a.member_first + sd);
+            to2 = __ldg(a.member_first + sd + 1);
+          }
           S.ds.last_prefetched_second = second;
-          S.st.treelets_prefetched++;
+          st.treelets_prefetched++;
         }
       }
       S.quiet = quiet ? 1u : 0u;
     }
+    from2 = __shfl_sync(kFull, from2, 0);
+    to2 = __shfl_sync(kFull, to2, 0);
+    push_list(from2, to2, false);
+    __syncwarp();
+  }
+
+  // Queues members [j0, j1), with their treelets' metadata first when the
+  // model loads it.
+  __device__ void push_list(unsigned long long j0, unsigned long long j1, bool with_metadata) {
+    if (j0 >= j1) return;
+    if (!(with_metadata && cfg.load_metadata) && a.members_apart && push_members(j0, j1)) return;
+    if (lane == 0)
+      for (unsigned long long j = j0; j < j1; ++j) push_member(j, with_metadata);
     __syncwarp();
   }
 
@@ -649,7 +790,7 @@ struct WUnit {
   __device__ uint32_t matching_lanes(uint32_t slot) const {
     const WarpSlot& w = sh.warps[slot];
     const uint32_t lp = S.ds.last_prefetched;
-    const bool m = lp != kNone && w.ptr[lane] < w.end[lane] && lane_root(w, lane) == lp;
+    const bool m = lp != kNone && w.ptr[lane] < w.end[lane] && w.root[lane] == lp;
     return __popc(__ballot_sync(kFull, m));
   }
 
@@ -685,7 +826,7 @@ struct WUnit {
   __device__ void start_round(uint32_t slot) {
     WarpSlot& w = sh.warps[slot];
     const bool has = w.ptr[lane] < w.end[lane];
-    const uint32_t v = has ? __ldg(a.visits + (unsigned long long)(w.gid * 32 + lane) * a.capacity + w.ptr[lane]) : 0u;
+    const uint32_t v = has ? w.next[lane] : 0u;
     const uint32_t size = tx_size(v & 7);
     const unsigned long long key = has ? (((unsigned long long)(v >> 3) << 8) | size) : ~0ull;
     const uint32_t peers = __match_any_sync(kFull, key);
@@ -699,7 +840,10 @@ struct WUnit {
     }
     const uint32_t total = __shfl_sync(kFull, incl, 31);
     const unsigned long long addr = (unsigned long long)(v >> 3) * 64;
-    for (uint32_t i = 0; i < nch; ++i) sh.chunk[incl - nch + i] = Request{addr + 32ull * i, addr, i == 0 ? 1u : 0u, 0u};
+    for (uint32_t i = 0; i < nch; ++i) {
+      sh.chunk[incl - nch + i] = Request{addr + 32ull * i, addr, i == 0 ? 1u : 0u, 0u};
+      if (cfg.prefetcher != RT_UNIT_PF_NONE) touch_tables(addr + 32ull * i);
+    }
     uint32_t il = has ? intersection_latency(v & 7) : 0u;
     il = __reduce_max_sync(kFull, il);
     const uint32_t issued = __ballot_sync(kFull, has);
@@ -758,11 +902,23 @@ struct WUnit {
       const uint32_t o = __ffs(m) - 1;
       WarpSlot& w = sh.warps[S.order[o]];
       const uint32_t issued = w.issued;
-      if ((issued >> lane) & 1u) w.ptr[lane]++;
+      const bool mine = (issued >> lane) & 1u;
+      const uint32_t old_root = w.root[lane];
+      if (mine) {
+        w.ptr[lane]++;
+        fetch_next(w);
+      }
+      if (cfg.prefetcher == RT_UNIT_PF_TREELET) {
+        __syncwarp();
+        if (!hist_renew()) {
+          hist_add(old_root, mine, ~0u);
+          hist_add(w.root[lane], mine && has_next(w), 1u);
+        }
+      }
       const uint32_t live = __ballot_sync(kFull, w.ptr[lane] < w.end[lane]);
       __syncwarp();
       if (lane == 0) {
-        S.st.transactions += __popc(issued);
+        st.transactions += __popc(issued);
         w.issued = 0;
         w.in_flight = 0;
         w.live = live;
@@ -779,7 +935,7 @@ struct WUnit {
       if (lane < n_res && !gone) S.order[__popc(keep & lanemask_lt())] = slot;
       __syncwarp();
       if (lane == 0) {
-        S.st.warps += __popc(leave);
+        st.warps += __popc(leave);
         S.n_res = __popc(keep);
         S.hist_dirty = 1;
       }
@@ -791,12 +947,14 @@ struct WUnit {
       WarpSlot& w = sh.warps[slot];
       const uint32_t gid = S.next_gid;
       const uint32_t r = gid * 32 + lane;
+      if (lane == 0) w.gid = gid;
       w.ptr[lane] = 0;
       w.end[lane] = r < a.n ? min(a.hits[r].n_visits, a.capacity) : 0u;
+      __syncwarp();
+      fetch_next(w);
       const uint32_t live = __ballot_sync(kFull, w.end[lane] != 0);
       __syncwarp();
       if (lane == 0) {
-        w.gid = gid;
         w.wid = S.local++ % cfg.max_warps;
         w.in_flight = w.all_sent = 0;
         w.ready = w.ilat = w.issued = 0;
@@ -807,6 +965,7 @@ struct WUnit {
         S.hist_dirty = 1;
       }
       __syncwarp();
+      if (cfg.prefetcher == RT_UNIT_PF_TREELET && !hist_renew()) hist_add(w.root[lane], has_next(w), 1u);
     }
     // when to look again: the earliest round due, or the next cycle for a
     // warp that came in without a transaction
@@ -824,7 +983,6 @@ struct WUnit {
   __device__ void run(uint32_t u) {
     const uint32_t n_warps = (a.n + 31) / 32;
     if (lane == 0) {
-      S.st = rt_unit_stats{};
       S.most_recent_metadata = 0;
       S.ds = rt_prefetch_state{kNone, kNone, kNone, 0};
       S.pq_head = S.pq_tail = S.pq_live = 0;
@@ -833,8 +991,7 @@ struct WUnit {
       S.n_res = 0;
       S.free_mask = (1u << cfg.max_warps) - 1u;
       S.mr_head = S.mr_tail = 0;
-      S.n_keys = 0;
-      S.best = kNone;
+      S.best = S.best_of = kNone;
       S.best_cnt = S.total = S.distinct = S.best_nodes = 0;
       S.best_dense = S.second = kNone;
       S.hist_dirty = 1;
@@ -844,6 +1001,7 @@ struct WUnit {
       S.next_gid = u;
       S.local = 0;
     }
+    hist_clear();
     if (lane < kMaxResident) sh.stride[lane].has = sh.stride[lane].n = 0;
     if (a.lines_shared)
       for (uint32_t i = lane; i < cfg.l1_sets * cfg.l1_ways; i += 32) lines[i].flags = 0;
@@ -855,13 +1013,13 @@ struct WUnit {
     for (uint32_t t = 0;; ++t) {
       if (t >= S.next_retire) retire_and_admit(t, n_warps);
       if (S.n_res == 0) {
-        if (lane == 0) S.st.cycles = t;
+        if (lane == 0) st.cycles = t;
         break;
       }
       if (t >= tcap) {
         if (lane == 0) {
-          S.st.cycles = t;
-          S.st.status |= 2;
+          st.cycles = t;
+          st.status |= 2;
         }
         break;
       }
@@ -927,31 +1085,12 @@ struct WUnit {
         t = until - 1u;
       }
     }
-    if (lane == 0) S.st.decisions = decisions;
+    if (lane == 0) st.decisions = decisions;
     __syncwarp();
-    // final tally (gpu-sim.cc:1749-1790): lanes take sector-map slices
-    const uint32_t n_sec = 1u << a.sec_log2;
-    unsigned long long eff[5] = {0, 0, 0, 0, 0}, uba = 0;
-    for (uint32_t i = lane; i < n_sec; i += 32) {
-      const SectorEntry& e = sec[i];
-      if (!e.key) continue;
-      const uint32_t classified = e.count[0] + e.count[1] + e.count[2] + e.count[3];
-      if (classified) {
-        uba += e.n_unclassified;
-        for (uint32_t c = 0; c < 4; ++c) eff[c] += e.count[c];
-      } else {
-        eff[RT_PF_NEVER_USED] += e.n_unclassified;
-      }
-    }
-#pragma unroll
-    for (int s = 16; s > 0; s >>= 1) {
-      uba += __shfl_xor_sync(kFull, uba, s);
-      for (int c = 0; c < 5; ++c) eff[c] += __shfl_xor_sync(kFull, eff[c], s);
-    }
     if (lane == 0) {
-      for (int c = 0; c < 5; ++c) S.st.effectiveness[c] = eff[c];
-      S.st.unclassified_but_accessed = uba;
-      if (S.full) S.st.status |= 1;
+      st.effectiveness[RT_PF_NEVER_USED] = uncl - uncl_accessed;
+      st.unclassified_but_accessed = uncl_accessed;
+      if (S.full) st.status |= 1;
     }
     __syncwarp();
   }
@@ -964,7 +1103,8 @@ __global__ void __launch_bounds__(32) unit_replay_kernel(ReplayArgs a) {
   const uint32_t u = blockIdx.x;
   WUnit unit(a, u, sh, smem_lines);
   unit.run(u);
-  if ((threadIdx.x & 31u) == 0) a.stats[u] = sh.s.st;
+  rtd::touch_l1_done();
+  if ((threadIdx.x & 31u) == 0) a.stats[u] = unit.st;
 }
 
 }  // namespace rtr
