@@ -80,8 +80,7 @@ struct Request {
 };
 
 struct WarpSlot {
-  uint32_t gid, wid, in_flight, all_sent, ready, ilat, issued;
-  uint32_t live;  // lanes with transactions left
+  uint32_t gid, wid, issued;
   uint32_t ptr[32], end[32];
   uint32_t next[32], root[32];  // each lane's next transaction (visit entry) and its treelet root
 };
@@ -102,15 +101,11 @@ struct MetaReturn {
 struct UnitState {
   unsigned long long most_recent_metadata;
   rt_prefetch_state ds;
-  uint32_t pq_head, pq_tail, pq_live;
-  uint32_t ch_head, ch_tail, serving;
-  uint32_t order[kMaxResident], n_res, free_mask;
   uint32_t mr_head, mr_tail;
   // histogram summary of the lanes' next treelets
-  uint32_t hist_used, best, best_cnt, total, distinct, best_of, best_dense, best_nodes, second, hist_dirty;
-  uint32_t quiet;         // deciding again changes nothing until the histogram does
-  uint32_t next_retire;   // earliest cycle at which a round is retired or a warp leaves
-  uint32_t full, next_gid, local;
+  uint32_t hist_used, best, best_cnt, total, distinct, best_of, best_dense, best_nodes, second;
+  uint32_t full;
+  uint32_t moved[kMaxResident];  // where resident warps move from when some leave
 };
 
 struct ReplayArgs {
@@ -131,7 +126,7 @@ struct ReplayArgs {
   // scratch
   uint8_t* scratch;
   unsigned long long unit_bytes;
-  uint32_t sec_log2, queued_log2, pq_cap;
+  uint32_t sec_log2, queued_log2, pq_cap;  // pq_cap: a power of two
   uint32_t cycle_cap;     // per unit: the model's own bound on its cycles (or max_cycles)
   uint32_t lines_shared;  // 1: the L1 lines live in shared memory
   uint32_t members_apart; // no two members of a treelet share an address
@@ -174,15 +169,6 @@ __device__ __forceinline__ unsigned long long warp_max64(unsigned long long v) {
   return v;
 }
 
-__device__ __forceinline__ unsigned long long warp_min64(unsigned long long v) {
-#pragma unroll
-  for (int s = 16; s > 0; s >>= 1) {
-    const unsigned long long o = __shfl_xor_sync(kFull, v, s);
-    v = o < v ? o : v;
-  }
-  return v;
-}
-
 __device__ __forceinline__ uint32_t warp_sum(uint32_t v) { return __reduce_add_sync(kFull, v); }
 
 struct WUnit {
@@ -202,6 +188,21 @@ struct WUnit {
   // sectors that have a classified one
   rt_unit_stats st;
   unsigned long long uncl, uncl_accessed;
+  // Resident warps in order, warp o in lane o's registers: its slot, whether
+  // its round is in flight and all sent, when the round's data is back, its
+  // lanes with transactions left.
+  uint32_t r_slot, r_ready, r_live;
+  bool r_fly, r_sent;
+  // The same in every lane: warps resident, free slots, the prefetch queue's
+  // ends and live requests, the round being sent (its requests, the order of
+  // its warp, when its data is back so far, its intersection latency), whether
+  // the histogram changed, whether deciding again changes nothing until it
+  // does, and the earliest cycle at which a round retires or a warp leaves.
+  // (Kept in shared memory, every one of them was a 30-cycle read on the path
+  // of each modeled cycle.)
+  uint32_t n_res, free_mask, pq_head, pq_tail, pq_live, ch_head, ch_tail, serving, ch_ready, ch_ilat;
+  uint32_t next_retire, next_gid, local;
+  bool hist_dirty, quiet;
 
   __device__ WUnit(const ReplayArgs& args, uint32_t u, UnitShared& shm, Line* smem_lines)
       : a(args), cfg(args.cfg), lane(threadIdx.x & 31u), sh(shm), S(shm.s) {
@@ -215,6 +216,24 @@ struct WUnit {
     metaret = reinterpret_cast<MetaReturn*>(base + a.off_meta);
     st = rt_unit_stats{};
     uncl = uncl_accessed = 0;
+    r_slot = r_ready = r_live = 0;
+    r_fly = r_sent = false;
+    n_res = 0;
+    free_mask = (1u << cfg.max_warps) - 1u;
+    pq_head = pq_tail = pq_live = 0;
+    ch_head = ch_tail = ch_ready = ch_ilat = 0;
+    serving = kNone;
+    next_retire = 0;
+    next_gid = u;
+    local = 0;
+    hist_dirty = true;
+    quiet = false;
+  }
+  // After lane 0 has changed the queue on its own.
+  __device__ void share_queue() {
+    pq_head = __shfl_sync(kFull, pq_head, 0);
+    pq_tail = __shfl_sync(kFull, pq_tail, 0);
+    pq_live = __shfl_sync(kFull, pq_live, 0);
   }
 
   // ------------------------------------------------------------ tables (lane 0)
@@ -264,7 +283,7 @@ struct WUnit {
   // unclassified records of the sectors with a classified one and of the
   // others; both are kept here (scanning the table at the end took a fifth of
   // a replay).
-  __device__ void classify(SectorEntry* e, uint32_t cls) {  // lane 0
+  __device__ __forceinline__ void classify(SectorEntry* e, uint32_t cls) {  // lane 0
     e->n_unclassified--;
     --uncl;
     st.effectiveness[cls]++;
@@ -275,7 +294,7 @@ struct WUnit {
       uncl_accessed += e->n_unclassified;
     }
   }
-  __device__ void classify(unsigned long long sector, uint32_t cls) {
+  __device__ __forceinline__ void classify(unsigned long long sector, uint32_t cls) {
     SectorEntry* e = sector_entry(sector, false);
     if (e) classify(e, cls);
   }
@@ -298,8 +317,9 @@ struct WUnit {
     const Line* set = set_of(block);
     const uint32_t inv = __ballot_sync(kFull, lane < cfg.l1_ways && !(set[lane].flags & kLineValid));
     if (inv) return __ffs(inv) - 1;
-    const unsigned long long k = lane < cfg.l1_ways ? (((unsigned long long)set[lane].lru << 5) | lane) : ~0ull;
-    return (int)(warp_min64(k) & 31u);
+    const uint32_t lru = lane < cfg.l1_ways ? set[lane].lru : 0xFFFFFFFFu;
+    const uint32_t oldest = __reduce_min_sync(kFull, lru);
+    return __ffs(__ballot_sync(kFull, lane < cfg.l1_ways && lru == oldest)) - 1;
   }
 
   // Lane 0: installs `block` in way `w`, recording evicted prefetched sectors.
@@ -326,7 +346,10 @@ struct WUnit {
     const uint32_t k = (uint32_t)((addr >> 5) & 3);
     const bool sector_valid = way >= 0 && ((set[way].flags >> k) & 1u);
     const int vic = (way < 0) ? victim_way(block) : -1;
-    uint32_t ret = 0;
+    // every lane finds the cycle the data is there; lane 0 updates the model
+    const uint32_t back = sector_valid ? set[way].ready[k] : 0u;
+    const uint32_t ret = !sector_valid ? t + cfg.miss_latency : (back <= t ? t + cfg.hit_latency : back);
+    __syncwarp();
     if (lane == 0) {
       const unsigned long long sector = addr >> 5;
       st.demand_requests++;
@@ -334,20 +357,18 @@ struct WUnit {
         Line* l = set + way;
         l->lru = t;
         const bool pf_uncl = (l->flags >> (4 + k)) & (l->flags >> (8 + k)) & 1u;
-        if (l->ready[k] <= t) {
+        if (back <= t) {
           st.demand_hits++;
           if (pf_uncl) {
             classify(sector, RT_PF_TIMELY);
             l->flags &= ~(1u << (8 + k));
           }
-          ret = t + cfg.hit_latency;
         } else {
           st.demand_hit_reserved++;
           if (pf_uncl) {
             classify(sector, RT_PF_LATE);
             l->flags &= ~(1u << (8 + k));
           }
-          ret = l->ready[k];
         }
       } else {
         st.demand_misses++;
@@ -360,11 +381,10 @@ struct WUnit {
         l->lru = t;
         l->flags = (l->flags | (1u << k)) & ~((1u << (4 + k)) | (1u << (8 + k)));
         l->ready[k] = t + cfg.miss_latency;
-        ret = t + cfg.miss_latency;
       }
     }
     __syncwarp();
-    return __shfl_sync(kFull, ret, 0);
+    return ret;
   }
 
   __device__ bool is_metadata(unsigned long long base) const {
@@ -378,6 +398,7 @@ struct WUnit {
     const uint32_t k = (uint32_t)((addr >> 5) & 3);
     const bool sector_valid = way >= 0 && ((set[way].flags >> k) & 1u);
     const int vic = (way < 0) ? victim_way(block) : -1;
+    __syncwarp();
     if (lane == 0) {
       st.prefetch_issued++;
       SectorEntry* e = sector_entry(addr >> 5, true);
@@ -415,26 +436,26 @@ struct WUnit {
   // ------------------------------------------------------------ prefetch queue
   __device__ void pq_push(unsigned long long addr, unsigned long long base) {  // lane 0
     st.prefetch_queued++;
-    if (S.pq_tail - S.pq_head >= a.pq_cap) {  // ring full (live + erased entries)
+    if (pq_tail - pq_head >= a.pq_cap) {  // ring full (live + erased entries)
       S.full = 1;
       return;
     }
-    const uint32_t i = S.pq_tail % a.pq_cap;
+    const uint32_t i = pq_tail & (a.pq_cap - 1u);
     pq[2 * i] = addr;
     pq[2 * i + 1] = base;
     dead[i] = 0;
     pq_next[i] = 0;
-    const uint32_t at = ++S.pq_tail;  // position + 1
-    ++S.pq_live;
+    const uint32_t at = ++pq_tail;  // position + 1
+    ++pq_live;
     QueuedEntry* q = queued_entry(addr, true);
     if (!q) return;
-    if (q->first) pq_next[(q->last - 1u) % a.pq_cap] = at;
+    if (q->first) pq_next[(q->last - 1u) & (a.pq_cap - 1u)] = at;
     else q->first = at;
     q->last = at;
   }
 
   __device__ void pq_drop_dead() {  // lane 0
-    while (S.pq_head != S.pq_tail && dead[S.pq_head % a.pq_cap]) ++S.pq_head;
+    while (pq_head != pq_tail && dead[pq_head & (a.pq_cap - 1u)]) ++pq_head;
   }
 
   // Erases queued prefetches of `addr`, stepping past the entry that follows
@@ -442,34 +463,38 @@ struct WUnit {
   // live entry between them the second stays.  Follows the address's own
   // requests (almost always one).
   __device__ void remove_queued(unsigned long long addr) {
+    QueuedEntry* q = nullptr;
+    uint32_t at = 0;
     if (lane == 0) {
-      QueuedEntry* q = queued_entry(addr, false);
-      uint32_t at = q ? q->first : 0u;
-      if (at) {
+      q = queued_entry(addr, false);
+      at = q ? q->first : 0u;
+    }
+    if (!__shfl_sync(kFull, at, 0)) return;
+    if (lane == 0) {
         uint32_t kept = 0;  // last live request kept, position + 1
         q->first = 0;
         while (at) {
-          const uint32_t i = (at - 1u) % a.pq_cap, next = pq_next[i];
+          const uint32_t i = (at - 1u) & (a.pq_cap - 1u), next = pq_next[i];
           dead[i] = 1;
-          --S.pq_live;
+          --pq_live;
           st.prefetch_removed++;
           uint32_t p = at;  // the entry stepped past: the next live one (positions at .. tail - 1)
-          while (p != S.pq_tail && dead[p % a.pq_cap]) ++p;
+          while (p != pq_tail && dead[p & (a.pq_cap - 1u)]) ++p;
           at = next;
           if (next && p + 1u == next) {  // it is the address's next request: it stays
-            const uint32_t k = p % a.pq_cap;
-            if (kept) pq_next[(kept - 1u) % a.pq_cap] = next;
+            const uint32_t k = p & (a.pq_cap - 1u);
+            if (kept) pq_next[(kept - 1u) & (a.pq_cap - 1u)] = next;
             else q->first = next;
             kept = next;
             at = pq_next[k];
           }
         }
-        if (kept) pq_next[(kept - 1u) % a.pq_cap] = 0;
+        if (kept) pq_next[(kept - 1u) & (a.pq_cap - 1u)] = 0;
         q->last = kept;
         pq_drop_dead();
-      }
     }
     __syncwarp();
+    share_queue();
   }
 
   __device__ uint32_t dense_of(uint32_t root) const {
@@ -514,11 +539,11 @@ struct WUnit {
         if ((int)lane >= s) incl += o;
       }
       const uint32_t total = __shfl_sync(kFull, incl, 31);
-      const uint32_t tail = S.pq_tail;
-      if (tail - S.pq_head + total > a.pq_cap) return jb == j0 ? false : push_rest(jb, j1);
+      const uint32_t tail = pq_tail;
+      if (tail - pq_head + total > a.pq_cap) return jb == j0 ? false : push_rest(jb, j1);
       for (uint32_t i = 0; i < n; ++i) {
         const unsigned long long at_addr = addr + 32ull * i;
-        const uint32_t p = tail + incl - n + i, k = p % a.pq_cap;
+        const uint32_t p = tail + incl - n + i, k = p & (a.pq_cap - 1u);
         pq[2 * k] = at_addr;
         pq[2 * k + 1] = addr;
         dead[k] = 0;
@@ -526,17 +551,14 @@ struct WUnit {
         touch_tables(at_addr);
         QueuedEntry* q = queued_claim(at_addr);
         if (!q) continue;
-        if (q->first) pq_next[(q->last - 1u) % a.pq_cap] = p + 1u;
+        if (q->first) pq_next[(q->last - 1u) & (a.pq_cap - 1u)] = p + 1u;
         else q->first = p + 1u;
         q->last = p + 1u;
       }
       __syncwarp();
-      if (lane == 0) {
-        S.pq_tail = tail + total;
-        S.pq_live += total;
-        st.prefetch_queued += total;
-      }
-      __syncwarp();
+      pq_tail = tail + total;
+      pq_live += total;
+      if (lane == 0) st.prefetch_queued += total;
     }
     return true;
   }
@@ -545,6 +567,7 @@ struct WUnit {
     if (lane == 0)
       for (unsigned long long j = j0; j < j1; ++j) push_member(j, false);
     __syncwarp();
+    share_queue();
     return true;
   }
 
@@ -604,8 +627,8 @@ struct WUnit {
     if (S.hist_used + 32u <= kHistSize * 3 / 4) return false;
     __syncwarp();
     hist_clear();
-    for (uint32_t o = 0; o < S.n_res; ++o) {
-      const WarpSlot& w = sh.warps[S.order[o]];
+    for (uint32_t o = 0; o < n_res; ++o) {
+      const WarpSlot& w = sh.warps[__shfl_sync(kFull, r_slot, o)];
       hist_add(w.root[lane], has_next(w), 1u);
     }
     return true;
@@ -650,20 +673,20 @@ struct WUnit {
                            ? 0u
                            : (uint32_t)(__ldg(a.member_first + S.best_dense + 1) - __ldg(a.member_first + S.best_dense));
       }
-      S.hist_dirty = 0;
     }
+    hist_dirty = false;
     __syncwarp();
   }
 
   // The RT unit's decision (shader.cc:3419-3683; as prefetch_decide_kernel).
   __device__ void decide() {
-    if (S.hist_dirty) summarize_histogram();
-    else if (S.quiet) return;
+    if (hist_dirty) summarize_histogram();
+    else if (quiet) return;
     const rt_prefetch_params& p = cfg.decision;
     __syncwarp();
     // lane 0 decides which members are queued: [from, to) of the lists
     unsigned long long from = 0, to = 0;
-    bool quiet = true;
+    bool still = true;  // lane 0: deciding again would change nothing
     if (lane == 0) {
       const uint32_t best = S.best;
       bool submit = false;
@@ -689,8 +712,8 @@ struct WUnit {
       if (submit && best != kNone && bd != kNone && S.ds.last_prefetched != best && S.ds.last_prefetched_second != best) {
         const bool partial = p.heuristic == RT_PREFETCH_PARTIAL || p.heuristic == RT_PREFETCH_LATTER;
         const int num = partial ? num_nodes : n_nodes;
-        quiet = false;  // submitted, or waiting for room in the queue
-        if ((unsigned long long)num + S.pq_live <= p.max_queue) {
+        still = false;  // submitted, or waiting for room in the queue
+        if ((unsigned long long)num + pq_live <= p.max_queue) {
           const int j0 = p.heuristic == RT_PREFETCH_LATTER ? n_nodes - num : 0;
           const int j1 = p.heuristic == RT_PREFETCH_LATTER ? n_nodes : num;
           const unsigned long long mf = __ldg(a.member_first + bd);
@@ -703,7 +726,7 @@ struct WUnit {
     }
     from = __shfl_sync(kFull, from, 0);
     to = __shfl_sync(kFull, to, 0);
-    const unsigned long long live = S.pq_live;
+    const unsigned long long live = pq_live;
     push_list(from, to, true);
     unsigned long long from2 = 0, to2 = 0;
     if (lane == 0) {
@@ -716,7 +739,7 @@ struct WUnit {
       // the second treelet may follow as soon as the queue is empty
       if (p.second_prefetch && S.total > 0 && S.distinct > 1 && S.second != kNone &&
           S.ds.last_prefetched_second != S.second)
-        quiet = false;
+        still = false;
       if (p.second_prefetch && queue == 0 && S.total > 0 && S.distinct > 1 && S.ds.last_prefetched == best &&
           best != kNone) {
         // the first maximum among treelets other than the last prefetched one,
@@ -732,12 +755,11 @@ struct WUnit {
           st.treelets_prefetched++;
         }
       }
-      S.quiet = quiet ? 1u : 0u;
     }
     from2 = __shfl_sync(kFull, from2, 0);
     to2 = __shfl_sync(kFull, to2, 0);
     push_list(from2, to2, false);
-    __syncwarp();
+    quiet = __shfl_sync(kFull, still ? 1u : 0u, 0) != 0;
   }
 
   // Queues members [j0, j1), with their treelets' metadata first when the
@@ -748,6 +770,7 @@ struct WUnit {
     if (lane == 0)
       for (unsigned long long j = j0; j < j1; ++j) push_member(j, with_metadata);
     __syncwarp();
+    share_queue();
   }
 
   // ------------------------------------------------------------ stride (Lee MICRO'10), lane 0
@@ -780,7 +803,7 @@ struct WUnit {
         largest_count = s.count[i];
       }
     const unsigned long long pa = next_addr + (unsigned long long)(long long)largest;
-    if (cfg.decision.max_queue <= S.pq_live) {
+    if (cfg.decision.max_queue <= pq_live) {
       pq_push(pa, pa);
       pq_push(pa + 32, pa);
     }
@@ -794,37 +817,36 @@ struct WUnit {
     return __popc(__ballot_sync(kFull, m));
   }
 
-  // rt_unit::schedule_next_warp (shader.cc:4307-4392); kNone if no warp is ready
+  // rt_unit::schedule_next_warp (shader.cc:4307-4392): the order of the warp
+  // to serve, kNone if no warp is ready
   __device__ uint32_t schedule() const {
-    const uint32_t n_res = S.n_res;
-    const bool rd = lane < n_res && !sh.warps[S.order[lane]].in_flight && sh.warps[S.order[lane]].live;
-    const uint32_t ready = __ballot_sync(kFull, rd);
+    const uint32_t ready = __ballot_sync(kFull, lane < n_res && !r_fly && r_live);
     if (!ready) return kNone;
     const bool treelet = cfg.prefetcher == RT_UNIT_PF_TREELET;
     if (treelet && cfg.scheduler == RT_UNIT_SCHED_OMR) {
       for (uint32_t m = ready; m; m &= m - 1) {
         const uint32_t o = __ffs(m) - 1;
-        if (matching_lanes(S.order[o]) > 0) return S.order[o];
+        if (matching_lanes(__shfl_sync(kFull, r_slot, o)) > 0) return o;
       }
     } else if (treelet && cfg.scheduler == RT_UNIT_SCHED_PMR) {
       uint32_t b = kNone, bc = 0;
       for (uint32_t m = ready; m; m &= m - 1) {
         const uint32_t o = __ffs(m) - 1;
-        const uint32_t c = matching_lanes(S.order[o]);
+        const uint32_t c = matching_lanes(__shfl_sync(kFull, r_slot, o));
         if (c > bc) {
-          b = S.order[o];
+          b = o;
           bc = c;
         }
       }
       if (b != kNone) return b;
     }
-    return S.order[__ffs(ready) - 1];
+    return __ffs(ready) - 1;
   }
 
   // A round: each lane's next transaction, identical (address, size) pairs
   // once in lane order, split into 32-byte requests.
-  __device__ void start_round(uint32_t slot) {
-    WarpSlot& w = sh.warps[slot];
+  __device__ void start_round(uint32_t o) {
+    WarpSlot& w = sh.warps[__shfl_sync(kFull, r_slot, o)];
     const bool has = w.ptr[lane] < w.end[lane];
     const uint32_t v = has ? w.next[lane] : 0u;
     const uint32_t size = tx_size(v & 7);
@@ -844,45 +866,42 @@ struct WUnit {
       sh.chunk[incl - nch + i] = Request{addr + 32ull * i, addr, i == 0 ? 1u : 0u, 0u};
       if (cfg.prefetcher != RT_UNIT_PF_NONE) touch_tables(addr + 32ull * i);
     }
-    uint32_t il = has ? intersection_latency(v & 7) : 0u;
-    il = __reduce_max_sync(kFull, il);
+    ch_ilat = __reduce_max_sync(kFull, has ? intersection_latency(v & 7) : 0u);
     const uint32_t issued = __ballot_sync(kFull, has);
-    __syncwarp();
-    if (lane == 0) {
-      w.issued = issued;
-      w.in_flight = 1;
-      w.all_sent = 0;
-      w.ready = 0;
-      w.ilat = il;
-      S.ch_head = 0;
-      S.ch_tail = total;
-      S.serving = slot;
+    if (lane == 0) w.issued = issued;
+    if (lane == o) {
+      r_fly = true;
+      r_sent = false;
     }
+    ch_head = 0;
+    ch_tail = total;
+    ch_ready = 0;
+    serving = o;
     __syncwarp();
   }
 
   __device__ void send_demand(uint32_t t) {
-    const Request r = sh.chunk[S.ch_head];
+    const Request r = sh.chunk[ch_head];
     if (cfg.prefetcher == RT_UNIT_PF_TREELET || cfg.prefetcher == RT_UNIT_PF_STRIDE) remove_queued(r.addr);
-    WarpSlot& w = sh.warps[S.serving];
-    if (lane == 0 && cfg.prefetcher == RT_UNIT_PF_STRIDE && r.first) stride_prefetch(w.wid, r.addr);
-    __syncwarp();
-    const uint32_t ret = demand(r.addr, t);
-    if (lane == 0) {
-      ++S.ch_head;
-      w.ready = max(w.ready, ret);
-      if (S.ch_head == S.ch_tail) {
-        w.all_sent = 1;
-        w.ready += w.ilat;
-        S.next_retire = min(S.next_retire, w.ready);
-        S.serving = kNone;
-      }
+    if (cfg.prefetcher == RT_UNIT_PF_STRIDE && r.first) {
+      const uint32_t wid = sh.warps[__shfl_sync(kFull, r_slot, serving)].wid;
+      if (lane == 0) stride_prefetch(wid, r.addr);
+      __syncwarp();
+      share_queue();
     }
-    __syncwarp();
+    ch_ready = max(ch_ready, demand(r.addr, t));
+    if (++ch_head == ch_tail) {
+      const uint32_t ready = ch_ready + ch_ilat;
+      if (lane == serving) {
+        r_sent = true;
+        r_ready = ready;
+      }
+      next_retire = min(next_retire, ready);
+      serving = kNone;
+    }
   }
 
-  __device__ bool prefetch_issuable() const {  // lane 0
-    const unsigned long long base = pq[2 * (S.pq_head % a.pq_cap) + 1];
+  __device__ bool prefetch_issuable(unsigned long long base) const {
     if (!cfg.wait_metadata || is_metadata(base)) return true;
     // shader.cc:4469-4476: the metadata of the treelet the request's base node belongs to
     const unsigned long long unit = base >> 6;
@@ -894,13 +913,11 @@ struct WUnit {
   // Rounds whose data is back advance their lanes; warps with no lanes left
   // leave; new warps come in, in order.
   __device__ void retire_and_admit(uint32_t t, uint32_t n_warps) {
-    const uint32_t n_res = S.n_res;
-    const WarpSlot* wl = lane < n_res ? &sh.warps[S.order[lane]] : nullptr;
-    const bool done_round = wl && wl->in_flight && wl->all_sent && wl->ready <= t;
-    const uint32_t rounds = __ballot_sync(kFull, done_round);
+    const bool treelets = cfg.prefetcher == RT_UNIT_PF_TREELET;
+    const uint32_t rounds = __ballot_sync(kFull, lane < n_res && r_fly && r_sent && r_ready <= t);
     for (uint32_t m = rounds; m; m &= m - 1) {
       const uint32_t o = __ffs(m) - 1;
-      WarpSlot& w = sh.warps[S.order[o]];
+      WarpSlot& w = sh.warps[__shfl_sync(kFull, r_slot, o)];
       const uint32_t issued = w.issued;
       const bool mine = (issued >> lane) & 1u;
       const uint32_t old_root = w.root[lane];
@@ -908,76 +925,77 @@ struct WUnit {
         w.ptr[lane]++;
         fetch_next(w);
       }
-      if (cfg.prefetcher == RT_UNIT_PF_TREELET) {
+      if (treelets) {
         __syncwarp();
         if (!hist_renew()) {
           hist_add(old_root, mine, ~0u);
           hist_add(w.root[lane], mine && has_next(w), 1u);
         }
       }
-      const uint32_t live = __ballot_sync(kFull, w.ptr[lane] < w.end[lane]);
-      __syncwarp();
-      if (lane == 0) {
-        st.transactions += __popc(issued);
-        w.issued = 0;
-        w.in_flight = 0;
-        w.live = live;
-        S.hist_dirty = 1;
+      const uint32_t live = __ballot_sync(kFull, has_next(w));
+      if (lane == 0) st.transactions += __popc(issued);
+      if (lane == o) {
+        r_fly = false;
+        r_live = live;
       }
-      __syncwarp();
+      hist_dirty = true;
     }
-    const bool gone = lane < n_res && !sh.warps[S.order[lane]].in_flight && sh.warps[S.order[lane]].live == 0;
+    const bool gone = lane < n_res && !r_fly && r_live == 0;
     const uint32_t leave = __ballot_sync(kFull, gone);
     if (leave) {
-      const uint32_t slot = lane < n_res ? S.order[lane] : 0u;
       const uint32_t keep = __ballot_sync(kFull, lane < n_res && !gone);
+      free_mask |= __reduce_or_sync(kFull, gone ? 1u << r_slot : 0u);
+      if (lane < n_res && !gone) S.moved[__popc(keep & lanemask_lt())] = lane;
       __syncwarp();
-      if (lane < n_res && !gone) S.order[__popc(keep & lanemask_lt())] = slot;
-      __syncwarp();
-      if (lane == 0) {
-        st.warps += __popc(leave);
-        S.n_res = __popc(keep);
-        S.hist_dirty = 1;
-      }
-      if (gone) atomicOr(&S.free_mask, 1u << slot);
+      if (lane == 0) st.warps += __popc(leave);
+      n_res = __popc(keep);
+      const uint32_t from = lane < n_res ? S.moved[lane] : lane;
+      r_slot = __shfl_sync(kFull, r_slot, from);
+      r_ready = __shfl_sync(kFull, r_ready, from);
+      r_live = __shfl_sync(kFull, r_live, from);
+      r_fly = __shfl_sync(kFull, r_fly ? 1u : 0u, from) != 0;
+      r_sent = __shfl_sync(kFull, r_sent ? 1u : 0u, from) != 0;
+      if (serving != kNone) serving = __popc(keep & ((1u << serving) - 1u));
+      hist_dirty = true;
       __syncwarp();
     }
-    while (S.n_res < cfg.max_warps && S.next_gid < n_warps) {
-      const uint32_t slot = __ffs(S.free_mask) - 1;
+    while (n_res < cfg.max_warps && next_gid < n_warps) {
+      const uint32_t slot = __ffs(free_mask) - 1;
       WarpSlot& w = sh.warps[slot];
-      const uint32_t gid = S.next_gid;
+      const uint32_t gid = next_gid;
       const uint32_t r = gid * 32 + lane;
-      if (lane == 0) w.gid = gid;
+      if (lane == 0) {
+        w.gid = gid;
+        w.wid = local % cfg.max_warps;
+        w.issued = 0;
+      }
       w.ptr[lane] = 0;
       w.end[lane] = r < a.n ? min(a.hits[r].n_visits, a.capacity) : 0u;
       __syncwarp();
       fetch_next(w);
-      const uint32_t live = __ballot_sync(kFull, w.end[lane] != 0);
-      __syncwarp();
-      if (lane == 0) {
-        w.wid = S.local++ % cfg.max_warps;
-        w.in_flight = w.all_sent = 0;
-        w.ready = w.ilat = w.issued = 0;
-        w.live = live;
-        S.free_mask &= ~(1u << slot);
-        S.order[S.n_res++] = slot;
-        S.next_gid = gid + cfg.n_rt_units;
-        S.hist_dirty = 1;
+      const uint32_t live = __ballot_sync(kFull, has_next(w));
+      if (lane == n_res) {
+        r_slot = slot;
+        r_live = live;
+        r_fly = r_sent = false;
+        r_ready = 0;
       }
+      ++local;
+      ++n_res;
+      free_mask &= ~(1u << slot);
+      next_gid = gid + cfg.n_rt_units;
+      hist_dirty = true;
       __syncwarp();
-      if (cfg.prefetcher == RT_UNIT_PF_TREELET && !hist_renew()) hist_add(w.root[lane], has_next(w), 1u);
+      if (treelets && !hist_renew()) hist_add(w.root[lane], has_next(w), 1u);
     }
     // when to look again: the earliest round due, or the next cycle for a
     // warp that came in without a transaction
     uint32_t due = 0xFFFFFFFFu;
-    if (lane < S.n_res) {
-      const WarpSlot& w = sh.warps[S.order[lane]];
-      if (w.in_flight && w.all_sent) due = w.ready;
-      else if (!w.in_flight && w.live == 0) due = t + 1;
+    if (lane < n_res) {
+      if (r_fly && r_sent) due = r_ready;
+      else if (!r_fly && r_live == 0) due = t + 1;
     }
-    due = __reduce_min_sync(kFull, due);
-    if (lane == 0) S.next_retire = due;
-    __syncwarp();
+    next_retire = __reduce_min_sync(kFull, due);
   }
 
   __device__ void run(uint32_t u) {
@@ -985,21 +1003,11 @@ struct WUnit {
     if (lane == 0) {
       S.most_recent_metadata = 0;
       S.ds = rt_prefetch_state{kNone, kNone, kNone, 0};
-      S.pq_head = S.pq_tail = S.pq_live = 0;
-      S.ch_head = S.ch_tail = 0;
-      S.serving = kNone;
-      S.n_res = 0;
-      S.free_mask = (1u << cfg.max_warps) - 1u;
       S.mr_head = S.mr_tail = 0;
       S.best = S.best_of = kNone;
       S.best_cnt = S.total = S.distinct = S.best_nodes = 0;
       S.best_dense = S.second = kNone;
-      S.hist_dirty = 1;
-      S.quiet = 0;
-      S.next_retire = 0;
       S.full = 0;
-      S.next_gid = u;
-      S.local = 0;
     }
     hist_clear();
     if (lane < kMaxResident) sh.stride[lane].has = sh.stride[lane].n = 0;
@@ -1011,8 +1019,8 @@ struct WUnit {
     unsigned long long decisions = 0;
     uint32_t next_decide = 0;  // the next multiple of prefetch_delay
     for (uint32_t t = 0;; ++t) {
-      if (t >= S.next_retire) retire_and_admit(t, n_warps);
-      if (S.n_res == 0) {
+      if (t >= next_retire) retire_and_admit(t, n_warps);
+      if (n_res == 0) {
         if (lane == 0) st.cycles = t;
         break;
       }
@@ -1036,7 +1044,7 @@ struct WUnit {
         ++decisions;
         next_decide += cfg.prefetch_delay;
       }
-      if (S.ch_head != S.ch_tail) {
+      if (ch_head != ch_tail) {
         send_demand(t);
         continue;
       }
@@ -1046,36 +1054,30 @@ struct WUnit {
         send_demand(t);
         continue;
       }
-      uint32_t go = 0;
-      if (cfg.prefetcher != RT_UNIT_PF_NONE && S.pq_live > 0) {
-        unsigned long long addr = 0, base = 0;
-        if (lane == 0 && prefetch_issuable()) {
-          const uint32_t i = S.pq_head % a.pq_cap;
-          addr = pq[2 * i];
-          base = pq[2 * i + 1];
-          dead[i] = 1;
-          --S.pq_live;
-          QueuedEntry* q = queued_entry(addr, false);
-          if (q) q->first = pq_next[i];  // the queue's head is its address's oldest request
-          pq_drop_dead();
-          go = 1;
-        }
-        __syncwarp();
-        go = __shfl_sync(kFull, go, 0);
-        if (go) {
-          addr = __shfl_sync(kFull, addr, 0);
-          base = __shfl_sync(kFull, base, 0);
+      if (cfg.prefetcher != RT_UNIT_PF_NONE && pq_live > 0) {
+        const uint32_t i = pq_head & (a.pq_cap - 1u);
+        const unsigned long long addr = pq[2 * i], base = pq[2 * i + 1];
+        if (prefetch_issuable(base)) {
+          __syncwarp();
+          if (lane == 0) {
+            dead[i] = 1;
+            QueuedEntry* q = queued_entry(addr, false);
+            if (q) q->first = pq_next[i];  // the queue's head is its address's oldest request
+            pq_drop_dead();
+          }
+          --pq_live;
+          pq_head = __shfl_sync(kFull, pq_head, 0);
           prefetch(addr, base, t);
+          continue;
         }
       }
-      if (go) continue;
       // An idle cycle: every resident warp waits for its round (schedule()
       // found none ready and no request is left to send).  Until the earliest
       // round is due nothing happens but decisions that change nothing and
       // metadata returns, which matter to a queued request that waits for one.
-      uint32_t until = min(S.next_retire, tcap);
-      if (treelets && (S.hist_dirty || !S.quiet)) until = min(until, next_decide);
-      if (S.pq_live > 0 && S.mr_head != S.mr_tail) until = min(until, metaret[S.mr_head % kMetaRing].t);
+      uint32_t until = min(next_retire, tcap);
+      if (treelets && (hist_dirty || !quiet)) until = min(until, next_decide);
+      if (pq_live > 0 && S.mr_head != S.mr_tail) until = min(until, metaret[S.mr_head % kMetaRing].t);
       if (until > t + 1) {
         if (treelets && next_decide < until) {
           const uint32_t k = (until - next_decide + cfg.prefetch_delay - 1u) / cfg.prefetch_delay;
@@ -1096,7 +1098,7 @@ struct WUnit {
   }
 };
 
-__global__ void __launch_bounds__(32) unit_replay_kernel(ReplayArgs a) {
+__global__ void __launch_bounds__(32, 1) unit_replay_kernel(ReplayArgs a) {
   extern __shared__ __align__(16) uint8_t replay_smem[];
   UnitShared& sh = *reinterpret_cast<UnitShared*>(replay_smem);
   Line* smem_lines = reinterpret_cast<Line*>(replay_smem + ((sizeof(UnitShared) + 15) & ~(size_t)15));
