@@ -6,9 +6,13 @@
 // access of every resident lane, takes the first maximum in ascending root
 // order, applies the heuristic, and queues the treelet's members as 32-byte
 // requests unless it was the last (or last second) treelet prefetched.  Here
-// the lanes' roots are sorted in shared memory (bitonic), runs give the
-// counts, and thread 0 applies the same heuristic arithmetic (IEEE double for
-// the popularity share, as in the reference).
+// the lanes count their roots in a shared-memory table, the two most popular
+// roots come out of one reduction, and the first warp applies the same
+// heuristic arithmetic (IEEE double for the popularity share, as in the
+// reference), searching the roots and adding up the members' requests 32 at a
+// time.  A decision is a chain of small steps, bound by their latency: 152 units
+// of 512 lanes take 7.7 us on a GB300; sorting the roots and walking the runs in
+// one thread took 43.7.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -33,68 +37,104 @@ struct PrefetchArgs {
   uint32_t n_treelets;
 };
 
+// Dense id of a treelet root, kNone if it is none: 32 probes at a time (a full
+// warp calls with the same root).
 __device__ __forceinline__ uint32_t dense_of_root(const PrefetchArgs& a, uint32_t root) {
-  uint32_t lo = 0, hi = a.n_treelets;
+  const uint32_t lane = threadIdx.x & 31u;
+  uint32_t lo = 0, hi = a.n_treelets;  // the first root >= `root` is in [lo, hi]
   while (lo < hi) {
-    const uint32_t mid = (lo + hi) >> 1;
-    if (a.roots[mid] < root) lo = mid + 1;
-    else hi = mid;
+    const uint32_t step = (hi - lo + 31u) / 32u, at = lo + lane * step;
+    // probes below `root` are a prefix of the lanes
+    const uint32_t less = __popc(__ballot_sync(0xffffffffu, at < hi && a.roots[at] < root));
+    if (less == 0) {
+      hi = lo;
+    } else {
+      hi = min(hi, lo + less * step);
+      lo += (less - 1u) * step + 1u;
+    }
   }
   return (lo < a.n_treelets && a.roots[lo] == root) ? lo : kNone;
 }
 
+// Requests of members [j0, j1) (a full warp calls).
+__device__ __forceinline__ uint32_t member_chunks(const PrefetchArgs& a, unsigned long long j0, unsigned long long j1) {
+  uint32_t c = 0;
+  for (unsigned long long j = j0 + (threadIdx.x & 31u); j < j1; j += 32) c += (a.member_bytes[j] + 31u) / 32u;
+  return __reduce_add_sync(0xffffffffu, c);
+}
+
+constexpr uint32_t kCountLog2 = 11, kCountSize = 1u << kCountLog2;  // at most 1,024 roots
+
 __global__ void __launch_bounds__(512) prefetch_decide_kernel(PrefetchArgs a) {
-  __shared__ uint32_t keys[kMaxLanes];
-  __shared__ uint32_t nkeys;
+  __shared__ uint32_t key[kCountSize], cnt[kCountSize];
+  __shared__ unsigned long long top[2][16];
+  __shared__ uint32_t sums[2][16];
   const uint32_t g = blockIdx.x;
-  const uint32_t tid = threadIdx.x;
-  uint32_t padded = 1;
-  while (padded < a.lanes) padded <<= 1;
-  for (uint32_t l = tid; l < padded; l += blockDim.x) {
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+  for (uint32_t i = tid; i < kCountSize; i += blockDim.x) {
+    key[i] = kNone;
+    cnt[i] = 0;
+  }
+  __syncthreads();
+  for (uint32_t l0 = 0; l0 < a.lanes; l0 += blockDim.x) {
+    const uint32_t l = l0 + tid;
     uint32_t k = kNone;
     if (l < a.lanes) {
       const uint32_t u = a.next_unit[(uint64_t)g * a.lanes + l];
       if (u != kNone && u < a.n_units) k = a.meta[u].x;
     }
-    keys[l] = k;
+    const uint32_t peers = __match_any_sync(0xffffffffu, k);
+    if (k != kNone && (uint32_t)(__ffs(peers) - 1) == lane) {
+      uint32_t i = (k * 0x9E3779B1u) >> (32 - kCountLog2);
+      for (;; i = (i + 1) & (kCountSize - 1)) {
+        const uint32_t old = atomicCAS(&key[i], kNone, k);
+        if (old == kNone || old == k) break;
+      }
+      atomicAdd(&cnt[i], (uint32_t)__popc(peers));
+    }
   }
   __syncthreads();
-  // bitonic sort ascending (kNone sorts last)
-  for (uint32_t size = 2; size <= padded; size <<= 1) {
-    for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
-      for (uint32_t i = tid; i < padded; i += blockDim.x) {
-        const uint32_t j = i ^ stride;
-        if (j > i) {
-          const bool up = (i & size) == 0;
-          const uint32_t x = keys[i], y = keys[j];
-          if ((x > y) == up) {
-            keys[i] = y;
-            keys[j] = x;
-          }
-        }
-      }
-      __syncthreads();
-    }
+  // the most popular root and the next one, (count << 32 | ~root): ties go to the lowest root
+  unsigned long long b0 = 0, b1 = 0;
+  uint32_t total = 0, distinct = 0;
+  for (uint32_t i = tid; i < kCountSize; i += blockDim.x) {
+    const uint32_t c = cnt[i];
+    if (!c) continue;
+    total += c;
+    ++distinct;
+    const unsigned long long v = ((unsigned long long)c << 32) | (unsigned long long)(~key[i]);
+    b1 = v > b0 ? b0 : (v > b1 ? v : b1);
+    b0 = v > b0 ? v : b0;
   }
-  if (tid != 0) return;
-  // runs: first maximum in ascending order; distinct count; total
-  uint32_t total = 0, distinct = 0, best = kNone, best_cnt = 0;
-  {
-    uint32_t i = 0;
-    while (i < padded && keys[i] != kNone) {
-      uint32_t j = i;
-      while (j < padded && keys[j] == keys[i]) ++j;
-      const uint32_t c = j - i;
-      total += c;
-      ++distinct;
-      if (best == kNone || c > best_cnt) {  // strict >: the lowest root wins ties
-        best = keys[i];
-        best_cnt = c;
-      }
-      i = j;
+  auto top_two = [](unsigned long long& x0, unsigned long long& x1) {
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) {
+      const unsigned long long y0 = __shfl_xor_sync(0xffffffffu, x0, s), y1 = __shfl_xor_sync(0xffffffffu, x1, s);
+      const unsigned long long lo = x0 > y0 ? y0 : x0, hi1 = x1 > y1 ? x1 : y1;
+      x0 = x0 > y0 ? x0 : y0;
+      x1 = lo > hi1 ? lo : hi1;
     }
-    nkeys = i;
+  };
+  top_two(b0, b1);
+  total = __reduce_add_sync(0xffffffffu, total);
+  distinct = __reduce_add_sync(0xffffffffu, distinct);
+  if (lane == 0) {
+    top[0][warp] = b0;
+    top[1][warp] = b1;
+    sums[0][warp] = total;
+    sums[1][warp] = distinct;
   }
+  __syncthreads();
+  if (warp != 0) return;
+  const uint32_t warps = blockDim.x / 32u;
+  b0 = lane < warps ? top[0][lane] : 0ull;
+  b1 = lane < warps ? top[1][lane] : 0ull;
+  top_two(b0, b1);
+  total = __reduce_add_sync(0xffffffffu, lane < warps ? sums[0][lane] : 0u);
+  distinct = __reduce_add_sync(0xffffffffu, lane < warps ? sums[1][lane] : 0u);
+  const uint32_t best = b0 ? ~(uint32_t)b0 : kNone, best_cnt = (uint32_t)(b0 >> 32);
+  const uint32_t next = b1 ? ~(uint32_t)b1 : kNone;
+  // every lane of the warp decides alike; lane 0 writes
   rt_prefetch_state st = a.state[g];
   const uint32_t copy = a.p.variant & 3u;
   const bool pipelined = copy == RT_PREFETCH_PIPELINED_QUEUE;
@@ -122,9 +162,8 @@ __global__ void __launch_bounds__(512) prefetch_decide_kernel(PrefetchArgs a) {
     // unless it was the last one prefetched; an empty histogram names no
     // treelet (an empty member list) and is recorded as the last one
     if (st.last_prefetched != best && (uint64_t)n_nodes + queue <= a.p.max_queue) {
-      uint32_t chunks = 0;
-      if (bd != kNone)
-        for (int j = 0; j < n_nodes; ++j) chunks += (a.member_bytes[a.member_first[bd] + j] + 31u) / 32u;
+      const uint32_t chunks =
+          bd != kNone ? member_chunks(a, a.member_first[bd], a.member_first[bd] + (unsigned long long)n_nodes) : 0u;
       queue += chunks;
       d.submitted = best != kNone ? 1u : 0u;
       d.n_members = (uint32_t)n_nodes;
@@ -132,8 +171,11 @@ __global__ void __launch_bounds__(512) prefetch_decide_kernel(PrefetchArgs a) {
       st.last_prefetched = best;
     }
     st.queue_len = (uint32_t)queue;
-    a.state[g] = st;
-    a.out[g] = d;
+    __syncwarp();  // every lane has read the state
+    if (lane == 0) {
+      a.state[g] = st;
+      a.out[g] = d;
+    }
     return;
   }
   if (a.p.heuristic == RT_PREFETCH_ALWAYS) {
@@ -162,8 +204,8 @@ __global__ void __launch_bounds__(512) prefetch_decide_kernel(PrefetchArgs a) {
         if (flush) queue = 0;
         const int j0 = a.p.heuristic == RT_PREFETCH_LATTER ? n_nodes - num : 0;
         const int j1 = a.p.heuristic == RT_PREFETCH_LATTER ? n_nodes : num;
-        uint32_t chunks = 0;
-        for (int j = j0; j < j1; ++j) chunks += (a.member_bytes[a.member_first[bd] + j] + 31u) / 32u;
+        const unsigned long long mf = a.member_first[bd];
+        const uint32_t chunks = member_chunks(a, mf + j0, mf + j1);
         queue += chunks;
         d.submitted = 1;
         d.first_member = (uint32_t)j0;
@@ -175,34 +217,22 @@ __global__ void __launch_bounds__(512) prefetch_decide_kernel(PrefetchArgs a) {
   }
   if (a.p.second_prefetch && !pipelined && queue == 0 && total > 0 && distinct > 1 && st.last_prefetched == best &&
       best != kNone) {
-    // next most popular treelet other than the last prefetched one
-    uint32_t second = kNone, scnt = 0;
-    uint32_t i = 0;
-    while (i < nkeys) {
-      uint32_t j = i;
-      while (j < nkeys && keys[j] == keys[i]) ++j;
-      const uint32_t c = j - i;
-      if (keys[i] != st.last_prefetched && (second == kNone || c > scnt)) {
-        second = keys[i];
-        scnt = c;
-      }
-      i = j;
-    }
-    if (second != kNone && st.last_prefetched_second != second) {
-      const uint32_t sd = dense_of_root(a, second);
-      uint32_t chunks = 0;
-      if (sd != kNone)
-        for (unsigned long long j = a.member_first[sd]; j < a.member_first[sd + 1]; ++j)
-          chunks += (a.member_bytes[j] + 31u) / 32u;
+    // next most popular treelet other than the last prefetched one, `best`
+    if (next != kNone && st.last_prefetched_second != next) {
+      const uint32_t sd = dense_of_root(a, next);
+      const uint32_t chunks = sd != kNone ? member_chunks(a, a.member_first[sd], a.member_first[sd + 1]) : 0u;
       queue += chunks;
       d.chunks += chunks;
-      d.second_treelet = second;
-      st.last_prefetched_second = second;
+      d.second_treelet = next;
+      st.last_prefetched_second = next;
     }
   }
   st.queue_len = (uint32_t)queue;
-  a.state[g] = st;
-  a.out[g] = d;
+  __syncwarp();  // every lane has read the state
+  if (lane == 0) {
+    a.state[g] = st;
+    a.out[g] = d;
+  }
 }
 
 }  // namespace rtk
