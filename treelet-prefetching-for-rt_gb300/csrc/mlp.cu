@@ -11,7 +11,7 @@
 // runs on the fifth-generation tensor cores (tcgen05.mma with accumulators in
 // tensor memory) fused with the softmax cross-entropy, so the batch x
 // treelets logits are never stored (mlp_tc.cuh).  The two hidden layers
-// (4096 x 64 x 64 at most) run on mma.sync m16n8k16 tiles.
+// (4096 x 64 x 64 at most) run on mma.sync m16n8k16 tiles, one fused kernel each way.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -30,14 +30,13 @@ constexpr int XIN = 22;           // real inputs
 constexpr int XP = 32;            // padded input width
 using bf16 = __nv_bfloat16;
 
-// ----------------------------------------------------------------- GEMM
-// C[M x N] (+)= A[M x K] * B[K x N].  A is read row-major (AT = false:
-// A[m * lda + k]) or transposed (AT = true: A[k * lda + m]); B is read
-// row-major (BT = false: B[k * ldb + n]) or transposed (BT = true:
-// B[n * ldb + k]).  64 x 64 CTA tile, 4 warps of 32 x 32, K in steps of 32;
-// gridDim.z splits K, partial sums are added atomically (EPI_ACC).
-enum Epi { EPI_STORE = 0, EPI_ACC = 1, EPI_BIAS_GELU = 2, EPI_BIAS = 3 };
-
+// ------------------------------------------------------------ hidden layers
+// One CTA of eight warps per 64 samples runs both hidden layers, forward or
+// backward, with its operands in shared memory; warp w owns rows 16 (w % 4) ..
+// + 15 and column half w / 4 of a product's output (mma.sync m16n8k16, K
+// ascending).  As separate products and elementwise kernels of 10-64 CTAs each,
+// the two directions took 15 launches and 150 us of a 4,096-sample step on a
+// GB300, nearly all of it latency; fused they take 24 us.
 __device__ __forceinline__ float gelu(float x) { return 0.5f * x * (1.0f + erff(x * 0.70710678118654752f)); }
 __device__ __forceinline__ float gelu_grad(float x) {
   const float cdf = 0.5f * (1.0f + erff(x * 0.70710678118654752f));
@@ -45,152 +44,251 @@ __device__ __forceinline__ float gelu_grad(float x) {
   return cdf + x * pdf;
 }
 
-template <bool AT, bool BT, int EPI>
-__global__ void __launch_bounds__(128) gemm_kernel(int M, int N, int K, const bf16* __restrict__ A, int lda,
-                                                   const bf16* __restrict__ B, int ldb, float* __restrict__ C,
-                                                   int ldc, const float* __restrict__ bias, bf16* __restrict__ Hout) {
-  constexpr int BM = 64, BN = 64, BK = 32, PAD = 8;
-  __shared__ __align__(16) bf16 As[BM][BK + PAD];
-  __shared__ __align__(16) bf16 Bs[BN][BK + PAD];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int wm = (warp >> 1) * 32, wn = (warp & 1) * 32;
-  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-  // K range of this split
-  const int splits = gridDim.z;
-  const int kchunk = ((K + splits * BK - 1) / (splits * BK)) * BK;
-  const int kbeg = blockIdx.z * kchunk, kend = min(K, kbeg + kchunk);
-  float acc[2][4][4];
+constexpr int HB = 64;        // samples per CTA
+constexpr int HT = 256;       // threads per CTA
+constexpr int HP = H + 8;     // padded rows of the 64-wide tiles (16-byte rows, fragments on distinct banks)
+constexpr int XPP = XP + 8;   // padded rows of the 32-wide tiles
+
+__device__ __forceinline__ uint32_t pair_at(const bf16* p) { return *reinterpret_cast<const uint32_t*>(p); }
+
+// acc[j] (16 rows from `row0`, columns col0 + 8j .. + 7) = A[row][k] . B[n][k]^T,
+// both K-contiguous in shared memory, over K = 16 KS.
+template <int NT, int KS, int LDA, int LDB>
+__device__ __forceinline__ void tile_mma(float (&acc)[NT][4], const bf16 (*A)[LDA], int row0, const bf16 (*B)[LDB],
+                                         int col0) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
 #pragma unroll
-  for (int i = 0; i < 2; ++i)
+  for (int j = 0; j < NT; ++j)
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
+    for (int r = 0; r < 4; ++r) acc[j][r] = 0.0f;
 #pragma unroll
-      for (int r = 0; r < 4; ++r) acc[i][j][r] = 0.0f;
-  const bf16 zero = __float2bfloat16(0.0f);
-  for (int k0 = kbeg; k0 < kend; k0 += BK) {
-    for (int e = tid; e < BM * BK; e += 128) {
-      const int r = e / BK, c = e % BK;
-      const int m = m0 + r, k = k0 + c;
-      bf16 v = zero;
-      if (m < M && k < kend) v = AT ? A[(size_t)k * lda + m] : A[(size_t)m * lda + k];
-      As[r][c] = v;
+  for (int ks = 0; ks < KS; ++ks) {
+    const int k = ks * 16 + 2 * t;
+    const uint32_t a0 = pair_at(&A[row0 + g][k]), a1 = pair_at(&A[row0 + g + 8][k]);
+    const uint32_t a2 = pair_at(&A[row0 + g][k + 8]), a3 = pair_at(&A[row0 + g + 8][k + 8]);
+#pragma unroll
+    for (int j = 0; j < NT; ++j) {
+      const uint32_t b0 = pair_at(&B[col0 + j * 8 + g][k]), b1 = pair_at(&B[col0 + j * 8 + g][k + 8]);
+      asm volatile(
+          "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+          "{%0,%1,%2,%3};\n"
+          : "+f"(acc[j][0]), "+f"(acc[j][1]), "+f"(acc[j][2]), "+f"(acc[j][3])
+          : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
     }
-    for (int e = tid; e < BN * BK; e += 128) {
-      const int r = e / BK, c = e % BK;
-      const int n = n0 + r, k = k0 + c;
-      bf16 v = zero;
-      if (n < N && k < kend) v = BT ? B[(size_t)n * ldb + k] : B[(size_t)k * ldb + n];
-      Bs[r][c] = v;
-    }
-    __syncthreads();
-    const int g = lane >> 2, t = lane & 3;
-#pragma unroll
-    for (int kk = 0; kk < BK; kk += 16) {
-      uint32_t af[2][4], bfr[4][2];
-#pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const int rb = wm + i * 16;
-        af[i][0] = *reinterpret_cast<const uint32_t*>(&As[rb + g][kk + 2 * t]);
-        af[i][1] = *reinterpret_cast<const uint32_t*>(&As[rb + g + 8][kk + 2 * t]);
-        af[i][2] = *reinterpret_cast<const uint32_t*>(&As[rb + g][kk + 2 * t + 8]);
-        af[i][3] = *reinterpret_cast<const uint32_t*>(&As[rb + g + 8][kk + 2 * t + 8]);
-      }
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int nb = wn + j * 8;
-        bfr[j][0] = *reinterpret_cast<const uint32_t*>(&Bs[nb + g][kk + 2 * t]);
-        bfr[j][1] = *reinterpret_cast<const uint32_t*>(&Bs[nb + g][kk + 2 * t + 8]);
-      }
-#pragma unroll
-      for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-          asm volatile(
-              "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-              "{%0,%1,%2,%3};\n"
-              : "+f"(acc[i][j][0]), "+f"(acc[i][j][1]), "+f"(acc[i][j][2]), "+f"(acc[i][j][3])
-              : "r"(af[i][0]), "r"(af[i][1]), "r"(af[i][2]), "r"(af[i][3]), "r"(bfr[j][0]), "r"(bfr[j][1]));
-    }
-    __syncthreads();
   }
-  const int g = lane >> 2, t = lane & 3;
+}
+
+// Row and column of accumulator element (j, r) of the calling lane.
+__device__ __forceinline__ int acc_row(int row0, int r) { return row0 + ((threadIdx.x & 31) >> 2) + (r >= 2 ? 8 : 0); }
+__device__ __forceinline__ int acc_col(int col0, int j, int r) { return col0 + j * 8 + 2 * (threadIdx.x & 3) + (r & 1); }
+
+// Eight consecutive elements at once.
+struct Eight {
+  bf16 v[8];
+};
+__device__ __forceinline__ Eight load8(const bf16* p) {
+  Eight e;
+  *reinterpret_cast<uint4*>(e.v) = *reinterpret_cast<const uint4*>(p);
+  return e;
+}
+__device__ __forceinline__ void store8(bf16* p, const Eight& e) {
+  *reinterpret_cast<uint4*>(p) = *reinterpret_cast<const uint4*>(e.v);
+}
+__device__ __forceinline__ void load8f(const float* p, float* v) {
+  *reinterpret_cast<float4*>(v) = *reinterpret_cast<const float4*>(p);
+  *reinterpret_cast<float4*>(v + 4) = *reinterpret_cast<const float4*>(p + 4);
+}
+
+// x = [origin, dir, E[current]] (a sample whose current treelet is out of range
+// gets a zero embedding); h1 = GELU(x W1 + b1), h2 = GELU(h1 W2 + b2).  Stores
+// x, z1, h1, z2, h2 and, for the output layer's dW3 product, [h2^T ; ones ;
+// zeros] (h2x, 80 x ldx, columns past n zero).
+__global__ void __launch_bounds__(HT) hidden_forward_kernel(
+    const rt_mlp_sample* __restrict__ s, int n, const bf16* __restrict__ E, uint32_t C, const bf16* __restrict__ W1,
+    const float* __restrict__ b1, const bf16* __restrict__ W2, const float* __restrict__ b2, bf16* __restrict__ X,
+    float* __restrict__ Z1, bf16* __restrict__ H1, float* __restrict__ Z2, bf16* __restrict__ H2,
+    bf16* __restrict__ H2X, int ldx) {
+  __shared__ __align__(16) bf16 xs[HB][XPP], w1[H][XPP], w2[H][HP], h1[HB][HP], h2t[tcm::HX][HP];
+  const int tid = threadIdx.x, row0 = ((tid >> 5) & 3) * 16, col0 = (tid >> 7) * 32, base = blockIdx.x * HB;
+  {  // four threads a sample: origin and direction, the embedding's halves, zeros
+    const int b = tid >> 2, part = tid & 3;
+    Eight e;
 #pragma unroll
-  for (int i = 0; i < 2; ++i)
+    for (int q = 0; q < 8; ++q) e.v[q] = __float2bfloat16(0.0f);
+    if (base + b < n) {
+      const rt_mlp_sample q = s[base + b];
+      const bool has = q.current < C;
+      if (part == 0) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
-#pragma unroll
-      for (int r = 0; r < 4; ++r) {
-        const int m = m0 + wm + i * 16 + g + (r >= 2 ? 8 : 0);
-        const int n = n0 + wn + j * 8 + 2 * t + (r & 1);
-        if (m >= M || n >= N) continue;
-        float v = acc[i][j][r];
-        float* dst = C + (size_t)m * ldc + n;
-        if (EPI == EPI_ACC) {
-          atomicAdd(dst, v);
-        } else if (EPI == EPI_STORE) {
-          *dst = v;
-        } else {
-          v += bias[n];
-          *dst = v;
-          if (EPI == EPI_BIAS_GELU) Hout[(size_t)m * ldc + n] = __float2bfloat16(gelu(v));
+        for (int k = 0; k < 3; ++k) {
+          e.v[k] = __float2bfloat16(q.origin[k]);
+          e.v[3 + k] = __float2bfloat16(q.dir[k]);
         }
+        if (has) e.v[6] = E[(size_t)q.current * EMB], e.v[7] = E[(size_t)q.current * EMB + 1];
+      } else if (has) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+          if (part * 8 + k < XIN) e.v[k] = E[(size_t)q.current * EMB + part * 8 + k - 6];
       }
-}
-
-template <bool AT, bool BT, int EPI>
-void gemm(int M, int N, int K, const bf16* A, int lda, const bf16* B, int ldb, float* C, int ldc, const float* bias,
-          bf16* Hout, int splits, cudaStream_t st) {
-  dim3 grid((N + 63) / 64, (M + 63) / 64, splits);
-  gemm_kernel<AT, BT, EPI><<<grid, 128, 0, st>>>(M, N, K, A, lda, B, ldb, C, ldc, bias, Hout);
-}
-
-// ------------------------------------------------------------ elementwise
-// A sample whose current treelet is out of range gets a zero embedding.
-__global__ void gather_inputs(const rt_mlp_sample* __restrict__ s, int n, const bf16* __restrict__ E, uint32_t C,
-                              bf16* __restrict__ X) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n * XP) return;
-  const int b = i / XP, c = i % XP;
-  float v = 0.0f;
-  if (c < 3) v = s[b].origin[c];
-  else if (c < 6) v = s[b].dir[c - 3];
-  else if (c < XIN) {
-    const uint32_t cur = s[b].current;
-    X[i] = cur < C ? E[(size_t)cur * EMB + (c - 6)] : __float2bfloat16(0.0f);
-    return;
+      store8(X + (size_t)(base + b) * XP + part * 8, e);
+    }
+    store8(&xs[b][part * 8], e);
   }
-  X[i] = __float2bfloat16(v);
+  {  // W1 (32 x 64) and W2 (64 x 64) transposed
+    const Eight e = load8(W1 + tid * 8), f = load8(W2 + tid * 8), g = load8(W2 + (HT + tid) * 8);
+    const int r = tid / 8, c = tid % 8 * 8;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      w1[c + q][r] = e.v[q];
+      w2[c + q][r] = f.v[q];
+      w2[c + q][r + 32] = g.v[q];
+    }
+  }
+  __syncthreads();
+  float acc[4][4];
+  tile_mma<4, XP / 16, XPP, XPP>(acc, xs, row0, w1, col0);
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const int m = acc_row(row0, r), c = acc_col(col0, j, r);
+      const float z = acc[j][r] + b1[c];
+      const bf16 h = __float2bfloat16(gelu(z));
+      h1[m][c] = h;
+      if (base + m < n) {
+        Z1[(size_t)(base + m) * H + c] = z;
+        H1[(size_t)(base + m) * H + c] = h;
+      }
+    }
+  __syncthreads();
+  tile_mma<4, H / 16, HP, HP>(acc, h1, row0, w2, col0);
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const int m = acc_row(row0, r), c = acc_col(col0, j, r);
+      const float z = acc[j][r] + b2[c];
+      const bool in = base + m < n;
+      const bf16 h = __float2bfloat16(in ? gelu(z) : 0.0f);
+      h2t[c][m] = h;
+      if (in) {
+        Z2[(size_t)(base + m) * H + c] = z;
+        H2[(size_t)(base + m) * H + c] = h;
+      }
+    }
+  for (int i = tid; i < (tcm::HX - H) * HB; i += HT)
+    h2t[H + i / HB][i % HB] = __float2bfloat16(i / HB == 0 && base + i % HB < n ? 1.0f : 0.0f);
+  __syncthreads();
+  // ldx is a multiple of HB: every CTA writes whole rows of its columns
+  for (int i = tid; i < tcm::HX * (HB / 8); i += HT) {
+    const int k = i / (HB / 8), q = (i % (HB / 8)) * 8;
+    store8(H2X + (size_t)k * ldx + base + q, load8(&h2t[k][q]));
+  }
 }
 
-// dZ = dH * GELU'(Z) as BF16.
-__global__ void gelu_back(const float* __restrict__ dH, const float* __restrict__ Z, bf16* __restrict__ dZ, int count) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < count) dZ[i] = __float2bfloat16(dH[i] * gelu_grad(Z[i]));
-}
-
-// out[c] += sum_r X[r][c]: one block per 128 rows, one thread per column
-// (out starts at zero).  One block over all rows took 0.22 ms for 4,096 x 64.
-__global__ void col_sum(const bf16* __restrict__ X, int rows, int cols, float* __restrict__ out) {
-  const int c = threadIdx.x;
-  if (c >= cols) return;
-  const int r0 = blockIdx.x * 128, r1 = min(rows, r0 + 128);
-  float s = 0.0f;
-  for (int r = r0; r < r1; ++r) s += __bfloat162float(X[(size_t)r * cols + c]);
-  atomicAdd(out + c, s);
-}
-
-__global__ void embed_grad(const float* __restrict__ dX, const rt_mlp_sample* __restrict__ s, int n, uint32_t C,
-                           float* __restrict__ gE) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n * EMB) return;
-  const int b = i / EMB, j = i % EMB;
-  const uint32_t cur = s[b].current;
-  if (cur < C) atomicAdd(gE + (size_t)cur * EMB + j, dX[(size_t)b * XP + 6 + j]);
-}
-
-__global__ void copy_rows(const float* __restrict__ src, int src_ld, float* __restrict__ dst, int rows, int cols) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < rows * cols) dst[i] = src[(size_t)(i / cols) * src_ld + (i % cols)];
+// dz2 = dh2 * GELU'(z2), [dW2, db2] += h1^T [dz2], dh1 = dz2 W2^T, dz1 = dh1 *
+// GELU'(z1), [dW1, db1] += x^T [dz1], dx = dz1 W1^T into the embedding's rows.
+// The dz are BF16, products FP32; weight gradients are added into G.
+__global__ void __launch_bounds__(HT) hidden_backward_kernel(
+    const rt_mlp_sample* __restrict__ s, int n, uint32_t C, const bf16* __restrict__ W1, const bf16* __restrict__ W2,
+    const bf16* __restrict__ X, const float* __restrict__ Z1, const bf16* __restrict__ H1,
+    const float* __restrict__ Z2, const float* __restrict__ dH2, float* __restrict__ gE, float* __restrict__ gW1,
+    float* __restrict__ gb1, float* __restrict__ gW2, float* __restrict__ gb2) {
+  __shared__ __align__(16) bf16 dz[HB][HP], dzt[H][HP], ht[H][HP], w[H][HP], xt[XP][HP];
+  const int tid = threadIdx.x, warp = tid >> 5, row0 = (warp & 3) * 16, col0 = (warp >> 2) * 32, base = blockIdx.x * HB;
+  const bf16 zero = __float2bfloat16(0.0f);
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {  // eight columns of a sample at a time
+    const int i = h * HT + tid, b = i / 8, c = i % 8 * 8;
+    Eight d, e;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) d.v[q] = e.v[q] = zero;
+    if (base + b < n) {
+      float g[8], z[8];
+      load8f(dH2 + (size_t)(base + b) * H + c, g);
+      load8f(Z2 + (size_t)(base + b) * H + c, z);
+      e = load8(H1 + (size_t)(base + b) * H + c);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) d.v[q] = __float2bfloat16(g[q] * gelu_grad(z[q]));
+    }
+    store8(&dz[b][c], d);
+    store8(&w[b][c], load8(W2 + i * 8));  // 64 x 64 as well: W2[k][c] row-major
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      dzt[c + q][b] = d.v[q];
+      ht[c + q][b] = e.v[q];
+    }
+  }
+  {
+    const int b = tid >> 2, c = (tid & 3) * 8;
+    Eight e;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) e.v[q] = zero;
+    if (base + b < n) e = load8(X + (size_t)(base + b) * XP + c);
+#pragma unroll
+    for (int q = 0; q < 8; ++q) xt[c + q][b] = e.v[q];
+  }
+  // z1 of this thread's accumulator elements, on its way while the products run
+  float z1[4][4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const int b = base + acc_row(row0, r);
+      z1[j][r] = b < n ? Z1[(size_t)b * H + acc_col(col0, j, r)] : 0.0f;
+    }
+  __syncthreads();
+  float acc[4][4];
+  // dW2[i][c] = sum_b h1[b][i] dz2[b][c]
+  tile_mma<4, HB / 16, HP, HP>(acc, ht, row0, dzt, col0);
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+#pragma unroll
+    for (int r = 0; r < 4; ++r) atomicAdd(gW2 + acc_row(row0, r) * H + acc_col(col0, j, r), acc[j][r]);
+  auto column_sum = [&](int c, float* out) {  // four threads a column
+    float sum = 0.0f;
+#pragma unroll
+    for (int b = 0; b < HB / 4; ++b) sum += __bfloat162float(dzt[c >> 2][(c & 3) * (HB / 4) + b]);
+    sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+    sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+    if ((c & 3) == 0) atomicAdd(out + (c >> 2), sum);
+  };
+  column_sum(tid, gb2);
+  // dh1[b][k] = sum_c dz2[b][c] W2[k][c]
+  tile_mma<4, H / 16, HP, HP>(acc, dz, row0, w, col0);
+  __syncthreads();  // every reader of dz, dzt and w is done
+  store8(&w[tid / 8][tid % 8 * 8], load8(W1 + tid * 8));
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const int b = acc_row(row0, r), c = acc_col(col0, j, r);
+      const bf16 d = base + b < n ? __float2bfloat16(acc[j][r] * gelu_grad(z1[j][r])) : zero;
+      dz[b][c] = d;
+      dzt[c][b] = d;
+    }
+  __syncthreads();
+  column_sum(tid, gb1);
+  if (row0 < XP) {  // dW1[i][c] = sum_b x[b][i] dz1[b][c], 22 of the 32 padded rows
+    tile_mma<4, HB / 16, HP, HP>(acc, xt, row0, dzt, col0);
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+        if (acc_row(row0, r) < XIN) atomicAdd(gW1 + acc_row(row0, r) * H + acc_col(col0, j, r), acc[j][r]);
+  }
+  // dx[b][i] = sum_c dz1[b][c] W1[i][c]; columns 6 .. 21 are the embedding's
+  float dx[2][4];
+  tile_mma<2, H / 16, HP, HP>(dx, dz, row0, w, col0 / 2);
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const int b = acc_row(row0, r), c = acc_col(col0 / 2, j, r);
+      if (c < 6 || c >= XIN || base + b >= n) continue;
+      const uint32_t cur = s[base + b].current;
+      if (cur < C) atomicAdd(gE + (size_t)cur * EMB + (c - 6), dx[j][r]);
+    }
 }
 
 __global__ void adam(float* __restrict__ p, float* __restrict__ m, float* __restrict__ v, const float* __restrict__ g,
@@ -245,11 +343,11 @@ struct rt_mlp {
   bf16 *E16 = nullptr, *W1_16 = nullptr, *W2_16 = nullptr;
   bf16 *W3T = nullptr, *W3P = nullptr, *H2X = nullptr;  // output-layer operands (mlp_tc.cuh)
   uint32_t Cp = 0;                                     // treelets padded to the output chunk
-  bf16 *X = nullptr, *H1 = nullptr, *H2 = nullptr, *dZ2 = nullptr, *dZ1 = nullptr;
-  float *Z1 = nullptr, *Z2 = nullptr, *dH2 = nullptr, *dH1 = nullptr, *dX = nullptr, *dW1 = nullptr;
+  bf16 *X = nullptr, *H1 = nullptr, *H2 = nullptr;
+  float *Z1 = nullptr, *Z2 = nullptr, *dH2 = nullptr;
   float *lse = nullptr, *part = nullptr;
   uint32_t* tstatus = nullptr;                         // bit 0: a bounded wait of the output layer gave up
-  float* loss = nullptr;
+  double* loss = nullptr;                              // sum over the samples of their loss / n
   uint64_t step = 0;
   cudaStream_t st = nullptr;
 };
@@ -328,62 +426,41 @@ void output_forward(rt_mlp* m, const rt_mlp_sample* s, uint32_t n, uint32_t* top
     return;
   }
   tcm::out_stats_kernel<false><<<grid, tcm::kThreads, kSmemStats, m->st>>>(a);
-  tcm::out_lse_kernel<<<blocks(n), 256, 0, m->st>>>(m->part, 2 * a.splits, n, s, m->C, m->lse, m->loss);
+  tcm::out_lse_kernel<<<blocks(n, tcm::kLseRows), tcm::kLseWarps * 32, 0, m->st>>>(m->part, 2 * a.splits, n, s, m->C,
+                                                                                  m->lse, m->loss);
 }
 
 // Gradients of the output layer: dW3, db3 into G, dH2 (zeroed first).
 void output_backward(rt_mlp* m, const rt_mlp_sample* s, uint32_t n) {
   const tcm::OutArgs a = out_args(m, s, n);
-  tcm::h2x_kernel<<<blocks((uint64_t)tcm::HX * RT_MLP_MAX_BATCH), 256, 0, m->st>>>(m->H2, n, RT_MLP_MAX_BATCH,
-                                                                                   m->H2X);
   tcm::out_dh2_kernel<<<dim3((n + tcm::TM - 1) / tcm::TM, a.splits), tcm::kThreads, kSmemDh2, m->st>>>(a);
   // two row halves per chunk, added into the zeroed gradient: 1,494 CTAs
   // (4.9 waves of 304) instead of 747 (2.5 waves)
   tcm::out_dw3_kernel<<<dim3(m->Cp / tcm::TN, 2), tcm::kThreads, kSmemDw3, m->st>>>(a);
 }
 
-int ksplit(int K, int tiles) {
-  // enough CTAs to cover the GPU when the output has few tiles
-  int s = 1;
-  while (tiles * s < 304 && K / (s * 2) >= 256) s *= 2;
-  return s;
-}
-
 // Forward (and, when grads is true, backward into G) for n samples.
 rt_status run(rt_mlp* m, const rt_mlp_sample* s, uint32_t n, bool grads, uint32_t* top4) {
   const int B = (int)n;
   cudaStream_t st = m->st;
-  gather_inputs<<<blocks((uint64_t)B * XP), 256, 0, st>>>(s, B, m->E16, m->C, m->X);
-  gemm<false, false, EPI_BIAS_GELU>(B, H, XP, m->X, XP, m->W1_16, H, m->Z1, H, m->P + m->offb1, m->H1, 1, st);
-  gemm<false, false, EPI_BIAS_GELU>(B, H, H, m->H1, H, m->W2_16, H, m->Z2, H, m->P + m->offb2, m->H2, 1, st);
+  // whole 128-row tiles: the output layer reads h2x's columns past n as zero
+  hidden_forward_kernel<<<(B + tcm::TM - 1) / tcm::TM * (tcm::TM / HB), HT, 0, st>>>(s, B, m->E16, m->C, m->W1_16, m->P + m->offb1, m->W2_16,
+                                                           m->P + m->offb2, m->X, m->Z1, m->H1, m->Z2, m->H2, m->H2X,
+                                                           (int)RT_MLP_MAX_BATCH);
   if (top4) {
     output_forward(m, s, n, top4);
     return RT_OK;
   }
-  MLP_CUDA(cudaMemsetAsync(m->loss, 0, sizeof(float), st));
+  MLP_CUDA(cudaMemsetAsync(m->loss, 0, sizeof(double), st));
   output_forward(m, s, n, nullptr);
   if (!grads) return RT_OK;
   MLP_CUDA(cudaMemsetAsync(m->G, 0, sizeof(float) * m->n_params, st));
   // W3, b3 and dH2 = dz W3^T, on the tensor cores without the logits
   MLP_CUDA(cudaMemsetAsync(m->dH2, 0, sizeof(float) * B * H, st));
   output_backward(m, s, n);
-  gelu_back<<<blocks((uint64_t)B * H), 256, 0, st>>>(m->dH2, m->Z2, m->dZ2, B * H);
-  // W2, b2
-  gemm<true, false, EPI_ACC>(H, H, B, m->H1, H, m->dZ2, H, m->G + m->offW2, H, nullptr, nullptr, ksplit(B, 1), st);
-  col_sum<<<(B + 127) / 128, H, 0, st>>>(m->dZ2, B, H, m->G + m->offb2);
-  // dH1 = dZ2 W2^T
-  MLP_CUDA(cudaMemsetAsync(m->dH1, 0, sizeof(float) * B * H, st));
-  gemm<false, true, EPI_ACC>(B, H, H, m->dZ2, H, m->W2_16, H, m->dH1, H, nullptr, nullptr, 1, st);
-  gelu_back<<<blocks((uint64_t)B * H), 256, 0, st>>>(m->dH1, m->Z1, m->dZ1, B * H);
-  // W1 (first 22 rows of the padded product), b1
-  MLP_CUDA(cudaMemsetAsync(m->dW1, 0, sizeof(float) * XP * H, st));
-  gemm<true, false, EPI_ACC>(XP, H, B, m->X, XP, m->dZ1, H, m->dW1, H, nullptr, nullptr, ksplit(B, 1), st);
-  copy_rows<<<blocks(XIN * H), 256, 0, st>>>(m->dW1, H, m->G + m->offW1, XIN, H);
-  col_sum<<<(B + 127) / 128, H, 0, st>>>(m->dZ1, B, H, m->G + m->offb1);
-  // dX = dZ1 W1^T -> embedding rows
-  MLP_CUDA(cudaMemsetAsync(m->dX, 0, sizeof(float) * B * XP, st));
-  gemm<false, true, EPI_ACC>(B, XP, H, m->dZ1, H, m->W1_16, H, m->dX, XP, nullptr, nullptr, 1, st);
-  embed_grad<<<blocks((uint64_t)B * EMB), 256, 0, st>>>(m->dX, s, B, m->C, m->G);
+  hidden_backward_kernel<<<(B + HB - 1) / HB, HT, 0, st>>>(s, B, m->C, m->W1_16, m->W2_16, m->X, m->Z1, m->H1, m->Z2,
+                                                            m->dH2, m->G, m->G + m->offW1, m->G + m->offb1,
+                                                            m->G + m->offW2, m->G + m->offb2);
   return RT_OK;
 }
 
@@ -436,17 +513,12 @@ rt_status rt_mlp_create(rt_ctx* ctx, uint32_t n_treelets, uint64_t seed, rt_mlp*
   chk(mk(&m->X, MB * XP));
   chk(mk(&m->H1, MB * H));
   chk(mk(&m->H2, MB * H));
-  chk(mk(&m->dZ2, MB * H));
-  chk(mk(&m->dZ1, MB * H));
   chk(mk(&m->Z1, MB * H));
   chk(mk(&m->Z2, MB * H));
   chk(mk(&m->lse, MB));
   chk(mk(&m->part, 8 * 152 * 2 * MB));  // 2 x 152 partial results of 8 floats per row
   chk(mk(&m->tstatus, 1));
   chk(mk(&m->dH2, MB * H));
-  chk(mk(&m->dH1, MB * H));
-  chk(mk(&m->dX, MB * XP));
-  chk(mk(&m->dW1, XP * H));
   chk(mk(&m->loss, 1));
   chk(cudaStreamCreateWithFlags(&m->st, cudaStreamNonBlocking));
   chk(cudaFuncSetAttribute(tcm::out_stats_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemStats));
@@ -476,8 +548,7 @@ rt_status rt_mlp_destroy(rt_mlp* m) {
   if (!m) return RT_OK;
   cudaSetDevice(m->device);
   void* ptrs[] = {m->P, m->M, m->V, m->G, m->E16, m->W1_16, m->W2_16, m->W3T, m->W3P, m->H2X, m->X, m->H1,
-                  m->H2, m->dZ2, m->dZ1, m->Z1, m->Z2, m->dH2, m->dH1, m->dX, m->dW1, m->lse, m->part,
-                  m->tstatus, m->loss};
+                  m->H2, m->Z1, m->Z2, m->dH2, m->lse, m->part, m->tstatus, m->loss};
   for (void* p : ptrs) cudaFree(p);
   if (m->st) cudaStreamDestroy(m->st);
   delete m;
@@ -518,7 +589,11 @@ rt_status rt_mlp_loss_grad(rt_mlp* m, const rt_mlp_sample* s, uint32_t n, float*
   MLP_CUDA(cudaStreamSynchronize(m->st));
   st = check_status(m, "rt_mlp_loss_grad");
   if (st != RT_OK) return st;
-  if (loss) MLP_CUDA(cudaMemcpy(loss, m->loss, sizeof(float), cudaMemcpyDeviceToHost));
+  if (loss) {
+    double sum = 0.0;
+    MLP_CUDA(cudaMemcpy(&sum, m->loss, sizeof(sum), cudaMemcpyDeviceToHost));
+    *loss = (float)sum;
+  }
   if (grads_host) MLP_CUDA(cudaMemcpy(grads_host, m->G, sizeof(float) * m->n_params, cudaMemcpyDeviceToHost));
   return RT_OK;
 }
@@ -535,8 +610,10 @@ rt_status rt_mlp_train_step(rt_mlp* m, const rt_mlp_sample* s, uint32_t n, float
   refresh_bf16(m);
   MLP_CUDA(cudaGetLastError());
   if (loss) {
-    MLP_CUDA(cudaMemcpyAsync(loss, m->loss, sizeof(float), cudaMemcpyDeviceToHost, m->st));
+    double sum = 0.0;
+    MLP_CUDA(cudaMemcpyAsync(&sum, m->loss, sizeof(sum), cudaMemcpyDeviceToHost, m->st));
     MLP_CUDA(cudaStreamSynchronize(m->st));
+    *loss = (float)sum;
     return check_status(m, "rt_mlp_train_step");
   }
   return RT_OK;
