@@ -139,3 +139,48 @@ def test_launch_sizes(ctx, n):
         assert_hits_equal(got, hits, f"untraced hits, mode {mode}, {n} rays")
         assert scene.stats()["node_bytes"] == node_bytes
     scene.close()
+
+
+@pytest.mark.parametrize("n", [1, 8192, 8193, 16384, 16385, 131073])
+@pytest.mark.parametrize("pinned", [True, False])
+def test_packed_call_sizes(ctx, n, pinned):
+    """Packed traces where the call changes its way: one block or four kernels
+    for the offsets, straight into page-locked arrays or through copies, one or
+    two chunks; arrays one entry too small; treelet ids alone."""
+    import ctypes as C
+
+    import torch
+
+    import treelet_rt as rt
+
+    scene = rt.Scene(ctx, rt.Blob.gen(rt.SCENE_CUBE_PLANE, 3000, 6))
+    scene.form_treelets(1024)
+    cam = rt.default_camera(rt.SCENE_CUBE_PLANE)
+    rays = np.resize(rt.camera_rays(cam, 190, 97, 1, 2, 1e-4, 1e30), n)
+    cap = 24  # some rays have more
+    hits, vis, tids = scene.trace_host(rays, rt.MODE_TREELET, capacity=cap, want_visits=True, want_treelets=True)
+    keep = np.arange(cap)[None, :] < hits["n_visits"][:, None]
+    total = int(keep.sum())
+    want_off = np.concatenate([[0], np.cumsum(keep.sum(axis=1))])
+
+    def array(a):
+        t = torch.from_numpy(a)
+        return t.pin_memory() if pinned else t.clone()
+
+    d_rays = array(rays.view(np.uint8).copy())
+    for visits, room in ((True, total), (True, total - 1), (False, total)):
+        h, off = array(np.zeros(n * 64, np.uint8)), array(np.zeros(n + 1, np.int64))
+        v, t = array(np.zeros(max(room, 1), np.int32)), array(np.zeros(max(room, 1), np.int32))
+        got = C.c_uint64(0)
+        st = rt.lib().rt_trace_host_packed(scene.handle, d_rays.data_ptr(), None, 1, n, rt.MODE_TREELET, cap,
+                                           h.data_ptr(), off.data_ptr(), v.data_ptr() if visits else None,
+                                           t.data_ptr(), room, C.byref(got))
+        assert st == (0 if room >= total else 6), rt.lib().rt_last_error().decode()
+        assert got.value == total
+        assert np.array_equal(off.numpy(), want_off)
+        assert_hits_equal(h.numpy().view(rt.HIT_DTYPE), hits, "packed hits")
+        if room >= total:
+            assert np.array_equal(t.numpy().view(np.uint32)[:total], tids[keep])
+            if visits:
+                assert np.array_equal(v.numpy().view(np.uint32)[:total], vis[keep])
+    scene.close()

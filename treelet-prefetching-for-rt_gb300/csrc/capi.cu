@@ -126,6 +126,17 @@ struct QueueScratch {
 
 }  // namespace rti
 
+namespace rti {
+
+// Counters, status word and ray hand-out counters of a scene's (or a batch's)
+// launches: one block, so that one memset clears them.
+struct Control {
+  unsigned long long stats[rtk::ST_COUNT];
+  uint32_t status, queue[kHostChunks];
+};
+
+}  // namespace rti
+
 struct rt_scene {
   rt_ctx* ctx = nullptr;
   std::vector<uint8_t> host_blob;
@@ -172,9 +183,10 @@ struct rt_scene {
   };
   std::vector<PinImage> pin_cache;
   // per-launch counters and status (library scratch)
-  unsigned long long* d_stats = nullptr;
+  rti::Control* d_ctl = nullptr;
+  unsigned long long* d_stats = nullptr;  // in d_ctl
   uint32_t* d_status = nullptr;
-  uint32_t* d_queue = nullptr;  // ray hand-out counter of the persistent kernels
+  uint32_t* d_queue = nullptr;  // ray hand-out counters of the persistent kernels
   rt_tuning tuning{128, 256, 16, RT_TUNING_OFF, 8, 2048, 8, 96, 4096, rtk::kWaitTries, RT_TUNING_OFF, RT_TUNING_OFF};
   // host-buffer path: a copy-in stream, two trace streams (chunk c on
   // stream / stream2 by parity, so one chunk's launch fills the SMs that the
@@ -185,7 +197,9 @@ struct rt_scene {
   size_t io_bytes = 0;
   void* d_pack = nullptr;  // packed access traces of rt_trace_host_packed
   size_t pack_bytes = 0;
-  unsigned long long* h_tot = nullptr;  // page-locked chunk totals of rt_trace_host_packed
+  // page-locked words the host path's kernels and copies write: the chunks'
+  // totals of rt_trace_host_packed, then the status word
+  unsigned long long* h_words = nullptr;
   rti::QueueScratch qs;  // treelet queues of RT_MODE_STAGED with queue_rounds
 };
 
@@ -566,19 +580,16 @@ rt_status launch_group(rtk::TraceArgs& a, bool treelet, uint32_t depth, cudaStre
   return RT_OK;
 }
 
-// Zeroes the launch's queue (and its counters unless `keep` is set: chunks of
-// one call add up), then launches the kernel of `mode` with stack depth CAP.
+// Zeroes the launch's control block (a.stats is its start; unless `keep` is
+// set: the chunks of one call add up, and the caller has cleared it), then
+// launches the kernel of `mode` with stack depth CAP.
 template <int CAP>
 rt_status launch_cap(rtk::TraceArgs& a, uint32_t mode, const rt_tuning& t, uint32_t largest_image, cudaStream_t st,
                      bool keep, const rti::QueueScratch* qs) {
   a.epoch = t.staged_epoch;
   a.refill = t.refill_lanes;
   a.wait_tries = t.wait_tries;
-  if (!keep) {
-    RT_CUDA(cudaMemsetAsync(a.stats, 0, sizeof(unsigned long long) * rtk::ST_COUNT, st));
-    RT_CUDA(cudaMemsetAsync(a.status, 0, sizeof(uint32_t), st));
-  }
-  RT_CUDA(cudaMemsetAsync(a.queue, 0, sizeof(uint32_t), st));
+  if (!keep) RT_CUDA(cudaMemsetAsync(a.stats, 0, sizeof(rti::Control), st));
   // A launch that writes traces runs the walks compiled with the trace code
   // (TRACED).  They write their rows a whole 32-byte sector at a time through
   // shared memory (rtk::trace_put) when every row starts on a 32-byte
@@ -754,19 +765,19 @@ rt_status rt_scene_create(rt_ctx* ctx, const rt_blob* blob, rt_scene** out) {
   if (st == RT_OK) st = dalloc(&s->d_walk, s->blob_bytes);
   s->mixed_roles = roles.mixed;
   if (st == RT_OK && !roles.mixed) st = dalloc(&s->d_internal, sizeof(uint32_t) * roles.internal.size());
-  if (st == RT_OK) st = dalloc(&s->d_stats, sizeof(unsigned long long) * rtk::ST_COUNT);
-  if (st == RT_OK) st = dalloc(&s->d_status, sizeof(uint32_t));
-  if (st == RT_OK) st = dalloc(&s->d_queue, sizeof(uint32_t) * rti::kHostChunks);
+  if (st == RT_OK) st = dalloc(&s->d_ctl, sizeof(rti::Control));
   if (st != RT_OK) {
     rt_scene_destroy(s);
     return st;
   }
+  s->d_stats = s->d_ctl->stats;
+  s->d_status = &s->d_ctl->status;
+  s->d_queue = s->d_ctl->queue;
   cudaError_t e = cudaMemcpy(s->d_blob, blob->bytes.data(), s->blob_bytes, cudaMemcpyHostToDevice);
   if (e == cudaSuccess && s->d_internal)
     e = cudaMemcpy(s->d_internal, roles.internal.data(), sizeof(uint32_t) * roles.internal.size(), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = make_walk_nodes(s, nullptr);
-  if (e == cudaSuccess) e = cudaMemset(s->d_stats, 0, sizeof(unsigned long long) * rtk::ST_COUNT);
-  if (e == cudaSuccess) e = cudaMemset(s->d_status, 0, sizeof(uint32_t));
+  if (e == cudaSuccess) e = cudaMemset(s->d_ctl, 0, sizeof(rti::Control));
   for (cudaStream_t* x : {&s->stream, &s->stream2, &s->xin, &s->xout})
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(x, cudaStreamNonBlocking);
   for (uint32_t c = 0; c < rti::kHostChunks; ++c) {
@@ -788,12 +799,10 @@ rt_status rt_scene_destroy(rt_scene* s) {
   cudaFree(s->d_blob);
   cudaFree(s->d_walk);
   cudaFree(s->d_internal);
-  cudaFree(s->d_stats);
-  cudaFree(s->d_status);
-  cudaFree(s->d_queue);
+  cudaFree(s->d_ctl);
   cudaFree(s->d_io);
   cudaFree(s->d_pack);
-  if (s->h_tot) cudaFreeHost(s->h_tot);
+  if (s->h_words) cudaFreeHost(s->h_words);
   cudaFree(s->qs.base);
   for (uint32_t c = 0; c < rti::kHostChunks; ++c) {
     if (s->ev_in[c]) cudaEventDestroy(s->ev_in[c]);
@@ -1033,6 +1042,43 @@ void* mapped_host(const void* p) {
   return at.type == cudaMemoryTypeHost ? at.devicePointer : nullptr;
 }
 
+// The same for an array of `bytes` bytes, all of it page-locked.
+void* mapped_range(const void* p, size_t bytes) {
+  uint8_t* first = static_cast<uint8_t*>(mapped_host(p));
+  if (!first || bytes == 0) return first;
+  return mapped_host(static_cast<const uint8_t*>(p) + bytes - 1) == first + bytes - 1 ? first : nullptr;
+}
+
+rt_status timeout_status(uint32_t status, const char* who) {
+  if (!(status & rtk::kStatusTimeout)) return RT_OK;
+  return rti::fail(RT_ERR_TIMEOUT, std::string(who) +
+                                       ": a bounded staging wait gave up (hit records are valid; staging was switched "
+                                       "off for the rest of the launch)");
+}
+
+// The scene's page-locked words, allocated by its first host call.
+rt_status ensure_host_words(rt_scene* s) {
+  if (s->h_words) return RT_OK;
+  const cudaError_t e = cudaHostAlloc(&s->h_words, sizeof(unsigned long long) * (rti::kHostChunks + 1), cudaHostAllocDefault);
+  if (e == cudaSuccess) return RT_OK;
+  s->h_words = nullptr;
+  return cuda_fail(e, "cudaHostAlloc");
+}
+
+// Ends a host call that used only s->stream: the status word follows the work
+// on the stream, and one wait covers both.
+rt_status finish_stream(rt_scene* s, rt_status st, const char* who, bool status_written) {
+  cudaError_t e = cudaSuccess;
+  uint32_t* word = reinterpret_cast<uint32_t*>(s->h_words + rti::kHostChunks);
+  if (st == RT_OK && !status_written)
+    e = cudaMemcpyAsync(word, s->d_status, sizeof(uint32_t), cudaMemcpyDeviceToHost, s->stream);
+  const cudaError_t ex = cudaStreamSynchronize(s->stream);
+  if (e == cudaSuccess) e = ex;
+  if (st != RT_OK) return st;
+  if (e != cudaSuccess) return cuda_fail(e, who);
+  return timeout_status(*reinterpret_cast<volatile uint32_t*>(word), who);
+}
+
 // Waits for every stream of the host path; returns `st` (or the first CUDA
 // error if `st` is RT_OK).
 rt_status host_finish(rt_scene* s, rt_status st) {
@@ -1058,11 +1104,7 @@ rt_status check_device_status(rt_scene* s, const char* who) {
   uint32_t status = 0;
   const cudaError_t e = cudaMemcpy(&status, s->d_status, sizeof(status), cudaMemcpyDeviceToHost);
   if (e != cudaSuccess) return cuda_fail(e, who);
-  if (status & rtk::kStatusTimeout)
-    return fail(RT_ERR_TIMEOUT, std::string(who) +
-                                    ": a bounded staging wait gave up (hit records are valid; staging was switched "
-                                    "off for the rest of the launch)");
-  return RT_OK;
+  return timeout_status(status, who);
 }
 
 }  // namespace rti
@@ -1117,6 +1159,8 @@ rt_status rt_trace_host(rt_scene* s, const rt_ray* rays, const uint32_t* flags, 
   rt_status st = check_trace(s, mode, trace, "rt_trace_host");
   if (st != RT_OK) return st;
   RT_CUDA(cudaSetDevice(s->ctx->device));
+  st = ensure_host_words(s);
+  if (st != RT_OK) return st;
   const uint32_t cap = (trace && (trace->visits || trace->treelets)) ? trace->capacity : 0;
   auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
   // Page-locked hit records: the kernel writes them straight into host memory
@@ -1132,7 +1176,7 @@ rt_status rt_trace_host(rt_scene* s, const rt_ray* rays, const uint32_t* flags, 
     if (mapped_rays && (!flags || mapped_flags)) {
       st = trace_launch(s, mapped_rays, mapped_flags, default_flags, n, mode, mapped_hits, nullptr, s->stream,
                         s->d_queue, false);
-      return host_finish(s, st);
+      return finish_stream(s, st, "rt_trace_host", false);
     }
     if (mapped_hits) {
       const size_t b_rays = al(sizeof(rt_ray) * (size_t)n), b_flags = flags ? sizeof(uint32_t) * (size_t)n : 0;
@@ -1149,10 +1193,10 @@ rt_status rt_trace_host(rt_scene* s, const rt_ray* rays, const uint32_t* flags, 
       cudaError_t e = cudaMemcpyAsync(d_rays, rays, sizeof(rt_ray) * (size_t)n, cudaMemcpyHostToDevice, s->stream);
       if (e == cudaSuccess && flags)
         e = cudaMemcpyAsync(d_flags, flags, sizeof(uint32_t) * (size_t)n, cudaMemcpyHostToDevice, s->stream);
-      if (e != cudaSuccess) return host_finish(s, cuda_fail(e, "rt_trace_host"));
+      if (e != cudaSuccess) return finish_stream(s, cuda_fail(e, "rt_trace_host"), "rt_trace_host", false);
       st = trace_launch(s, d_rays, d_flags, default_flags, n, mode, mapped_hits, nullptr, s->stream, s->d_queue,
                         false);
-      return host_finish(s, st);
+      return finish_stream(s, st, "rt_trace_host", false);
     }
   }
   const size_t b_rays = al(sizeof(rt_ray) * (size_t)n), b_flags = flags ? al(sizeof(uint32_t) * (size_t)n) : 0;
@@ -1183,10 +1227,28 @@ rt_status rt_trace_host(rt_scene* s, const rt_ray* rays, const uint32_t* flags, 
   bound[0] = 0;
   bound[1] = n;
   if (!queued(s, mode)) chunks = rti::host_chunk_bounds(n, bound);
-  // counters of the whole call start at zero, ahead of every chunk's copy-in
-  RT_CUDA(cudaMemsetAsync(s->d_stats, 0, sizeof(unsigned long long) * rtk::ST_COUNT, s->xin));
-  RT_CUDA(cudaMemsetAsync(s->d_status, 0, sizeof(uint32_t), s->xin));
   cudaError_t e = cudaSuccess;
+  if (chunks == 1) {
+    // a call that runs whole has nothing to overlap: one stream, one wait
+    e = cudaMemcpyAsync(d_rays, rays, sizeof(rt_ray) * (size_t)n, cudaMemcpyHostToDevice, s->stream);
+    if (e == cudaSuccess && flags)
+      e = cudaMemcpyAsync(d_flags, flags, sizeof(uint32_t) * (size_t)n, cudaMemcpyHostToDevice, s->stream);
+    if (e == cudaSuccess) {
+      rt_trace_buf tb{d_vis, d_tl, cap};
+      st = trace_launch(s, d_rays, d_flags, default_flags, n, mode, d_hits, cap ? &tb : nullptr, s->stream, s->d_queue,
+                        false);
+    }
+    if (st == RT_OK && e == cudaSuccess)
+      e = cudaMemcpyAsync(hits, d_hits, sizeof(rt_hit) * (size_t)n, cudaMemcpyDeviceToHost, s->stream);
+    if (st == RT_OK && e == cudaSuccess && d_vis)
+      e = cudaMemcpyAsync(trace->visits, d_vis, sizeof(uint32_t) * (size_t)n * cap, cudaMemcpyDeviceToHost, s->stream);
+    if (st == RT_OK && e == cudaSuccess && d_tl)
+      e = cudaMemcpyAsync(trace->treelets, d_tl, sizeof(uint32_t) * (size_t)n * cap, cudaMemcpyDeviceToHost, s->stream);
+    if (st == RT_OK && e != cudaSuccess) st = cuda_fail(e, "rt_trace_host");
+    return finish_stream(s, st, "rt_trace_host", false);
+  }
+  // counters of the whole call start at zero, ahead of every chunk's copy-in
+  RT_CUDA(cudaMemsetAsync(s->d_ctl, 0, sizeof(rti::Control), s->xin));
   for (uint32_t c = 0; c < chunks && e == cudaSuccess && st == RT_OK; ++c) {
     const size_t lo = bound[c], m = bound[c + 1] - bound[c];
     e = cudaMemcpyAsync(d_rays + lo, rays + lo, sizeof(rt_ray) * m, cudaMemcpyHostToDevice, s->xin);
@@ -1401,9 +1463,7 @@ struct rt_batch {
   uint32_t* d_item_scene = nullptr;
   uint32_t n_items = 0, n_rays = 0;
   std::vector<uint32_t> item_begin, item_scene;  // host copies (staged batches launch per item)
-  unsigned long long* d_stats = nullptr;
-  uint32_t* d_status = nullptr;
-  uint32_t* d_queue = nullptr;
+  rti::Control* d_ctl = nullptr;
   rt_tuning tuning{128, 128, 16, 1, 8, 2048, 2, 96, RT_TUNING_OFF, rtk::kWaitTries, RT_TUNING_OFF,
                    RT_TUNING_OFF};  // batches pin nothing
   cudaGraph_t graph = nullptr;
@@ -1458,9 +1518,9 @@ rt_status batch_args(rt_batch* b, const rt_ray* rays, const uint32_t* flags, uin
   a.default_flags = default_flags;
   a.n = b->n_rays;
   a.hits = hits;
-  a.stats = b->d_stats;
-  a.status = b->d_status;
-  a.queue = b->d_queue;
+  a.stats = b->d_ctl->stats;
+  a.status = &b->d_ctl->status;
+  a.queue = b->d_ctl->queue;
   return RT_OK;
 }
 
@@ -1517,9 +1577,7 @@ rt_status rt_batch_create(rt_ctx* ctx, rt_scene* const* scenes, uint32_t n_scene
   b->ctx = ctx;
   b->scenes.assign(scenes, scenes + n_scenes);
   rt_status st = dalloc(&b->d_views, sizeof(rtk::SceneView) * n_scenes);
-  if (st == RT_OK) st = dalloc(&b->d_stats, sizeof(unsigned long long) * rtk::ST_COUNT);
-  if (st == RT_OK) st = dalloc(&b->d_status, sizeof(uint32_t));
-  if (st == RT_OK) st = dalloc(&b->d_queue, sizeof(uint32_t));
+  if (st == RT_OK) st = dalloc(&b->d_ctl, sizeof(rti::Control));
   if (st != RT_OK) {
     rt_batch_destroy(b);
     return st;
@@ -1553,9 +1611,7 @@ rt_status rt_batch_destroy(rt_batch* b) {
   cudaFree(b->d_views);
   cudaFree(b->d_item_begin);
   cudaFree(b->d_item_scene);
-  cudaFree(b->d_stats);
-  cudaFree(b->d_status);
-  cudaFree(b->d_queue);
+  cudaFree(b->d_ctl);
   delete b;
   return RT_OK;
 }
@@ -1657,31 +1713,91 @@ __global__ void trace_counts_kernel(const rt_hit* __restrict__ hits, uint32_t n,
 }
 
 // Turns the block-local exclusive offsets of bin_scan_kernel into offsets
-// within the chunk (in place) and writes the chunk's total.
+// within the chunk (in place) and writes the chunk's total, to device and to
+// host memory.
 __global__ void trace_offsets_kernel(uint32_t* __restrict__ off, const uint32_t* __restrict__ block_sum,
                                      const rt_hit* __restrict__ hits, uint32_t n, uint32_t cap,
-                                     unsigned long long* __restrict__ total) {
+                                     unsigned long long* __restrict__ total, volatile unsigned long long* h_total,
+                                     const uint32_t* __restrict__ status, volatile uint32_t* h_status) {
   const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= n) return;
   const uint32_t o = block_sum[r / rtk::kBinScanItems] + off[r];
   off[r] = o;
-  if (r == n - 1) *total = (unsigned long long)o + min(hits[r].n_visits, cap);
+  if (r == n - 1) {
+    *total = *h_total = (unsigned long long)o + min(hits[r].n_visits, cap);
+    *h_status = *status;
+  }
+}
+
+// Chunks of a packed call: two from 2^17 rays on, four from 2^19.  Overlapping
+// the copies with the next chunk's trace pays for the second launch's tail of
+// long rays from there: 307,200 primary rays with both traces (144 MB out) take
+// 1.46 ms in one chunk on a GB300, 1.35 in two, 1.41 in three, 1.68 in four.
+constexpr uint32_t kPackedChunkRays = 1u << 17;
+constexpr uint32_t kPackedFewChunks = 2;
+// Rays up to which a call into page-locked arrays packs straight into them.
+// That saves a wait for the total and five copies (32 rays: 96 -> 50 us), but the
+// kernel stores to host memory at 120 GB/s, the copy engines at 200: 307,200 rays
+// 1.79 ms that way.
+constexpr uint32_t kPackDirectRays = 1u << 14;
+
+// Counts, offsets and total of a call of at most kScanRays rays in one block
+// (its four kernels' launches took longer than their work).
+constexpr uint32_t kScanRays = 1u << 13;
+__global__ void __launch_bounds__(1024) trace_scan_kernel(const rt_hit* __restrict__ hits, uint32_t n, uint32_t cap,
+                                                          uint32_t* __restrict__ off,
+                                                          unsigned long long* __restrict__ total,
+                                                          volatile unsigned long long* h_total,
+                                                          const uint32_t* __restrict__ status,
+                                                          volatile uint32_t* h_status) {
+  __shared__ uint32_t warp_sum[32];
+  const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
+  uint32_t base = 0;
+  for (uint32_t r0 = 0; r0 < n; r0 += 1024) {
+    const uint32_t r = r0 + threadIdx.x;
+    const uint32_t c = r < n ? min(hits[r].n_visits, cap) : 0u;
+    uint32_t x = c;  // inclusive scan
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, x, d);
+      if ((int)lane >= d) x += y;
+    }
+    __syncthreads();  // the last turn's sums are read
+    if (lane == 31) warp_sum[wid] = x;
+    __syncthreads();
+    uint32_t before = lane < wid ? warp_sum[lane] : 0u;
+    before = __reduce_add_sync(0xffffffffu, before);
+    if (r < n) off[r] = base + before + x - c;
+    base += __reduce_add_sync(0xffffffffu, warp_sum[lane]);
+  }
+  if (threadIdx.x == 0) {
+    *total = *h_total = base;
+    *h_status = *status;
+  }
 }
 
 // One warp per ray: the ray's global offset (base + chunk offset) into
 // `goff`, and the used prefix of its trace rows to its place in the packed
-// staging arrays (NULL: not written).  The rows are visits when `vis` is
-// written (a treelet id is then looked up for each), else treelet ids.
+// arrays (NULL: not written; not written either when the chunk's `total`
+// exceeds `room`).  The rows are visits when `vis` is written (a treelet id is
+// then looked up for each), else treelet ids.  With hits_out the hit records
+// are copied too: the outputs may be the caller's own page-locked arrays.
 __global__ void trace_pack_kernel(const uint32_t* __restrict__ rows, const uint2* __restrict__ meta, bool rows_tl,
-                                  const uint32_t* __restrict__ off, uint32_t n, uint32_t cap, uint32_t chunk_total,
+                                  const uint32_t* __restrict__ off, uint32_t n, uint32_t cap,
+                                  const unsigned long long* __restrict__ total, unsigned long long room,
                                   unsigned long long base, unsigned long long* __restrict__ goff,
-                                  uint32_t* __restrict__ vis, uint32_t* __restrict__ tl) {
+                                  uint32_t* __restrict__ vis, uint32_t* __restrict__ tl,
+                                  const rt_hit* __restrict__ hits, rt_hit* __restrict__ hits_out) {
   const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31u;
   const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+  const unsigned long long all = *total;
+  const bool fits = all <= room;
   for (uint32_t r = warp; r < n; r += warps) {
     const uint32_t o = off[r];
-    const uint32_t m = (r + 1 < n ? off[r + 1] : chunk_total) - o;
+    const uint32_t m = (r + 1 < n ? off[r + 1] : (uint32_t)all) - o;
     if (lane == 0) goff[r] = base + o;
+    if (hits_out && lane < 16) reinterpret_cast<uint32_t*>(hits_out + r)[lane] = reinterpret_cast<const uint32_t*>(hits + r)[lane];
+    if (!fits) continue;
     const uint64_t row = (uint64_t)r * cap;
     for (uint32_t j = lane; j < m; j += 32) {
       const uint32_t x = __ldcs(rows + row + j);
@@ -1689,6 +1805,20 @@ __global__ void trace_pack_kernel(const uint32_t* __restrict__ rows, const uint2
       if (tl) tl[o + j] = rows_tl ? x : meta[x >> 3].x;
     }
   }
+}
+
+}  // namespace
+
+namespace {
+
+// The end of a packed call whose entries are `count` in all.
+rt_status packed_total(uint64_t count, uint64_t capacity, uint64_t* offsets, uint32_t n, uint64_t* total) {
+  offsets[n] = count;
+  *total = count;
+  if (count > capacity)
+    return rti::fail(RT_ERR_TOO_LARGE, "rt_trace_host_packed: " + std::to_string(count) +
+                                           " trace entries exceed the arrays' capacity (hits and offsets are filled)");
+  return RT_OK;
 }
 
 }  // namespace
@@ -1723,14 +1853,14 @@ extern "C" rt_status rt_trace_host_packed(rt_scene* s, const rt_ray* rays, const
   RT_CUDA(cudaSetDevice(s->ctx->device));
   const uint32_t cap = row_capacity;
   auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
-  // four equal chunks from 2^19 rays on (a queued staged launch runs whole:
+  // equal chunks from kPackedChunkRays rays on (a queued staged launch runs whole:
   // its queues are the scene's, one set)
   uint64_t bound[rti::kHostChunks + 1];
   uint32_t chunks = 1;
   bound[0] = 0;
   bound[1] = n;
-  if (!queued(s, mode) && n >= (1u << 19)) {
-    chunks = rti::kHostChunks;
+  if (!queued(s, mode) && n >= kPackedChunkRays) {
+    chunks = n >= (1u << 19) ? rti::kHostChunks : kPackedFewChunks;
     for (uint32_t c = 0; c <= chunks; ++c) bound[c] = (uint64_t)n * c / chunks;
   }
   const size_t b_rays = al(sizeof(rt_ray) * (size_t)n), b_flags = flags ? al(sizeof(uint32_t) * (size_t)n) : 0;
@@ -1748,13 +1878,8 @@ extern "C" rt_status rt_trace_host_packed(rt_scene* s, const rt_ray* rays, const
     if (st != RT_OK) return st;
     s->io_bytes = need;
   }
-  if (!s->h_tot) {
-    cudaError_t e = cudaHostAlloc(&s->h_tot, sizeof(unsigned long long) * rti::kHostChunks, cudaHostAllocDefault);
-    if (e != cudaSuccess) {
-      s->h_tot = nullptr;
-      return cuda_fail(e, "rt_trace_host_packed: cudaHostAlloc");
-    }
-  }
+  st = ensure_host_words(s);
+  if (st != RT_OK) return st;
   uint8_t* p = (uint8_t*)s->d_io;
   auto take = [&](size_t b) {
     uint8_t* r = p;
@@ -1772,9 +1897,57 @@ extern "C" rt_status rt_trace_host_packed(rt_scene* s, const rt_ray* rays, const
   unsigned long long* d_tot = (unsigned long long*)take(b_tot);
   const size_t blk_stride = al(sizeof(uint32_t) * rtk::kBinScanItems) / sizeof(uint32_t);
 
-  RT_CUDA(cudaMemsetAsync(s->d_stats, 0, sizeof(unsigned long long) * rtk::ST_COUNT, s->xin));
-  RT_CUDA(cudaMemsetAsync(s->d_status, 0, sizeof(uint32_t), s->xin));
+  volatile unsigned long long* const h_tot = s->h_words;
+  volatile uint32_t* const h_status = reinterpret_cast<uint32_t*>(s->h_words + rti::kHostChunks);
   cudaError_t e = cudaSuccess;
+  // counts, offsets within the chunk and total of a traced chunk
+  auto offsets_of = [&](const rt_hit* h, uint32_t m, uint32_t* cnt, uint32_t* off, uint32_t* blk,
+                        unsigned long long* tot, volatile unsigned long long* ht, cudaStream_t cs) {
+    if (m <= kScanRays) {
+      trace_scan_kernel<<<1, 1024, 0, cs>>>(h, m, cap, off, tot, ht, s->d_status, h_status);
+      return;
+    }
+    const uint32_t nb = (m + rtk::kBinScanItems - 1) / rtk::kBinScanItems;
+    trace_counts_kernel<<<(m + 255) / 256, 256, 0, cs>>>(h, m, cap, cnt);
+    rtk::bin_scan_kernel<<<nb, 1024, 0, cs>>>(cnt, off, blk, m);
+    rtk::bin_scan_top_kernel<<<1, 1024, 0, cs>>>(blk, nb);
+    trace_offsets_kernel<<<(m + 255) / 256, 256, 0, cs>>>(off, blk, h, m, cap, tot, ht, s->d_status, h_status);
+  };
+  auto pack_grid = [](uint32_t m) { return std::min<uint32_t>((m + 3) / 4, 152 * 8); };
+  // A small call into page-locked arrays packs straight into them: the total is
+  // checked on the device, and the host waits once, at the end.
+  if (chunks == 1 && n <= kPackDirectRays) {
+    rt_hit* m_hits = (rt_hit*)mapped_range(hits, sizeof(rt_hit) * (size_t)n);
+    auto* m_off = m_hits ? (unsigned long long*)mapped_range(offsets, sizeof(uint64_t) * ((size_t)n + 1)) : nullptr;
+    uint32_t* m_vis = m_off && visits ? (uint32_t*)mapped_range(visits, sizeof(uint32_t) * (size_t)capacity) : nullptr;
+    uint32_t* m_tl = m_off && treelets ? (uint32_t*)mapped_range(treelets, sizeof(uint32_t) * (size_t)capacity) : nullptr;
+    if (m_off && (!visits || m_vis) && (!treelets || m_tl)) {
+      const rt_ray* in = (const rt_ray*)mapped_range(rays, sizeof(rt_ray) * (size_t)n);
+      const uint32_t* in_flags = flags ? (const uint32_t*)mapped_range(flags, sizeof(uint32_t) * (size_t)n) : nullptr;
+      if (!in || (flags && !in_flags)) {
+        in = d_rays;
+        in_flags = d_flags;
+        e = cudaMemcpyAsync(d_rays, rays, sizeof(rt_ray) * (size_t)n, cudaMemcpyHostToDevice, s->stream);
+        if (e == cudaSuccess && flags)
+          e = cudaMemcpyAsync(d_flags, flags, sizeof(uint32_t) * (size_t)n, cudaMemcpyHostToDevice, s->stream);
+      }
+      if (e == cudaSuccess) {
+        rt_trace_buf rows{visits ? d_rows : nullptr, visits ? nullptr : d_rows, cap};
+        st = trace_launch(s, in, in_flags, default_flags, n, mode, d_hits, &rows, s->stream, s->d_queue, false);
+        if (st == RT_OK) {
+          offsets_of(d_hits, n, d_cnt, d_off, d_blk, d_tot, h_tot, s->stream);
+          trace_pack_kernel<<<pack_grid(n), 128, 0, s->stream>>>(d_rows, s->d_meta, !visits, d_off, n, cap, d_tot,
+                                                                 capacity, 0ull, m_off, m_vis, m_tl, d_hits, m_hits);
+          e = cudaGetLastError();
+        }
+      }
+      if (st == RT_OK && e != cudaSuccess) st = cuda_fail(e, "rt_trace_host_packed");
+      st = finish_stream(s, st, "rt_trace_host_packed", true);
+      if (st != RT_OK) return st;
+      return packed_total(h_tot[0], capacity, offsets, n, total);
+    }
+  }
+  RT_CUDA(cudaMemsetAsync(s->d_ctl, 0, sizeof(rti::Control), s->xin));
   // every chunk's rays in
   for (uint32_t c = 0; c < chunks && e == cudaSuccess; ++c) {
     const size_t lo = bound[c];
@@ -1784,8 +1957,8 @@ extern "C" rt_status rt_trace_host_packed(rt_scene* s, const rt_ray* rays, const
       e = cudaMemcpyAsync(d_flags + lo, flags + lo, sizeof(uint32_t) * m, cudaMemcpyHostToDevice, s->xin);
     if (e == cudaSuccess) e = cudaEventRecord(s->ev_in[c], s->xin);
   }
-  // chunk c's trace, counts, offsets and total (copied to the page-locked
-  // h_tot[c]), ending in ev_done[c]
+  // chunk c's trace, counts, offsets and total (written to the page-locked
+  // h_tot[c] too), ending in ev_done[c]
   auto trace_chunk = [&](uint32_t c) -> bool {
     const size_t lo = bound[c];
     const uint32_t m = (uint32_t)(bound[c + 1] - bound[c]);
@@ -1796,15 +1969,8 @@ extern "C" rt_status rt_trace_host_packed(rt_scene* s, const rt_ray* rays, const
     st = trace_launch(s, d_rays + lo, d_flags ? d_flags + lo : nullptr, default_flags, m, mode, d_hits + lo, &rows, cs,
                       s->d_queue + c, true);
     if (st != RT_OK) return false;
-    const uint32_t nb = (m + rtk::kBinScanItems - 1) / rtk::kBinScanItems;
-    uint32_t* blk = d_blk + c * blk_stride;
-    trace_counts_kernel<<<(m + 255) / 256, 256, 0, cs>>>(d_hits + lo, m, cap, d_cnt + lo);
-    rtk::bin_scan_kernel<<<nb, 1024, 0, cs>>>(d_cnt + lo, d_off + lo, blk, m);
-    rtk::bin_scan_top_kernel<<<1, 1024, 0, cs>>>(blk, nb);
-    trace_offsets_kernel<<<(m + 255) / 256, 256, 0, cs>>>(d_off + lo, blk, d_hits + lo, m, cap, d_tot + c);
+    offsets_of(d_hits + lo, m, d_cnt + lo, d_off + lo, d_blk + c * blk_stride, d_tot + c, h_tot + c, cs);
     e = cudaGetLastError();
-    if (e == cudaSuccess)
-      e = cudaMemcpyAsync(s->h_tot + c, d_tot + c, sizeof(unsigned long long), cudaMemcpyDeviceToHost, cs);
     if (e == cudaSuccess) e = cudaEventRecord(s->ev_done[c], cs);
     return e == cudaSuccess;
   };
@@ -1820,7 +1986,7 @@ extern "C" rt_status rt_trace_host_packed(rt_scene* s, const rt_ray* rays, const
     const uint32_t m = (uint32_t)(bound[c + 1] - bound[c]);
     e = cudaEventSynchronize(s->ev_done[c]);
     if (e != cudaSuccess) break;
-    const unsigned long long tot_c = reinterpret_cast<volatile unsigned long long*>(s->h_tot)[c];
+    const unsigned long long tot_c = h_tot[c];
     fits = fits && base + tot_c <= capacity;
     uint32_t *dst_vis = nullptr, *dst_tl = nullptr;
     if (fits && tot_c > 0) {
@@ -1844,8 +2010,8 @@ extern "C" rt_status rt_trace_host_packed(rt_scene* s, const rt_ray* rays, const
     e = cudaStreamWaitEvent(s->xout, s->ev_done[c], 0);
     if (e != cudaSuccess) break;
     unsigned long long* goff = d_goff + lo;
-    trace_pack_kernel<<<std::min<uint32_t>((m + 3) / 4, 152 * 8), 128, 0, s->xout>>>(
-        d_rows + lo * cap, s->d_meta, !visits, d_off + lo, m, cap, (uint32_t)tot_c, base, goff, dst_vis, dst_tl);
+    trace_pack_kernel<<<pack_grid(m), 128, 0, s->xout>>>(d_rows + lo * cap, s->d_meta, !visits, d_off + lo, m, cap,
+                                                         d_tot + c, ~0ull, base, goff, dst_vis, dst_tl, nullptr, nullptr);
     e = cudaGetLastError();
     if (e == cudaSuccess && c + 1 < chunks && !trace_chunk(c + 1)) break;
     if (e == cudaSuccess)
@@ -1861,10 +2027,5 @@ extern "C" rt_status rt_trace_host_packed(rt_scene* s, const rt_ray* rays, const
   if (st == RT_OK && e != cudaSuccess) st = cuda_fail(e, "rt_trace_host_packed");
   st = host_finish(s, st);
   if (st != RT_OK) return st;
-  offsets[n] = base;
-  *total = base;
-  if (base > capacity)
-    return rti::fail(RT_ERR_TOO_LARGE, "rt_trace_host_packed: " + std::to_string(base) +
-                                           " trace entries exceed the arrays' capacity (hits and offsets are filled)");
-  return RT_OK;
+  return packed_total(base, capacity, offsets, n, total);
 }
