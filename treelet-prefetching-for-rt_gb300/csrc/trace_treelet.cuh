@@ -449,11 +449,12 @@ struct Walker {
 // registers (stacks inside it would leave every field in local memory).
 // 72 registers: seven 128-thread CTAs per SM.  GB300, ms for 1M traced bounce
 // rays / 2M any-hit rays: 2.36 / 1.64; 64 registers (eight CTAs) 2.44 / 1.64,
-// 56 2.51 / 1.67, 85 2.49 / 1.76.
-constexpr int kTreeletRegs = 72;
+// 56 2.51 / 1.67, 85 2.49 / 1.76.  A batch's walk, which looks its scene up per
+// ray, spills at 72: 48 scenes in one launch 0.69 ms, at 80 0.65.
+constexpr int kTreeletRegs = 72, kTreeletBatchRegs = 80;
 
 template <int CAP, bool MULTI, bool TRACED>
-__global__ void __maxnreg__(kTreeletRegs) trace_treelet_kernel(TraceArgs a) {
+__global__ void __maxnreg__(MULTI ? kTreeletBatchRegs : kTreeletRegs) trace_treelet_kernel(TraceArgs a) {
   using W = Walker<CAP, false, MULTI, false, TRACED>;
   unsigned long long stack[W::kWords];
   W w;
@@ -534,11 +535,10 @@ __device__ __forceinline__ SlotLookup<F> slot_lookup(F f) {
 
 constexpr int kMaxSlots = 8;  // slots per warp
 constexpr uint32_t kWaitTries = 1u << 22;
-// Three 256-thread CTAs per SM, at most 85 registers a thread (no spills with
-// one ray context held): 2M primary rays 2.86 ms on a GB300 against 3.12 ms
-// with both rays held and 52 bytes of spills.
+// Four 256-thread CTAs per SM, 64 registers a thread (96 bytes of spills): 2M
+// primary rays 2.50 ms on a GB300 against 2.56 with three CTAs at 80 registers.
 constexpr int kStagedMaxThreads = 256;
-constexpr int kStagedMinBlocks = 3;
+constexpr int kStagedMinBlocks = 4;
 constexpr uint32_t kPinChunk = 32768;  // bytes per bulk copy of the pinned image
 
 // Per-warp staging state in shared memory.
