@@ -1022,8 +1022,10 @@ rt_status trace_launch(rt_scene* s, const rt_ray* rays, const uint32_t* flags, u
   if (queues) rs = ensure_queue_scratch(s, n);
   if (rs == RT_OK) rs = launch_trace(a, mode, s->tuning, s->slot_bytes, st, keep, queues ? &s->qs : nullptr);
   if (rs == RT_OK && visits && treelets) {
-    auto ids = rtk::trace_treelet_ids_kernel;
-    ids<<<persistent_grid((const void*)ids, 256, (uint32_t)std::min<uint64_t>(32ull * n, 0xffffffffull)), 256, 0, st>>>(
+    const bool wide = a.cap % 4 == 0 && (((uintptr_t)visits | (uintptr_t)treelets) & 15u) == 0;
+    auto ids = wide ? rtk::trace_treelet_ids_kernel<true> : rtk::trace_treelet_ids_kernel<false>;
+    const uint64_t threads = (wide ? 8ull : 32ull) * n;
+    ids<<<persistent_grid((const void*)ids, 256, (uint32_t)std::min<uint64_t>(threads, 0xffffffffull)), 256, 0, st>>>(
         visits, hits, s->d_meta, n, a.cap, treelets);
     RT_CUDA(cudaGetLastError());
   }

@@ -173,17 +173,33 @@ __device__ __forceinline__ void trace_drain(const TraceArgs& a, uint32_t r, uint
   for (uint32_t j = 0; j < k; ++j) row[j] = b[j * 32];
 }
 
-// The treelet id of every recorded visit (one warp per ray): reads and writes
-// whole rows in order, the scattered part is the 8-byte table entry.
+// The treelet id of every recorded visit: reads and writes the rows in order,
+// the scattered part is the 8-byte table entry.  WIDE: eight lanes take a row,
+// four entries each (rows that start on 16-byte boundaries), so that a warp has
+// up to 128 table reads on their way; with one warp per row and one entry a
+// lane the pass was bound by two dependent loads (282 us for 1M bounce rays' 63M
+// entries on a GB300; WIDE 208, by then bound by L2 sectors).
+template <bool WIDE>
 __global__ void __launch_bounds__(256) trace_treelet_ids_kernel(const uint32_t* __restrict__ visits,
                                                                 const rt_hit* __restrict__ hits,
                                                                 const uint2* __restrict__ meta, uint32_t n,
                                                                 uint32_t cap, uint32_t* __restrict__ treelets) {
-  const uint32_t lane = threadIdx.x & 31u, warps = (gridDim.x * blockDim.x) >> 5;
-  for (uint32_t r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < n; r += warps) {
+  constexpr uint32_t kLanes = WIDE ? 8u : 32u, kEach = WIDE ? 4u : 1u;
+  const uint32_t lane = threadIdx.x % kLanes, rows = gridDim.x * blockDim.x / kLanes;
+  for (uint32_t r = (blockIdx.x * blockDim.x + threadIdx.x) / kLanes; r < n; r += rows) {
     const uint32_t m = min(hits[r].n_visits, cap);
     const uint64_t row = (uint64_t)r * cap;
-    for (uint32_t j = lane; j < m; j += 32) __stcs(treelets + row + j, meta[__ldcs(visits + row + j) >> 3].x);
+#pragma unroll 2
+    for (uint32_t j = lane * kEach; j < m; j += kLanes * kEach) {
+      if (WIDE && j + 4 <= m) {
+        const uint4 x = __ldcs(reinterpret_cast<const uint4*>(visits + row + j));
+        __stcs(reinterpret_cast<uint4*>(treelets + row + j),
+               make_uint4(__ldg(&meta[x.x >> 3].x), __ldg(&meta[x.y >> 3].x), __ldg(&meta[x.z >> 3].x),
+                          __ldg(&meta[x.w >> 3].x)));
+      } else {
+        for (uint32_t k = j; k < min(j + kEach, m); ++k) treelets[row + k] = __ldg(&meta[visits[row + k] >> 3].x);
+      }
+    }
   }
 }
 
