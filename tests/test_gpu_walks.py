@@ -98,9 +98,9 @@ def test_unit_that_is_node_and_leaf(ctx):
     scene.close()
 
 
-@pytest.mark.parametrize("n", [1, 7, 33, 4864, 4865, 9729, 32768, 32769, 40001])
+@pytest.mark.parametrize("n", [1, 7, 33, 4864, 4865, 9729, 24576, 24577, 32768, 32769, 40001])
 def test_launch_sizes(ctx, n):
-    """Eight lanes a ray (one, two or four rays a warp) up to 32,768 rays, one
+    """Eight lanes a ray (one, two or four rays a warp) up to 32,768 rays (24,576 staged), one
     lane a ray above: hits and traces, any-hit rays among them, with a row
     capacity that some rays exceed and rows that start off a 32-byte boundary."""
     import torch
@@ -117,7 +117,7 @@ def test_launch_sizes(ctx, n):
     flags = np.random.default_rng(n + 1).choice(np.array([0, 1, 5], np.uint32), size=n)
     d_rays = torch.from_numpy(rays.view(np.uint8).copy()).cuda()
     d_flags = torch.from_numpy(flags.view(np.uint8).copy()).cuda()
-    for mode, omode in ((rt.MODE_PLAIN, 0), (rt.MODE_TREELET, 1)):
+    for mode, omode in ((rt.MODE_PLAIN, 0), (rt.MODE_TREELET, 1), (rt.MODE_STAGED, 1)):
         for cap, skew in ((48, 0), (48, 1), (45, 0)):
             d_hits = torch.zeros(n * 64, dtype=torch.uint8, device="cuda")
             d_vis = torch.zeros(n * cap + skew, dtype=torch.int32, device="cuda")[skew:]
@@ -131,6 +131,7 @@ def test_launch_sizes(ctx, n):
             assert_traces_equal(d_vis.cpu().numpy().view(np.uint32).reshape(n, cap), ov, oh["n_visits"], "visits")
             assert_traces_equal(d_tl.cpu().numpy().view(np.uint32).reshape(n, cap), ot, oh["n_visits"], "treelet ids")
             node_bytes = scene.stats()["node_bytes"]
+            assert mode != rt.MODE_STAGED or scene.stats()["smem_reads"] > 0
         untraced = torch.zeros(n * 64, dtype=torch.uint8, device="cuda")
         scene.trace(d_rays, untraced, mode, flags=d_flags, n=n)
         torch.cuda.synchronize()

@@ -558,19 +558,33 @@ constexpr uint32_t kGroupRays = 1u << 15;
 // the start: 9,216 bounce rays 303 against 257 us).
 constexpr uint32_t kGroupRaysPerSplit = 152 * 32;
 
-bool group_launch(const rtk::TraceArgs& a, uint32_t mode, const rt_tuning& t) {
-  if (a.n_items || t.short_stack == 1) return false;
-  return (mode == RT_MODE_PLAIN || mode == RT_MODE_TREELET) && a.n <= kGroupRays;
+// Rays and pinned bytes up to which a staged launch does: each of its CTAs of
+// four warps copies the image.  Eight lanes / one, pinned image of 4 KiB:
+//                                    32        1,024      4,096      16,384     25,600     30,976
+//   131K-tri terrain, primary        57 / 124  90 / 230   116 / 249  198 / 274  226 / 273  304 / 275
+//   131K-tri terrain, bounce         88 / 186  140 / 331  173 / 358  332 / 410  375 / 419  413 / 434
+//   16K-tri cube, bounce             32 / 54   47 / 99    57 / 110   76 / 109   103 / 120  122 / 115
+// With 16 KiB pinned, terrain bounce: 89 / 189 at 32 rays, 324 / 429 at 16,384, 430 / 452 at 24,480.
+constexpr uint32_t kGroupStagedRays = 3u << 13;
+constexpr uint32_t kGroupPinBytes = 16384;
+
+bool group_launch(const rtk::TraceArgs& a, uint32_t mode, const rt_tuning& t, const rti::QueueScratch* qs) {
+  if (a.n_items || a.n > kGroupRays) return false;
+  if (mode == RT_MODE_STAGED)
+    return !qs && t.staged_slots == RT_TUNING_OFF && a.pin_bytes <= kGroupPinBytes && a.n <= kGroupStagedRays;
+  return mode != RT_MODE_PLAIN || t.short_stack != 1;
 }
 
-rt_status launch_group(rtk::TraceArgs& a, bool treelet, uint32_t depth, cudaStream_t st) {
+rt_status launch_group(rtk::TraceArgs& a, uint32_t mode, uint32_t depth, cudaStream_t st) {
   void (*kern)(rtk::TraceArgs, uint32_t, uint32_t);
-  if (treelet) kern = a.cap ? rtk::trace_group_kernel<true, true> : rtk::trace_group_kernel<true, false>;
+  const bool treelet = mode != RT_MODE_PLAIN, staged = mode == RT_MODE_STAGED;
+  if (staged) kern = a.cap ? rtk::trace_group_kernel<true, true, true> : rtk::trace_group_kernel<true, false, true>;
+  else if (treelet) kern = a.cap ? rtk::trace_group_kernel<true, true> : rtk::trace_group_kernel<true, false>;
   else kern = a.cap ? rtk::trace_group_kernel<false, true> : rtk::trace_group_kernel<false, false>;
   const uint32_t warps = rtk::kGroupThreads / 32;
   uint32_t rpw = 1;
   while (rpw < 4 && a.n > rpw * kGroupRaysPerSplit) rpw *= 2;
-  const size_t dyn = (size_t)warps * rpw * rtk::group_stack_bytes(treelet, depth);
+  const size_t dyn = (staged ? a.pin_bytes : 0u) + (size_t)warps * rpw * rtk::group_stack_bytes(treelet, depth) + 128;
   RT_CUDA(ensure_dyn_smem((const void*)kern, dyn));
   // CTAs for every ray, or as many as are resident at once
   const uint32_t full = persistent_grid((const void*)kern, rtk::kGroupThreads, 0xffffffffu, dyn);
@@ -599,7 +613,7 @@ rt_status launch_cap(rtk::TraceArgs& a, uint32_t mode, const rt_tuning& t, uint3
   const uint32_t stage_warp_bytes = rtk::kTraceBufWarpBytes;
   a.tbuf_off = rtk::kNone;
   a.ss_off = rtk::kNone;
-  if (group_launch(a, mode, t)) return launch_group(a, mode == RT_MODE_TREELET, (uint32_t)CAP, st);
+  if (group_launch(a, mode, t, qs)) return launch_group(a, mode, (uint32_t)CAP, st);
   if (mode == RT_MODE_PLAIN || mode == RT_MODE_TREELET) {
     const uint32_t bt = t.block_threads;
     size_t dyn = stage_rows ? (size_t)(bt / 32) * stage_warp_bytes + 128 : 0;

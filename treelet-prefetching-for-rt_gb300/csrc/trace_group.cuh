@@ -8,7 +8,9 @@
 // consecutive leaves on the stack's top are tested at once; what the ray's
 // state says is computed by all its lanes alike.  The visits, their order and
 // every value are those of PlainWalker and Walker.  A warp holds `rpw` rays
-// (1, 2 or 4): with one, no ray waits for another's branch.
+// (1, 2 or 4): with one, no ray waits for another's branch.  STAGED reads
+// pinned treelets' nodes from the CTA's copy of the pinned image, as
+// trace_staged_kernel does.
 #pragma once
 #include <type_traits>
 
@@ -27,7 +29,7 @@ __host__ __device__ constexpr uint32_t group_stack_bytes(bool treelet, uint32_t 
 
 
 // One ray's walk over its eight lanes.
-template <bool TREELET, bool TRACED>
+template <bool TREELET, bool TRACED, bool STAGED>
 struct GroupWalk {
   using Entry = std::conditional_t<TREELET, unsigned long long, uint32_t>;
   static constexpr uint32_t kShift = TREELET ? kEShift : 2u;
@@ -38,6 +40,7 @@ struct GroupWalk {
   Entry* const cu;  // the stack (plain), the current-treelet stack
   Entry* const ot;  // the other-treelet stack
   const uint32_t scratch;  // touch_l1's word
+  const uint32_t pin_base, pin_root;  // STAGED: shared address of the pinned records, the TLAS root's record (0: none)
   uint32_t r;
   rtm::V3 O, D, I;  // the world ray
   RayCtx cx;
@@ -46,6 +49,7 @@ struct GroupWalk {
   int extra, ncu, not_;
   Entry e;        // the entry visited next, 0 = none popped
   bool from_cu;   // the stack it came from
+  uint32_t smem_reads, gmem_reads;
 
   __device__ __forceinline__ uint32_t ballot(bool p) const {
     return (__ballot_sync(mask, p) >> (threadIdx.x & 24u)) & 0xffu;
@@ -78,6 +82,26 @@ struct GroupWalk {
     cx.fast = (flags & kRayWorldFast) != 0;
   }
   __device__ __forceinline__ uint32_t inst() const { return TREELET ? (uint32_t)((unsigned long long)e >> 32) : 0u; }
+  static __device__ __forceinline__ bool pinned(uint32_t code) { return STAGED && (code & kEPin); }
+  // A node's address: its pinned record, else unit `unit` of `from`.  `unit`
+  // is read from the record of a pinned node.
+  __device__ __forceinline__ const uint4* locate(uint32_t code, const uint4* from, uint32_t& unit) const {
+    if (pinned(code)) {
+      const uint32_t saddr = pin_base + (code >> kShift) * 16u;
+      unit = rtd::ld_shared_u32(saddr + ((code & kLeaf) ? 0u : rtp::IN_UNIT));
+      return reinterpret_cast<const uint4*>(__cvta_shared_to_generic(saddr));
+    }
+    unit = code >> kShift;
+    return from + (uint64_t)unit * 4;
+  }
+  static __device__ __forceinline__ uint4 ld16(const uint4* p) { return STAGED ? *p : __ldg(p); }
+  static __device__ __forceinline__ uint8_t ld1(const uint8_t* p) { return STAGED ? *p : __ldg(p); }
+  __device__ __forceinline__ void count_reads(uint32_t shared, uint32_t all) {
+    if (STAGED) {
+      smem_reads += shared;
+      gmem_reads += all - shared;
+    }
+  }
   static __device__ __forceinline__ Entry make(uint32_t code, uint32_t in) {
     if constexpr (TREELET) return (unsigned long long)code | ((unsigned long long)in << 32);
     else return code;
@@ -105,7 +129,7 @@ struct GroupWalk {
     float th;
     if (rtm::ray_box_test(bmin, bmax, I, O, tmin, tmax, th)) {
       const uint32_t code = ((uint32_t)(root_off >> 6) << kShift) | kTop;
-      e = make(code, 0);
+      e = make(STAGED && pin_root ? ((pin_root << kShift) | kEPin | kTop) : code, 0);
       if constexpr (TREELET) {  // current_treelet_root starts as the TLAS header, unit 0 (:1707)
         const uint32_t unit = code >> kShift;
         from_cu = (unit < v.n_units ? __ldg(&v.meta[unit].x) : kNone) == 0u;
@@ -130,11 +154,11 @@ struct GroupWalk {
   }
 
   // Lane j's slab test of child j.
-  __device__ __forceinline__ bool hit_child(uint32_t unit, const uint4 q0, const uint4 q1, float t0, float t1,
-                                            float cull) const {
+  __device__ __forceinline__ bool hit_child(const uint4* src, uint32_t unit, const uint4 q0, const uint4 q1, float t0,
+                                            float t1, float cull) const {
     const uint32_t c = min(j, 5u);
     if (cx.fast && !(q1.y & rtw::kExact)) {
-      const uint8_t* b = reinterpret_cast<const uint8_t*>(v.walk + (uint64_t)unit * 4) + c;
+      const uint8_t* b = reinterpret_cast<const uint8_t*>(src) + c;
       const uint32_t hi = c < 4u ? 36u : 30u;  // child c's upper bound, axis x (walk_node.h)
       const float s[3] = {__uint_as_float((q1.x << 23) & 0x7f800000u), __uint_as_float((q1.x << 15) & 0x7f800000u),
                           __uint_as_float((q1.x << 7) & 0x7f800000u)};
@@ -143,8 +167,8 @@ struct GroupWalk {
       float lo[3], up[3];
 #pragma unroll
       for (int k = 0; k < 3; ++k) {
-        lo[k] = (__fmaf_rn((float)__ldg(b + 28 + 12 * k), s[k], org[k]) - o[k]) * id[k];
-        up[k] = (__fmaf_rn((float)__ldg(b + hi + 12 * k), s[k], org[k]) - o[k]) * id[k];
+        lo[k] = (__fmaf_rn((float)ld1(b + 28 + 12 * k), s[k], org[k]) - o[k]) * id[k];
+        up[k] = (__fmaf_rn((float)ld1(b + hi + 12 * k), s[k], org[k]) - o[k]) * id[k];
       }
       const float tn = fmaxf(rtd::max3(fminf(lo[0], up[0]), fminf(lo[1], up[1]), fminf(lo[2], up[2])), t0);
       const float tf = fminf(rtd::min3(fmaxf(lo[0], up[0]), fmaxf(lo[1], up[1]), fmaxf(lo[2], up[2])), t1);
@@ -154,39 +178,46 @@ struct GroupWalk {
   }
 
   __device__ __forceinline__ void internal() {
-    const uint32_t code = (uint32_t)e, unit = code >> kShift, in = inst(), level = code & kTop;
-    if (unit >= v.n_units) return stop(RT_RAY_BAD_NODE);
-    const uint4 q0 = __ldg(v.walk + (uint64_t)unit * 4), q1 = __ldg(v.walk + (uint64_t)unit * 4 + 1);
+    const uint32_t code = (uint32_t)e, in = inst(), level = code & kTop;
+    uint32_t unit;
+    const uint4* src = locate(code, v.walk, unit);
+    if (!pinned(code) && unit >= v.n_units) return stop(RT_RAY_BAD_NODE);
+    const uint4 q0 = ld16(src), q1 = ld16(src + 1);
+    uint32_t so = 0;  // a pinned parent names its pinned children's records: lane j's child
+    if (pinned(code)) so = rtd::ld_shared_u16(pin_base + (code >> kShift) * 16u + rtp::IN_CHILD_SOFF + 2u * min(j, 5u));
+    count_reads(pinned(code) ? 1u : 0u, 1u);
     record(unit, rtf::TX_INTERNAL);
     if (level && cx.unit != kNone) world();
     const uint32_t valid = (q1.y | (q1.y >> rtw::kLeafShift)) & rtw::kChildMask;
-    const bool h = hit_child(unit, q0, q1, tmin * cx.mult, tmax * cx.mult, min_thit * cx.mult);
+    const bool h = hit_child(src, unit, q0, q1, tmin * cx.mult, tmax * cx.mult, min_thit * cx.mult);
     uint32_t hit = ballot(h) & valid;
     // hit children start on their way to L1 while the ray is elsewhere
-    if ((hit >> j) & 1u) {
+    if ((hit >> j) & 1u && !so) {
       const uint4* const child = v.walk + (uint64_t)(q0.w + ((q1.z >> (4 * j)) & 15u)) * 4;
       rtd::touch_l1(scratch, child);
       rtd::touch_l1(scratch, child + 2);
     }
-    auto entry_of = [&](uint32_t i) {
+    auto entry_of = [&](uint32_t i, uint32_t so_i) {
       const uint32_t c = q0.w + ((q1.z >> (4 * i)) & 15u);
-      return make((c << kShift) | level | ((q1.y >> (i + rtw::kLeafShift)) & kLeaf), in);
+      const uint32_t at = STAGED && so_i ? ((so_i << kShift) | kEPin) : c << kShift;
+      return make(at | level | ((q1.y >> (i + rtw::kLeafShift)) & kLeaf), in);
     };
+    auto entry_for_all = [&](uint32_t i) { return entry_of(i, STAGED ? from_lane(so, (int)i) : 0u); };
     const uint32_t below = (1u << j) - 1u;
     e = 0;
     if constexpr (TREELET) {
       const uint32_t same = q1.y >> (from_cu ? rtw::kSameShift : rtw::kOtherShift);
       const uint32_t to_cu = hit & same, to_ot = hit & ~same;
       if ((hit >> j) & 1u) {
-        if ((to_cu >> j) & 1u) cu[ncu + __popc(to_cu & below)] = entry_of(j);
-        else ot[not_ + __popc(to_ot & below)] = entry_of(j);
+        if ((to_cu >> j) & 1u) cu[ncu + __popc(to_cu & below)] = entry_of(j, so);
+        else ot[not_ + __popc(to_ot & below)] = entry_of(j, so);
       }
       ncu += __popc(to_cu);
       not_ += __popc(to_ot);
       __syncwarp(mask);
       if (ncu > depth + 1 || not_ > depth) return stop(RT_RAY_STACK_OVERFLOW);
       if (to_cu) {  // the entry just put on top
-        e = entry_of(31u - __clz(to_cu));
+        e = entry_for_all(31u - __clz(to_cu));
         from_cu = true;
         --ncu;
       }
@@ -194,15 +225,15 @@ struct GroupWalk {
       const uint32_t inner = hit & q1.y;  // the first hit internal child is visited next
       if (inner) {
         const uint32_t i = __ffs(inner) - 1;
-        e = entry_of(i);
+        e = entry_for_all(i);
         hit &= ~(1u << i);
       }
-      if ((hit >> j) & 1u) cu[ncu + __popc(hit & below)] = entry_of(j);
+      if ((hit >> j) & 1u) cu[ncu + __popc(hit & below)] = entry_of(j, so);
       ncu += __popc(hit);
       __syncwarp(mask);
       if (ncu > depth) return stop(RT_RAY_STACK_OVERFLOW);
       if (!e && hit) {
-        e = entry_of(31u - __clz(hit));
+        e = entry_for_all(31u - __clz(hit));
         --ncu;
       }
     }
@@ -219,14 +250,24 @@ struct GroupWalk {
       ok = ((uint32_t)x & (kLeaf | kTop)) == kLeaf;
       if constexpr (TREELET) ok = ok && (uint32_t)(x >> 32) == cx.unit;
     }
-    const uint32_t unit = (uint32_t)x >> kShift;
-    int k = __ffs(~ballot(ok && unit < v.n_units)) - 1;  // leaves of this batch
+    uint32_t unit = 0;
+    const uint4* src = v.blob;
+    if (ok) src = locate((uint32_t)x, v.blob, unit);
+    int k = __ffs(~ballot(ok && (pinned((uint32_t)x) || unit < v.n_units))) - 1;  // leaves of this batch
     if (k == 0) return stop(RT_RAY_BAD_NODE);
     rtd::Node64 q;
     bool quad = false, hit = false;
     float t = 0.0f, wt = 0.0f;
     if ((int)j < k) {
-      rtd::load64(v.blob + (uint64_t)unit * 4, 0, q);
+      if (STAGED) {
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+          const uint4 y = src[w];
+          q.w[4 * w] = y.x, q.w[4 * w + 1] = y.y, q.w[4 * w + 2] = y.z, q.w[4 * w + 3] = y.w;
+        }
+      } else {
+        rtd::load64(src, 0, q);
+      }
       quad = rtf::leaf_type_of(q.w[1]) == 0;
       if (quad) {
         const rtm::V3 v0 = rtm::v3(__uint_as_float(q.w[4]), __uint_as_float(q.w[5]), __uint_as_float(q.w[6]));
@@ -256,6 +297,7 @@ struct GroupWalk {
       }
     }
     if (ballot((int)j < k && !quad)) flags |= RT_RAY_HIT_PROCEDURAL;
+    if (STAGED) count_reads(__popc(ballot((int)j < k && pinned((uint32_t)x))), (uint32_t)k);
     if ((int)j < k) {
       put(n_tx + 2 * j, unit, rtf::TX_LEAF_DESC);
       put(n_tx + 2 * j + 1, unit,
@@ -274,24 +316,50 @@ struct GroupWalk {
   __device__ __forceinline__ void entry() {
     const uint32_t code = (uint32_t)e;
     const bool top = code & kTop;
-    const uint32_t unit = top ? code >> kShift : inst();
-    if (top && unit + 2 > v.n_units) return stop(RT_RAY_BAD_NODE);
+    const bool rec = top && pinned(code);  // a pinned record: decoded rows, units and route bits
+    uint32_t unit = inst();
+    const uint4* src = v.blob;
+    if (top) {
+      src = locate(code, v.blob, unit);
+      if (!rec && unit + 2 > v.n_units) return stop(RT_RAY_BAD_NODE);
+      count_reads(rec ? 1u : 0u, 1u);
+    }
     rtd::Instance in;
-    rtd::load_instance(v.blob + (uint64_t)unit * 4, 0, in);
+    uint4 head = make_uint4(0, 0, 0, 0);
+    if (rec) {
+      head = src[0];
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        const uint4 y = src[rtp::IL_W2O / 16 + k];
+        const uint32_t w[4] = {y.x, y.y, y.z, y.w};
+#pragma unroll
+        for (int q = 0; q < 4; ++q) in.w2o.m[(4 * k + q) / 3][(4 * k + q) % 3] = __uint_as_float(w[q]);
+      }
+    } else {
+      rtd::load_instance(v.blob + (uint64_t)unit * 4, 0, in);
+    }
     enter_instance(in, unit, O, D, tmin, tmax, cx);
     if (!top) return;
     record(unit, rtf::TX_INSTANCE_LEAF);
     extra += kInstanceExtra;
-    const uint64_t hdr = (uint64_t)unit * 64 + in.bvh_address;
-    if ((hdr & 63) || hdr / 64 >= v.n_units) return stop(RT_RAY_BAD_NODE);
-    const uint4 h0 = __ldg(v.blob + (hdr >> 4));
-    const uint64_t broot = hdr + ((uint64_t)h0.x | ((uint64_t)h0.y << 32));
-    record((uint32_t)(hdr >> 6), rtf::TX_STRUCTURE);
-    const uint32_t next = (uint32_t)(broot >> 6) << kShift;
+    uint32_t hdr_unit = head.y, next = 0;
+    if (rec) {
+      const uint32_t so = head.w >> 16;
+      next = so ? ((so << kShift) | kEPin) : head.z << kShift;
+    } else {
+      const uint64_t hdr = (uint64_t)unit * 64 + in.bvh_address;
+      if ((hdr & 63) || hdr / 64 >= v.n_units) return stop(RT_RAY_BAD_NODE);
+      const uint4 h0 = __ldg(v.blob + (hdr >> 4));
+      const uint64_t broot = hdr + ((uint64_t)h0.x | ((uint64_t)h0.y << 32));
+      hdr_unit = (uint32_t)(hdr >> 6);
+      next = (uint32_t)(broot >> 6) << kShift;
+    }
+    record(hdr_unit, rtf::TX_STRUCTURE);
     if constexpr (TREELET) {
       // visited next from the stack its route bit names: cu is popped first,
       // and ot only when cu is empty
-      const bool same = (__ldg(v.route + unit) >> (kRouteInst + (from_cu ? 0u : 1u))) & 1u;
+      const uint32_t route = rec ? head.w & 0xffffu : __ldg(v.route + unit);
+      const bool same = (route >> (kRouteInst + (from_cu ? 0u : 1u))) & 1u;
       if (same ? ncu + 1 > depth + 1 : not_ + 1 > depth) return stop(RT_RAY_STACK_OVERFLOW);
       e = make(next, unit);
       if (same || ncu == 0) {
@@ -326,17 +394,45 @@ struct GroupWalk {
 };
 
 // rays r = group index, + groups of the launch, ...; dynamic shared memory:
-// group_stack_bytes per group of the CTA.
-template <bool TREELET, bool TRACED>
+// the pinned image (STAGED), then group_stack_bytes per group of the CTA.
+template <bool TREELET, bool TRACED, bool STAGED = false>
 __global__ void __launch_bounds__(kGroupThreads) trace_group_kernel(TraceArgs a, uint32_t depth, uint32_t rpw) {
-  using W = GroupWalk<TREELET, TRACED>;
+  using W = GroupWalk<TREELET, TRACED, STAGED>;
   extern __shared__ __align__(128) uint8_t dyn_smem[];
+  __shared__ uint64_t pin_bar;
+  __shared__ uint32_t pin_ok;
+  uint8_t* const smem0 = dyn_smem + ((128u - (smem_u32(dyn_smem) & 127u)) & 127u);
+  if (STAGED) {  // as trace_staged_kernel
+    if (threadIdx.x == 0) {
+      pin_ok = 0;
+      if (a.pin_bytes) {
+        mbar_init(&pin_bar, 1);
+        mbar_expect_tx(&pin_bar, a.pin_bytes);
+        for (uint32_t off = 0; off < a.pin_bytes; off += kPinChunk)
+          bulk_copy_g2s(smem0 + off, reinterpret_cast<const uint8_t*>(a.pin_image) + off,
+                        min(kPinChunk, a.pin_bytes - off), &pin_bar);
+        pin_ok = mbar_wait(&pin_bar, 0, a.wait_tries) ? 1u : 0u;
+        if (!pin_ok) atomicOr(a.status, kStatusTimeout);
+      }
+    }
+    __syncthreads();
+  }
   const uint32_t lane = threadIdx.x & 31u, g = lane / kGroup, warps = blockDim.x / 32u;
   if (g >= rpw) return;
   const uint32_t slot = (threadIdx.x >> 5) * rpw + g;
-  typename W::Entry* stack = reinterpret_cast<typename W::Entry*>(dyn_smem + slot * group_stack_bytes(TREELET, depth));
-  W w{a,    scene_of<false>(a, 0), lane % kGroup, 0xffu << (g * kGroup), (int)depth, stack, stack + depth + kStackPad,
-      smem_u32(dyn_smem) + (slot + 1) * group_stack_bytes(TREELET, depth) - 16u};
+  uint8_t* const mine = smem0 + (STAGED ? a.pin_bytes : 0u) + slot * group_stack_bytes(TREELET, depth);
+  typename W::Entry* stack = reinterpret_cast<typename W::Entry*>(mine);
+  W w{a,
+      scene_of<false>(a, 0),
+      lane % kGroup,
+      0xffu << (g * kGroup),
+      (int)depth,
+      stack,
+      stack + depth + kStackPad,
+      smem_u32(mine) + group_stack_bytes(TREELET, depth) - 16u,
+      STAGED && pin_ok ? smem_u32(smem0) : 0u,
+      STAGED && pin_ok ? a.pin_root : 0u};
+  w.smem_reads = w.gmem_reads = 0;
   unsigned long long bytes = 0;
   for (uint32_t r = blockIdx.x * warps * rpw + slot; r < a.n; r += gridDim.x * warps * rpw) {
     w.run(r);
@@ -344,7 +440,22 @@ __global__ void __launch_bounds__(kGroupThreads) trace_group_kernel(TraceArgs a,
     __syncwarp(w.mask);
   }
   rtd::touch_l1_done();
-  if (a.stats && lane % kGroup == 0 && bytes) atomicAdd(a.stats + ST_NODE_BYTES, bytes);
+  // a pinned image still in flight must land before the CTA's shared memory goes away
+  if (STAGED && threadIdx.x == 0 && a.pin_bytes && !pin_ok) {
+    if (!mbar_wait(&pin_bar, 0, kWaitTries)) atomicOr(a.status, kStatusTimeout);
+  }
+  if (a.stats && lane % kGroup == 0 && bytes) {
+    atomicAdd(a.stats + ST_NODE_BYTES, bytes);
+    if (STAGED) {
+      atomicAdd(a.stats + ST_SMEM_READS, (unsigned long long)w.smem_reads);
+      atomicAdd(a.stats + ST_GMEM_READS, (unsigned long long)w.gmem_reads);
+    }
+  }
+  if (STAGED && a.stats && threadIdx.x == 0 && pin_ok && blockIdx.x == 0) {
+    // the pinned image counts once as staged bytes (copied by every CTA)
+    atomicAdd(a.stats + ST_STAGED_BYTES, (unsigned long long)a.pin_bytes * gridDim.x);
+    atomicAdd(a.stats + ST_STAGINGS, (unsigned long long)gridDim.x);
+  }
 }
 
 }  // namespace rtk
