@@ -101,14 +101,12 @@ __device__ __forceinline__ void load8f(const float* p, float* v) {
 
 // x = [origin, dir, E[current]] (a sample whose current treelet is out of range
 // gets a zero embedding); h1 = GELU(x W1 + b1), h2 = GELU(h1 W2 + b2).  Stores
-// x, z1, h1, z2, h2 and, for the output layer's dW3 product, [h2^T ; ones ;
-// zeros] (h2x, 80 x ldx, columns past n zero).
+// x, z1, h1, z2 and h2.
 __global__ void __launch_bounds__(HT) hidden_forward_kernel(
     const rt_mlp_sample* __restrict__ s, int n, const bf16* __restrict__ E, uint32_t C, const bf16* __restrict__ W1,
     const float* __restrict__ b1, const bf16* __restrict__ W2, const float* __restrict__ b2, bf16* __restrict__ X,
-    float* __restrict__ Z1, bf16* __restrict__ H1, float* __restrict__ Z2, bf16* __restrict__ H2,
-    bf16* __restrict__ H2X, int ldx) {
-  __shared__ __align__(16) bf16 xs[HB][XPP], w1[H][XPP], w2[H][HP], h1[HB][HP], h2t[tcm::HX][HP];
+    float* __restrict__ Z1, bf16* __restrict__ H1, float* __restrict__ Z2, bf16* __restrict__ H2) {
+  __shared__ __align__(16) bf16 xs[HB][XPP], w1[H][XPP], w2[H][HP], h1[HB][HP];
   const int tid = threadIdx.x, row0 = ((tid >> 5) & 3) * 16, col0 = (tid >> 7) * 32, base = blockIdx.x * HB;
   {  // four threads a sample: origin and direction, the embedding's halves, zeros
     const int b = tid >> 2, part = tid & 3;
@@ -168,22 +166,11 @@ __global__ void __launch_bounds__(HT) hidden_forward_kernel(
     for (int r = 0; r < 4; ++r) {
       const int m = acc_row(row0, r), c = acc_col(col0, j, r);
       const float z = acc[j][r] + b2[c];
-      const bool in = base + m < n;
-      const bf16 h = __float2bfloat16(in ? gelu(z) : 0.0f);
-      h2t[c][m] = h;
-      if (in) {
+      if (base + m < n) {
         Z2[(size_t)(base + m) * H + c] = z;
-        H2[(size_t)(base + m) * H + c] = h;
+        H2[(size_t)(base + m) * H + c] = __float2bfloat16(gelu(z));
       }
     }
-  for (int i = tid; i < (tcm::HX - H) * HB; i += HT)
-    h2t[H + i / HB][i % HB] = __float2bfloat16(i / HB == 0 && base + i % HB < n ? 1.0f : 0.0f);
-  __syncthreads();
-  // ldx is a multiple of HB: every CTA writes whole rows of its columns
-  for (int i = tid; i < tcm::HX * (HB / 8); i += HT) {
-    const int k = i / (HB / 8), q = (i % (HB / 8)) * 8;
-    store8(H2X + (size_t)k * ldx + base + q, load8(&h2t[k][q]));
-  }
 }
 
 // dz2 = dh2 * GELU'(z2), [dW2, db2] += h1^T [dz2], dh1 = dz2 W2^T, dz1 = dh1 *
@@ -341,7 +328,7 @@ struct rt_mlp {
   uint64_t n_params = 0, offW1 = 0, offb1 = 0, offW2 = 0, offb2 = 0, offW3 = 0, offb3 = 0;
   float *P = nullptr, *M = nullptr, *V = nullptr, *G = nullptr;
   bf16 *E16 = nullptr, *W1_16 = nullptr, *W2_16 = nullptr;
-  bf16 *W3T = nullptr, *W3P = nullptr, *H2X = nullptr;  // output-layer operands (mlp_tc.cuh)
+  bf16 *W3T = nullptr;                                 // output-layer operand (mlp_tc.cuh)
   uint32_t Cp = 0;                                     // treelets padded to the output chunk
   bf16 *X = nullptr, *H1 = nullptr, *H2 = nullptr;
   float *Z1 = nullptr, *Z2 = nullptr, *dH2 = nullptr;
@@ -374,8 +361,7 @@ void refresh_bf16(rt_mlp* m) {
   to_bf16<<<blocks((uint64_t)m->C * EMB), 256, 0, m->st>>>(m->P, m->E16, (uint64_t)m->C * EMB);
   w1_to_bf16<<<blocks(XP * H), 256, 0, m->st>>>(m->P + m->offW1, m->W1_16);
   to_bf16<<<blocks(H * H), 256, 0, m->st>>>(m->P + m->offW2, m->W2_16, H * H);
-  tcm::w3_operands_kernel<<<m->Cp / 32, 256, 0, m->st>>>(m->P + m->offW3, m->C, m->Cp, m->W3T,
-                                                                          m->W3P);
+  tcm::w3_operand_kernel<<<m->Cp / 32, 256, 0, m->st>>>(m->P + m->offW3, m->C, m->W3T);
 }
 
 // Column splits of the row-tile passes of the output layer: two waves of
@@ -390,16 +376,11 @@ uint32_t out_splits(const rt_mlp* m, uint32_t n) {
 // Shared memory per CTA.  Pass 1 needs 49 KiB but asks for 80, so that
 // exactly two CTAs share an SM (and its 512 TMEM columns).
 constexpr size_t kSmemStats = 80 * 1024;
-constexpr size_t kSmemDh2 = 16384 + 16384 + 32768 + 16384 + 512;
-constexpr size_t kSmemDw3 = 16384 + 16384 + tcm::kDztBytes + 20480 + 512;
 
 tcm::OutArgs out_args(rt_mlp* m, const rt_mlp_sample* s, uint32_t n) {
   tcm::OutArgs a{};
   a.h2 = m->H2;
-  a.h2x = m->H2X;
-  a.ldx = RT_MLP_MAX_BATCH;
   a.w3t = m->W3T;
-  a.w3p = m->W3P;
   a.b3 = m->P + m->offb3;
   a.s = s;
   a.n = n;
@@ -433,20 +414,17 @@ void output_forward(rt_mlp* m, const rt_mlp_sample* s, uint32_t n, uint32_t* top
 // Gradients of the output layer: dW3, db3 into G, dH2 (zeroed first).
 void output_backward(rt_mlp* m, const rt_mlp_sample* s, uint32_t n) {
   const tcm::OutArgs a = out_args(m, s, n);
-  tcm::out_dh2_kernel<<<dim3((n + tcm::TM - 1) / tcm::TM, a.splits), tcm::kThreads, kSmemDh2, m->st>>>(a);
-  // two row halves per chunk, added into the zeroed gradient: 1,494 CTAs
-  // (4.9 waves of 304) instead of 747 (2.5 waves)
-  tcm::out_dw3_kernel<<<dim3(m->Cp / tcm::TN, 2), tcm::kThreads, kSmemDw3, m->st>>>(a);
+  // one CTA per SM, each with an even share of the splits' tiles
+  const uint32_t units = (n + tcm::TM - 1) / tcm::TM * a.splits;
+  tcm::out_grad_kernel<<<std::min(units, 152u), tcm::kGradThreads, tcm::kGradSmem, m->st>>>(a);
 }
 
 // Forward (and, when grads is true, backward into G) for n samples.
 rt_status run(rt_mlp* m, const rt_mlp_sample* s, uint32_t n, bool grads, uint32_t* top4) {
   const int B = (int)n;
   cudaStream_t st = m->st;
-  // whole 128-row tiles: the output layer reads h2x's columns past n as zero
-  hidden_forward_kernel<<<(B + tcm::TM - 1) / tcm::TM * (tcm::TM / HB), HT, 0, st>>>(s, B, m->E16, m->C, m->W1_16, m->P + m->offb1, m->W2_16,
-                                                           m->P + m->offb2, m->X, m->Z1, m->H1, m->Z2, m->H2, m->H2X,
-                                                           (int)RT_MLP_MAX_BATCH);
+  hidden_forward_kernel<<<(B + HB - 1) / HB, HT, 0, st>>>(s, B, m->E16, m->C, m->W1_16, m->P + m->offb1, m->W2_16,
+                                                          m->P + m->offb2, m->X, m->Z1, m->H1, m->Z2, m->H2);
   if (top4) {
     output_forward(m, s, n, top4);
     return RT_OK;
@@ -508,8 +486,6 @@ rt_status rt_mlp_create(rt_ctx* ctx, uint32_t n_treelets, uint64_t seed, rt_mlp*
   chk(mk(&m->W2_16, H * H));
   m->Cp = (uint32_t)((C + tcm::TN - 1) / tcm::TN * tcm::TN);
   chk(mk(&m->W3T, (size_t)m->Cp * H));
-  chk(mk(&m->W3P, (size_t)m->Cp * H));
-  chk(mk(&m->H2X, (size_t)tcm::HX * MB));
   chk(mk(&m->X, MB * XP));
   chk(mk(&m->H1, MB * H));
   chk(mk(&m->H2, MB * H));
@@ -523,8 +499,7 @@ rt_status rt_mlp_create(rt_ctx* ctx, uint32_t n_treelets, uint64_t seed, rt_mlp*
   chk(cudaStreamCreateWithFlags(&m->st, cudaStreamNonBlocking));
   chk(cudaFuncSetAttribute(tcm::out_stats_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemStats));
   chk(cudaFuncSetAttribute(tcm::out_stats_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemStats));
-  chk(cudaFuncSetAttribute(tcm::out_dh2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemDh2));
-  chk(cudaFuncSetAttribute(tcm::out_dw3_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemDw3));
+  chk(cudaFuncSetAttribute(tcm::out_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tcm::kGradSmem));
   if (e == cudaSuccess) e = cudaMemset(m->tstatus, 0, sizeof(uint32_t));
   if (e != cudaSuccess) {
     rt_mlp_destroy(m);
@@ -547,7 +522,7 @@ rt_status rt_mlp_create(rt_ctx* ctx, uint32_t n_treelets, uint64_t seed, rt_mlp*
 rt_status rt_mlp_destroy(rt_mlp* m) {
   if (!m) return RT_OK;
   cudaSetDevice(m->device);
-  void* ptrs[] = {m->P, m->M, m->V, m->G, m->E16, m->W1_16, m->W2_16, m->W3T, m->W3P, m->H2X, m->X, m->H1,
+  void* ptrs[] = {m->P, m->M, m->V, m->G, m->E16, m->W1_16, m->W2_16, m->W3T, m->X, m->H1,
                   m->H2, m->Z1, m->Z2, m->dH2, m->lse, m->part, m->tstatus, m->loss};
   for (void* p : ptrs) cudaFree(p);
   if (m->st) cudaStreamDestroy(m->st);

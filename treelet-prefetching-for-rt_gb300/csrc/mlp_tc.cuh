@@ -7,24 +7,21 @@
 //   dz      = (softmax(z) - onehot(target)) / n
 //   dW3 = h2^T dz,  db3 = column sums of dz,  dh2 = dz W3^T
 //
-// Three passes recompute the logits tile by tile instead of storing them:
+// Two passes compute the logits tile by tile instead of storing them:
 //   out_stats_kernel  per (128-row tile, column split): the online max and
 //                     exp-sum of every row, and the target's logit (or, for
 //                     prediction, the four largest logits);
-//   out_dh2_kernel    per (row tile, column split): dz for the tile, then
-//                     dh2 += dz . W3 on the tensor cores, summed across
-//                     splits with atomics;
-//   out_dw3_kernel    per 128-column chunk and half of the row tiles: dz^T,
-//                     then [dW3 | db3]^T += dz^T . [h2 | 1] on the tensor
-//                     cores, added into the zeroed gradient.
+//   out_grad_kernel   per (up to four row tiles, column split): dz of a tile,
+//                     then both products of it, dh2 += dz . W3 and
+//                     [dW3 | db3]^T += dz^T . [h2 | 1], on the tensor cores.
 //
 // Operands live in shared memory in the canonical K-major layout without
 // swizzle: 8-row x 16-byte core matrices, core matrices of one row group
-// 128 bytes apart along K (the leading-dimension offset; 144 in the dW3
-// pass's dz^T tile), row groups 16 * (K extent) bytes apart (the
-// stride-dimension offset).  One thread issues
-// the MMAs and commits them to an mbarrier; every wait is bounded and a wait
-// that gives up sets the status word instead of hanging.
+// 128 bytes apart along K (the leading-dimension offset), row groups 16 * (K
+// extent) bytes apart (the stride-dimension offset).  A product whose K runs
+// along a tile's rows reads the same tile as an MN-major operand.  One thread
+// issues the MMAs and commits them to an mbarrier; every wait is bounded and a
+// wait that gives up sets the status word instead of hanging.
 #pragma once
 #include <cuda_bf16.h>
 #include <stdint.h>
@@ -61,6 +58,15 @@ __device__ __forceinline__ uint64_t sdesc(uint32_t addr, uint32_t sbo) {
   return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)(128u >> 4) << 16) | ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) |
          ((uint64_t)1 << 46);
 }
+
+// The same tile read the other way round, its row index as K (MN-major, no
+// swizzle): core matrices 128 bytes apart along M or N (the stride-dimension
+// offset), the given distance apart along K (the leading-dimension offset).
+__device__ __forceinline__ uint64_t sdesc_mn(uint32_t addr, uint32_t lbo) {
+  return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) | ((uint64_t)(128u >> 4) << 32) |
+         ((uint64_t)1 << 46);
+}
+constexpr uint32_t kAMn = 1u << 15, kBMn = 1u << 16;  // instruction descriptor: A, B MN-major
 
 // Instruction descriptor of kind::f16: BF16 A and B (both K-major), FP32 accumulator.
 __host__ __device__ constexpr uint32_t idesc(int m, int n) {
@@ -102,14 +108,15 @@ __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.a
 __device__ __forceinline__ void tc_before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_after_sync() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-// kTmemCols TMEM columns for the CTA (one warp allocates); returns the base address.
+// COLS TMEM columns for the CTA (one warp allocates); returns the base address.
 // The .sync.aligned tcgen05 instructions need their whole warp converged,
 // hence the __syncwarp before each.
+template <uint32_t COLS = kTmemCols>
 __device__ __forceinline__ uint32_t tmem_alloc(uint32_t* slot, int warp) {
   __syncwarp();
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(su32(slot)),
-                 "n"(kTmemCols));
+                 "n"(COLS));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
   tc_before_sync();
@@ -118,11 +125,12 @@ __device__ __forceinline__ uint32_t tmem_alloc(uint32_t* slot, int warp) {
   return *slot;
 }
 
+template <uint32_t COLS = kTmemCols>
 __device__ __forceinline__ void tmem_free(uint32_t base, int warp) {
   tc_before_sync();
   __syncthreads();
   __syncwarp();
-  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(base), "n"(kTmemCols));
+  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(base), "n"(COLS));
 }
 
 // 32 consecutive FP32 columns of this thread's TMEM lane; every lane of the
@@ -141,6 +149,20 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
   for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
+}
+
+// 16 of them.
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
+  uint32_t r[16];
+  __syncwarp();
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr));
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
 }
 
 // Byte offset of element (row r, k) of a K-major tile whose K extent is kx.
@@ -174,10 +196,7 @@ __device__ __forceinline__ void load_tile(uint8_t* tile, const bf16* g, uint64_t
 
 struct OutArgs {
   const bf16* h2;       // [n][64] hidden activations of the last layer
-  const bf16* h2x;      // [80][ldx]: h2^T, then a row of ones for valid rows, zeros
-  uint32_t ldx;         // row stride of h2x (elements)
   const bf16* w3t;      // [cp][64]: W3^T, rows past C zero
-  const bf16* w3p;      // [64][cp]: W3, columns past C zero
   const float* b3;      // [C]
   const rt_mlp_sample* s;
   uint32_t n, C, cp;    // rows, treelets, padded treelets (multiple of TN)
@@ -450,232 +469,204 @@ __global__ void out_top4_kernel(const float* __restrict__ part, uint32_t splits,
   for (int q = 0; q < 4; ++q) out[(uint64_t)b * 4 + q] = ti[q];
 }
 
-// dz of element (row, col) from its logit z (bias included, -inf where not
-// live): (softmax - onehot) / n, with sh = lse * log2(e).
-__device__ __forceinline__ float dz_of(float z, float sh, uint32_t col, uint32_t tgt, float inv_n) {
-  return (ex2(fmaf(z, kLog2e, -sh)) - (col == tgt ? 1.0f : 0.0f)) * inv_n;
-}
+// Pass 2, both gradients from one recomputation.  A CTA takes up to kTiles
+// 128-row tiles through the chunks of a column split; per chunk and tile the
+// logits (A = h2 tile, B = W3^T chunk), dz from them into shared memory, and
+// from that one tile
+//   dh2[tile]            += dz . W3             (A = dz,   B = W3^T chunk, read along its rows)
+//   [dW3 | db3]^T[chunk] += dz^T . [h2 | 1]     (A = dz read along its rows, B = [h2 | 1] tile, too)
+// so that neither operand is kept or stored a second time in transposed form.
+// Tensor memory holds the logits, the chunk's dW3 and every tile's dh2; dh2
+// leaves it once per split, dW3 once per chunk, added into the zeroed gradient.
+//
+// What bounds it: the exponentials and the epilogue around them.  The next
+// logits and the last gradient products run on the tensor pipe while sixteen
+// warps are in an epilogue; W3 chunks arrive two ahead.  GB300, 4,096 samples, about
+// 22,150 treelets: 90 us; as two passes with the logits recomputed in each,
+// the products waited for and dz^T stored apart, 111 and 148.
+constexpr uint32_t kTiles = 4;
+constexpr uint32_t kColDw3 = TN, kColDh2 = kColDw3 + 96;  // TMEM columns (dW3 uses 80)
+static_assert(kColDh2 + kTiles * HK <= 512, "tensor memory");
+constexpr int kGradThreads = 512;  // warp w: TMEM lanes 32 (w % 4) .. + 31, column quarter w / 4 of a chunk
+constexpr uint32_t kH2Bytes = TM * HX * 2, kW3Bytes = TN * HK * 2, kDzBytes = TM * TN * 2;
+constexpr uint32_t kW3Bufs = 3;    // read until a chunk's last product, loaded two chunks ahead
+constexpr uint32_t kGradSmem = kTiles * kH2Bytes + kW3Bufs * (kW3Bytes + TN * 4) + kDzBytes;
 
-// Pass 2: dh2[tile] += dz[tile, split's columns] . W3^T.
-__global__ void __launch_bounds__(kThreads, 2) out_dh2_kernel(OutArgs a) {
+__global__ void __launch_bounds__(kGradThreads, 1) out_grad_kernel(OutArgs a) {
   extern __shared__ __align__(1024) uint8_t smem[];
-  uint8_t* a_tile = smem;                     // h2 tile 128 x 64: 16 KiB
-  uint8_t* bz = smem + 16384;                 // W3^T chunk 128 x 64: 16 KiB
-  uint8_t* dz = smem + 32768;                 // dz tile 128 x 128 (K-major, K = 128): 32 KiB
-  uint8_t* bw = smem + 65536;                 // W3 tile 64 x 128 (K-major, K = 128): 16 KiB
-  float* bias = reinterpret_cast<float*>(smem + 81920);
-  __shared__ __align__(8) uint64_t bar;
-  __shared__ uint32_t tmem_slot;
-  const int tid = threadIdx.x, warp = tid >> 5, quad = warp & 3, half = warp >> 2;
-  const uint32_t row0 = blockIdx.x * TM;
-  uint32_t c_beg, c_end;
-  split_range(a, blockIdx.y, c_beg, c_end);
-  if (tid == 0) bar_init(&bar);
-  const uint32_t tmem = tmem_alloc(&tmem_slot, warp);
-  const uint32_t lanes = tmem + ((uint32_t)(quad * 32) << 16);
-  const uint32_t d_h = tmem + TN;  // dh2 accumulator: 64 columns after the logits
-  const uint32_t r = (uint32_t)(quad * 32) + (uint32_t)(tid & 31), row = row0 + r;
-  const bool valid_row = row < a.n;
-  const uint32_t tgt = valid_row ? a.s[row].target : 0xFFFFFFFFu;
-  const float sh = valid_row ? a.lse[row] * kLog2e : 0.0f;
+  uint8_t* const h2 = smem;                          // the tiles' [h2 | 1 | 0], 128 x 80 each
+  uint8_t* const w3 = h2 + kTiles * kH2Bytes;        // W3^T chunks, 128 x 64 each
+  uint8_t* const dz = w3 + kW3Bufs * kW3Bytes;       // 128 x 128
+  float* const bias = reinterpret_cast<float*>(dz + kDzBytes);
+  __shared__ __align__(8) uint64_t bar_l, bar_g;     // logits ready; gradient products done
+  __shared__ uint32_t tmem_slot, s_tgt[kTiles][TM];
+  __shared__ float s_sh[kTiles][TM];                 // lse * log2(e)
+  const uint32_t tid = threadIdx.x, warp = tid >> 5, quad = warp & 3u, quarter = warp >> 2;
+  if (tid == 0) {
+    bar_init(&bar_l);
+    bar_init(&bar_g);
+  }
+  const uint32_t tmem = tmem_alloc<512>(&tmem_slot, (int)warp);
+  const uint32_t lanes = tmem + ((quad * 32u) << 16);
+  const uint32_t r = quad * 32u + (tid & 31u);
   const float inv_n = 1.0f / (float)a.n;
-  uint32_t phase = 0;
+  {  // the one and the zeros behind every h2 row
+    *reinterpret_cast<uint4*>(h2 + (tid / TM) * kH2Bytes + koff(tid % TM, HK, HX)) = make_uint4(0x3f80u, 0, 0, 0);
+    *reinterpret_cast<uint4*>(h2 + (tid / TM) * kH2Bytes + koff(tid % TM, HK + 8, HX)) = make_uint4(0, 0, 0, 0);
+  }
+  const uint32_t tiles = (a.n + TM - 1) / TM, units = a.splits * tiles;  // unit: a split of a tile
+  const uint32_t u_end = (uint32_t)((uint64_t)units * (blockIdx.x + 1u) / gridDim.x);
+  uint32_t u = (uint32_t)((uint64_t)units * blockIdx.x / gridDim.x), par_l = 0, par_g = 0;
   bool ok = true;
-  load_tile(a_tile, a.h2, HK, row0, TM, a.n, 0, HK);
-  for (uint32_t c = c_beg; c < c_end; ++c) {
-    load_tile(bz, a.w3t, HK, c * TN, TN, a.cp, 0, HK);
-    load_tile(bw, a.w3p, a.cp, 0, HK, HK, c * TN, TN);
-    load_bias(bias, a.b3, c, a.C);
+  auto load_chunk = [&](uint32_t c, uint32_t buf) {
+    load_tile(w3 + buf * kW3Bytes, a.w3t, HK, c * TN, TN, a.cp, 0, HK);
+    load_bias(bias + buf * TN, a.b3, c, a.C);
     cp_commit();
+  };
+  auto issue_logits = [&](uint32_t i, uint32_t buf) {
+    tc_after_sync();
+#pragma unroll
+    for (uint32_t kk = 0; kk < HK / 16; ++kk)
+      mma(tmem, sdesc(su32(h2 + i * kH2Bytes) + kk * 256u, HX * 16u), sdesc(su32(w3 + buf * kW3Bytes) + kk * 256u, HK * 16u),
+          idesc(TM, TN), kk > 0 ? 1u : 0u);
+    commit(&bar_l);
+  };
+  auto next = [](uint32_t buf) { return buf + 1 == kW3Bufs ? 0u : buf + 1; };
+  // lane r of the accumulator is the chunk's column r: 64 weight gradients, then the bias gradient
+  auto add_dw3 = [&](uint32_t c) {
+    const uint32_t col = c * TN + r, k0 = quarter * 16u;
+    float v[16];
+    tmem_ld16(lanes + kColDw3 + k0, v);
+    if (col < a.C) {
+#pragma unroll
+      for (int k = 0; k < 16; ++k) atomicAdd(a.dw3 + (uint64_t)(k0 + k) * a.C + col, v[k]);
+    }
+    if (quarter == 0) {
+      tmem_ld16(lanes + kColDw3 + HK, v);
+      if (col < a.C) atomicAdd(a.db3 + col, v[0]);
+    }
+  };
+  while (u < u_end) {
+    // this CTA's tiles t0 .. t0 + nt - 1 of one split
+    const uint32_t t0 = u % tiles, nt = min(min(tiles - t0, u_end - u), kTiles);
+    uint32_t c_beg, c_end;
+    split_range(a, u / tiles, c_beg, c_end);
+    u += nt;
+    if (c_beg >= c_end) continue;
+    for (uint32_t x = tid; x < nt * TM * (HK / 8u); x += kGradThreads) {
+      const uint32_t row = x / (HK / 8u), k = x % (HK / 8u) * 8u;
+      uint8_t* dst = h2 + row / TM * kH2Bytes + koff(row % TM, k, HX);
+      if (t0 * TM + row < a.n) cp16(dst, a.h2 + (uint64_t)(t0 * TM + row) * HK + k);
+      else *reinterpret_cast<uint4*>(dst) = make_uint4(0, 0, 0, 0);
+    }
+    if (tid < nt * TM) {
+      const uint32_t row = t0 * TM + tid;
+      s_tgt[tid / TM][tid % TM] = row < a.n ? a.s[row].target : 0xFFFFFFFFu;
+      s_sh[tid / TM][tid % TM] = row < a.n ? a.lse[row] * kLog2e : 0.0f;
+    }
+    load_chunk(c_beg, 0);
+    if (c_beg + 1 < c_end) load_chunk(c_beg + 1, 1);
     cp_wait_all();
     fence_async_smem();
     tc_before_sync();
     __syncthreads();
-    if (tid == 0) {
-      tc_after_sync();
-      mma_logits(tmem, a_tile, bz);
-      commit(&bar);
-    }
-    if (!bar_wait(&bar, phase)) ok = false;
-    phase ^= 1u;
-    tc_after_sync();
-#pragma unroll 1
-    for (int sl = 0; sl < 2; ++sl) {
-      const uint32_t cl0 = (uint32_t)(half * 64 + sl * 32);
-      const uint32_t col0 = c * TN + cl0;
-      float v[32];
-      logits32(lanes + cl0, bias + cl0, col0, a.C, valid_row, v);
+    if (tid == 0) issue_logits(0, 0);
+    uint32_t buf = 0;
+    for (uint32_t c = c_beg; c < c_end; ++c) {
+      for (uint32_t i = 0; i < nt; ++i) {
+        const bool first = i == 0 && c == c_beg, last = i + 1 == nt && c + 1 == c_end;
+        const uint32_t tgt = s_tgt[i][r];
+        const float sh = s_sh[i][r];
+        if (!bar_wait(&bar_l, par_l)) ok = false;
+        par_l ^= 1u;
+        tc_after_sync();
+        const uint32_t cl0 = quarter * 32u, col0 = c * TN + cl0;
+        float v[32];
+        logits32(lanes + cl0, bias + buf * TN + cl0, col0, a.C, (t0 + i) * TM + r < a.n, v);
+        cp_wait_all();
+        fence_async_smem();
+        tc_before_sync();
+        __syncthreads();  // every warp has its logits; the chunk asked for one chunk ago is in place
+        if (tid == 0 && !last) issue_logits(i + 1 == nt ? 0u : i + 1, i + 1 == nt ? next(buf) : buf);
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        uint32_t w[4];
+        for (int k = 0; k < 32; ++k) v[k] = ex2(fmaf(v[k], kLog2e, -sh));  // ex2(-inf) = 0: dead columns give 0
+        if (tgt - col0 < 32u) {
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int j = q * 8 + 2 * e;
-          const float d0 = dz_of(v[j], sh, col0 + j, tgt, inv_n);  // ex2(-inf) = 0: dead columns give 0
-          const float d1 = dz_of(v[j + 1], sh, col0 + j + 1, tgt, inv_n);
-          const __nv_bfloat162 pr = __floats2bfloat162_rn(d0, d1);
-          w[e] = *reinterpret_cast<const uint32_t*>(&pr);
+          for (int k = 0; k < 32; ++k)
+            if (col0 + k == tgt) v[k] -= 1.0f;
         }
-        *reinterpret_cast<uint4*>(dz + koff(r, cl0 + (uint32_t)(q * 8), TN)) = make_uint4(w[0], w[1], w[2], w[3]);
+        uint32_t w[16];
+#pragma unroll
+        for (int k = 0; k < 16; ++k) {
+          const __nv_bfloat162 pr = __floats2bfloat162_rn(v[2 * k] * inv_n, v[2 * k + 1] * inv_n);
+          w[k] = *reinterpret_cast<const uint32_t*>(&pr);
+        }
+        if (!first) {
+          if (!bar_wait(&bar_g, par_g)) ok = false;  // the last products have read dz
+          par_g ^= 1u;
+          tc_after_sync();
+        }
+        if (i == 0) {
+          if (c > c_beg) add_dw3(c - 1);
+          if (c + 2 < c_end) load_chunk(c + 2, next(next(buf)));  // over chunk c - 1
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          *reinterpret_cast<uint4*>(dz + koff(r, cl0 + (uint32_t)(q * 8), TN)) =
+              make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
+        fence_async_smem();
+        tc_before_sync();
+        __syncthreads();
+        if (tid == 0) {
+          tc_after_sync();
+#pragma unroll
+          for (uint32_t kk = 0; kk < TN / 16; ++kk)
+            mma(tmem + kColDh2 + i * HK, sdesc(su32(dz) + kk * 256u, TN * 16u),
+                sdesc_mn(su32(w3 + buf * kW3Bytes) + kk * (2u * HK * 16u), HK * 16u), idesc(TM, HK) | kBMn,
+                (c > c_beg || kk > 0) ? 1u : 0u);
+#pragma unroll
+          for (uint32_t kk = 0; kk < TM / 16; ++kk)
+            mma(tmem + kColDw3, sdesc_mn(su32(dz) + kk * (2u * TN * 16u), TN * 16u),
+                sdesc_mn(su32(h2 + i * kH2Bytes) + kk * (2u * HX * 16u), HX * 16u), idesc(TM, HX) | kAMn | kBMn,
+                (i > 0 || kk > 0) ? 1u : 0u);
+          commit(&bar_g);
+        }
+      }
+      buf = next(buf);
+    }
+    if (!bar_wait(&bar_g, par_g)) ok = false;
+    par_g ^= 1u;
+    tc_after_sync();
+    add_dw3(c_end - 1);
+    for (uint32_t i = 0; i < nt; ++i) {  // a quarter of the tile's columns each
+      float v[16];
+      tmem_ld16(lanes + kColDh2 + i * HK + quarter * 16u, v);
+      const uint32_t row = (t0 + i) * TM + r;
+      if (row < a.n) {
+        float4* p = reinterpret_cast<float4*>(a.dh2 + (uint64_t)row * HK + quarter * 16u);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) atomicAdd(p + q, make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]));
       }
     }
-    fence_async_smem();
     tc_before_sync();
-    __syncthreads();
-    if (tid == 0) {
-      tc_after_sync();
-#pragma unroll
-      for (int kk = 0; kk < TN / 16; ++kk)
-        mma(d_h, sdesc(su32(dz) + kk * 256u, TN * 16u), sdesc(su32(bw) + kk * 256u, TN * 16u), idesc(TM, HK),
-            (c > c_beg || kk > 0) ? 1u : 0u);
-      commit(&bar);
-    }
-    if (!bar_wait(&bar, phase)) ok = false;  // dz and bw are read before they are rewritten
-    phase ^= 1u;
+    __syncthreads();  // the next tiles' operands and accumulators may replace these
     tc_after_sync();
   }
   if (!ok) atomicOr(a.status, 1u);
-  cp_wait_all();  // no copy may still be landing when the CTA exits
-  if (c_beg < c_end) {
-    // tcgen05.ld is warp-collective: every lane loads, valid rows store; the
-    // two column halves of the CTA take 32 of the 64 columns each
-    float v[32];
-    tmem_ld32(d_h + ((uint32_t)(quad * 32) << 16) + (uint32_t)(half * 32), v);
-    if (valid_row) {
-#pragma unroll
-      for (int j = 0; j < 32; ++j) atomicAdd(a.dh2 + (uint64_t)row * HK + half * 32 + j, v[j]);
-    }
-  }
-  tmem_free(tmem, warp);
+  tmem_free<512>(tmem, (int)warp);
 }
 
-// dz^T tile of pass 3 (128 treelet columns x 128 batch rows, K-major along
-// the rows) with its K-adjacent core matrices 144 bytes apart instead of
-// 128: a warp writes one column's 32 rows, and with 128-byte spacing rows r
-// and r + 8 fell on the same banks (40M conflicts of 65M shared-memory
-// wavefronts in pass 3); 144 bytes spreads the four groups of 8 rows over
-// 16 banks.
-constexpr uint32_t kDztLbo = 144, kDztSbo = 16 * kDztLbo;  // 16 K groups per 8-column group
-constexpr uint32_t kDztBytes = 16 * kDztSbo;               // 36 KiB
-__device__ __forceinline__ uint32_t dzt_off(uint32_t col, uint32_t row) {
-  return (col >> 3) * kDztSbo + (row >> 3) * kDztLbo + (col & 7u) * 16u + (row & 7u) * 2u;
-}
-__device__ __forceinline__ uint64_t sdesc_lbo(uint32_t addr, uint32_t lbo, uint32_t sbo) {
-  return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) |
-         ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | ((uint64_t)1 << 46);
-}
-
-// Pass 3: per 128-column chunk and half of the row tiles (blockIdx.y),
-// [dW3 | db3]^T += sum over those row tiles of dz^T . [h2 | 1], added into
-// the zeroed gradient.
-__global__ void __launch_bounds__(kThreads, 2) out_dw3_kernel(OutArgs a) {
-  extern __shared__ __align__(1024) uint8_t smem[];
-  uint8_t* bz = smem;                          // W3^T chunk 128 x 64: 16 KiB (the CTA's, fixed)
-  uint8_t* a_tile = smem + 16384;              // h2 tile 128 x 64: 16 KiB
-  uint8_t* dzt = smem + 32768;                 // dz^T 128 x 128 (K-major, K = 128 rows, padded): 36 KiB
-  uint8_t* bx = smem + 32768 + kDztBytes;      // [h2 | 1]^T tile 80 x 128 (K-major): 20 KiB
-  float* bias = reinterpret_cast<float*>(smem + 32768 + kDztBytes + 20480);
-  __shared__ __align__(8) uint64_t bar;
-  __shared__ uint32_t tmem_slot;
-  const int tid = threadIdx.x, warp = tid >> 5, quad = warp & 3, half = warp >> 2;
-  const uint32_t c = blockIdx.x;  // chunk
-  if (tid == 0) bar_init(&bar);
-  const uint32_t tmem = tmem_alloc(&tmem_slot, warp);
-  const uint32_t lanes = tmem + ((uint32_t)(quad * 32) << 16);
-  const uint32_t d_w = tmem + TN;  // [dW3 | db3]^T accumulator: 80 columns after the logits
-  const float inv_n = 1.0f / (float)a.n;
-  const uint32_t tiles = (a.n + TM - 1) / TM, per = (tiles + gridDim.y - 1) / gridDim.y;
-  const uint32_t t_beg = min(tiles, blockIdx.y * per), t_end = min(tiles, t_beg + per);
-  const uint32_t r = (uint32_t)(quad * 32) + (uint32_t)(tid & 31);
-  uint32_t phase = 0;
-  bool ok = true;
-  load_tile(bz, a.w3t, HK, c * TN, TN, a.cp, 0, HK);
-  load_bias(bias, a.b3, c, a.C);
-  for (uint32_t t = t_beg; t < t_end; ++t) {
-    const uint32_t row0 = t * TM, row = row0 + r;
-    const bool valid_row = row < a.n;
-    const uint32_t tgt = valid_row ? a.s[row].target : 0xFFFFFFFFu;
-    const float sh = valid_row ? a.lse[row] * kLog2e : 0.0f;
-    load_tile(a_tile, a.h2, HK, row0, TM, a.n, 0, HK);
-    load_tile(bx, a.h2x, a.ldx, 0, HX, HX, row0, TM);
-    cp_commit();
-    cp_wait_all();
-    fence_async_smem();
-    tc_before_sync();
-    __syncthreads();
-    if (tid == 0) {
-      tc_after_sync();
-      mma_logits(tmem, a_tile, bz);
-      commit(&bar);
-    }
-    if (!bar_wait(&bar, phase)) ok = false;
-    phase ^= 1u;
-    tc_after_sync();
-#pragma unroll 1
-    for (int sl = 0; sl < 2; ++sl) {
-      const uint32_t cl0 = (uint32_t)(half * 64 + sl * 32);
-      const uint32_t col0 = c * TN + cl0;
-      float v[32];
-      logits32(lanes + cl0, bias + cl0, col0, a.C, valid_row, v);
-#pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        // dz^T: element (column cl0 + j, row r)
-        *reinterpret_cast<bf16*>(dzt + dzt_off(cl0 + (uint32_t)j, r)) =
-            __float2bfloat16_rn(dz_of(v[j], sh, col0 + j, tgt, inv_n));
-      }
-    }
-    fence_async_smem();
-    tc_before_sync();
-    __syncthreads();
-    if (tid == 0) {
-      tc_after_sync();
-#pragma unroll
-      for (int kk = 0; kk < TM / 16; ++kk)
-        mma(d_w, sdesc_lbo(su32(dzt) + kk * 2u * kDztLbo, kDztLbo, kDztSbo), sdesc(su32(bx) + kk * 256u, TM * 16u),
-            idesc(TM, HX), (t > t_beg || kk > 0) ? 1u : 0u);
-      commit(&bar);
-    }
-    if (!bar_wait(&bar, phase)) ok = false;
-    phase ^= 1u;
-    tc_after_sync();
-  }
-  if (!ok) atomicOr(a.status, 1u);
-  cp_wait_all();
-  // lane r of the accumulator is column c * 128 + r: 64 weight gradients,
-  // then the bias gradient; column half 0 takes k 0..31, half 1 k 32..95
-  // (the last load reads past the 80 columns, within the allocation)
-  if (t_beg < t_end) {
-    const uint32_t col = c * TN + r;
-    float v[32];
-    for (int q = half; q < (half ? 3 : 1); ++q) {
-      tmem_ld32(d_w + ((uint32_t)(quad * 32) << 16) + (uint32_t)(q * 32), v);
-      if (col < a.C) {
-#pragma unroll
-        for (int j = 0; j < 32; ++j) {
-          const int k = q * 32 + j;
-          if (k < HK) atomicAdd(a.dw3 + (uint64_t)k * a.C + col, v[j]);
-          else if (k == HK) atomicAdd(a.db3 + col, v[j]);
-        }
-      }
-    }
-  }
-  tmem_free(tmem, warp);
-}
-
-// W3 (FP32 master, [64][C]) as the two padded BF16 operands: W3 itself
-// ([64][cp]) and W3^T ([cp][64]).  One block per 32 columns: W3's rows are
-// read and written along the columns, W3^T's through a shared-memory
-// transpose (one thread per column wrote 2-byte entries 128 bytes apart).
-__global__ void __launch_bounds__(256) w3_operands_kernel(const float* __restrict__ w3, uint32_t C, uint32_t cp,
-                                                          bf16* __restrict__ w3t, bf16* __restrict__ w3p) {
+// W3 (FP32 master, [64][C]) as the padded BF16 operand W3^T ([cp][64]).  One
+// block per 32 columns: W3's rows are read along the columns, W3^T's written
+// through a shared-memory transpose (one thread per column wrote 2-byte entries
+// 128 bytes apart).
+__global__ void __launch_bounds__(256) w3_operand_kernel(const float* __restrict__ w3, uint32_t C,
+                                                         bf16* __restrict__ w3t) {
   __shared__ __align__(4) bf16 t[32][HK + 2];  // [column][k]: rows 132 bytes apart, no bank conflicts
   const uint32_t c0 = blockIdx.x * 32, tx = threadIdx.x & 31u, ty = threadIdx.x >> 5;
   const uint32_t c = c0 + tx;
-  for (uint32_t k = ty; k < (uint32_t)HK; k += 8) {
-    const bf16 v = __float2bfloat16_rn(c < C ? w3[(uint64_t)k * C + c] : 0.0f);
-    w3p[(uint64_t)k * cp + c] = v;
-    t[tx][k] = v;
-  }
+  for (uint32_t k = ty; k < (uint32_t)HK; k += 8)
+    t[tx][k] = __float2bfloat16_rn(c < C ? w3[(uint64_t)k * C + c] : 0.0f);
   __syncthreads();
   for (uint32_t i = threadIdx.x; i < 32u * (HK / 2); i += blockDim.x) {
     const uint32_t cl = i / (HK / 2), kp = i % (HK / 2);
