@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "f32x2.cuh"
 #include "format.h"
 #include "rtmath.h"
 #include "walk_node.h"
@@ -76,41 +77,6 @@ __device__ __forceinline__ uint4 load16(const uint4* g, uint32_t saddr, int q) {
 }
 
 __device__ __forceinline__ float f32_at(const Node64& n, int b) { return __uint_as_float(n.w[b >> 2]); }
-
-// Two-wide FP32 arithmetic (add / sub / mul / fma .rn.f32x2, sm_100 and
-// later): one instruction computes two lanes, each rounded exactly as the
-// scalar instruction rounds it (IEEE round to nearest even, subnormals
-// kept), so the results are bit for bit those of two scalar operations.  The
-// slab test pairs a child's x and y planes in them.
-__device__ __forceinline__ unsigned long long f2_pack(float x, float y) {
-  unsigned long long r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
-  return r;
-}
-__device__ __forceinline__ unsigned long long f2_pack_bits(uint32_t x, uint32_t y) {
-  unsigned long long r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(x), "r"(y));
-  return r;
-}
-__device__ __forceinline__ void f2_unpack(unsigned long long r, float& x, float& y) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(r));
-}
-__device__ __forceinline__ unsigned long long f2_sub(unsigned long long a, unsigned long long b) {
-  unsigned long long r;
-  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ unsigned long long f2_mul(unsigned long long a, unsigned long long b) {
-  unsigned long long r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ unsigned long long f2_fma(unsigned long long a, unsigned long long b,
-                                                     unsigned long long c) {
-  unsigned long long r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
 
 // A bound's byte q becomes a float by one byte permute, which places it in the
 // mantissa of 2^23, and a subtraction of 2^23 (both exact).  The child bound

@@ -175,12 +175,13 @@ __global__ void __launch_bounds__(HT) hidden_forward_kernel(
 
 // dz2 = dh2 * GELU'(z2), [dW2, db2] += h1^T [dz2], dh1 = dz2 W2^T, dz1 = dh1 *
 // GELU'(z1), [dW1, db1] += x^T [dz1], dx = dz1 W1^T into the embedding's rows.
-// The dz are BF16, products FP32; weight gradients are added into G.
+// The dz are BF16, products FP32; weight gradients are added into G.  dh2
+// arrives as one partial sum per column split of the output layer.
 __global__ void __launch_bounds__(HT) hidden_backward_kernel(
     const rt_mlp_sample* __restrict__ s, int n, uint32_t C, const bf16* __restrict__ W1, const bf16* __restrict__ W2,
     const bf16* __restrict__ X, const float* __restrict__ Z1, const bf16* __restrict__ H1,
-    const float* __restrict__ Z2, const float* __restrict__ dH2, float* __restrict__ gE, float* __restrict__ gW1,
-    float* __restrict__ gb1, float* __restrict__ gW2, float* __restrict__ gb2) {
+    const float* __restrict__ Z2, const float* __restrict__ dH2, uint32_t splits, float* __restrict__ gE,
+    float* __restrict__ gW1, float* __restrict__ gb1, float* __restrict__ gW2, float* __restrict__ gb2) {
   __shared__ __align__(16) bf16 dz[HB][HP], dzt[H][HP], ht[H][HP], w[H][HP], xt[XP][HP];
   const int tid = threadIdx.x, warp = tid >> 5, row0 = (warp & 3) * 16, col0 = (warp >> 2) * 32, base = blockIdx.x * HB;
   const bf16 zero = __float2bfloat16(0.0f);
@@ -192,7 +193,15 @@ __global__ void __launch_bounds__(HT) hidden_backward_kernel(
     for (int q = 0; q < 8; ++q) d.v[q] = e.v[q] = zero;
     if (base + b < n) {
       float g[8], z[8];
-      load8f(dH2 + (size_t)(base + b) * H + c, g);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) g[q] = 0.0f;
+#pragma unroll 8
+      for (uint32_t k = 0; k < splits; ++k) {  // in the splits' order: the sum is the same on every run
+        float p[8];
+        load8f(dH2 + ((size_t)k * n + base + b) * H + c, p);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) g[q] += p[q];
+      }
       load8f(Z2 + (size_t)(base + b) * H + c, z);
       e = load8(H1 + (size_t)(base + b) * H + c);
 #pragma unroll
@@ -331,7 +340,7 @@ struct rt_mlp {
   bf16 *W3T = nullptr;                                 // output-layer operand (mlp_tc.cuh)
   uint32_t Cp = 0;                                     // treelets padded to the output chunk
   bf16 *X = nullptr, *H1 = nullptr, *H2 = nullptr;
-  float *Z1 = nullptr, *Z2 = nullptr, *dH2 = nullptr;
+  float *Z1 = nullptr, *Z2 = nullptr;
   float *lse = nullptr, *part = nullptr;
   uint32_t* tstatus = nullptr;                         // bit 0: a bounded wait of the output layer gave up
   double* loss = nullptr;                              // sum over the samples of their loss / n
@@ -364,8 +373,8 @@ void refresh_bf16(rt_mlp* m) {
   tcm::w3_operand_kernel<<<m->Cp / 32, 256, 0, m->st>>>(m->P + m->offW3, m->C, m->W3T);
 }
 
-// Column splits of the row-tile passes of the output layer: two waves of
-// two CTAs per SM over the row tiles of the batch (at most 152 splits: the
+// Column splits of the row-tile passes of the output layer: one wave of
+// four CTAs per SM over the row tiles of the batch (at most 152 splits: the
 // partial-result buffer holds 2 x 152 per row).
 uint32_t out_splits(const rt_mlp* m, uint32_t n) {
   const uint32_t tiles = (n + tcm::TM - 1) / tcm::TM, chunks = m->Cp / tcm::TN;
@@ -373,9 +382,8 @@ uint32_t out_splits(const rt_mlp* m, uint32_t n) {
   return std::max<uint32_t>(1, std::min(std::min(chunks, want), 152u));
 }
 
-// Shared memory per CTA.  Pass 1 needs 49 KiB but asks for 80, so that
-// exactly two CTAs share an SM (and its 512 TMEM columns).
-constexpr size_t kSmemStats = 80 * 1024;
+// Shared memory per CTA of pass 1: an h2 tile, two W3 chunks and their biases.
+constexpr size_t kSmemStats = 16384 + 2 * 16384 + 1024;
 
 tcm::OutArgs out_args(rt_mlp* m, const rt_mlp_sample* s, uint32_t n) {
   tcm::OutArgs a{};
@@ -389,7 +397,7 @@ tcm::OutArgs out_args(rt_mlp* m, const rt_mlp_sample* s, uint32_t n) {
   a.splits = out_splits(m, n);
   a.part = m->part;
   a.lse = m->lse;
-  a.dh2 = m->dH2;
+  a.dh2 = m->part;  // pass 1's partial results are used up by then
   a.dw3 = m->G + m->offW3;
   a.db3 = m->G + m->offb3;
   a.status = m->tstatus;
@@ -411,12 +419,12 @@ void output_forward(rt_mlp* m, const rt_mlp_sample* s, uint32_t n, uint32_t* top
                                                                                   m->lse, m->loss);
 }
 
-// Gradients of the output layer: dW3, db3 into G, dH2 (zeroed first).
+// Gradients of the output layer: dW3 and db3 into the zeroed G, dH2 as partial sums into part.
 void output_backward(rt_mlp* m, const rt_mlp_sample* s, uint32_t n) {
   const tcm::OutArgs a = out_args(m, s, n);
   // one CTA per SM, each with an even share of the splits' tiles
   const uint32_t units = (n + tcm::TM - 1) / tcm::TM * a.splits;
-  tcm::out_grad_kernel<<<std::min(units, 152u), tcm::kGradThreads, tcm::kGradSmem, m->st>>>(a);
+  tcm::out_grad_kernel<<<std::min(units, 152u), tcm::kGradThreads + 32, tcm::kGradSmem, m->st>>>(a);
 }
 
 // Forward (and, when grads is true, backward into G) for n samples.
@@ -433,12 +441,11 @@ rt_status run(rt_mlp* m, const rt_mlp_sample* s, uint32_t n, bool grads, uint32_
   output_forward(m, s, n, nullptr);
   if (!grads) return RT_OK;
   MLP_CUDA(cudaMemsetAsync(m->G, 0, sizeof(float) * m->n_params, st));
-  // W3, b3 and dH2 = dz W3^T, on the tensor cores without the logits
-  MLP_CUDA(cudaMemsetAsync(m->dH2, 0, sizeof(float) * B * H, st));
   output_backward(m, s, n);
   hidden_backward_kernel<<<(B + HB - 1) / HB, HT, 0, st>>>(s, B, m->C, m->W1_16, m->W2_16, m->X, m->Z1, m->H1, m->Z2,
-                                                            m->dH2, m->G, m->G + m->offW1, m->G + m->offb1,
-                                                            m->G + m->offW2, m->G + m->offb2);
+                                                           m->part, tcm::live_splits(m->Cp, out_splits(m, n)), m->G,
+                                                           m->G + m->offW1, m->G + m->offb1, m->G + m->offW2,
+                                                           m->G + m->offb2);
   return RT_OK;
 }
 
@@ -492,9 +499,11 @@ rt_status rt_mlp_create(rt_ctx* ctx, uint32_t n_treelets, uint64_t seed, rt_mlp*
   chk(mk(&m->Z1, MB * H));
   chk(mk(&m->Z2, MB * H));
   chk(mk(&m->lse, MB));
-  chk(mk(&m->part, 8 * 152 * 2 * MB));  // 2 x 152 partial results of 8 floats per row
+  // 2 x 152 partial results of 8 floats per row; or dH2's partial sums: at most
+  // 4 x 152 + 31 row tiles' splits (out_splits) of 128 x 64 floats
+  static_assert(8 * 152 * 2 * (uint64_t)RT_MLP_MAX_BATCH >= (4 * 152 + RT_MLP_MAX_BATCH / tcm::TM) * (uint64_t)tcm::TM * H);
+  chk(mk(&m->part, 8 * 152 * 2 * MB));
   chk(mk(&m->tstatus, 1));
-  chk(mk(&m->dH2, MB * H));
   chk(mk(&m->loss, 1));
   chk(cudaStreamCreateWithFlags(&m->st, cudaStreamNonBlocking));
   chk(cudaFuncSetAttribute(tcm::out_stats_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemStats));
@@ -523,7 +532,7 @@ rt_status rt_mlp_destroy(rt_mlp* m) {
   if (!m) return RT_OK;
   cudaSetDevice(m->device);
   void* ptrs[] = {m->P, m->M, m->V, m->G, m->E16, m->W1_16, m->W2_16, m->W3T, m->X, m->H1,
-                  m->H2, m->Z1, m->Z2, m->dH2, m->lse, m->part, m->tstatus, m->loss};
+                  m->H2, m->Z1, m->Z2, m->lse, m->part, m->tstatus, m->loss};
   for (void* p : ptrs) cudaFree(p);
   if (m->st) cudaStreamDestroy(m->st);
   delete m;

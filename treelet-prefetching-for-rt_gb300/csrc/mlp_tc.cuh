@@ -26,6 +26,8 @@
 #include <cuda_bf16.h>
 #include <stdint.h>
 
+#include "f32x2.cuh"
+
 namespace tcm {
 
 using bf16 = __nv_bfloat16;
@@ -37,9 +39,9 @@ constexpr int HX = 80;           // [h2 | 1 | 0 ...] rows of the dW3 operand
 // Eight warps a CTA: warp w reads TMEM lanes 32 (w % 4) .. 32 (w % 4) + 31
 // (the lanes a warp may access) and column half w / 4 of every chunk.
 constexpr int kThreads = 256;
-// TMEM columns a CTA allocates: two CTAs share an SM's 512, so one CTA's
-// epilogue runs while the other's MMAs and copies do.
-constexpr uint32_t kTmemCols = 256;
+// TMEM columns a CTA of pass 1 allocates: four CTAs share an SM's 512, and one's
+// epilogue runs while the others' MMAs and copies do.
+constexpr uint32_t kTmemCols = 128;
 constexpr uint32_t kTries = 1u << 22;
 constexpr float kLog2e = 1.4426950408889634f;
 
@@ -177,6 +179,13 @@ __device__ __forceinline__ void cp16(void* dst, const void* src) {
 __device__ __forceinline__ void cp4(void* dst, const void* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(su32(dst)), "l"(src) : "memory");
 }
+// Named barrier of `threads` threads: arrive without waiting, or wait.
+__device__ __forceinline__ void nb_arrive(int id, int threads) {
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+__device__ __forceinline__ void nb_sync(int id, int threads) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cp_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
@@ -203,11 +212,17 @@ struct OutArgs {
   uint32_t splits;      // column splits of the row-tile passes
   float* part;          // [3][splits][n]: max, exp-sum, target logit (stats); or [splits][n][8] top-4 (pairs)
   const float* lse;     // [n]
-  float* dh2;           // [n][64], summed atomically
+  float* dh2;           // [splits][n][64]: a partial sum per split that has chunks
   float* dw3;           // [64][C]
   float* db3;           // [C]
   uint32_t* status;     // bit 0: a bounded wait gave up
 };
+
+// Splits that have chunks: the first so many.
+__host__ __device__ constexpr uint32_t live_splits(uint32_t cp, uint32_t splits) {
+  const uint32_t chunks = cp / TN, per = (chunks + splits - 1) / splits;
+  return (chunks + per - 1) / per;
+}
 
 // Columns [c_beg, c_end) of split `sp`, in whole chunks.
 __device__ __forceinline__ void split_range(const OutArgs& a, uint32_t sp, uint32_t& c_beg, uint32_t& c_end) {
@@ -240,7 +255,11 @@ __device__ __forceinline__ void logits32(uint32_t taddr, const float* bias, uint
   tmem_ld32(taddr, v);
   if (valid_row && col0 + 32 <= C) {
 #pragma unroll
-    for (int j = 0; j < 32; ++j) v[j] += bias[j];
+    for (int j = 0; j < 32; j += 4) {
+      const float4 b = *reinterpret_cast<const float4*>(bias + j);
+      rtd::f2_unpack(rtd::f2_add(rtd::f2_pack(v[j], v[j + 1]), rtd::f2_pack(b.x, b.y)), v[j], v[j + 1]);
+      rtd::f2_unpack(rtd::f2_add(rtd::f2_pack(v[j + 2], v[j + 3]), rtd::f2_pack(b.z, b.w)), v[j + 2], v[j + 3]);
+    }
   } else {
 #pragma unroll
     for (int j = 0; j < 32; ++j) v[j] = (valid_row && col0 + j < C) ? v[j] + bias[j] : -INFINITY;
@@ -248,36 +267,34 @@ __device__ __forceinline__ void logits32(uint32_t taddr, const float* bias, uint
 }
 
 __device__ __forceinline__ float max32(const float* v) {
-  float t[16];
+  float t[11];
 #pragma unroll
-  for (int j = 0; j < 16; ++j) t[j] = fmaxf(v[j], v[j + 16]);
-#pragma unroll
-  for (int w = 8; w > 0; w >>= 1)
-#pragma unroll
-    for (int j = 0; j < w; ++j) t[j] = fmaxf(t[j], t[j + w]);
-  return t[0];
+  for (int j = 0; j < 10; ++j) t[j] = fmaxf(fmaxf(v[3 * j], v[3 * j + 1]), v[3 * j + 2]);
+  t[10] = fmaxf(v[30], v[31]);
+  const float a = fmaxf(fmaxf(t[0], t[1]), t[2]), b = fmaxf(fmaxf(t[3], t[4]), t[5]);
+  const float c = fmaxf(fmaxf(t[6], t[7]), t[8]), d = fmaxf(t[9], t[10]);
+  return fmaxf(fmaxf(fmaxf(a, b), c), d);
 }
 
 // Pass 1: per row, the running maximum and exp-sum over the split's columns
 // and the target's logit (TOPK = false); or the four largest logits (TOPK).
 // Each thread covers one row and one column half of every chunk, so a row's
 // results are written as two partial results (index 2 * split + half).
+// Four CTAs per SM hide one another's waits: 48 us for 4,096 samples and about
+// 22,150 treelets on a GB300, two CTAs with two logits buffers each 57.
 template <bool TOPK>
-__global__ void __launch_bounds__(kThreads, 2) out_stats_kernel(OutArgs a) {
+__global__ void __launch_bounds__(kThreads, 4) out_stats_kernel(OutArgs a) {
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* a_tile = smem;                                        // 128 x 64 bf16: 16 KiB
   uint8_t* b_tile0 = smem + 16384;                               // 128 x 64 bf16: 16 KiB, two buffers
   float* bias = reinterpret_cast<float*>(smem + 16384 + 32768);  // 2 x 128
-  __shared__ __align__(8) uint64_t bars[2];
+  __shared__ __align__(8) uint64_t bar;
   __shared__ uint32_t tmem_slot;
   const int tid = threadIdx.x, warp = tid >> 5, quad = warp & 3, half = warp >> 2;
   const uint32_t row0 = blockIdx.x * TM;
   uint32_t c_beg, c_end;
   split_range(a, blockIdx.y, c_beg, c_end);
-  if (tid == 0) {
-    bar_init(&bars[0]);
-    bar_init(&bars[1]);
-  }
+  if (tid == 0) bar_init(&bar);
   const uint32_t tmem = tmem_alloc(&tmem_slot, warp);
   const uint32_t lanes = tmem + ((uint32_t)(quad * 32) << 16);
   const uint32_t row = row0 + (uint32_t)(quad * 32) + (uint32_t)(tid & 31);
@@ -286,54 +303,42 @@ __global__ void __launch_bounds__(kThreads, 2) out_stats_kernel(OutArgs a) {
   float m = -INFINITY, ssum = 0.0f, zt = -INFINITY;
   float tv[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
   uint32_t ti[4] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu};
-  uint32_t phases = 0;  // bit b: the parity of buffer b's next phase
+  uint32_t phase = 0;
   bool ok = true;
-  auto load_chunk = [&](uint32_t c, int buf) {
+  auto load_chunk = [&](uint32_t c, uint32_t buf) {
     load_tile(b_tile0 + buf * 16384, a.w3t, HK, c * TN, TN, a.cp, 0, HK);
     load_bias(bias + buf * TN, a.b3, c, a.C);
+    cp_commit();
+  };
+  auto issue = [&](uint32_t buf) {  // once the chunk's operands are in place
+    cp_wait_all();
+    fence_async_smem();
+    tc_before_sync();
+    __syncthreads();
+    if (tid == 0) {
+      tc_after_sync();
+      mma_logits(tmem, a_tile, b_tile0 + buf * 16384);
+      commit(&bar);
+    }
   };
   if (c_beg < c_end) {
     load_tile(a_tile, a.h2, HK, row0, TM, a.n, 0, HK);
     load_chunk(c_beg, 0);
-    cp_commit();
-    cp_wait_all();
-    fence_async_smem();
-    __syncthreads();
-    if (tid == 0) {
-      tc_after_sync();
-      mma_logits(tmem, a_tile, b_tile0);
-      commit(&bars[0]);
-    }
+    issue(0);
   }
   for (uint32_t c = c_beg; c < c_end; ++c) {
-    const int buf = (int)((c - c_beg) & 1u);
-    // the next chunk's operand into the other buffer (its last reader, the
-    // MMA of chunk c - 1, finished before that chunk's epilogue)
-    if (c + 1 < c_end) {
-      load_chunk(c + 1, buf ^ 1);
-      cp_commit();
-    }
-    if (!bar_wait(&bars[buf], (phases >> buf) & 1u)) ok = false;
-    phases ^= 1u << buf;
+    const uint32_t buf = (c - c_beg) & 1u;
+    // into the other buffer: its last reader, the MMA of chunk c - 1, is done
+    if (c + 1 < c_end) load_chunk(c + 1, buf ^ 1u);
+    if (!bar_wait(&bar, phase)) ok = false;
+    phase ^= 1u;
     tc_after_sync();
-    if (c + 1 < c_end) {
-      cp_wait_all();
-      fence_async_smem();
-    }
-    tc_before_sync();
-    __syncthreads();  // the next operand is in place, every thread saw chunk c's MMA complete
-    if (c + 1 < c_end && tid == 0) {
-      tc_after_sync();
-      mma_logits(tmem + (uint32_t)((buf ^ 1) * TN), a_tile, b_tile0 + (buf ^ 1) * 16384);
-      commit(&bars[buf ^ 1]);
-    }
-    // epilogue of chunk c, overlapping the next chunk's MMA
 #pragma unroll 1
     for (int sl = 0; sl < 2; ++sl) {
       const uint32_t cl0 = (uint32_t)(half * 64 + sl * 32);  // column within the chunk
       const uint32_t col0 = c * TN + cl0;
       float v[32];
-      logits32(lanes + (uint32_t)(buf * TN) + cl0, bias + buf * TN + cl0, col0, a.C, valid_row, v);
+      logits32(lanes + cl0, bias + buf * TN + cl0, col0, a.C, valid_row, v);
       if (TOPK) {
 #pragma unroll
         for (int j = 0; j < 32; ++j) {
@@ -367,19 +372,21 @@ __global__ void __launch_bounds__(kThreads, 2) out_stats_kernel(OutArgs a) {
         const float mx = max32(v);
         if (mx > -INFINITY) {
           const float mn = fmaxf(m, mx), sh = mn * kLog2e;
-          float acc0 = ssum * ex2(fmaf(m, kLog2e, -sh)), acc1 = 0.0f;
+          unsigned long long acc = rtd::f2_pack(ssum * ex2(fmaf(m, kLog2e, -sh)), 0.0f);
 #pragma unroll
           for (int j = 0; j < 32; j += 2) {
-            acc0 += ex2(fmaf(v[j], kLog2e, -sh));
-            acc1 += ex2(fmaf(v[j + 1], kLog2e, -sh));
+            float x, y;
+            rtd::f2_unpack(rtd::f2_fma(rtd::f2_pack(v[j], v[j + 1]), rtd::f2_pack(kLog2e, kLog2e), rtd::f2_pack(-sh, -sh)), x, y);
+            acc = rtd::f2_add(acc, rtd::f2_pack(ex2(x), ex2(y)));
           }
+          float acc0, acc1;
+          rtd::f2_unpack(acc, acc0, acc1);
           ssum = acc0 + acc1;
           m = mn;
         }
       }
     }
-    tc_before_sync();
-    __syncthreads();  // chunk c's TMEM columns are free for chunk c + 2
+    if (c + 1 < c_end) issue(buf ^ 1u);  // every thread has read chunk c's logits
   }
   if (!ok) atomicOr(a.status, 1u);
   cp_wait_all();  // no copy may still be landing when the CTA exits
@@ -477,22 +484,30 @@ __global__ void out_top4_kernel(const float* __restrict__ part, uint32_t splits,
 //   [dW3 | db3]^T[chunk] += dz^T . [h2 | 1]     (A = dz read along its rows, B = [h2 | 1] tile, too)
 // so that neither operand is kept or stored a second time in transposed form.
 // Tensor memory holds the logits, the chunk's dW3 and every tile's dh2; dh2
-// leaves it once per split, dW3 once per chunk, added into the zeroed gradient.
+// leaves it once per split, as a partial sum, dW3 once per chunk, added into the
+// zeroed gradient.
 //
-// What bounds it: the exponentials and the epilogue around them.  The next
-// logits and the last gradient products run on the tensor pipe while sixteen
-// warps are in an epilogue; W3 chunks arrive two ahead.  GB300, 4,096 samples, about
-// 22,150 treelets: 90 us; as two passes with the logits recomputed in each,
-// the products waited for and dz^T stored apart, 111 and 148.
+// What bounds it: each tile's chain from logits through tensor memory, the
+// exponentials and dz to the products (tensor pipe 46% of the time, issue 35%).
+// The next logits and the last products run under the epilogue of sixteen
+// warps; a seventeenth issues them, so that no warp waits for another but at a
+// chunk's start; W3 chunks arrive two ahead.  GB300, 4,096 samples, about
+// 22,150 treelets: 68 us; with CTA-wide barriers and one thread of the epilogue
+// issuing 90; with dz in two buffers 76 (spills); as two kernels that
+// recompute the logits each and wait for every product, 111 and 148.
 constexpr uint32_t kTiles = 4;
 constexpr uint32_t kColDw3 = TN, kColDh2 = kColDw3 + 96;  // TMEM columns (dW3 uses 80)
 static_assert(kColDh2 + kTiles * HK <= 512, "tensor memory");
-constexpr int kGradThreads = 512;  // warp w: TMEM lanes 32 (w % 4) .. + 31, column quarter w / 4 of a chunk
+// Epilogue threads: warp w has TMEM lanes 32 (w % 4) .. + 31 and column quarter
+// w / 4 of a chunk.  One more warp issues the products.
+constexpr int kGradThreads = 512;
 constexpr uint32_t kH2Bytes = TM * HX * 2, kW3Bytes = TN * HK * 2, kDzBytes = TM * TN * 2;
 constexpr uint32_t kW3Bufs = 3;    // read until a chunk's last product, loaded two chunks ahead
 constexpr uint32_t kGradSmem = kTiles * kH2Bytes + kW3Bufs * (kW3Bytes + TN * 4) + kDzBytes;
 
-__global__ void __launch_bounds__(kGradThreads, 1) out_grad_kernel(OutArgs a) {
+constexpr int kBarRead = 1, kBarDz = 2, kBarChunk = 3;  // named barriers
+
+__global__ void __launch_bounds__(kGradThreads + 32, 1) out_grad_kernel(OutArgs a) {
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* const h2 = smem;                          // the tiles' [h2 | 1 | 0], 128 x 80 each
   uint8_t* const w3 = h2 + kTiles * kH2Bytes;        // W3^T chunks, 128 x 64 each
@@ -510,7 +525,7 @@ __global__ void __launch_bounds__(kGradThreads, 1) out_grad_kernel(OutArgs a) {
   const uint32_t lanes = tmem + ((quad * 32u) << 16);
   const uint32_t r = quad * 32u + (tid & 31u);
   const float inv_n = 1.0f / (float)a.n;
-  {  // the one and the zeros behind every h2 row
+  if (tid < kGradThreads) {  // the one and the zeros behind every h2 row
     *reinterpret_cast<uint4*>(h2 + (tid / TM) * kH2Bytes + koff(tid % TM, HK, HX)) = make_uint4(0x3f80u, 0, 0, 0);
     *reinterpret_cast<uint4*>(h2 + (tid / TM) * kH2Bytes + koff(tid % TM, HK + 8, HX)) = make_uint4(0, 0, 0, 0);
   }
@@ -518,8 +533,11 @@ __global__ void __launch_bounds__(kGradThreads, 1) out_grad_kernel(OutArgs a) {
   const uint32_t u_end = (uint32_t)((uint64_t)units * (blockIdx.x + 1u) / gridDim.x);
   uint32_t u = (uint32_t)((uint64_t)units * blockIdx.x / gridDim.x), par_l = 0, par_g = 0;
   bool ok = true;
-  auto load_chunk = [&](uint32_t c, uint32_t buf) {
-    load_tile(w3 + buf * kW3Bytes, a.w3t, HK, c * TN, TN, a.cp, 0, HK);
+  auto load_chunk = [&](uint32_t c, uint32_t buf) {  // by the epilogue threads
+    for (uint32_t x = tid; x < TN * (HK / 8u); x += kGradThreads) {
+      const uint32_t row = x / (HK / 8u), k = x % (HK / 8u) * 8u;
+      cp16(w3 + buf * kW3Bytes + koff(row, k, HK), a.w3t + (uint64_t)(c * TN + row) * HK + k);
+    }
     load_bias(bias + buf * TN, a.b3, c, a.C);
     cp_commit();
   };
@@ -530,6 +548,20 @@ __global__ void __launch_bounds__(kGradThreads, 1) out_grad_kernel(OutArgs a) {
       mma(tmem, sdesc(su32(h2 + i * kH2Bytes) + kk * 256u, HX * 16u), sdesc(su32(w3 + buf * kW3Bytes) + kk * 256u, HK * 16u),
           idesc(TM, TN), kk > 0 ? 1u : 0u);
     commit(&bar_l);
+  };
+  auto issue_products = [&](uint32_t i, uint32_t buf, bool more) {
+    tc_after_sync();
+#pragma unroll
+    for (uint32_t kk = 0; kk < TN / 16; ++kk)
+      mma(tmem + kColDh2 + i * HK, sdesc(su32(dz) + kk * 256u, TN * 16u),
+          sdesc_mn(su32(w3 + buf * kW3Bytes) + kk * (2u * HK * 16u), HK * 16u), idesc(TM, HK) | kBMn,
+          (more || kk > 0) ? 1u : 0u);
+#pragma unroll
+    for (uint32_t kk = 0; kk < TM / 16; ++kk)
+      mma(tmem + kColDw3, sdesc_mn(su32(dz) + kk * (2u * TN * 16u), TN * 16u),
+          sdesc_mn(su32(h2 + i * kH2Bytes) + kk * (2u * HX * 16u), HX * 16u), idesc(TM, HX) | kAMn | kBMn,
+          (i > 0 || kk > 0) ? 1u : 0u);
+    commit(&bar_g);
   };
   auto next = [](uint32_t buf) { return buf + 1 == kW3Bufs ? 0u : buf + 1; };
   // lane r of the accumulator is the chunk's column r: 64 weight gradients, then the bias gradient
@@ -548,12 +580,12 @@ __global__ void __launch_bounds__(kGradThreads, 1) out_grad_kernel(OutArgs a) {
   };
   while (u < u_end) {
     // this CTA's tiles t0 .. t0 + nt - 1 of one split
-    const uint32_t t0 = u % tiles, nt = min(min(tiles - t0, u_end - u), kTiles);
+    const uint32_t split = u / tiles, t0 = u % tiles, nt = min(min(tiles - t0, u_end - u), kTiles);
     uint32_t c_beg, c_end;
-    split_range(a, u / tiles, c_beg, c_end);
+    split_range(a, split, c_beg, c_end);
     u += nt;
     if (c_beg >= c_end) continue;
-    for (uint32_t x = tid; x < nt * TM * (HK / 8u); x += kGradThreads) {
+    for (uint32_t x = tid; x < nt * TM * (HK / 8u); x += blockDim.x) {
       const uint32_t row = x / (HK / 8u), k = x % (HK / 8u) * 8u;
       uint8_t* dst = h2 + row / TM * kH2Bytes + koff(row % TM, k, HX);
       if (t0 * TM + row < a.n) cp16(dst, a.h2 + (uint64_t)(t0 * TM + row) * HK + k);
@@ -564,88 +596,94 @@ __global__ void __launch_bounds__(kGradThreads, 1) out_grad_kernel(OutArgs a) {
       s_tgt[tid / TM][tid % TM] = row < a.n ? a.s[row].target : 0xFFFFFFFFu;
       s_sh[tid / TM][tid % TM] = row < a.n ? a.lse[row] * kLog2e : 0.0f;
     }
-    load_chunk(c_beg, 0);
-    if (c_beg + 1 < c_end) load_chunk(c_beg + 1, 1);
+    if (tid < kGradThreads) {
+      load_chunk(c_beg, 0);
+      if (c_beg + 1 < c_end) load_chunk(c_beg + 1, 1);
+    }
     cp_wait_all();
     fence_async_smem();
     tc_before_sync();
     __syncthreads();
-    if (tid == 0) issue_logits(0, 0);
-    uint32_t buf = 0;
-    for (uint32_t c = c_beg; c < c_end; ++c) {
-      for (uint32_t i = 0; i < nt; ++i) {
-        const bool first = i == 0 && c == c_beg, last = i + 1 == nt && c + 1 == c_end;
-        const uint32_t tgt = s_tgt[i][r];
-        const float sh = s_sh[i][r];
-        if (!bar_wait(&bar_l, par_l)) ok = false;
-        par_l ^= 1u;
-        tc_after_sync();
-        const uint32_t cl0 = quarter * 32u, col0 = c * TN + cl0;
-        float v[32];
-        logits32(lanes + cl0, bias + buf * TN + cl0, col0, a.C, (t0 + i) * TM + r < a.n, v);
-        cp_wait_all();
-        fence_async_smem();
-        tc_before_sync();
-        __syncthreads();  // every warp has its logits; the chunk asked for one chunk ago is in place
-        if (tid == 0 && !last) issue_logits(i + 1 == nt ? 0u : i + 1, i + 1 == nt ? next(buf) : buf);
-#pragma unroll
-        for (int k = 0; k < 32; ++k) v[k] = ex2(fmaf(v[k], kLog2e, -sh));  // ex2(-inf) = 0: dead columns give 0
-        if (tgt - col0 < 32u) {
-#pragma unroll
-          for (int k = 0; k < 32; ++k)
-            if (col0 + k == tgt) v[k] -= 1.0f;
+    if (warp == kGradThreads / 32) {
+      if (tid == kGradThreads) issue_logits(0, 0);
+      uint32_t buf = 0;
+      for (uint32_t c = c_beg; c < c_end; ++c, buf = next(buf))
+        for (uint32_t i = 0; i < nt; ++i) {
+          const bool last = i + 1 == nt && c + 1 == c_end;
+          nb_sync(kBarRead, kGradThreads + 32);
+          if (tid == kGradThreads && !last) issue_logits(i + 1 == nt ? 0u : i + 1, i + 1 == nt ? next(buf) : buf);
+          __syncwarp();
+          nb_sync(kBarDz, kGradThreads + 32);
+          if (tid == kGradThreads) issue_products(i, buf, c > c_beg);
+          __syncwarp();
         }
-        uint32_t w[16];
-#pragma unroll
-        for (int k = 0; k < 16; ++k) {
-          const __nv_bfloat162 pr = __floats2bfloat162_rn(v[2 * k] * inv_n, v[2 * k + 1] * inv_n);
-          w[k] = *reinterpret_cast<const uint32_t*>(&pr);
-        }
-        if (!first) {
-          if (!bar_wait(&bar_g, par_g)) ok = false;  // the last products have read dz
-          par_g ^= 1u;
+    } else {
+      uint32_t buf = 0;
+      for (uint32_t c = c_beg; c < c_end; ++c, buf = next(buf)) {
+        if (c > c_beg) nb_sync(kBarChunk, kGradThreads);  // every thread's part of the chunk's biases is in place
+        for (uint32_t i = 0; i < nt; ++i) {
+          const uint32_t tgt = s_tgt[i][r];
+          const float sh = s_sh[i][r];
+          if (!bar_wait(&bar_l, par_l)) ok = false;
+          par_l ^= 1u;
           tc_after_sync();
-        }
-        if (i == 0) {
-          if (c > c_beg) add_dw3(c - 1);
-          if (c + 2 < c_end) load_chunk(c + 2, next(next(buf)));  // over chunk c - 1
-        }
+          const uint32_t cl0 = quarter * 32u, col0 = c * TN + cl0;
+          float v[32];
+          logits32(lanes + cl0, bias + buf * TN + cl0, col0, a.C, (t0 + i) * TM + r < a.n, v);
+          cp_wait_all();  // the chunk asked for one chunk ago
+          fence_async_smem();
+          tc_before_sync();
+          nb_arrive(kBarRead, kGradThreads + 32);
 #pragma unroll
-        for (int q = 0; q < 4; ++q)
-          *reinterpret_cast<uint4*>(dz + koff(r, cl0 + (uint32_t)(q * 8), TN)) =
-              make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
-        fence_async_smem();
-        tc_before_sync();
-        __syncthreads();
-        if (tid == 0) {
-          tc_after_sync();
+          for (int k = 0; k < 32; k += 2) {  // ex2(-inf) = 0: dead columns give 0
+            rtd::f2_unpack(rtd::f2_fma(rtd::f2_pack(v[k], v[k + 1]), rtd::f2_pack(kLog2e, kLog2e), rtd::f2_pack(-sh, -sh)), v[k], v[k + 1]);
+            v[k] = ex2(v[k]);
+            v[k + 1] = ex2(v[k + 1]);
+          }
+          if (tgt - col0 < 32u) {
 #pragma unroll
-          for (uint32_t kk = 0; kk < TN / 16; ++kk)
-            mma(tmem + kColDh2 + i * HK, sdesc(su32(dz) + kk * 256u, TN * 16u),
-                sdesc_mn(su32(w3 + buf * kW3Bytes) + kk * (2u * HK * 16u), HK * 16u), idesc(TM, HK) | kBMn,
-                (c > c_beg || kk > 0) ? 1u : 0u);
+            for (int k = 0; k < 32; ++k)
+              if (col0 + k == tgt) v[k] -= 1.0f;
+          }
+          uint32_t w[16];
 #pragma unroll
-          for (uint32_t kk = 0; kk < TM / 16; ++kk)
-            mma(tmem + kColDw3, sdesc_mn(su32(dz) + kk * (2u * TN * 16u), TN * 16u),
-                sdesc_mn(su32(h2 + i * kH2Bytes) + kk * (2u * HX * 16u), HX * 16u), idesc(TM, HX) | kAMn | kBMn,
-                (i > 0 || kk > 0) ? 1u : 0u);
-          commit(&bar_g);
+          for (int k = 0; k < 16; ++k) {
+            float x, y;
+            rtd::f2_unpack(rtd::f2_mul(rtd::f2_pack(v[2 * k], v[2 * k + 1]), rtd::f2_pack(inv_n, inv_n)), x, y);
+            const __nv_bfloat162 pr = __floats2bfloat162_rn(x, y);
+            w[k] = *reinterpret_cast<const uint32_t*>(&pr);
+          }
+          if (i > 0 || c > c_beg) {
+            if (!bar_wait(&bar_g, par_g)) ok = false;  // the last products have read dz
+            par_g ^= 1u;
+            tc_after_sync();
+          }
+          if (i == 0) {
+            if (c > c_beg) add_dw3(c - 1);
+            if (c + 2 < c_end) load_chunk(c + 2, next(next(buf)));  // over chunk c - 1
+          }
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            *reinterpret_cast<uint4*>(dz + koff(r, cl0 + (uint32_t)(q * 8), TN)) =
+                make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
+          fence_async_smem();
+          tc_before_sync();
+          nb_arrive(kBarDz, kGradThreads + 32);
         }
       }
-      buf = next(buf);
-    }
-    if (!bar_wait(&bar_g, par_g)) ok = false;
-    par_g ^= 1u;
-    tc_after_sync();
-    add_dw3(c_end - 1);
-    for (uint32_t i = 0; i < nt; ++i) {  // a quarter of the tile's columns each
-      float v[16];
-      tmem_ld16(lanes + kColDh2 + i * HK + quarter * 16u, v);
-      const uint32_t row = (t0 + i) * TM + r;
-      if (row < a.n) {
-        float4* p = reinterpret_cast<float4*>(a.dh2 + (uint64_t)row * HK + quarter * 16u);
+      if (!bar_wait(&bar_g, par_g)) ok = false;
+      par_g ^= 1u;
+      tc_after_sync();
+      add_dw3(c_end - 1);
+      for (uint32_t i = 0; i < nt; ++i) {  // a quarter of the tile's columns each
+        float v[16];
+        tmem_ld16(lanes + kColDh2 + i * HK + quarter * 16u, v);
+        const uint32_t row = (t0 + i) * TM + r;
+        if (row < a.n) {
+          float4* p = reinterpret_cast<float4*>(a.dh2 + ((uint64_t)split * a.n + row) * HK + quarter * 16u);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) atomicAdd(p + q, make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]));
+          for (int q = 0; q < 4; ++q) p[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+        }
       }
     }
     tc_before_sync();
