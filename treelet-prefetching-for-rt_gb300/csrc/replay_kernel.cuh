@@ -6,14 +6,14 @@
 // request per cycle, so a unit is a sequential loop.  The warp works the
 // parts of a cycle that have lanes in them: the L1 set (one lane per way),
 // the resident warps (one lane per warp), a round's 32 lanes (one lane per
-// RT lane, identical requests merged with __match_any_sync), the sorted
-// histogram of next treelets, and the prefetch-queue scans.  Lane 0 keeps
-// the unit's counters and makes the single-request updates.
+// RT lane, identical requests merged with __match_any_sync), and the members
+// of a treelet that is pushed onto the prefetch queue.  Lane 0 keeps the
+// unit's counters and makes the single-request updates.
 //
 // Per unit, in shared memory: the unit's scalar state, the resident warps
 // (per RT lane a trace cursor), the current round's requests, the histogram
-// keys, the stride tables and, when they fit, the L1 lines.  In a slice of
-// one device scratch buffer:
+// of next treelets (a table of counts kept as lanes move on), the stride tables
+// and, when they fit, the L1 lines.  In a slice of one device scratch buffer:
 //   lines     sectored L1 (128 B lines, 4 x 32 B sectors, LRU stamps), when
 //             they do not fit in shared memory
 //   sectors   open-addressing map keyed by 32 B sector: prefetch records of
