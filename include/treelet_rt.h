@@ -313,7 +313,8 @@ typedef struct rt_tuning {
   uint32_t staged_threads;    /* threads per CTA for RT_MODE_STAGED (32..256) */
   uint32_t staged_epoch;      /* node visits of a warp between staging votes */
   uint32_t staged_slots;      /* shared-memory treelet slots per warp (1..8; RT_TUNING_OFF: none) */
-  uint32_t refill_lanes;      /* idle lanes of a warp that make it fetch new rays (1..32) */
+  uint32_t refill_lanes;      /* idle lanes of a warp that make it fetch new rays (1..32; large staged
+                               * launches wait for all 32 where a warp holds neighbouring camera rays) */
   uint32_t staged_slot_bytes; /* bytes per slot: a treelet's first bytes when smaller than it */
   uint32_t staged_min_votes;  /* lanes of a warp that must want a treelet to stage it (1..32) */
   uint32_t stack_depth;       /* traversal stack entries per ray: 48, 96 or 160 (deeper rays are flagged) */

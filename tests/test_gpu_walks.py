@@ -185,3 +185,32 @@ def test_packed_call_sizes(ctx, n, pinned):
             if visits:
                 assert np.array_equal(v.numpy().view(np.uint32)[:total], vis[keep])
     scene.close()
+
+
+@pytest.mark.parametrize("n", [(1 << 19) - 1, 1 << 19, (1 << 19) + 33])
+def test_staged_rays_taken_together(ctx, n):
+    """Staged launches on both sides of the size from which a warp of
+    neighbouring camera rays waits for its last one: camera rays, then the same
+    from other points and in other directions, mixed within the warps."""
+    import torch
+
+    import treelet_rt as rt
+    from oracle import oracle as orc
+
+    blob = rt.Blob.gen(rt.SCENE_TERRAIN_INSTANCES, 2 * 40 * 40, 5)
+    scene = rt.Scene(ctx, blob)
+    scene.form_treelets(1024)
+    rays = np.resize(rt.camera_rays(rt.default_camera(rt.SCENE_TERRAIN_INSTANCES), 1024, 512, 1, 3, 1e-4, 1e30), n)
+    rng = np.random.default_rng(n)
+    spread = np.arange(n) % 4096 > 3000
+    spread &= rng.random(n) < 0.5
+    rays["origin"][spread] += rng.uniform(-0.1, 0.1, (int(spread.sum()), 3)).astype(np.float32)
+    rays["dir"][spread] = rng.normal(size=(int(spread.sum()), 3)).astype(np.float32)
+    rays["dir"][7::5001] = np.nan
+    d_rays = torch.from_numpy(rays.view(np.uint8).copy()).cuda()
+    hits = torch.zeros(n * 64, dtype=torch.uint8, device="cuda")
+    scene.trace(d_rays, hits, rt.MODE_STAGED, n=n)
+    torch.cuda.synchronize()
+    oh, _, _ = orc.trace(blob.bytes(), rays, 1, orc.Treelets(blob.bytes(), 1024), threads=8)
+    assert_hits_equal(hits.cpu().numpy().view(rt.HIT_DTYPE), oh, "staged")
+    scene.close()

@@ -549,6 +549,32 @@ struct WarpStage {
   uint32_t pending_slot, pending_id, pending_units, phase, victim, disabled;
 };
 
+// Whether the calling warp's 32 rays, just taken, leave one point within a
+// narrow cone of each other (kCone: cosine squared, 14 degrees), as a camera's
+// neighbouring rays do.
+constexpr float kCone = 0.94f;
+
+__device__ __forceinline__ bool rays_together(rtm::V3 o, rtm::V3 d) {
+  const float ox = __shfl_sync(0xffffffffu, o.x, 0), oy = __shfl_sync(0xffffffffu, o.y, 0);
+  const float oz = __shfl_sync(0xffffffffu, o.z, 0), dx = __shfl_sync(0xffffffffu, d.x, 0);
+  const float dy = __shfl_sync(0xffffffffu, d.y, 0), dz = __shfl_sync(0xffffffffu, d.z, 0);
+  const float dot = d.x * dx + d.y * dy + d.z * dz;
+  const float len = (d.x * d.x + d.y * d.y + d.z * d.z) * (dx * dx + dy * dy + dz * dz);
+  return __all_sync(0xffffffffu, o.x == ox && o.y == oy && o.z == oz && dot > 0.0f && dot * dot >= kCone * len);
+}
+
+// Rays from which on a staged launch waits for the last ray of a warp whose rays
+// are together, to take 32 neighbours again: neighbours walk the same nodes, and a
+// ray taken alone walks beside rays that are far ahead.  GB300, primary rays,
+// waiting / refilling at 8 idle lanes, us: 2M-triangle terrain 1M rays 1199 /
+// 1292, 2M (two a pixel) 2247 / 2500, 4M 4350 / 4919; traced 1495 /
+// 1660 at 1M; 1M-triangle blobs 594 / 604 at 1M.  At 307,200 rays, two per
+// lane of the chip, the warps' uneven ends cost what it gains (blobs 379 / 358).
+// Bounce rays: 2102 / 2101 us at 1M, 3850 / 3830 at 2M.  The unstaged treelet
+// walk gains as much on such rays but pays 0.4% on all others for the check,
+// and the plain walk gains nothing (1036 / 1025): neither does it.
+constexpr uint32_t kTogetherRays = 1u << 19;
+
 // The staged walk.  Persistent warps with ray refill (as run_persistent).
 //
 // Pinned treelets: at launch each CTA copies the pinned image (the treelets
@@ -624,24 +650,25 @@ __global__ void __launch_bounds__(kStagedMaxThreads, kStagedMinBlocks) trace_sta
   w.smem_reads = w.gmem_reads = 0;
   w.pin_base = pin_ok ? smem_u32(smem0) : 0u;
   w.pin_root = pin_ok ? a.pin_root : 0u;
-  bool have = false, ended = false, exhausted = false;
+  bool have = false, ended = false;
+  int spare = (int)a.refill;  // idle lanes that end a turn; 33 once no rays are left
   uint32_t r = 0, it = 0;
   unsigned long long bytes = 0, staged = 0, stagings = 0;
   for (;; ++it) {
     // --- records of finished rays, then new rays for idle lanes (as run_persistent)
     const uint32_t need = __ballot_sync(0xffffffffu, !have);
-    if (need == 0xffffffffu || (!exhausted && __popc(need) >= (int)a.refill)) {
+    if (need == 0xffffffffu || __popc(need) >= spare) {
       if (ended) {
         w.finish(a, r);
         bytes += 64ull * w.n_tx;
         ended = false;
       }
-      if (exhausted) break;  // every lane is idle
+      if (spare > 32) break;  // every lane is idle
       const int leader = __ffs(need) - 1;
       uint32_t base = 0;
       if ((int)lane == leader) base = atomicAdd(a.queue, (uint32_t)__popc(need));
       base = __shfl_sync(0xffffffffu, base, leader);
-      if (base + (uint32_t)__popc(need) >= a.n) exhausted = true;
+      if (base + (uint32_t)__popc(need) >= a.n) spare = 33;
       if (!have) {
         const uint32_t rr = base + (uint32_t)__popc(need & ((1u << lane) - 1u));
         if (rr < a.n) {
@@ -650,6 +677,8 @@ __global__ void __launch_bounds__(kStagedMaxThreads, kStagedMinBlocks) trace_sta
           have = true;
         }
       }
+      if (need == 0xffffffffu && spare <= 32 && a.n >= kTogetherRays)
+        spare = rays_together(w.cx.o, w.dir()) ? 32 : (int)a.refill;
     }
     // --- staging: land a finished copy, then vote for the next one
     if (SLOTS && slots > 0 && (it % a.epoch) == 0) {
@@ -706,8 +735,8 @@ __global__ void __launch_bounds__(kStagedMaxThreads, kStagedMinBlocks) trace_sta
       __syncwarp();
     }
     // --- node visits
-    if (SLOTS) warp_turn(a, w, r, have, ended, exhausted ? 33 : (int)a.refill, lookup);
-    else warp_turn(a, w, r, have, ended, exhausted ? 33 : (int)a.refill, NoLookup());
+    if (SLOTS) warp_turn(a, w, r, have, ended, spare, lookup);
+    else warp_turn(a, w, r, have, ended, spare, NoLookup());
   }
   rtd::touch_l1_done();
   // copies still in flight must land before the CTA's shared memory goes away
