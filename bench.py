@@ -53,21 +53,20 @@ def _peaks():
 
 
 # DRAM bytes per ray of the staged kernel (dram__bytes_read.sum + dram__bytes_write.sum) from
-# the ncu capture summarised in profiles/trace_kernels_terrain_instances.md: the same scene with
-# 262,144 rays per launch (the full launch of 2,097,152 rays is too large to capture with
-# --set full); scaled to a full launch by the ray count.
-STAGED_DRAM_BYTES_PER_RAY = {"primary": (103.862784e6 + 16.576000e6) / 262144,
-                             "bounce": (172.382720e6 + 34.174464e6) / 262144}
+# the ncu capture summarised in profiles/walks_and_output_layer.md: the same scene with 262,144
+# rays per launch, scaled to a full launch by the ray count.
+STAGED_DRAM_BYTES_PER_RAY = {"primary": (113.36e6 + 26.39e6) / 262144,
+                             "bounce": (205.54e6 + 66.53e6) / 262144}
 
 
 # What binds the staged walk, from the same ncu capture (bounce launch): it
 # moves a small fraction of the HBM roofline's bytes, and is bound by SIMT
 # divergence and issue instead.
 LIMITER = {"kind": "issue / SIMT divergence (dependent loads of a pointer-chasing walk), not HBM bandwidth",
-           "source": "profiles/trace_kernels_terrain_instances.md, staged walk, 262,144 bounce rays",
-           "lanes_active_of_32": 8.93, "issue_slots_active_pct": 66.7, "warps_per_sm": 20.0,
-           "dram_busy_pct": 2.8, "l1_hit_pct": 54.8, "l2_hit_pct": 71.0, "l1_throughput_pct": 24.7,
-           "l2_throughput_pct": 12.8, "smem_pipe_pct": 1.9}
+           "source": "profiles/walks_and_output_layer.md, staged walk, 262,144 bounce rays",
+           "lanes_active_of_32": 11.04, "issue_slots_active_pct": 71.9, "warps_per_sm": 25.5,
+           "dram_busy_pct": 3.9, "l1_hit_pct": 54.0, "l2_hit_pct": 71.9, "l1_throughput_pct": 43.8,
+           "l2_throughput_pct": 18.6}
 
 
 def _traffic_per_ray():
