@@ -98,6 +98,48 @@ def test_unit_that_is_node_and_leaf(ctx):
     scene.close()
 
 
+@pytest.mark.parametrize("n", [256, 40001])
+def test_node_of_both_levels(ctx, n):
+    """A node the TLAS root lists as its child and an instance has as its BLAS
+    root: as a top-level node its quad leaf is an instance leaf, whose BLAS is
+    reached no other way."""
+    import kat_blob as K
+
+    import treelet_rt as rt
+    from oracle import oracle as orc
+
+    def box(size, typ):
+        return size, typ, (0, 0, 0), (64, 64, 64)
+
+    wide = (-262144.0,) * 3
+    second = bytearray(64)  # the second half of the quad leaf's instance: its BLAS header is unit 8
+    second[0:8] = np.uint64(128).tobytes()
+    units = [
+        K._header(128, (-1, -1, 0), (3, 3, 4)),                             # 0: TLAS root is unit 2
+        K._header(128, (-1, -1, 0), (3, 3, 4)),                             # 1: BLAS root is unit 3
+        K._internal((-1, -1, 0), 1, (4, 4, 4), [box(1, 0), box(2, 1)]),     # 2
+        K._internal((-1, -1, 0), 3, (4, 4, 4), [box(1, 4)]),                # 3: a node of both levels
+        K._instance((1 << 64) - 192, 7),                                    # 4-5: BLAS header is unit 1
+        K._quad(1.0, 100),                                                  # 6
+        bytes(second),                                                      # 7
+        K._header(64, (-1, -1, 0), (3, 3, 4)),                              # 8: BLAS root is unit 9
+        K._internal(wide, 1, (20, 20, 20), [(1, 4, (0, 0, 0), (128, 128, 128)), (1, 0, (0, 0, 0), (128, 128, 128))]),
+        K._quad(2.0, 200),                                                  # 10
+        K._internal(wide, 1, (20, 20, 20), [(1, 4, (0, 0, 0), (128, 128, 128))]),  # 11
+        K._quad(3.0, 300),                                                  # 12
+    ]
+    b = np.frombuffer(b"".join(units), np.uint8).copy()
+    rays = np.resize(K.grid_rays(16), n)
+    oh, ov, _ = orc.trace(b, rays, 0, None, capacity=32, want_visits=True, threads=8)
+    reached = ov[np.arange(32)[None, :] < np.minimum(oh["n_visits"], 32)[:, None]] >> 3
+    assert {3, 6, 9, 11} <= set(reached.tolist())
+    scene = rt.Scene(ctx, rt.Blob.wrap(b))
+    hits, vis, _ = scene.trace_host(rays, rt.MODE_PLAIN, capacity=32, want_visits=True)
+    assert_hits_equal(hits, oh, "hits")
+    assert_traces_equal(vis, ov, oh["n_visits"], "visits")
+    scene.close()
+
+
 @pytest.mark.parametrize("n", [1, 7, 33, 4864, 4865, 9729, 24576, 24577, 32768, 32769, 40001])
 def test_launch_sizes(ctx, n):
     """Eight lanes a ray (one, two or four rays a warp) up to 32,768 rays (24,576 staged), one

@@ -58,6 +58,55 @@ def test_blob_validation_rejects_corruption(built):
         assert e.value.status == 4, name
 
 
+@pytest.mark.parametrize("child_off,bvh_address,node_first,ok", [
+    (6, 192, False, True), (6, 192, True, True),          # both uses are in order
+    (1 << 27, 192, False, False), (1 << 27, 192, True, False),  # the node's children lie outside the blob
+    (6, 64 * 4000, False, False), (6, 64 * 4000, True, False)])  # the instance's header does
+def test_blob_validation_checks_both_uses_of_a_unit(built, child_off, bvh_address, node_first, ok):
+    """A unit that is an instance leaf and another node's internal child is
+    checked as both, whichever of the two is met first."""
+    import treelet_rt as rt
+
+    full = ((0, 0, 0), (64, 64, 64))
+    leaf = bytearray(K._instance(bvh_address, 7))
+    leaf[12:16] = np.int32(child_off).tobytes()
+    leaf[22] = 1  # as a node: one internal child
+    # units: 0 header, 1 root, 2 and 3 nodes, 4-5 the leaf, 6 spare, 7 BLAS header, 8 BLAS root, 9 quad, 10 empty node
+    as_node, as_leaf = (1, 0) + full, (2, 1) + full
+    uses = [[as_leaf], [as_node]] if node_first else [[as_node], [as_leaf]]  # the last child of unit 1 is checked first
+    units = [
+        K._header(64, (-1, -1, 0), (3, 3, 3)),
+        K._internal((-1, -1, 0), 1, (4, 4, 4), [as_node, as_node]),
+        K._internal((-1, -1, 0), 2, (4, 4, 4), uses[0]),
+        K._internal((-1, -1, 0), 1, (4, 4, 4), uses[1]),
+        bytes(leaf),
+        bytes(64),
+        K._header(64, (-1, -1, 0), (3, 3, 3)),
+        K._internal((-1, -1, 0), 1, (4, 4, 4), [(1, 4) + full]),
+        K._quad(1.0, 100),
+        bytes(64),
+    ]
+    blob = rt.Blob.wrap(np.frombuffer(b"".join(units), np.uint8).copy())
+    if ok:
+        blob.validate()
+    else:
+        with pytest.raises(rt.RTError) as e:
+            blob.validate()
+        assert e.value.status == 4
+
+
+def test_walk_nodes_name_no_unit_far_outside_the_blob(tmp_path):
+    import subprocess
+
+    exe = str(tmp_path / "walk_node_bounds")
+    here = os.path.dirname(os.path.abspath(__file__))
+    csrc = os.path.join(REPO, "treelet-prefetching-for-rt_gb300", "csrc")
+    subprocess.run(["g++", "-std=c++17", "-O2", "-I" + csrc, os.path.join(here, "walk_node_bounds.cpp"), "-o", exe],
+                   check=True)
+    r = subprocess.run([exe], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0 and "mismatches 0" in r.stdout, r.stdout
+
+
 def _partition_equal(blob, budget):
     import treelet_rt as rt
     from oracle import oracle as orc

@@ -44,14 +44,19 @@ bool validate_blob(const uint8_t* b, uint64_t n, std::string* err, BlobRoles* ro
     std::memcpy(&v, b + off, 8);
     return v;
   };
+  // what a unit has been checked as: a unit in both uses is checked in both
+  constexpr uint8_t kNodeChecked = 1, kInstanceChecked = 2;
   std::vector<uint8_t> seen(units, 0);
-  // roles: bit 0 internal node, bit 1 read as the blob's bytes (headers, leaves)
-  constexpr uint8_t kInternal = 1, kRaw = 2;
+  // roles: bit 0 internal node, bit 1 read as the blob's bytes (headers, leaves);
+  // bits 2 and 3: a node of the top, of a bottom level.  A node of both levels is
+  // checked as one of them only, and the walks may reach others from it that are
+  // not met here.
+  constexpr uint8_t kInternal = 1, kRaw = 2, kTop = 4, kBottom = 8;
   std::vector<uint8_t> role(units, 0);
   bool mixed = false;
   auto take = [&](uint64_t u, uint8_t r) {
     role[u] |= r;
-    mixed |= role[u] == (kInternal | kRaw);
+    mixed |= (role[u] & (kInternal | kRaw)) == (kInternal | kRaw) || (role[u] & (kTop | kBottom)) == (kTop | kBottom);
   };
   take(0, kRaw);
   struct Item {
@@ -65,9 +70,9 @@ bool validate_blob(const uint8_t* b, uint64_t n, std::string* err, BlobRoles* ro
   while (!work.empty()) {
     const Item it = work.back();
     work.pop_back();
-    take(it.unit, kInternal);
-    if (seen[it.unit]) continue;
-    seen[it.unit] = 1;
+    take(it.unit, kInternal | (it.top ? kTop : kBottom));
+    if (seen[it.unit] & kNodeChecked) continue;
+    seen[it.unit] |= kNodeChecked;
     const uint8_t* p = b + it.unit * 64;
     int32_t child_off;
     std::memcpy(&child_off, p + rtf::IN_CHILD_OFFSET, 4);
@@ -87,8 +92,8 @@ bool validate_blob(const uint8_t* b, uint64_t n, std::string* err, BlobRoles* ro
           if (ty != rtf::CT_INSTANCE || sz != 2) return bad("top-level leaf that is not a 128-byte instance leaf");
           take(c, kRaw);
           take(c + 1, kRaw);
-          if (!seen[c]) {
-            seen[c] = 1;
+          if (!(seen[c] & kInstanceChecked)) {
+            seen[c] |= kInstanceChecked;
             const uint64_t hdr = c * 64 + rd64(c * 64 + rtf::IL_BVH_ADDRESS);
             if (hdr % 64 || hdr / 64 >= units) return bad("instance BVHAddress out of range");
             const uint64_t broot = hdr + rd64(hdr + rtf::HDR_ROOT_OFFSET);
@@ -405,7 +410,7 @@ rt_status rebuild_pinned(rt_scene* s, bool keep_current) {
   for (const auto& [at, unit] : pin.internal) {
     uint32_t raw[16], node[16];
     std::memcpy(raw, s->host_blob.data() + (uint64_t)unit * 64, 64);
-    rtw::walk_node(raw, unit, s->route[unit], node);
+    rtw::walk_node(raw, unit, s->n_units, s->route[unit], node);
     std::memcpy(pin.bytes.data() + at, node, 64);
   }
   rt_status st = dalloc(&s->d_pin, pin.bytes.size());
@@ -776,7 +781,7 @@ rt_status rt_scene_create(rt_ctx* ctx, const rt_blob* blob, rt_scene** out) {
   s->blob_bytes = blob->bytes.size();
   s->n_units = (uint32_t)(s->blob_bytes / 64);
   rt_status st = dalloc(&s->d_blob, s->blob_bytes);
-  if (st == RT_OK) st = dalloc(&s->d_walk, s->blob_bytes);
+  if (st == RT_OK) st = dalloc(&s->d_walk, s->blob_bytes + 64ull * rtw::kPadUnits);
   s->mixed_roles = roles.mixed;
   if (st == RT_OK && !roles.mixed) st = dalloc(&s->d_internal, sizeof(uint32_t) * roles.internal.size());
   if (st == RT_OK) st = dalloc(&s->d_ctl, sizeof(rti::Control));

@@ -24,8 +24,8 @@ rt_status fail(rt_status s, const std::string& msg);
 
 // What a blob's units are to the walks.  internal: bit u % 32 of word u / 32
 // for every unit reached as an internal node; mixed: some unit is reached as
-// an internal node and also read as something else (then `internal` may miss
-// some).
+// an internal node and also read as something else, or as a node of the top and
+// of a bottom level (then `internal` may miss some).
 struct BlobRoles {
   std::vector<uint32_t> internal;
   bool mixed = false;

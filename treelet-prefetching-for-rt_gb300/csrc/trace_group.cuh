@@ -191,7 +191,7 @@ struct GroupWalk {
     const uint32_t valid = (q1.y | (q1.y >> rtw::kLeafShift)) & rtw::kChildMask;
     const bool h = hit_child(src, unit, q0, q1, tmin * cx.mult, tmax * cx.mult, min_thit * cx.mult);
     uint32_t hit = ballot(h) & valid;
-    // hit children start on their way to L1 while the ray is elsewhere
+    // hit children start on their way to L1 while the ray is elsewhere (touch_node)
     if ((hit >> j) & 1u && !so) {
       const uint4* const child = v.walk + (uint64_t)(q0.w + ((q1.z >> (4 * j)) & 15u)) * 4;
       rtd::touch_l1(scratch, child);

@@ -58,7 +58,7 @@ __global__ void __launch_bounds__(256) walk_nodes_kernel(const uint4* __restrict
     const uint4 x = __ldcs(blob + (uint64_t)u * 4 + q);
     raw[4 * q] = x.x, raw[4 * q + 1] = x.y, raw[4 * q + 2] = x.z, raw[4 * q + 3] = x.w;
   }
-  rtw::walk_node(raw, u, route ? route[u] : 0u, node);
+  rtw::walk_node(raw, u, n_units, route ? route[u] : 0u, node);
   const bool keep = internal && !((internal[u >> 5] >> (u & 31u)) & 1u);
 #pragma unroll
   for (int q = 0; q < 16; ++q) node[q] = keep ? raw[q] : node[q];
@@ -139,7 +139,8 @@ __device__ __forceinline__ uint32_t* trace_buf(uint32_t off) {
 // terrain, 49K bounce rays plain 441 / 386, treelet order 521 / 424, staged 571 /
 // 463; 2M rays 2124 / 2059, 2683 / 2607, 2997 / 2852; 1M-triangle blobs, 1M bounce
 // rays 764 / 662, 941 / 741, 1016 / 772.  2M any-hit rays in treelet order lose
-// 1.7% (1636 / 1664).  (A prefetch into L2 only was slower than none.)
+// 1.7% (1636 / 1664).  (A prefetch into L2 only was slower than none.)  A child
+// outside the blob is within the array's padding (rtw::kPadUnits).
 __device__ __forceinline__ void touch_node(const uint4* walk, uint32_t unit) {
   __shared__ uint32_t scratch;
   const uint32_t s = (uint32_t)__cvta_generic_to_shared(&scratch);

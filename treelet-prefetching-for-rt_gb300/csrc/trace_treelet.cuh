@@ -308,7 +308,7 @@ struct Walker {
       uint32_t raw[16];
 #pragma unroll
       for (int k = 0; k < 16; ++k) raw[k] = nd.w[k];
-      rtw::walk_node(raw, unit, __ldg(v.route + unit), nd.w);
+      rtw::walk_node(raw, unit, v.n_units, __ldg(v.route + unit), nd.w);
     }
     e = 0;
     popped = 0;
