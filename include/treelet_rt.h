@@ -187,7 +187,9 @@ rt_status rt_scene_device_blob(const rt_scene* scene, const void** dptr, uint64_
 /* Treelet partition of the scene with a byte budget per treelet
  * (createTreelets, vulkan_ray_tracing.cc:823-1470, with the node -> treelet
  * map of buildNodeToRootMap, :475-489).  Must precede RT_MODE_TREELET /
- * RT_MODE_STAGED traces.  Re-forming replaces the previous partition. */
+ * RT_MODE_STAGED traces.  Re-forming replaces the previous partition.  Waits
+ * for the work in flight on the device (so not while a stream is captured):
+ * traces of every mode read nodes that it rewrites in place. */
 typedef struct rt_treelet_info {
   uint32_t n_treelets;
   uint32_t max_treelet_bytes;
@@ -368,7 +370,8 @@ rt_status rt_scene_pinned_info(rt_scene* scene, rt_pinned_info* info);
  * other-treelet stack; RT_MODE_TREELET and RT_MODE_STAGED then reproduce
  * that order.  RT_MODE_PLAIN is unaffected.  Visit traces name blob units
  * either way (the reference's transaction address is unit * 64 plus the
- * offset). */
+ * offset).  With treelets formed, a call that changes the order waits for the
+ * work in flight on the device, as rt_treelets_form does. */
 rt_status rt_scene_set_device_offset(rt_scene* scene, uint64_t device_offset);
 
 /* Counters of the last rt_trace on this scene (read after the stream is

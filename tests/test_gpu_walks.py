@@ -256,3 +256,31 @@ def test_staged_rays_taken_together(ctx, n):
     oh, _, _ = orc.trace(blob.bytes(), rays, 1, orc.Treelets(blob.bytes(), 1024), threads=8)
     assert_hits_equal(hits.cpu().numpy().view(rt.HIT_DTYPE), oh, "staged")
     scene.close()
+
+
+def test_forming_treelets_waits_for_traces_in_flight(ctx):
+    """Plain traces queued on a stream of the caller's own are over when
+    rt_treelets_form, or a change of the device offset, returns: both rewrite
+    nodes that the traces read."""
+    import torch
+
+    import treelet_rt as rt
+
+    n = 1 << 21
+    scene = rt.Scene(ctx, rt.Blob.gen(rt.SCENE_CUBE_PLANE, 3000, 6))
+    rays = np.resize(rt.camera_rays(rt.default_camera(rt.SCENE_CUBE_PLANE), 190, 97, 1, 2, 1e-4, 1e30), n)
+    d_rays = torch.from_numpy(rays.view(np.uint8).copy()).cuda()
+    want = torch.zeros(n * 64, dtype=torch.uint8, device="cuda")
+    scene.trace(d_rays, want, rt.MODE_PLAIN, n=n)
+    torch.cuda.synchronize()
+    stream = torch.cuda.Stream()
+    for change in (lambda: scene.form_treelets(1024), lambda: scene.form_treelets(2048),
+                   lambda: scene.set_device_offset(64), lambda: scene.set_device_offset(0)):
+        hits = [torch.zeros(n * 64, dtype=torch.uint8, device="cuda") for _ in range(4)]
+        torch.cuda.synchronize()
+        for k in range(200):  # at least a tenth of a second of work: longer than the calls take by themselves
+            scene.trace(d_rays, hits[k % 4], rt.MODE_PLAIN, n=n, stream=stream.cuda_stream)
+        change()
+        assert stream.query()
+        assert all(torch.equal(h, want) for h in hits)
+    scene.close()

@@ -342,7 +342,7 @@ void drop_pin_cache(rt_scene* s) {
 }
 
 // Writes the scene's walk nodes with the given route bits (null: none) and
-// waits for them.
+// waits for them.  Nothing on the device may be reading them.
 cudaError_t make_walk_nodes(rt_scene* s, const uint16_t* d_route) {
   rtk::walk_nodes_kernel<<<(s->n_units + 255) / 256, 256>>>(reinterpret_cast<const uint4*>(s->d_blob), s->d_internal,
                                                             d_route, s->n_units, reinterpret_cast<uint4*>(s->d_walk));
@@ -363,6 +363,10 @@ rt_status upload_route(rt_scene* s) {
   rtt::route_masks(s->host_blob.data(), s->blob_bytes, s->part, s->route);
   if (s->offset_quirk)
     for (uint16_t& r : s->route) r &= (uint16_t)~((0x3Fu << rtt::kRouteOtherShift) | (2u << rtt::kRouteInstShift));
+  // Launches in flight, plain ones too, read the walk nodes through the
+  // non-coherent path, and a caller's stream need not wait for the default one.
+  // (The nodes stay where they are: captured graphs of plain traces hold their address.)
+  RT_CUDA(cudaDeviceSynchronize());
   RT_CUDA(cudaMemcpy(s->d_route, s->route.data(), sizeof(uint16_t) * s->route.size(), cudaMemcpyHostToDevice));
   RT_CUDA(make_walk_nodes(s, s->d_route));
   drop_pin_cache(s);
