@@ -276,7 +276,9 @@ rt_status rt_trace_host(rt_scene* scene, const rt_ray* rays, const uint32_t* fla
  * RT_ERR_TOO_LARGE (call again with arrays of *total entries).  Calls of
  * 2^17 rays or more run as chunks whose packing and copies overlap the next
  * chunk's trace (page-locked arrays let the copies run at full speed); calls
- * of at most 2^14 rays pack straight into page-locked arrays.
+ * of at most 2^14 rays pack straight into page-locked arrays.  (An array lies
+ * in one page-locked allocation or registration, or is pageable: the copies of
+ * one that spans several fail, RT_ERR_CUDA.)
  * n x row_capacity must stay below 2^32 and n at most 2^24.  Synchronous. */
 rt_status rt_trace_host_packed(rt_scene* scene, const rt_ray* rays, const uint32_t* flags, uint32_t default_flags,
                                uint32_t n, uint32_t mode, uint32_t row_capacity, rt_hit* hits, uint64_t* offsets,

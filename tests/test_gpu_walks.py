@@ -284,3 +284,48 @@ def test_forming_treelets_waits_for_traces_in_flight(ctx):
         assert stream.query()
         assert all(torch.equal(h, want) for h in hits)
     scene.close()
+
+
+def test_packed_arrays_lie_in_one_registration(ctx):
+    """A small packed call packs into an array anywhere inside one page-locked
+    registration; an array across two of them (back to back here, so that all
+    of it is page-locked) is refused as the copies of larger calls refuse it, and
+    the next call is none the worse."""
+    import ctypes as C
+    import mmap
+
+    import torch
+
+    import treelet_rt as rt
+
+    n, cap, page = 300, 24, mmap.PAGESIZE
+    scene = rt.Scene(ctx, rt.Blob.gen(rt.SCENE_CUBE_PLANE, 3000, 6))
+    scene.form_treelets(1024)
+    rays = np.ascontiguousarray(rt.camera_rays(rt.default_camera(rt.SCENE_CUBE_PLANE), 30, 10, 1, 2, 1e-4, 1e30)[:n])
+    hits, vis, _ = scene.trace_host(rays, rt.MODE_TREELET, capacity=cap, want_visits=True)
+    keep = np.arange(cap)[None, :] < hits["n_visits"][:, None]
+    total = int(keep.sum())
+    half = -(-n * 64 // page) * page  # bytes of a registration: the hit records fit one
+    room = mmap.mmap(-1, 2 * half)
+    base = np.frombuffer(room, np.uint8)
+    cudart = torch.cuda.cudart()
+    for k in range(2):
+        assert int(cudart.cudaHostRegister(base.ctypes.data + k * half, half, 0)) == 0
+    off = torch.zeros(n + 1, dtype=torch.int64).pin_memory()
+    v = torch.zeros(total, dtype=torch.int32).pin_memory()
+    try:
+        for at, ok in ((0, True), (half, True), (half - 64 * 7, False), (2 * half - 64 * n, True)):
+            base[:] = 0
+            got = C.c_uint64(0)
+            st = rt.lib().rt_trace_host_packed(scene.handle, rays.ctypes.data, None, 1, n, rt.MODE_TREELET, cap,
+                                               base.ctypes.data + at, off.data_ptr(), v.data_ptr(), None, total,
+                                               C.byref(got))
+            assert st == (0 if ok else 2), rt.lib().rt_last_error().decode()
+            if ok:
+                assert got.value == total
+                assert_hits_equal(base[at:at + 64 * n].copy().view(rt.HIT_DTYPE), hits, "packed hits")
+                assert np.array_equal(v.numpy().view(np.uint32), vis[keep])
+    finally:
+        for k in range(2):
+            cudart.cudaHostUnregister(base.ctypes.data + k * half)
+    scene.close()

@@ -1,6 +1,7 @@
 // C ABI: contexts, device scenes, treelets, tracing, bounce rays and the
 // prefetch decision.  Every entry point returns an rt_status and records a
 // message for rt_last_error(); none aborts.
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -211,6 +212,7 @@ struct rt_scene {
 namespace {
 
 rt_status cuda_fail(cudaError_t e, const char* what) {
+  cudaGetLastError();  // reported here: the next launch's check is not to find it again
   return rti::fail(RT_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
 }
 
@@ -1067,11 +1069,36 @@ void* mapped_host(const void* p) {
   return at.type == cudaMemoryTypeHost ? at.devicePointer : nullptr;
 }
 
-// The same for an array of `bytes` bytes, all of it page-locked.
+// First byte and size of the allocation or registration that holds host byte
+// p, which is page-locked.
+bool host_allocation(const void* p, uintptr_t& first, size_t& size) {
+  using Query = CUresult (*)(unsigned, CUpointer_attribute*, void**, CUdeviceptr);
+  static const Query query = [] {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult found = cudaDriverEntryPointSymbolNotFound;
+    if (cudaGetDriverEntryPointByVersion("cuPointerGetAttributes", &f, 7000, cudaEnableDefault, &found) != cudaSuccess)
+      cudaGetLastError();
+    return found == cudaDriverEntryPointSuccess ? reinterpret_cast<Query>(f) : nullptr;
+  }();
+  CUdeviceptr start = 0;
+  size = 0;
+  CUpointer_attribute what[2] = {CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+  void* to[2] = {&start, &size};
+  if (!query || query(2, what, to, (CUdeviceptr)(uintptr_t)p) != CUDA_SUCCESS) return false;
+  first = (uintptr_t)start;
+  return size != 0;
+}
+
+// mapped_host for an array of `bytes` bytes that lies in one page-locked
+// allocation (two page-locked ends say nothing of what is between them).
 void* mapped_range(const void* p, size_t bytes) {
-  uint8_t* first = static_cast<uint8_t*>(mapped_host(p));
-  if (!first || bytes == 0) return first;
-  return mapped_host(static_cast<const uint8_t*>(p) + bytes - 1) == first + bytes - 1 ? first : nullptr;
+  void* const d = mapped_host(p);
+  uintptr_t first = 0;
+  size_t size = 0;
+  if (!d || bytes == 0) return d;
+  if (!host_allocation(p, first, size)) return nullptr;
+  const size_t before = (uintptr_t)p - first;
+  return before <= size && bytes <= size - before ? d : nullptr;
 }
 
 rt_status timeout_status(uint32_t status, const char* who) {
