@@ -329,3 +329,39 @@ def test_packed_arrays_lie_in_one_registration(ctx):
         for k in range(2):
             cudart.cudaHostUnregister(base.ctypes.data + k * half)
     scene.close()
+
+
+@pytest.mark.parametrize("epoch", [16, 64])
+def test_staged_epoch_counts_node_visits(ctx, epoch):
+    """Warp slots: a warp votes every staged_epoch visits.  A visit is of 32
+    nodes at most, on average of far fewer, so the warps vote more than (nodes
+    read) / (32 epoch) times; with one slot, one vote enough, and rays all over a
+    scene of many treelets, nearly every vote stages one.  And they vote no more
+    often than the visits allow, at once and then every epoch."""
+    import torch
+
+    import treelet_rt as rt
+
+    n = 2_000_000
+    scene = rt.Scene(ctx, rt.Blob.gen(rt.SCENE_BLOBS, 60000, 5))
+    info = scene.form_treelets(1024)
+    assert info["n_treelets"] > 1000
+    rng = np.random.default_rng(3)
+    rays = np.zeros(n, rt.RAY_DTYPE)
+    rays["origin"] = rng.uniform(0, 1, (n, 3))
+    rays["dir"] = rng.normal(size=(n, 3))
+    rays["tmax"] = 1e30
+    d_rays = torch.from_numpy(rays.view(np.uint8).copy()).cuda()
+    want = torch.zeros(n * 64, dtype=torch.uint8, device="cuda")
+    scene.trace(d_rays, want, rt.MODE_TREELET, n=n)
+    scene.set_tuning(staged_slots=1, staged_min_votes=1, staged_epoch=epoch, staged_threads=128,
+                     pinned_bytes=rt.TUNING_OFF)
+    hits = torch.zeros_like(want)
+    scene.trace(d_rays, hits, rt.MODE_STAGED, n=n)
+    torch.cuda.synchronize()
+    assert torch.equal(hits, want)
+    st = scene.stats()
+    nodes = st["smem_reads"] + st["gmem_reads"]
+    assert st["stagings"] > nodes / (32 * epoch)
+    assert st["stagings"] <= nodes / epoch + 152 * 64
+    scene.close()

@@ -582,7 +582,7 @@ constexpr uint32_t kTogetherRays = 1u << 19;
 // cp.async.bulk and keeps it for the whole launch; every node read that names
 // a record is served from it.
 //
-// Warp slots: every `epoch` node visits a warp votes: each lane names the
+// Warp slots: every `epoch` node visits of its lanes together a warp votes: each lane names the
 // treelet of its next access, __match_any_sync counts equal names, and the
 // most popular treelet that is not resident (ties to the lowest treelet, i.e.
 // the lowest root address, as the RT unit's decision in shader.cc:3424-3441)
@@ -652,9 +652,9 @@ __global__ void __launch_bounds__(kStagedMaxThreads, kStagedMinBlocks) trace_sta
   w.pin_root = pin_ok ? a.pin_root : 0u;
   bool have = false, ended = false;
   int spare = (int)a.refill;  // idle lanes that end a turn; 33 once no rays are left
-  uint32_t r = 0, it = 0;
+  uint32_t r = 0, left = 0;  // left: visits of the warp until it votes
   unsigned long long bytes = 0, staged = 0, stagings = 0;
-  for (;; ++it) {
+  for (;;) {
     // --- records of finished rays, then new rays for idle lanes (as run_persistent)
     const uint32_t need = __ballot_sync(0xffffffffu, !have);
     if (need == 0xffffffffu || __popc(need) >= spare) {
@@ -681,7 +681,8 @@ __global__ void __launch_bounds__(kStagedMaxThreads, kStagedMinBlocks) trace_sta
         spare = rays_together(w.cx.o, w.dir()) ? 32 : (int)a.refill;
     }
     // --- staging: land a finished copy, then vote for the next one
-    if (SLOTS && slots > 0 && (it % a.epoch) == 0) {
+    if (SLOTS && left == 0) {
+      left = a.epoch;
       if (lane == 0 && st.pending_slot != kNone && mbar_test(&st.bar, st.phase)) {
         st.resident[st.pending_slot] = st.pending_id;
         st.units[st.pending_slot] = st.pending_units;
@@ -735,8 +736,8 @@ __global__ void __launch_bounds__(kStagedMaxThreads, kStagedMinBlocks) trace_sta
       __syncwarp();
     }
     // --- node visits
-    if (SLOTS) warp_turn(a, w, r, have, ended, spare, lookup);
-    else warp_turn(a, w, r, have, ended, spare, NoLookup());
+    if (SLOTS) warp_turn(a, w, r, have, ended, spare, lookup, left);
+    else warp_turn(a, w, r, have, ended, spare, NoLookup(), left);
   }
   rtd::touch_l1_done();
   // copies still in flight must land before the CTA's shared memory goes away
