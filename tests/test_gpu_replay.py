@@ -95,3 +95,121 @@ def test_replay_bad_config_is_an_error(ctx):
         with pytest.raises(rt.RTError):
             scene.unit_replay(hits, vis, n, CAP, cfg, d_stats)
     scene.close()
+
+
+def _replay(scene, blob, budget, hits, vis, n, cfg):
+    """Counters of the replay and of the oracle's, for device traces."""
+    import torch
+
+    import treelet_rt as rt
+    from oracle import oracle as orc
+
+    d_stats = torch.zeros(cfg.n_rt_units * rt.UNIT_STATS_DTYPE.itemsize, dtype=torch.uint8, device="cuda")
+    scene.unit_replay(hits, vis, n, CAP, cfg, d_stats)
+    got = np.frombuffer(d_stats.cpu().numpy().tobytes(), rt.UNIT_STATS_DTYPE)
+    h = np.frombuffer(hits.cpu().numpy().tobytes(), rt.HIT_DTYPE)
+    v = vis.cpu().numpy().view(np.uint32).reshape(n, CAP)
+    return got, orc.unit_replay(orc.Treelets(blob.bytes(), budget), h, v, cfg)
+
+
+EDGES = [
+    dict(max_warps=16, l1_sets=64, l1_ways=32, prefetcher=1, heuristic=0),  # 2,048 lines: more than shared memory takes
+    dict(max_warps=16, l1_sets=128, l1_ways=16, prefetcher=2, max_queue=0),
+    dict(max_warps=16, l1_sets=16, l1_ways=32, prefetcher=1, heuristic=2, second_prefetch=1),
+    dict(max_warps=16, l1_sets=16, l1_ways=16, prefetcher=1, scheduler=1, load_metadata=1, wait_metadata=1, max_queue=2048),
+    dict(max_warps=16, l1_sets=1, l1_ways=1, prefetcher=1, scheduler=2, prefetch_delay=7),
+    dict(max_warps=1, l1_sets=8, l1_ways=4, prefetcher=1, heuristic=3, second_prefetch=1, prefetch_delay=2),
+    dict(max_warps=16, l1_sets=8, l1_ways=4, prefetcher=1, prefetch_delay=1000),
+    dict(max_warps=6, l1_sets=8, l1_ways=4, prefetcher=1, hit_latency=1, miss_latency=1),
+    dict(max_warps=6, l1_sets=8, l1_ways=4, prefetcher=1, miss_latency=4000, load_metadata=1, max_queue=2048, n_rt_units=40),
+    dict(max_warps=16, l1_sets=8, l1_ways=4, prefetcher=1, n_rt_units=150),  # units without warps
+]
+
+
+@pytest.mark.parametrize("kind,budget", [("cube_plane", 1024), ("terrain", 8192)])
+@pytest.mark.parametrize("extra", EDGES)
+def test_replay_at_its_limits(ctx, kind, budget, extra):
+    """As many resident warps as there may be and one, lines in shared memory
+    and outside it, rare decisions, equal and long latencies, idle units."""
+    import treelet_rt as rt
+
+    blob, scene, hits, vis, n = _gpu_traces(ctx, kind, budget)
+    cfg = rt.unit_config(**{**dict(n_rt_units=7, hit_latency=3, miss_latency=60), **extra})
+    got, exp = _replay(scene, blob, budget, hits, vis, n, cfg)
+    for f in rt.UNIT_STATS_DTYPE.names:
+        assert np.array_equal(got[f], exp[f]), (f, got[f], exp[f])
+    scene.close()
+
+
+@pytest.mark.parametrize("max_cycles", [1, 2, 61, 64, 777, 4096, 20011])
+def test_replay_stops_at_max_cycles(ctx, max_cycles):
+    """The limit falls where it may, into skipped idle cycles too."""
+    import treelet_rt as rt
+
+    blob, scene, hits, vis, n = _gpu_traces(ctx, "terrain", 8192)
+    for extra in (dict(prefetcher=0), dict(prefetcher=1, prefetch_delay=3), dict(prefetcher=1, prefetch_delay=100)):
+        cfg = rt.unit_config(n_rt_units=5, max_warps=2, l1_sets=8, l1_ways=4, hit_latency=3, miss_latency=60,
+                             max_cycles=max_cycles, **extra)
+        got, exp = _replay(scene, blob, 8192, hits, vis, n, cfg)
+        assert (exp["status"] == 2).all()
+        for f in rt.UNIT_STATS_DTYPE.names:
+            assert np.array_equal(got[f], exp[f]), (extra, f, got[f], exp[f])
+    scene.close()
+
+
+def test_replay_with_a_full_prefetch_ring(ctx):
+    """Prefetches that never issue (each waits for metadata that nobody loads)
+    pile up until the ring of 2^18 entries is full: that is reported, and the
+    counters that a full ring cannot change are the oracle's."""
+    import treelet_rt as rt
+
+    blob, scene, hits, vis, n = _gpu_traces(ctx, "terrain", 65536)
+    cfg = rt.unit_config(n_rt_units=5, max_warps=1, l1_sets=16, l1_ways=4, hit_latency=3, miss_latency=60,
+                         prefetcher=1, heuristic=0, wait_metadata=1, max_queue=1 << 31)
+    got, exp = _replay(scene, blob, 65536, hits, vis, n, cfg)
+    full = exp["prefetch_queued"] - exp["prefetch_removed"] > 1 << 18
+    assert full.any() and not exp["prefetch_issued"].any()
+    assert (got["status"][full] == 1).all()
+    for f in rt.UNIT_STATS_DTYPE.names:
+        if f not in ("status", "prefetch_removed"):
+            assert np.array_equal(got[f], exp[f]), (f, got[f], exp[f])
+    scene.close()
+
+
+@pytest.mark.parametrize("budget", [192, 256, 8192])
+@pytest.mark.parametrize("extra", [dict(heuristic=0), dict(heuristic=0, wait_metadata=1),
+                                   dict(heuristic=2, second_prefetch=1), dict(heuristic=0, max_queue=8)])
+def test_replay_of_members_that_share_addresses(ctx, budget, extra):
+    """A quad leaf in the second half of an instance leaf: both members of a
+    treelet queue requests of the same addresses."""
+    import kat_blob as K
+    import torch
+
+    import treelet_rt as rt
+
+    full = ((0, 0, 0), (64, 64, 64))
+    units = [
+        K._header(256, (-1, -1, 0), (3, 3, 4)),                     # 0: TLAS root is unit 4
+        K._header(64, (-1, -1, 0), (3, 3, 4)),                      # 1: BLAS root is unit 2
+        K._internal((-1, -1, 0), 4, (4, 4, 4), [(1, 4) + full] * 3),  # 2: leaves 6, 7, 8
+        bytes(64),
+        K._internal((-1, -1, 0), 1, (4, 4, 4), [(2, 1) + full]),    # 4
+        K._instance((1 << 64) - 256, 7),                            # 5-6: BLAS header is unit 1
+        K._quad(1.0, 100), K._quad(2.0, 101),                       # 7, 8
+    ]
+    data = np.frombuffer(b"".join(units), np.uint8).copy()
+    blob = rt.Blob.wrap(data)
+    scene = rt.Scene(ctx, blob)
+    scene.form_treelets(budget)
+    assert {5, 6} <= set(scene.treelets()["members"].tolist())
+    rays = np.resize(K.grid_rays(16), 1024)
+    h, v, _ = scene.trace_host(rays, rt.MODE_TREELET, capacity=CAP, want_visits=True)
+    hits = torch.from_numpy(h.view(np.uint8).copy()).cuda()
+    vis = torch.from_numpy(v.view(np.uint8).copy()).cuda().view(torch.int32)
+    cfg = rt.unit_config(n_rt_units=3, max_warps=4, l1_sets=1, l1_ways=2, hit_latency=3, miss_latency=40, prefetcher=1,
+                         **extra)
+    got, exp = _replay(scene, blob, budget, hits, vis, len(rays), cfg)
+    for f in rt.UNIT_STATS_DTYPE.names:
+        assert np.array_equal(got[f], exp[f]), (f, got[f], exp[f])
+    assert got["prefetch_queued"].sum() > 0
+    scene.close()
