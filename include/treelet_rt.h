@@ -274,7 +274,7 @@ rt_status rt_trace_host(rt_scene* scene, const rt_ray* rays, const uint32_t* fla
  * written; when it exceeds `capacity`, hits, offsets and *total are still
  * filled, the arrays' contents are unspecified and the call returns
  * RT_ERR_TOO_LARGE (call again with arrays of *total entries).  Calls of
- * 2^17 rays or more run as chunks whose packing and copies overlap the next
+ * 2^19 rays or more run as chunks whose packing and copies overlap the next
  * chunk's trace (page-locked arrays let the copies run at full speed); calls
  * of at most 2^14 rays pack straight into page-locked arrays.  (An array lies
  * in one page-locked allocation or registration, or is pageable: the copies of

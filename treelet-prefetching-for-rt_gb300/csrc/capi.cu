@@ -1781,20 +1781,30 @@ __global__ void trace_offsets_kernel(uint32_t* __restrict__ off, const uint32_t*
   }
 }
 
-// Chunks of a packed call: two from 2^17 rays on, four from 2^19.  Overlapping
-// the copies with the next chunk's trace pays for the second launch's tail of
-// long rays from there: 307,200 primary rays with both traces (144 MB out) take
-// 1.46 ms in one chunk on a GB300, 1.35 in two, 1.41 in three, 1.68 in four.
-constexpr uint32_t kPackedChunkRays = 1u << 17;
-constexpr uint32_t kPackedFewChunks = 2;
+// Rays from which a packed call runs as kHostChunks chunks.  Each chunk's trace
+// has a tail of long rays of its own, and starts when the one before it is packed;
+// the copies that overlap pay for that in large calls only.  GB300, both traces
+// out, us in one chunk / two, and / four from 2^19 rays on:
+//                                            131,072     200,000      307,200      450,000      524,288      1,000,000
+//   131K-tri terrain, primary, treelet order 818 / 1026  1071 / 1165  1453 / 1349  2006 / 1845  2277 / 2106  4094 / 3486
+//   the same, bounce, plain                  901 / 1193  1176 / 1405  1528 / 1716  2030 / 1997  2858 / 3073  5091 / 4207
+//   1M-tri blobs, primary, treelet order     518 / 804   648 / 849    807 / 979    1034 / 1127  1144 / 1401  1851 / 1894
+//   the same, bounce, plain                  504 / 752   617 / 896    775 / 954    943 / 1193   1149 / 1610  1854 / 2281
+constexpr uint32_t kPackedChunkRays = 1u << 19;
 // Rays up to which a call into page-locked arrays packs straight into them.
 // That saves a wait for the total and five copies (32 rays: 96 -> 50 us), but the
 // kernel stores to host memory at 120 GB/s, the copy engines at 200: 307,200 rays
-// 1.79 ms that way.
+// 1.79 ms that way.  The line is where the gain has become small (the calls above;
+// us straight / through the copies):
+//   32  99 / 129, 24 / 49, 105 / 142, 24 / 52       12,000  253 / 276, 277 / 297, 207 / 238, 207 / 238
+//   20,000  329 / 335, 349 / 359, 220 / 240, 227 / 251   32,768  437 / 429, 465 / 457, 272 / 279, 285 / 297
 constexpr uint32_t kPackDirectRays = 1u << 14;
 
 // Counts, offsets and total of a call of at most kScanRays rays in one block
-// (its four kernels' launches took longer than their work).
+// (its four kernels' launches took longer than their work).  The calls above, us in
+// one block / four kernels: 32 rays 99 / 107, 24 / 34, 105 / 115, 24 / 36; 8,192
+// 210 / 218, 205 / 212, 177 / 184, 201 / 209; 20,000 336 / 335, 362 / 359, 238 /
+// 240, 249 / 251; 65,536 588 / 560, 643 / 613, 454 / 436, 457 / 431.
 constexpr uint32_t kScanRays = 1u << 13;
 __global__ void __launch_bounds__(1024) trace_scan_kernel(const rt_hit* __restrict__ hits, uint32_t n, uint32_t cap,
                                                           uint32_t* __restrict__ off,
@@ -1912,7 +1922,7 @@ extern "C" rt_status rt_trace_host_packed(rt_scene* s, const rt_ray* rays, const
   bound[0] = 0;
   bound[1] = n;
   if (!queued(s, mode) && n >= kPackedChunkRays) {
-    chunks = n >= (1u << 19) ? rti::kHostChunks : kPackedFewChunks;
+    chunks = rti::kHostChunks;
     for (uint32_t c = 0; c <= chunks; ++c) bound[c] = (uint64_t)n * c / chunks;
   }
   const size_t b_rays = al(sizeof(rt_ray) * (size_t)n), b_flags = flags ? al(sizeof(uint32_t) * (size_t)n) : 0;
