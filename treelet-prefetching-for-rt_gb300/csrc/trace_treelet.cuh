@@ -550,9 +550,16 @@ struct WarpStage {
 };
 
 // Whether the calling warp's 32 rays, just taken, leave one point within a
-// narrow cone of each other (kCone: cosine squared, 14 degrees), as a camera's
-// neighbouring rays do.
-constexpr float kCone = 0.94f;
+// narrow cone of the first (kCone: cosine squared, 3 degrees), as a camera's
+// neighbouring rays do.  GB300, 1M primary rays staged, tiles of 8 x 4 pixels a
+// warp, us waiting / refilling (kTogetherRays), for frames whose tiles are ever
+// narrower:
+//                    32 x 32      64 x 64      128 x 128    192 x 192    256 x 256    512 x 512    1024 x 1024
+//   2M-tri terrain   1985 / 1673  1776 / 1638  1591 / 1591  1488 / 1562  1444 / 1543  1330 / 1449  1211 / 1304
+//   1M-tri blobs     934 / 698    772 / 672    684 / 659    648 / 654    659 / 651    611 / 626    607 / 620
+// A 192 x 192 frame's tile is 2.6 degrees across, a 128 x 128 frame's 3.9.  The same
+// camera's rays in random order 2520 / 1766 and 1565 / 715.
+constexpr float kCone = 0.9973f;
 
 __device__ __forceinline__ bool rays_together(rtm::V3 o, rtm::V3 d) {
   const float ox = __shfl_sync(0xffffffffu, o.x, 0), oy = __shfl_sync(0xffffffffu, o.y, 0);
