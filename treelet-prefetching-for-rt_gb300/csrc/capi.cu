@@ -556,26 +556,36 @@ rt_status launch_queued(rtk::TraceArgs& a, const rt_tuning& t, uint32_t largest_
 
 // Rays up to which a launch walks each with eight lanes (trace_group.cuh)
 // instead of one.  GB300, us of a launch, eight lanes / one:
-//                                    32        1,024      4,096      16,384     30,976     49,152
-//   131K-tri terrain, bounce, plain  69 / 126  126 / 281  158 / 321  210 / 369  298 / 372  440 / 370
-//   the same, treelet order          79 / 210  124 / 315  153 / 340  259 / 380  360 / 444  495 / 417
-//   16K-tri cube, bounce, plain      28 / 55   44 / 96    49 / 108   66 / 115   94 / 117   105 / 120
-//   the same, treelet order          31 / 65   44 / 106   50 / 114   67 / 116   107 / 126  124 / 117
-// Longer launches have enough rays to fill the lanes, and eight lanes a ray
-// then cost more instructions than one.
+//                                    32        1,024      4,096      16,384     25,600     32,768     49,152
+//   2M-tri terrain, primary, plain   66 / 117  93 / 175   97 / 182   169 / 209  183 / 224  253 / 212  292 / 234
+//   the same, bounce, plain          56 / 116  133 / 214  144 / 229  241 / 317  284 / 278  362 / 278  443 / 319
+//   the same, bounce, treelet order  63 / 140  115 / 244  161 / 277  249 / 328  321 / 359  372 / 371  509 / 403
+//   1M-tri blobs, bounce, plain      36 / 46   141 / 217  99 / 201   152 / 255  157 / 242  216 / 285  230 / 265
+//   the same, treelet order          36 / 46   118 / 189  116 / 228  153 / 272  175 / 277  221 / 332  298 / 343
+//   16K-tri cube, bounce, plain      26 / 35   47 / 74    50 / 84    68 / 92    79 / 99    93 / 97     140 / 112
+//   the same, treelet order          27 / 40   47 / 79    52 / 91    72 / 93    89 / 101   104 / 106  143 / 118
+// At the line some scenes still gain (131K-triangle terrain, 30,976 rays: 298 / 372,
+// 360 / 444) and the largest lose.  Longer launches have enough rays to fill the
+// lanes, and eight lanes a ray then cost more instructions than one.  Stacks of
+// 160 entries in treelet order take the line down, as fewer rays are resident:
+// 25,600 rays 268 / 256, 387 / 357 on the terrain (primary, bounce), 171 / 222, 186 /
+// 274 on the blobs, 70 / 83, 106 / 106 on the cube, 32,768 352 / 245, 424 / 372,
+// 191 / 220, 280 / 331, 97 / 84, 129 / 106; other depths are alike.
 constexpr uint32_t kGroupRays = 1u << 15;
-// A warp holds one ray up to this many, then two, then four: 32 warps of 64-72
+// A warp holds one ray up to this many, then two, then four: 24-28 warps of 72-80
 // registers are resident on each of 152 SMs (twice as many rays a warp from
 // the start: 9,216 bounce rays 303 against 257 us).
 constexpr uint32_t kGroupRaysPerSplit = 152 * 32;
 
 // Rays and pinned bytes up to which a staged launch does: each of its CTAs of
 // four warps copies the image.  Eight lanes / one, pinned image of 4 KiB:
-//                                    32        1,024      4,096      16,384     25,600     30,976
-//   131K-tri terrain, primary        57 / 124  90 / 230   116 / 249  198 / 274  226 / 273  304 / 275
-//   131K-tri terrain, bounce         88 / 186  140 / 331  173 / 358  332 / 410  375 / 419  413 / 434
-//   16K-tri cube, bounce             32 / 54   47 / 99    57 / 110   76 / 109   103 / 120  122 / 115
-// With 16 KiB pinned, terrain bounce: 89 / 189 at 32 rays, 324 / 429 at 16,384, 430 / 452 at 24,480.
+//                                    32        1,024      4,096      16,384     24,000     25,600     32,768
+//   2M-tri terrain, primary          76 / 144  114 / 254  115 / 257  214 / 290  226 / 287  235 / 298  275 / 283
+//   2M-tri terrain, bounce           71 / 162  131 / 333  190 / 373  300 / 437  378 / 463  414 / 439  456 / 436
+//   1M-tri blobs, bounce             41 / 53   139 / 223  139 / 269  189 / 325  207 / 329  213 / 322  267 / 379
+//   16K-tri cube, bounce             30 / 45   54 / 97    60 / 113   86 / 116   106 / 120  108 / 120  126 / 119
+// With stacks of 160 entries 24,000 rays 315 / 285, 454 / 464, 245 / 331, 123 / 122.
+// With 16 KiB pinned, 131K-triangle terrain, bounce: 89 / 189 at 32 rays, 324 / 429 at 16,384, 430 / 452 at 24,480.
 constexpr uint32_t kGroupStagedRays = 3u << 13;
 constexpr uint32_t kGroupPinBytes = 16384;
 
