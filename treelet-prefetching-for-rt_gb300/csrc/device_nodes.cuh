@@ -55,23 +55,13 @@ __device__ __forceinline__ void ld_global_v8(const uint4* p, uint32_t* w) {
       : "l"(p));
 }
 
-// Loads 64 bytes: from shared memory when saddr != 0, else from global.
-__device__ __forceinline__ void load64(const uint4* g, uint32_t saddr, Node64& n) {
-  if (!saddr) {
-    ld_global_v8(g, n.w);
-    ld_global_v8(g + 2, n.w + 8);
-    return;
-  }
-#pragma unroll
-  for (int q = 0; q < 4; ++q) {
-    const uint4 v = saddr ? ld_shared_v4(saddr + 16u * q) : ld_global_nc(g + q);
-    n.w[4 * q + 0] = v.x;
-    n.w[4 * q + 1] = v.y;
-    n.w[4 * q + 2] = v.z;
-    n.w[4 * q + 3] = v.w;
-  }
+// Loads a node's 64 bytes from global memory.
+__device__ __forceinline__ void load64(const uint4* g, Node64& n) {
+  ld_global_v8(g, n.w);
+  ld_global_v8(g + 2, n.w + 8);
 }
 
+// 16 bytes: from shared memory when saddr != 0, else from global.
 __device__ __forceinline__ uint4 load16(const uint4* g, uint32_t saddr, int q) {
   return saddr ? ld_shared_v4(saddr + 16u * q) : ld_global_nc(g + q);
 }
@@ -218,9 +208,9 @@ __device__ __forceinline__ void instance_from(const Node64& q, const uint4* g, u
   in.instance_id = d.z;
 }
 
-__device__ __forceinline__ void load_instance(const uint4* g, uint32_t saddr, Instance& in) {
-  const uint4 a = load16(g, saddr, 1), b = load16(g, saddr, 2), c = load16(g, saddr, 3);
-  const uint4 d = load16(g, saddr, 4), e = load16(g, saddr, 7);
+__device__ __forceinline__ void load_instance(const uint4* g, Instance& in) {
+  const uint4 a = ld_global_nc(g + 1), b = ld_global_nc(g + 2), c = ld_global_nc(g + 3);
+  const uint4 d = ld_global_nc(g + 4), e = ld_global_nc(g + 7);
   // bytes 16..51: world-to-object rows 0-2
   const uint32_t lin[9] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, c.x};
 #pragma unroll

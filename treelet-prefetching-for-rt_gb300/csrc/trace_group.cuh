@@ -266,7 +266,7 @@ struct GroupWalk {
           q.w[4 * w] = y.x, q.w[4 * w + 1] = y.y, q.w[4 * w + 2] = y.z, q.w[4 * w + 3] = y.w;
         }
       } else {
-        rtd::load64(src, 0, q);
+        rtd::load64(src, q);
       }
       quad = rtf::leaf_type_of(q.w[1]) == 0;
       if (quad) {
@@ -336,7 +336,7 @@ struct GroupWalk {
         for (int q = 0; q < 4; ++q) in.w2o.m[(4 * k + q) / 3][(4 * k + q) % 3] = __uint_as_float(w[q]);
       }
     } else {
-      rtd::load_instance(v.blob + (uint64_t)unit * 4, 0, in);
+      rtd::load_instance(v.blob + (uint64_t)unit * 4, in);
     }
     enter_instance(in, unit, O, D, tmin, tmax, cx);
     if (!top) return;

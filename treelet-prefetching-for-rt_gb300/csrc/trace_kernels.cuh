@@ -253,9 +253,9 @@ __device__ __forceinline__ void write_hit(const TraceArgs& a, const SceneView& v
   h.reserved = 0;
   if (hit) {
     rtd::Node64 q;
-    rtd::load64(v.blob + (uint64_t)c_leaf * 4, 0, q);
+    rtd::load64(v.blob + (uint64_t)c_leaf * 4, q);
     rtd::Instance in;
-    rtd::load_instance(v.blob + (uint64_t)c_inst * 4, 0, in);
+    rtd::load_instance(v.blob + (uint64_t)c_inst * 4, in);
     const rtm::ObjRay orr = rtm::make_transformed_ray(in.w2o, O, D, tmin, tmax);
     h.hit_geometry = 1;
     h.geometry_index = rtf::geometry_index_of(q.w[1]);
@@ -552,7 +552,7 @@ struct PlainWalker {
       stop(RT_RAY_BAD_NODE);
       return false;
     }
-    rtd::load64(from + (uint64_t)unit * 4, 0, q);
+    rtd::load64(from + (uint64_t)unit * 4, q);
     return true;
   }
 

@@ -289,7 +289,7 @@ struct Walker {
         nd.w[4 * k + 3] = w.w;
       }
     } else {
-      rtd::load64(src, 0, nd);
+      rtd::load64(src, nd);
     }
     return true;
   }
@@ -386,7 +386,7 @@ struct Walker {
         rtd::instance_from(nd, v.blob + (uint64_t)unit * 4, saddr, in);
       }
     } else {
-      rtd::load_instance(v.blob + (uint64_t)unit * 4, 0, in);
+      rtd::load_instance(v.blob + (uint64_t)unit * 4, in);
     }
     enter_instance(in, unit, world_o(), dir(), tmin, tmax, cx);
     if (!top) return;
