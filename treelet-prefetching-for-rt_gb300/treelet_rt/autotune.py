@@ -4,7 +4,9 @@ For one scene, one device ray batch and one mode it searches the launch
 parameters coordinate by coordinate (two passes over the parameters; each
 candidate timed with CUDA events, best of `reps` after a warm-up), keeping
 the fastest setting that produces no stack overflow.  None of the parameters
-changes a result; the treelet budget (searched only when `budgets` is given)
+changes a result, except that a ray which needs more stack entries than
+stack_depth is flagged: a depth below the default is kept only when it is more
+than 1% faster.  The treelet budget (searched only when `budgets` is given)
 selects a different partition, which the caller then forms for its own
 parity checks.  autotune_batch does the same for a many-scene batch launch
 (rt_batch_set_tuning: threads, refill lanes, stack depth).
@@ -47,6 +49,18 @@ def stages(cfg: dict) -> bool:
     all (pinned treelets, warp slots or treelet queues)."""
     return (cfg.get("pinned_bytes", OFF) != OFF or cfg.get("staged_slots", OFF) != OFF
             or cfg.get("queue_rounds", OFF) != OFF)
+
+
+def settle_depth(best: dict, best_ms: float, measure) -> tuple[float, dict]:
+    """The search's choice, at the default stack depth instead of a shallower
+    one when that is as fast (within 1%): the rays that were tuned on fit the
+    shallow stack, others may not."""
+    if best["stack_depth"] < DEFAULTS["stack_depth"]:
+        cand = {**best, "stack_depth": DEFAULTS["stack_depth"]}
+        ms = measure(cand)
+        if ms <= 1.01 * best_ms:
+            return ms, cand
+    return best_ms, best
 
 
 def time_trace(scene, d_rays, d_hits, n: int, mode: int, reps: int = 2, flush=None) -> float:
@@ -120,6 +134,7 @@ def autotune(scene, d_rays, n: int, mode: int, budgets=None, reps: int = 2, pass
                 ms = measure(cand)
                 if ms < best_ms:
                     best_ms, best = ms, cand
+    best_ms, best = settle_depth(best, best_ms, measure)
     scene.set_tuning(**best)
     return {"mode": int(mode), "budget": budget, "tuning": {k: best[k] for k in grid}, "ms": round(best_ms, 4),
             "mrays_s": round(n / best_ms / 1e3, 3), "candidates": len(table), "table": table}
@@ -170,6 +185,7 @@ def autotune_batch(batch, d_rays, n: int, mode: int, reps: int = 2, passes: int 
                 ms = measure(cand)
                 if ms < best_ms:
                     best_ms, best = ms, cand
+    best_ms, best = settle_depth(best, best_ms, measure)
     batch.set_tuning(**best)
     return {"mode": int(mode), "tuning": best, "ms": round(best_ms, 4), "mrays_s": round(n / best_ms / 1e3, 3),
             "candidates": len(table), "table": table}
