@@ -53,20 +53,22 @@ def _peaks():
 
 
 # DRAM bytes per ray of the staged kernel (dram__bytes_read.sum + dram__bytes_write.sum) from
-# the ncu capture summarised in profiles/walks_and_output_layer.md: the same scene with 262,144
-# rays per launch, scaled to a full launch by the ray count.
-STAGED_DRAM_BYTES_PER_RAY = {"primary": (113.36e6 + 26.39e6) / 262144,
-                             "bounce": (205.54e6 + 66.53e6) / 262144}
+# the ncu capture summarised in profiles/walks_and_output_layer.md: the same scene with 524,288
+# rays per launch (from that size on warps of neighbouring camera rays wait for their last one,
+# as in a full launch).  Scaled to a full launch by the ray count, an estimate: a larger launch
+# reads the scene's nodes no more often, so it moves fewer bytes a ray.
+STAGED_DRAM_BYTES_PER_RAY = {"primary": (167.36e6 + 53.26e6) / 524288,
+                             "bounce": (313.26e6 + 115.60e6) / 524288}
 
 
 # What binds the staged walk, from the same ncu capture (bounce launch): it
 # moves a small fraction of the HBM roofline's bytes, and is bound by SIMT
 # divergence and issue instead.
 LIMITER = {"kind": "issue / SIMT divergence (dependent loads of a pointer-chasing walk), not HBM bandwidth",
-           "source": "profiles/walks_and_output_layer.md, staged walk, 262,144 bounce rays",
-           "lanes_active_of_32": 11.04, "issue_slots_active_pct": 71.9, "warps_per_sm": 25.5,
-           "dram_busy_pct": 3.9, "l1_hit_pct": 54.0, "l2_hit_pct": 71.9, "l1_throughput_pct": 43.8,
-           "l2_throughput_pct": 18.6}
+           "source": "profiles/walks_and_output_layer.md, staged walk, 524,288 bounce rays",
+           "lanes_active_of_32": 11.96, "issue_slots_active_pct": 71.9, "warps_per_sm": 26.9,
+           "dram_busy_pct": 5.3, "l1_hit_pct": 52.2, "l2_hit_pct": 72.0, "l1_throughput_pct": 49.8,
+           "l2_throughput_pct": 22.8}
 
 
 def _traffic_per_ray():

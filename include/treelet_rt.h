@@ -169,14 +169,17 @@ rt_status rt_gen_bounce_rays_host(const rt_blob* blob, const rt_ray* rays, const
                                   uint64_t seed, float tmin, float tmax, rt_ray* out);
 
 /* Validates a blob: header, child pointers in range, child sizes/types legal.
- * Returns RT_ERR_BLOB with a message on the first problem. */
+ * A unit that is reached in two uses is checked in both.  Returns RT_ERR_BLOB
+ * with a message on the first problem. */
 rt_status rt_blob_validate(const rt_blob* blob);
 
 /* ---------------- device context and scenes ---------------- */
 rt_status rt_ctx_create(int device, rt_ctx** out);
 rt_status rt_ctx_destroy(rt_ctx* ctx);
 
-/* Uploads a blob (validated first). */
+/* Uploads a blob (validated first).  The scene holds it twice on the device, as
+ * it is and with its internal nodes in the walks' form: 2 x its bytes, 1 KiB and
+ * a bit per 64 bytes; treelets add their tables and images. */
 rt_status rt_scene_create(rt_ctx* ctx, const rt_blob* blob, rt_scene** out);
 rt_status rt_scene_destroy(rt_scene* scene);
 /* Device pointer and size of the uploaded blob. */
@@ -310,12 +313,17 @@ rt_status rt_trace_host_noalloc(rt_scene* scene, const rt_ray* rays, const uint3
 rt_status rt_scene_set_stage_hints(rt_scene* scene, const uint32_t* hints);
 
 /* Traversal tuning; 0 keeps the current value, RT_TUNING_OFF switches a
- * feature off where noted.  None of these changes any result, only speed. */
+ * feature off where noted.  None of these changes any result, only speed.
+ * A launch of at most 32,768 rays over one scene (RT_MODE_STAGED: 24,576, with
+ * no slots, no queues and at most 16 KiB pinned; RT_MODE_PLAIN: without the short
+ * stack) gives each ray eight lanes and has a launch shape of its own:
+ * block_threads, staged_threads and refill_lanes do not apply to it. */
 #define RT_TUNING_OFF 0xFFFFFFFFu
 typedef struct rt_tuning {
   uint32_t block_threads;     /* threads per CTA for RT_MODE_PLAIN / RT_MODE_TREELET (32..256) */
   uint32_t staged_threads;    /* threads per CTA for RT_MODE_STAGED (32..256) */
-  uint32_t staged_epoch;      /* node visits of a warp between staging votes */
+  uint32_t staged_epoch;      /* node visits of a warp (one node of each lane that takes part) between
+                                 staging votes */
   uint32_t staged_slots;      /* shared-memory treelet slots per warp (1..8; RT_TUNING_OFF: none) */
   uint32_t refill_lanes;      /* idle lanes of a warp that make it fetch new rays (1..32; large staged
                                * launches wait for all 32 where a warp holds neighbouring camera rays) */
@@ -337,7 +345,7 @@ typedef struct rt_tuning {
                                  stack in shared memory, lane-interleaved per warp (a warp-synchronous
                                  short stack: entry k of the warp's 32 rays in one row of 32 banks),
                                  the deeper ones in local memory; RT_TUNING_OFF (the default): the whole
-                                 stack in local memory, about 40% faster on a GB300 */
+                                 stack in local memory, 8% faster on a GB300 (2M bounce rays) */
 } rt_tuning;
 rt_status rt_scene_set_tuning(rt_scene* scene, const rt_tuning* t);
 rt_status rt_scene_get_tuning(const rt_scene* scene, rt_tuning* t);
@@ -345,9 +353,8 @@ rt_status rt_scene_get_tuning(const rt_scene* scene, rt_tuning* t);
 /* Pinned treelets (RT_MODE_STAGED; no reference counterpart).  Each CTA of a
  * staged launch copies the pinned image into shared memory once, with
  * cp.async.bulk, and serves every read of a pinned node from it for the
- * whole launch.  The image holds the pinned nodes' own bytes with their
- * route bits and the records of their pinned children, so results are
- * unchanged.  Treelets are pinned in `order`
+ * whole launch.  The image holds the pinned nodes with their route bits and the
+ * records of their pinned children, so results are unchanged.  Treelets are pinned in `order`
  * (dense ids, most wanted first) while they fit in tuning.pinned_bytes;
  * order == NULL restores the default order: the TLAS treelet, then treelets
  * by the surface-area probability of their root. */
@@ -593,7 +600,7 @@ typedef struct rt_unit_stats {
 /* hits / visits are the device outputs of rt_trace on `n` rays (visits with
  * `capacity` entries per ray; a ray replays min(n_visits, capacity) of them).
  * stats: device array of n_rt_units records.  Needs rt_treelets_form.  One
- * CUDA thread models one RT unit; the call allocates the units' tables,
+ * warp models one RT unit; the call allocates the units' tables,
  * synchronises `stream` and frees them before it returns. */
 rt_status rt_unit_replay(rt_scene* scene, const rt_hit* hits, const uint32_t* visits, uint32_t n, uint32_t capacity,
                          const rt_unit_config* config, rt_unit_stats* stats, void* stream);

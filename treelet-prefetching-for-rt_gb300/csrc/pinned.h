@@ -1,20 +1,20 @@
 // Shared-memory records of pinned treelets.
 //
 // The staged traversal keeps the most-visited treelets resident in shared
-// memory for the whole launch.  A record holds a node's own 64 bytes (so the
-// walk reads and tests it exactly as it would from the blob) plus what the
+// memory for the whole launch.  A record holds a node's 64 bytes plus what the
 // walk would otherwise fetch from other tables: the node's unit, its route
-// bits and the records of its pinned children.  Records are 16-byte aligned
-// and named by their offset in 16-byte units ("soff"); soff 0 is never a
-// record.
+// bits and the records of its pinned children.  Internal nodes are in the blob's
+// form in the image made here and in the walks' own (walk_node.h) in the copy
+// that goes to the device.  Records are 16-byte aligned and named by their
+// offset in 16-byte units ("soff"); soff 0 is never a record.
 #pragma once
 #include <stdint.h>
 
 namespace rtp {
 
 // internal node, 80 B: the blob's 64 bytes with bytes 16..17 (NodeType and
-// the pad byte, which the walk does not read) replaced by the node's route
-// bits, then a 16-byte tail
+// the pad byte) replaced by the node's route bits, then a 16-byte tail; on the
+// device the 64 bytes are the walk node, which has the route bits in its word 5
 constexpr uint32_t IN_ROUTE = 16;        // u16 route bits of the node
 constexpr uint32_t IN_UNIT = 64;         // u32 unit of the node
 constexpr uint32_t IN_CHILD_SOFF = 68;   // u16 x6: record of child i, 0 if the child is not pinned

@@ -11,8 +11,10 @@
 // heuristic arithmetic (IEEE double for the popularity share, as in the
 // reference), searching the roots and adding up the members' requests 32 at a
 // time.  A decision is a chain of small steps, bound by their latency: 152 units
-// of 512 lanes take 7.7 us on a GB300; sorting the roots and walking the runs in
-// one thread took 43.7.
+// of 512 lanes take 7.7 us on a GB300 when the most popular treelet was the last
+// one queued (with events around the call 10.9, and 10.9 when every unit queues
+// its treelet's 256 requests); sorting the roots and walking the runs in one
+// thread took 43.7 (47.8, and 49.8).
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>

@@ -536,7 +536,8 @@ __device__ __forceinline__ SlotLookup<F> slot_lookup(F f) {
 constexpr int kMaxSlots = 8;  // slots per warp
 constexpr uint32_t kWaitTries = 1u << 22;
 // Four 256-thread CTAs per SM, 64 registers a thread (96 bytes of spills): 2M
-// primary rays 2.50 ms on a GB300 against 2.56 with three CTAs at 80 registers.
+// primary rays 2.50 ms on a GB300 against 2.56 with three CTAs at 80 registers
+// (2.25 with four since neighbouring camera rays are kept together, below).
 constexpr int kStagedMaxThreads = 256;
 constexpr int kStagedMinBlocks = 4;
 constexpr uint32_t kPinChunk = 32768;  // bytes per bulk copy of the pinned image
@@ -589,12 +590,13 @@ constexpr uint32_t kTogetherRays = 1u << 19;
 // cp.async.bulk and keeps it for the whole launch; every node read that names
 // a record is served from it.
 //
-// Warp slots: every `epoch` node visits of its lanes together a warp votes: each lane names the
-// treelet of its next access, __match_any_sync counts equal names, and the
-// most popular treelet that is not resident (ties to the lowest treelet, i.e.
-// the lowest root address, as the RT unit's decision in shader.cc:3424-3441)
-// is copied with cp.async.bulk into the warp's least recently filled slot,
-// provided at least `min_votes` lanes want it.  A slot holds the first
+// Warp slots: every `epoch` visits (of all its lanes that are at a node of the
+// kind visited, one step each) a warp votes: each lane names the treelet of its
+// next access, __match_any_sync counts equal names, and the most popular treelet
+// that is not resident (ties to the lowest treelet, i.e. the lowest root address,
+// as the RT unit's decision in shader.cc:3424-3441) is copied with cp.async.bulk
+// into the warp's least recently filled slot, provided at least `min_votes` lanes
+// want it.  A slot holds the first
 // slot_bytes of the treelet's image (the whole image when it fits).  Node
 // reads that fall in a resident slot are served from shared memory.  A slot
 // is read only by its own warp; __syncwarp orders the slot's reads before it
