@@ -76,8 +76,17 @@ __device__ __forceinline__ uint32_t add_grouped(uint32_t* counter, uint32_t key,
 }
 
 // One binned round (FINAL = false) or the last round (FINAL = true).
+// Three 256-thread CTAs per SM, 80 registers, and nodes fetched ahead in the last
+// round only: in a binned round a ray stops at its treelet's end, and most nodes
+// it pushes are visited by another warp, or come from the slot.  GB300, 1 / 2 / 4 /
+// 8 / 16 rounds, ms: 2M bounce rays of the 2M-triangle terrain 5.29 / 5.99 / 6.64 /
+// 7.74 / 9.37; fetched ahead in every round 5.36 / 6.12 / 6.85 / 8.09 / 9.87, with
+// four CTAs at 64 registers too 5.59 / 6.43 / 7.22 / 8.51 / 10.45, in no round 5.31 /
+// 6.02 / 6.68 / 7.78 / 9.40; 518K bounce rays of 1M-triangle blobs 0.80 / 0.90 /
+// 1.13 / 1.39 / 1.96, in no round 1.02 / 1.03 / 1.29 / 1.60 / 2.11.
+constexpr int kQueueMinBlocks = 3;
 template <int CAP, bool FINAL>
-__global__ void __launch_bounds__(kStagedMaxThreads, kStagedMinBlocks) trace_queued_kernel(TraceArgs a, QueueArgs q) {
+__global__ void __launch_bounds__(kStagedMaxThreads, kQueueMinBlocks) trace_queued_kernel(TraceArgs a, QueueArgs q) {
   extern __shared__ __align__(128) uint8_t dyn_smem[];
   __shared__ uint64_t bars[kStagedMaxThreads / 32];
   __shared__ uint32_t slot_key[kStagedMaxThreads / 32], slot_units[kStagedMaxThreads / 32];
@@ -105,7 +114,7 @@ __global__ void __launch_bounds__(kStagedMaxThreads, kStagedMinBlocks) trace_que
     const uint32_t u = loc & ((1u << kSlotBitsDev) - 1u);
     return u < slot_units[warp] ? slot_base + u * 64u : 0u;
   });
-  using W = Walker<CAP, true, false, true>;
+  using W = Walker<CAP, true, false, true, true, FINAL>;
   unsigned long long stack[W::kWords];
   W w;
   w.stk = stack;

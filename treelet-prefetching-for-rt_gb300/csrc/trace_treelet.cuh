@@ -39,8 +39,8 @@ constexpr int kColdWords = 6;
 // walk (trace_queued.cuh).  The local array then holds only the current
 // stack and the cold tail.
 // TRACED = false compiles the walk of a launch without traces (no trace code
-// at all).
-template <int CAP, bool STAGED, bool MULTI, bool SLAB = false, bool TRACED = true>
+// at all), TOUCH = false one that fetches no pushed node ahead (touch_node).
+template <int CAP, bool STAGED, bool MULTI, bool SLAB = false, bool TRACED = true, bool TOUCH = true>
 struct Walker {
   // local array: cu, ot (unless SLAB), each with room for the entries a visit
   // may push before its depths are checked, then the cold words
@@ -328,7 +328,7 @@ struct Walker {
       if (pinned) so = rtd::ld_shared_u16(saddr + rtp::IN_CHILD_SOFF + 2u * i);
       const uint32_t c = nd.w[3] + ((nd.w[6] >> (4 * i)) & 15u);
       push((nd.w[5] >> (shift + i)) & 1u, (so ? (so << kEShift) | kEPin : c << kEShift) | level | lf, inst);
-      if (!so) touch_node(v.walk, c);
+      if (TOUCH && !so) touch_node(v.walk, c);
     }
     check_depth();
   }
