@@ -45,20 +45,13 @@ bool validate_blob(const uint8_t* b, uint64_t n, std::string* err, BlobRoles* ro
     std::memcpy(&v, b + off, 8);
     return v;
   };
-  // what a unit has been checked as: a unit in both uses is checked in both
-  constexpr uint8_t kNodeChecked = 1, kInstanceChecked = 2;
-  std::vector<uint8_t> seen(units, 0);
-  // roles: bit 0 internal node, bit 1 read as the blob's bytes (headers, leaves);
-  // bits 2 and 3: a node of the top, of a bottom level.  A node of both levels is
-  // checked as one of them only, and the walks may reach others from it that are
-  // not met here.
-  constexpr uint8_t kInternal = 1, kRaw = 2, kTop = 4, kBottom = 8;
-  std::vector<uint8_t> role(units, 0);
-  bool mixed = false;
-  auto take = [&](uint64_t u, uint8_t r) {
-    role[u] |= r;
-    mixed |= (role[u] & (kInternal | kRaw)) == (kInternal | kRaw) || (role[u] & (kTop | kBottom)) == (kTop | kBottom);
-  };
+  // What a unit is reached as: an internal node, of the top or of a bottom level
+  // (one of both levels is checked as one of them only, and the walks may reach
+  // others from it that are not met here); read as the blob's bytes (headers,
+  // leaves).  And what it has been checked as, a unit in both uses in both.
+  constexpr uint8_t kInternal = 1, kRaw = 2, kTop = 4, kBottom = 8, kNodeChecked = 16, kInstanceChecked = 64;
+  std::vector<uint8_t> mark(units, 0);
+  auto take = [&](uint64_t u, uint8_t r) { mark[u] |= r; };
   take(0, kRaw);
   struct Item {
     uint64_t unit;
@@ -72,8 +65,8 @@ bool validate_blob(const uint8_t* b, uint64_t n, std::string* err, BlobRoles* ro
     const Item it = work.back();
     work.pop_back();
     take(it.unit, kInternal | (it.top ? kTop : kBottom));
-    if (seen[it.unit] & kNodeChecked) continue;
-    seen[it.unit] |= kNodeChecked;
+    if (mark[it.unit] & kNodeChecked) continue;
+    take(it.unit, kNodeChecked);
     const uint8_t* p = b + it.unit * 64;
     int32_t child_off;
     std::memcpy(&child_off, p + rtf::IN_CHILD_OFFSET, 4);
@@ -93,8 +86,8 @@ bool validate_blob(const uint8_t* b, uint64_t n, std::string* err, BlobRoles* ro
           if (ty != rtf::CT_INSTANCE || sz != 2) return bad("top-level leaf that is not a 128-byte instance leaf");
           take(c, kRaw);
           take(c + 1, kRaw);
-          if (!(seen[c] & kInstanceChecked)) {
-            seen[c] |= kInstanceChecked;
+          if (!(mark[c] & kInstanceChecked)) {
+            take(c, kInstanceChecked);
             const uint64_t hdr = c * 64 + rd64(c * 64 + rtf::IL_BVH_ADDRESS);
             if (hdr % 64 || hdr / 64 >= units) return bad("instance BVHAddress out of range");
             const uint64_t broot = hdr + rd64(hdr + rtf::HDR_ROOT_OFFSET);
@@ -111,9 +104,20 @@ bool validate_blob(const uint8_t* b, uint64_t n, std::string* err, BlobRoles* ro
     }
   }
   if (roles) {
-    roles->mixed = mixed;
-    roles->internal.assign((units + 31) / 32, 0);
-    for (uint64_t u = 0; u < units; ++u) roles->internal[u / 32] |= (uint32_t)(role[u] & kInternal) << (u % 32);
+    roles->internal.resize((units + 31) / 32);
+    uint8_t both = 0;  // bit 0: a unit has both kInternal and kRaw, bit 2: both levels
+    for (uint64_t w = 0; w < roles->internal.size(); ++w) {
+      const uint64_t u0 = w * 32;
+      const uint32_t count = (uint32_t)std::min<uint64_t>(32, units - u0);
+      uint32_t bits = 0;
+      for (uint32_t i = 0; i < count; ++i) {
+        const uint8_t m = mark[u0 + i];
+        bits |= (uint32_t)(m & kInternal) << i;
+        both |= m & (m >> 1);
+      }
+      roles->internal[w] = bits;
+    }
+    roles->mixed = (both & (kInternal | kTop)) != 0;
   }
   return true;
 }
