@@ -584,12 +584,12 @@ constexpr uint32_t kGroupRaysPerSplit = 152 * 32;
 // Rays and pinned bytes up to which a staged launch does: each of its CTAs of
 // four warps copies the image.  Eight lanes / one, pinned image of 4 KiB:
 //                                    32        1,024      4,096      16,384     24,000     25,600     32,768
-//   2M-tri terrain, primary          76 / 144  114 / 254  115 / 257  214 / 290  226 / 287  235 / 298  275 / 283
-//   2M-tri terrain, bounce           71 / 162  131 / 333  190 / 373  300 / 437  378 / 463  414 / 439  456 / 436
-//   1M-tri blobs, bounce             41 / 53   139 / 223  139 / 269  189 / 325  207 / 329  213 / 322  267 / 379
-//   16K-tri cube, bounce             30 / 45   54 / 97    60 / 113   86 / 116   106 / 120  108 / 120  126 / 119
-// With stacks of 160 entries 24,000 rays 315 / 285, 454 / 464, 245 / 331, 123 / 122.
-// With 16 KiB pinned, 131K-triangle terrain, bounce: 89 / 189 at 32 rays, 324 / 429 at 16,384, 430 / 452 at 24,480.
+//   2M-tri terrain, primary          62 / 143  114 / 245  115 / 253  214 / 284  247 / 278  234 / 287  275 / 277
+//   2M-tri terrain, bounce           79 / 170  132 / 317  190 / 359  302 / 416  386 / 389  416 / 422  458 / 416
+//   1M-tri blobs, bounce             32 / 43   139 / 217  137 / 272  188 / 321  214 / 350  216 / 323  264 / 373
+//   16K-tri cube, bounce             25 / 33   50 / 87    53 / 84    90 / 94    83 / 95    82 / 95    94 / 96
+// With stacks of 160 entries 24,000 rays 357 / 279, 424 / 391, 228 / 356, 91 / 96.
+// With 16 KiB pinned, 131K-triangle terrain, bounce: 81 / 169 at 32 rays, 329 / 415 at 16,384, 378 / 421 at 24,000.
 constexpr uint32_t kGroupStagedRays = 3u << 13;
 constexpr uint32_t kGroupPinBytes = 16384;
 

@@ -535,11 +535,20 @@ __device__ __forceinline__ SlotLookup<F> slot_lookup(F f) {
 
 constexpr int kMaxSlots = 8;  // slots per warp
 constexpr uint32_t kWaitTries = 1u << 22;
-// Four 256-thread CTAs per SM, 64 registers a thread (96 bytes of spills): 2M
-// primary rays 2.50 ms on a GB300 against 2.56 with three CTAs at 80 registers
-// (2.25 with four since neighbouring camera rays are kept together, below).
+// 256-thread CTAs per SM: three at 80 registers; four at 64 spill 96 bytes.  GB300,
+// us, three / four:
+//                                     131,769    313,600    1,000,000    2,097,152
+//   2M-tri terrain, primary                      530 / 565  1122 / 1170  2152 / 2158
+//   the same, bounce                             865 / 949  2021 / 2041  3886 / 3845
+//   131K-tri terrain, bounce          601 / 675  827 / 899  1939 / 1961
+//   1M-tri blobs, bounce                                    797 / 856    1002 / 1055
+//   2,000-tri cube and plane, bounce  87 / 115   105 / 123  (810,000 rays: 164 / 177)
+// and traced: 1M bounce rays of the 2M-triangle terrain 2423 / 2528.  With warp slots
+// the lookups hide better behind more warps: four, one slot each, 2,013 bounce rays of
+// the terrain 598 / 524, 307,200 primary rays of the blobs 515 / 476 (2M primary rays of the
+// terrain 2847 / 3065).
 constexpr int kStagedMaxThreads = 256;
-constexpr int kStagedMinBlocks = 4;
+constexpr int kStagedMinBlocks = 3, kStagedSlotsMinBlocks = 4;
 constexpr uint32_t kPinChunk = 32768;  // bytes per bulk copy of the pinned image
 
 // Per-warp staging state in shared memory.
@@ -556,10 +565,11 @@ struct WarpStage {
 // warp, us waiting / refilling (kTogetherRays), for frames whose tiles are ever
 // narrower:
 //                    32 x 32      64 x 64      128 x 128    192 x 192    256 x 256    512 x 512    1024 x 1024
-//   2M-tri terrain   1985 / 1673  1776 / 1638  1591 / 1591  1488 / 1562  1444 / 1543  1330 / 1449  1211 / 1304
-//   1M-tri blobs     934 / 698    772 / 672    684 / 659    648 / 654    659 / 651    611 / 626    607 / 620
-// A 192 x 192 frame's tile is 2.6 degrees across, a 128 x 128 frame's 3.9.  The same
-// camera's rays in random order 2520 / 1766 and 1565 / 715.
+//   2M-tri terrain   2033 / 1682  1813 / 1644  1607 / 1616  1489 / 1562  1460 / 1557  1319 / 1461  1166 / 1314
+//   1M-tri blobs     932 / 651    782 / 640    697 / 636    654 / 620    652 / 624    623 / 613    596 / 602
+// A 192 x 192 frame's tile is 2.6 degrees across, a 128 x 128 frame's 3.9: from there on
+// waiting gains more on the one than it loses on the other.  The same camera's rays in
+// random order 2603 / 1758 and 1566 / 679.
 constexpr float kCone = 0.9973f;
 
 __device__ __forceinline__ bool rays_together(rtm::V3 o, rtm::V3 d) {
@@ -574,11 +584,11 @@ __device__ __forceinline__ bool rays_together(rtm::V3 o, rtm::V3 d) {
 // Rays from which on a staged launch waits for the last ray of a warp whose rays
 // are together, to take 32 neighbours again: neighbours walk the same nodes, and a
 // ray taken alone walks beside rays that are far ahead.  GB300, primary rays,
-// waiting / refilling at 8 idle lanes, us: 2M-triangle terrain 1M rays 1199 /
-// 1292, 2M (two a pixel) 2247 / 2500, 4M 4350 / 4919; traced 1495 /
-// 1660 at 1M; 1M-triangle blobs 594 / 604 at 1M.  At 307,200 rays, two per
-// lane of the chip, the warps' uneven ends cost what it gains (blobs 379 / 358).
-// Bounce rays: 2102 / 2101 us at 1M, 3850 / 3830 at 2M.  The unstaged treelet
+// waiting / refilling at 8 idle lanes, us: 2M-triangle terrain 537,600 rays 711 / 752,
+// 1M 1166 / 1314, 2M (two a pixel) 2230 / 2567, 4M 4360 / 5068; traced 1473 / 1622 at
+// 1M; 1M-triangle blobs 433 / 428, 596 / 602, 937 / 949, 1676 / 1677.  At 307,200
+// rays, three per lane of the chip, the warps' uneven ends cost what it gains (terrain
+// 501 / 516, blobs 354 / 339).  Bounce rays: 2101 / 2086 us at 1M, 3920 / 3899 at 2M.  The unstaged treelet
 // walk gains as much on such rays but pays 0.4% on all others for the check,
 // and the plain walk gains nothing (1036 / 1025): neither does it.
 constexpr uint32_t kTogetherRays = 1u << 19;
@@ -602,7 +612,8 @@ constexpr uint32_t kTogetherRays = 1u << 19;
 // is read only by its own warp; __syncwarp orders the slot's reads before it
 // is refilled.  SLOTS = false compiles the warp slots out (a.slots == 0).
 template <int CAP, bool SLOTS, bool TRACED>
-__global__ void __launch_bounds__(kStagedMaxThreads, kStagedMinBlocks) trace_staged_kernel(TraceArgs a) {
+__global__ void __launch_bounds__(kStagedMaxThreads, SLOTS ? kStagedSlotsMinBlocks : kStagedMinBlocks)
+    trace_staged_kernel(TraceArgs a) {
   extern __shared__ __align__(128) uint8_t dyn_smem[];
   __shared__ WarpStage ws[kStagedMaxThreads / 32];
   __shared__ uint64_t pin_bar;
