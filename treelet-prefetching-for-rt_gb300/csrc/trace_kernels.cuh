@@ -369,7 +369,7 @@ __device__ __forceinline__ void warp_turn(const TraceArgs& a, W& w, uint32_t r, 
 
 struct NoLookup {
   static constexpr bool kSlots = false;
-  __device__ __forceinline__ uint32_t operator()(uint32_t, const uint2*) const { return 0u; }
+  __device__ __forceinline__ uint32_t operator()(uint32_t, uint32_t, const uint2*) const { return 0u; }
 };
 
 // Finds a ray for every idle lane of the warp (one atomic per refill) and

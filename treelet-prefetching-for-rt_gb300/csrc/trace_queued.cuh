@@ -106,13 +106,13 @@ __global__ void __launch_bounds__(kStagedMaxThreads, kQueueMinBlocks) trace_queu
   const bool round0 = q.in_ray == nullptr;
   const uint32_t n_in = q.n_in ? *q.n_in : a.n;
   // nodes of the warp's staged treelet come from its slot
-  const auto lookup = slot_lookup([&](uint32_t unit, const uint2* meta) -> uint32_t {
+  const auto lookup = slot_lookup([&](uint32_t unit, uint32_t units, const uint2* meta) -> uint32_t {
     const uint32_t key = slot_key[warp];
     if (FINAL || key == kNone) return 0u;
     const uint32_t loc = __ldg(reinterpret_cast<const uint32_t*>(meta) + 2ull * unit + 1);
     if (loc == kNone || (loc >> kSlotBitsDev) != key) return 0u;
     const uint32_t u = loc & ((1u << kSlotBitsDev) - 1u);
-    return u < slot_units[warp] ? slot_base + u * 64u : 0u;
+    return u + units <= slot_units[warp] ? slot_base + u * 64u : 0u;
   });
   using W = Walker<CAP, true, false, true, true, FINAL>;
   unsigned long long stack[W::kWords];

@@ -251,8 +251,9 @@ struct Walker {
   __device__ __forceinline__ bool in_treelet() const { return ncu > 0; }
 
   // Where a popped node is: its unit, and the address of its pinned record or
-  // staged copy in shared memory (`lookup(unit, meta)`: a node staged in a
-  // warp slot), 0 when it is read from `from` (the walk nodes or the blob).
+  // staged copy in shared memory (`lookup(unit, units, meta)`: a node of so
+  // many units that lies whole in a warp slot), 0 when it is read from `from`
+  // (the walk nodes or the blob).
   // Loads its first 64 bytes (or the whole pinned record of an instance leaf).
   // False, and the ray stopped, when it lies outside the blob.
   template <class Lookup>
@@ -270,7 +271,7 @@ struct Walker {
         return false;
       }
       if (STAGED) {
-        saddr = lookup(unit, v.meta);
+        saddr = lookup(unit, units, v.meta);
         if (saddr) ++smem_reads;
         else ++gmem_reads;
       }
@@ -526,7 +527,9 @@ template <class F>
 struct SlotLookup {
   static constexpr bool kSlots = true;
   F f;
-  __device__ __forceinline__ uint32_t operator()(uint32_t unit, const uint2* meta) const { return f(unit, meta); }
+  __device__ __forceinline__ uint32_t operator()(uint32_t unit, uint32_t units, const uint2* meta) const {
+    return f(unit, units, meta);
+  }
 };
 template <class F>
 __device__ __forceinline__ SlotLookup<F> slot_lookup(F f) {
@@ -651,7 +654,7 @@ __global__ void __launch_bounds__(kStagedMaxThreads, SLOTS ? kStagedSlotsMinBloc
   }
   __syncthreads();
   // the node's location is read only while some slot of the warp is resident
-  const auto lookup = slot_lookup([&](uint32_t unit, const uint2* meta) -> uint32_t {
+  const auto lookup = slot_lookup([&](uint32_t unit, uint32_t units, const uint2* meta) -> uint32_t {
     bool any = false;
     for (uint32_t s = 0; s < slots; ++s) any |= st.resident[s] != kNone;
     if (!any) return 0u;
@@ -659,7 +662,7 @@ __global__ void __launch_bounds__(kStagedMaxThreads, SLOTS ? kStagedSlotsMinBloc
     if (loc == kNone) return 0u;
     const uint32_t d = loc >> kSlotBitsDev, u = loc & ((1u << kSlotBitsDev) - 1u);
     for (uint32_t s = 0; s < slots; ++s)
-      if (st.resident[s] == d && u < st.units[s]) return slot_base + s * a.slot_bytes + u * 64u;
+      if (st.resident[s] == d && u + units <= st.units[s]) return slot_base + s * a.slot_bytes + u * 64u;
     return 0u;
   });
   using W = Walker<CAP, true, false, false, TRACED>;  // staged launches trace one scene
