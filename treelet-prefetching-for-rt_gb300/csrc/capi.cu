@@ -614,8 +614,16 @@ rt_status launch_group(rtk::TraceArgs& a, uint32_t mode, uint32_t depth, cudaStr
   // CTAs for every ray, or as many as are resident at once
   const uint32_t full = persistent_grid((const void*)kern, rtk::kGroupThreads, 0xffffffffu, dyn);
   const uint32_t need = (a.n + warps * rpw - 1) / (warps * rpw);
+  // With one ray a warp the walk writes the treelet ids too, as each ray ends: the
+  // launch that does so otherwise (trace_launch) is longer than what it adds.  GB300,
+  // us, in the walk / a launch of its own: 1 ray 18 / 23, 4,096 rays of the 131K-triangle
+  // terrain 121 / 125 (bounce 204 / 206); with several rays a warp, one after the other, no longer: 25,600
+  // rays 384 / 369.
+  uint32_t* const ids = a.ids;
+  if (rpw > 1) a.ids = nullptr;
   kern<<<std::min(full, need), rtk::kGroupThreads, dyn, st>>>(a, depth, rpw);
   RT_CUDA(cudaGetLastError());
+  a.ids = rpw > 1 ? ids : nullptr;  // what is left to write
   return RT_OK;
 }
 
@@ -1042,6 +1050,7 @@ rt_status trace_launch(rt_scene* s, const rt_ray* rays, const uint32_t* flags, u
   a.rows = visits ? visits : treelets;
   a.rows_tl = visits ? 0u : 1u;
   a.cap = a.rows ? trace->capacity : 0;
+  a.ids = visits ? treelets : nullptr;
   a.meta = s->d_meta;
   a.route = s->d_route;
   if (mode == RT_MODE_STAGED && s->d_pin) {
@@ -1060,7 +1069,7 @@ rt_status trace_launch(rt_scene* s, const rt_ray* rays, const uint32_t* flags, u
   const bool queues = allow_queues && queued(s, mode);
   if (queues) rs = ensure_queue_scratch(s, n);
   if (rs == RT_OK) rs = launch_trace(a, mode, s->tuning, s->slot_bytes, st, keep, queues ? &s->qs : nullptr);
-  if (rs == RT_OK && visits && treelets) {
+  if (rs == RT_OK && a.ids) {  // not written by the walk
     const bool wide = a.cap % 4 == 0 && (((uintptr_t)visits | (uintptr_t)treelets) & 15u) == 0;
     auto ids = wide ? rtk::trace_treelet_ids_kernel<true> : rtk::trace_treelet_ids_kernel<false>;
     const uint64_t threads = (wide ? 8ull : 32ull) * n;

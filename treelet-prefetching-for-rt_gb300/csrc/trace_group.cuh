@@ -385,6 +385,13 @@ struct GroupWalk {
       else if (leaf) leaves();
       else internal();
     }
+    if (TRACED && a.ids) {  // the ids of the ray's visits, read back from its row
+      __syncwarp(mask);
+      const uint32_t m = min(n_tx, a.cap);
+      const uint64_t row = (uint64_t)r * a.cap;
+#pragma unroll 4
+      for (uint32_t k = j; k < m; k += kGroup) a.ids[row + k] = __ldg(&v.meta[a.rows[row + k] >> 3].x);
+    }
     if (j == 0) {
       const bool bad = flags & (RT_RAY_STACK_OVERFLOW | RT_RAY_BAD_NODE);
       write_hit(a, v, r, !bad && (min_thit < tmax), min_thit, O, D, tmin, tmax, c_leaf, c_inst, c_tobj, n_tx,

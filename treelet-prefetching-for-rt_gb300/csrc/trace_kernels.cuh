@@ -86,6 +86,7 @@ struct TraceArgs {
   uint32_t* rows;              // traced: n rows of `cap` entries, visits or (rows_tl) treelet ids, or null
   uint32_t rows_tl;
   uint32_t cap;
+  uint32_t* ids;               // rows of treelet ids beside the visits', or null (trace_group_kernel writes them)
   const uint2* meta;           // per unit: x = treelet root unit, y = dense << 10 | slot
   const uint16_t* route;       // per unit: routing bits of the treelet-ordered walk
   const uint4* pin_image;      // staged: pinned-treelet records (pinned.h), copied to shared memory per CTA
