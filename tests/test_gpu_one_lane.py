@@ -98,3 +98,30 @@ def test_stack_overflow(ctx):
     rays = rt.camera_rays(rt.default_camera(rt.SCENE_CUBE), 48, 48, 1, 3, 1e-4, 1e30)
     overlapping = rt.Blob.build([tris], [(0, ident, 0)])
     assert _check_overflow(ctx, overlapping, np.resize(rays, N), 8192, (48, 96, 160)) > 0
+
+
+@pytest.mark.parametrize("n,depth", [(786431, 96), (786432, 96), (786433, 48), (786432, 160)])
+def test_large_any_hit_launches(ctx, n, depth):
+    """Staged any-hit launches on both sides of the size from which they run four CTAs per SM."""
+    import torch
+
+    import treelet_rt as rt
+    from oracle import oracle as orc
+
+    blob = rt.Blob.gen(rt.SCENE_CUBE_PLANE, 2000, 4)
+    prim = rt.camera_rays(rt.default_camera(rt.SCENE_CUBE_PLANE), 64, 64, 1, 2, 1e-4, 1e30)
+    ph, _, _ = orc.trace(blob.bytes(), prim, 0)
+    few = np.concatenate([prim, rt.bounce_rays_host(blob, prim, ph, seed=5)])
+    flags = rt.RAY_FLAG_OPAQUE | rt.RAY_FLAG_TERMINATE_ON_FIRST_HIT
+    tl = orc.Treelets(blob.bytes(), 1024)
+    oh, _, _ = orc.trace(blob.bytes(), few, 1, tl, default_flags=flags, threads=8)
+    pick = np.resize(np.arange(len(few)), n)
+    scene = rt.Scene(ctx, blob)
+    scene.form_treelets(1024)
+    scene.set_tuning(stack_depth=depth)
+    d_rays = torch.from_numpy(few[pick].view(np.uint8)).cuda()
+    d_hits = torch.zeros(n * 64, dtype=torch.uint8, device="cuda")
+    scene.trace(d_rays, d_hits, rt.MODE_STAGED, default_flags=flags, n=n)
+    hits = d_hits.cpu().numpy().view(rt.HIT_DTYPE)
+    scene.close()
+    assert_hits_equal(hits, oh[pick], f"{n} any-hit rays, depth {depth}")

@@ -593,6 +593,17 @@ constexpr uint32_t kGroupRaysPerSplit = 152 * 32;
 constexpr uint32_t kGroupStagedRays = 3u << 13;
 constexpr uint32_t kGroupPinBytes = 16384;
 
+// Any-hit rays from which on a staged launch runs four CTAs of 64 registers per SM
+// instead of three of 80.  GB300, ambient-occlusion rays, us, four / three:
+//                          64,000     240,000    576,000    960,000      2,073,600    4,320,000
+//   1M-tri blobs           193 / 186  366 / 355  619 / 616  932 / 950    1824 / 1886  3614 / 3765
+//   4M-tri blobs           222 / 217  370 / 355  648 / 658  1002 / 1035  1941 / 1999  3828 / 3987
+//   2M-tri terrain         113 / 108  196 / 182  365 / 362  574 / 573    1156 / 1156  2330 / 2334
+//   300K-tri cube, plane   135 / 129  208 / 181  338 / 336  480 / 485    942 / 961    1895 / 1958
+//   100K-tri shared BLAS   173 / 164  314 / 304  583 / 591  895 / 918    1785 / 1851  3551 / 3687
+// Bounce rays are no faster with four until 2M (terrain 4131 / 4192, blobs 1212 / 1149).
+constexpr uint32_t kStagedAnyHitRays = 3u << 18;
+
 bool group_launch(const rtk::TraceArgs& a, uint32_t mode, const rt_tuning& t, const rti::QueueScratch* qs) {
   if (a.n_items || a.n > kGroupRays) return false;
   if (mode == RT_MODE_STAGED)
@@ -698,6 +709,9 @@ rt_status launch_cap(rtk::TraceArgs& a, uint32_t mode, const rt_tuning& t, uint3
     }
     auto kern = slots ? (traced ? rtk::trace_staged_kernel<CAP, true, true> : rtk::trace_staged_kernel<CAP, true, false>)
                       : (traced ? rtk::trace_staged_kernel<CAP, false, true> : rtk::trace_staged_kernel<CAP, false, false>);
+    if (!slots && !traced && !a.flags && (a.default_flags & rtf::RAY_FLAG_TERMINATE_ON_FIRST_HIT) &&
+        a.n >= kStagedAnyHitRays)
+      kern = rtk::trace_staged_kernel<CAP, false, false, rtk::kStagedAnyHitMinBlocks>;
     RT_CUDA(ensure_dyn_smem((const void*)kern, dyn));
     kern<<<persistent_grid((const void*)kern, bt, a.n, dyn), bt, dyn, st>>>(a);
   }

@@ -548,9 +548,10 @@ constexpr uint32_t kWaitTries = 1u << 22;
 //   2,000-tri cube and plane, bounce  87 / 115   105 / 123  (810,000 rays: 164 / 177)
 // and traced: 1M bounce rays of the 2M-triangle terrain 2423 / 2528.  With one slot a
 // warp: 2,013 bounce rays of the terrain 581 / 641, 307,200 primary rays 713 / 826, of the
-// blobs 527 / 548, 2M primary rays of the terrain 2848 / 3229.
+// blobs 527 / 548, 2M primary rays of the terrain 2848 / 3229.  Large launches of any-hit
+// rays, which end early and are taken at once, run four (kStagedAnyHitRays).
 constexpr int kStagedMaxThreads = 256;
-constexpr int kStagedMinBlocks = 3;
+constexpr int kStagedMinBlocks = 3, kStagedAnyHitMinBlocks = 4;
 constexpr uint32_t kPinChunk = 32768;  // bytes per bulk copy of the pinned image
 
 // Per-warp staging state in shared memory.
@@ -613,8 +614,8 @@ constexpr uint32_t kTogetherRays = 1u << 19;
 // reads that fall in a resident slot are served from shared memory.  A slot
 // is read only by its own warp; __syncwarp orders the slot's reads before it
 // is refilled.  SLOTS = false compiles the warp slots out (a.slots == 0).
-template <int CAP, bool SLOTS, bool TRACED>
-__global__ void __launch_bounds__(kStagedMaxThreads, kStagedMinBlocks) trace_staged_kernel(TraceArgs a) {
+template <int CAP, bool SLOTS, bool TRACED, int MIN_BLOCKS = kStagedMinBlocks>
+__global__ void __launch_bounds__(kStagedMaxThreads, MIN_BLOCKS) trace_staged_kernel(TraceArgs a) {
   extern __shared__ __align__(128) uint8_t dyn_smem[];
   __shared__ WarpStage ws[kStagedMaxThreads / 32];
   __shared__ uint64_t pin_bar;
