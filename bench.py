@@ -53,22 +53,20 @@ def _peaks():
 
 
 # DRAM bytes per ray of the staged kernel (dram__bytes_read.sum + dram__bytes_write.sum) from
-# the ncu capture summarised in profiles/walks_and_output_layer.md: the same scene with 524,288
-# rays per launch (from that size on warps of neighbouring camera rays wait for their last one,
-# as in a full launch).  Scaled to a full launch by the ray count, an estimate: a larger launch
-# reads the scene's nodes no more often, so it moves fewer bytes a ray.
-STAGED_DRAM_BYTES_PER_RAY = {"primary": (167.36e6 + 53.26e6) / 524288,
-                             "bounce": (313.26e6 + 115.60e6) / 524288}
+# the ncu capture summarised in profiles/walks_and_output_layer.md: the same scene and launches
+# of the same 2,097,152 rays.
+STAGED_DRAM_BYTES_PER_RAY = {"primary": (306.94e6 + 151.08e6) / 2097152,
+                             "bounce": (666.16e6 + 227.86e6) / 2097152}
 
 
 # What binds the staged walk, from the same ncu capture (bounce launch): it
 # moves a small fraction of the HBM roofline's bytes, and is bound by SIMT
 # divergence and issue instead.
 LIMITER = {"kind": "issue / SIMT divergence (dependent loads of a pointer-chasing walk), not HBM bandwidth",
-           "source": "profiles/walks_and_output_layer.md, staged walk, 524,288 bounce rays",
-           "lanes_active_of_32": 11.96, "issue_slots_active_pct": 71.9, "warps_per_sm": 26.9,
-           "dram_busy_pct": 5.3, "l1_hit_pct": 52.2, "l2_hit_pct": 72.0, "l1_throughput_pct": 49.8,
-           "l2_throughput_pct": 22.8}
+           "source": "profiles/walks_and_output_layer.md, staged walk, 2,097,152 bounce rays",
+           "lanes_active_of_32": 14.92, "issue_slots_active_pct": 67.9, "warps_per_sm": 23.4,
+           "dram_busy_pct": 2.9, "l1_hit_pct": 56.4, "l2_hit_pct": 77.5, "l1_throughput_pct": 60.9,
+           "l2_throughput_pct": 27.9}
 
 
 def _traffic_per_ray():
