@@ -365,3 +365,35 @@ def test_staged_epoch_counts_node_visits(ctx, epoch):
     assert st["stagings"] > nodes / (32 * epoch)
     assert st["stagings"] <= nodes / epoch + 152 * 64
     scene.close()
+
+
+@pytest.mark.parametrize("cap,skew", [(8, 0), (16, 0), (40, 0), (40, 1), (45, 0)])
+def test_ids_of_short_rows(ctx, cap, skew):
+    """Rows on both sides of eight entries (rays that miss, or leave the scene at once): the walk
+    writes the ids of shorter ones, the pass after it the others', and none past a row's entries."""
+    import torch
+
+    import treelet_rt as rt
+    from oracle import oracle as orc
+
+    blob = rt.Blob.gen(rt.SCENE_BLOBS, 2000, 5)
+    few = rt.camera_rays(rt.default_camera(rt.SCENE_BLOBS), 96, 80, 1, 3, 1e-4, 1e30)
+    tl = orc.Treelets(blob.bytes(), 1024)
+    n = 40003
+    pick = np.random.default_rng(1).integers(0, len(few), n)
+    d_rays = torch.from_numpy(few[pick].view(np.uint8)).cuda()
+    scene = rt.Scene(ctx, blob)
+    scene.form_treelets(1024)
+    for mode, omode in ((rt.MODE_PLAIN, 0), (rt.MODE_TREELET, 1), (rt.MODE_STAGED, 1)):
+        oh, ov, ot = orc.trace(blob.bytes(), few, omode, tl, capacity=cap, want_visits=True, want_treelets=True, threads=8)
+        assert (oh["n_visits"] < 8).any() and (oh["n_visits"] >= 8).any()
+        d_hits = torch.zeros(n * 64, dtype=torch.uint8, device="cuda")
+        d_vis = torch.full((n * cap + skew,), -1, dtype=torch.int32, device="cuda")[skew:]
+        d_tl = torch.full((n * cap,), -1, dtype=torch.int32, device="cuda")
+        scene.trace(d_rays, d_hits, mode, visits=d_vis, treelets=d_tl, capacity=cap, n=n)
+        keep = np.arange(cap)[None, :] < np.minimum(oh["n_visits"], cap)[pick][:, None]
+        for got, expect, what in ((d_vis, ov, "visits"), (d_tl, ot, "treelet ids")):
+            g = got.cpu().numpy().view(np.uint32).reshape(n, cap)
+            assert np.array_equal(g[keep], expect[pick][keep]), f"{what}, mode {mode}"
+            assert (g[~keep] == 0xFFFFFFFF).all(), f"{what} past a row's entries, mode {mode}"
+    scene.close()

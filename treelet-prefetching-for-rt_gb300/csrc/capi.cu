@@ -1086,9 +1086,10 @@ rt_status trace_launch(rt_scene* s, const rt_ray* rays, const uint32_t* flags, u
   if (rs == RT_OK && a.ids) {  // not written by the walk
     const bool wide = a.cap % 4 == 0 && (((uintptr_t)visits | (uintptr_t)treelets) & 15u) == 0;
     auto ids = wide ? rtk::trace_treelet_ids_kernel<true> : rtk::trace_treelet_ids_kernel<false>;
+    const uint32_t skip = a.tbuf_off != rtk::kNone ? rtk::kIdsSkip : 0u;
     const uint64_t threads = (wide ? 8ull : 32ull) * n;
     ids<<<persistent_grid((const void*)ids, 256, (uint32_t)std::min<uint64_t>(threads, 0xffffffffull)), 256, 0, st>>>(
-        visits, hits, s->d_meta, n, a.cap, treelets);
+        visits, hits, s->d_meta, n, a.cap, skip, treelets);
     RT_CUDA(cudaGetLastError());
   }
   return rs;

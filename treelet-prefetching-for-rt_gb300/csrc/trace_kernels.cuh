@@ -166,13 +166,17 @@ __device__ __forceinline__ void trace_put(const TraceArgs& a, uint32_t r, uint32
 }
 
 // Writes the staged entries of a ray's last partial sector; m = entries
-// recorded (at most the capacity).
-__device__ __forceinline__ void trace_drain(const TraceArgs& a, uint32_t r, uint32_t m) {
+// recorded (at most the capacity).  A row shorter than kIdsSkip is whole in the
+// staging area: its treelet ids are written too.
+constexpr uint32_t kIdsSkip = 8;
+__device__ __forceinline__ void trace_drain(const TraceArgs& a, uint32_t r, uint32_t m, const uint2* meta) {
   const uint32_t k = m & 7u;
   if (a.tbuf_off == kNone || k == 0) return;
   const uint32_t* b = trace_buf(a.tbuf_off);
-  uint32_t* row = a.rows + (uint64_t)r * a.cap + (m - k);
-  for (uint32_t j = 0; j < k; ++j) row[j] = b[j * 32];
+  const uint64_t at = (uint64_t)r * a.cap + (m - k);
+  for (uint32_t j = 0; j < k; ++j) a.rows[at + j] = b[j * 32];
+  if (a.ids && m < kIdsSkip)
+    for (uint32_t j = 0; j < k; ++j) a.ids[at + j] = __ldg(&meta[b[j * 32] >> 3].x);
 }
 
 // The treelet id of every recorded visit: reads and writes the rows in order,
@@ -180,17 +184,28 @@ __device__ __forceinline__ void trace_drain(const TraceArgs& a, uint32_t r, uint
 // four entries each (rows that start on 16-byte boundaries), so that a warp has
 // up to 128 table reads on their way; with one warp per row and one entry a
 // lane the pass was bound by two dependent loads (282 us for 1M bounce rays' 63M
-// entries on a GB300; WIDE 208, by then bound by L2 sectors).
+// entries on a GB300; WIDE 208, by then bound by L2 sectors; eight lanes a row
+// without WIDE are 4-11% faster for rows of a few entries, 3-5% slower for long
+// ones).  Rows shorter than `skip` have their ids already (trace_drain).  WIDE reads
+// a row's count one row ahead: 1M rays of 1M-triangle blobs, both traces, in treelet
+// order 728 / 710 us, 810,000 of 2,000-triangle blobs, nearly all of which miss, with
+// the skip 166 / 142.
 template <bool WIDE>
 __global__ void __launch_bounds__(256) trace_treelet_ids_kernel(const uint32_t* __restrict__ visits,
                                                                 const rt_hit* __restrict__ hits,
                                                                 const uint2* __restrict__ meta, uint32_t n,
-                                                                uint32_t cap, uint32_t* __restrict__ treelets) {
+                                                                uint32_t cap, uint32_t skip,
+                                                                uint32_t* __restrict__ treelets) {
   constexpr uint32_t kLanes = WIDE ? 8u : 32u, kEach = WIDE ? 4u : 1u;
-  const uint32_t lane = threadIdx.x % kLanes, rows = gridDim.x * blockDim.x / kLanes;
-  for (uint32_t r = (blockIdx.x * blockDim.x + threadIdx.x) / kLanes; r < n; r += rows) {
-    const uint32_t m = min(hits[r].n_visits, cap);
-    const uint64_t row = (uint64_t)r * cap;
+  const uint32_t lane = threadIdx.x % kLanes;
+  const uint64_t rows = (uint64_t)gridDim.x * blockDim.x / kLanes;
+  uint64_t r = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) / kLanes;
+  uint32_t next = r < n ? min(hits[r].n_visits, cap) : 0u;
+  for (; r < n; r += rows) {
+    const uint32_t m = WIDE ? next : min(hits[r].n_visits, cap);
+    if (WIDE && r + rows < n) next = min(hits[r + rows].n_visits, cap);
+    if (m < skip) continue;
+    const uint64_t row = r * cap;
 #pragma unroll 2
     for (uint32_t j = lane * kEach; j < m; j += kLanes * kEach) {
       if (WIDE && j + 4 <= m) {
@@ -659,7 +674,7 @@ struct PlainWalker {
 
   __device__ __forceinline__ void finish(const TraceArgs& a, uint32_t r) {
     const bool bad = flags & (RT_RAY_STACK_OVERFLOW | RT_RAY_BAD_NODE);
-    if (TRACED) trace_drain(a, r, min(n_tx, a.cap));
+    if (TRACED) trace_drain(a, r, min(n_tx, a.cap), v.meta);
     write_hit(a, v, r, !bad && (min_thit < tmax), min_thit, world_o(), world_d(), tmin, tmax, cold(9), cold(10),
               __uint_as_float(cold(11)), n_tx, flags & kRayStatusMask);
   }

@@ -440,7 +440,7 @@ struct Walker {
   __device__ __forceinline__ void finish(const TraceArgs& a, uint32_t r) {
     const bool bad = flags & (RT_RAY_STACK_OVERFLOW | RT_RAY_BAD_NODE);
     const unsigned long long h = cold(2);
-    if (TRACED) trace_drain(a, r, min(n_tx, a.cap));
+    if (TRACED) trace_drain(a, r, min(n_tx, a.cap), v.meta);
     write_hit(a, v, r, !bad && (min_thit < tmax), min_thit, world_o(), dir(), tmin, tmax, (uint32_t)h,
               (uint32_t)(h >> 32), hi(cold(1)), n_tx, flags & kRayStatusMask);
   }
