@@ -2,12 +2,12 @@
 //
 //   trace_plain_kernel    traceRay order (vulkan_ray_tracing.cc:2309-3076)
 //   trace_treelet_kernel  traceRayWithTreelets order (vulkan_ray_tracing.cc:1522-2307);
-//                         with STAGED = true, each CTA votes every epoch on the
-//                         treelet most of its rays need next (the treelet-prefetch
-//                         decision of shader.cc:3419-3441 with heuristic ALWAYS),
-//                         copies that treelet's image into shared memory with
-//                         cp.async.bulk, and serves node reads that fall in a
-//                         resident treelet from shared memory.  Staging changes
+//                         with STAGED = true, node reads that fall in a treelet
+//                         in shared memory are served from there: one pinned for
+//                         the launch, or one that the warp's lanes voted for (the
+//                         treelet-prefetch decision of shader.cc:3419-3441 with
+//                         heuristic ALWAYS) and copied into one of its slots.  Both
+//                         are copied with cp.async.bulk.  Staging changes
 //                         where a node's bytes come from, never which nodes a
 //                         ray visits or in which order.
 //
