@@ -97,7 +97,7 @@ bool validate_blob(const uint8_t* b, uint64_t n, std::string* err, BlobRoles* ro
           }
         } else {
           if (ty != rtf::CT_QUAD && ty != rtf::CT_PROCEDURAL) return bad("bottom-level leaf of unknown type");
-          for (uint32_t k = 0; k < sz; ++k) take(c + k, kRaw);
+          for (uint32_t k = 0; roles && k < sz; ++k) take(c + k, kRaw);  // only BlobRoles needs it
         }
       }
       c += sz;
